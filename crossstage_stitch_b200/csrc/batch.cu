@@ -67,6 +67,7 @@ void set_attributes_once() {
                              s2s3::kSortCap * static_cast<int>(sizeof(std::uint64_t)));
         s5k::enable_search_smem_once(
             reinterpret_cast<const void*>(s5k::search_kernel<s5k::JobTable<SearchJob>, true>));
+        s5k::enable_finish_smem_once(reinterpret_cast<const void*>(s5k::finish_kernel<s5k::JobTable<PairIO>>));
     });
 }
 
@@ -213,6 +214,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     sort_smem = s2s3::sort_smem_bytes(max_cand);
     rank_fallback = max_cand > s2s3::kSortCap;
     search_smem = s5k::search_smem_bytes(max_cap_m);
+    finish_smem = s5k::finish_smem_bytes(max_cap_m);
     // S4: one train partition per block unless the batch is too small to fill the GPU
     n_knn = 0;
     for (int i = 0; i < n; ++i) n_knn += pairs[i].s4.cross_check ? 2 : 1;
@@ -709,7 +711,7 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
                                reinterpret_cast<const int*>(T + offsets[kSearchPrefix]), n},
                      kMapSearch));
     mark();
-    if (go(n)) s5k::finish_kernel<PairSrc><<<n, s5k::kFinishThreads, 0, s>>>(pairsrc);
+    if (go(n)) s5k::finish_kernel<PairSrc><<<n, s5k::kFinishThreads, finish_smem, s>>>(pairsrc);
     mark();
     if (!marks_ok) return Status::CUDA_ERROR;
     note_launches(launches);

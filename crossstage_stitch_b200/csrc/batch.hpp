@@ -54,7 +54,7 @@ public:
     int rs_blocks[s2s3::kMaxLevels] = {};  // resize launch of layer kind + 1
     int knn_blocks = 0, merge_blocks = 0, n_knn = 0;
     int search_blocks = 0, fit_blocks = 0;
-    int sort_smem = 0, search_smem = 0;
+    int sort_smem = 0, search_smem = 0, finish_smem = 0;
     bool rank_fallback = false;
     int hpw = 8;
     // binary matcher of this plan's S4 launches (s4k::kMatcherPopc or

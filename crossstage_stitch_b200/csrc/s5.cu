@@ -90,6 +90,11 @@ int search_smem_bytes(int match_capacity) {
     return std::min(std::max(match_capacity, 1), kStagePoints) * static_cast<int>(sizeof(float4));
 }
 
+bool enable_finish_smem_once(const void* fn) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, finish_smem_bytes(kFinishStage)) ==
+           cudaSuccess;
+}
+
 bool enable_search_smem_once(const void* fn) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kStagePoints * static_cast<int>(sizeof(float4))) == cudaSuccess;
@@ -133,7 +138,11 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
         note_launches(1);
         if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     }
-    finish_kernel<OneJob<PairIO>><<<1, kFinishThreads, 0, stream>>>(OneJob<PairIO>{io});
+    static const bool finish_ok =
+        enable_finish_smem_once(reinterpret_cast<const void*>(finish_kernel<OneJob<PairIO>>));
+    (void)finish_ok;
+    finish_kernel<OneJob<PairIO>>
+        <<<1, kFinishThreads, finish_smem_bytes(matches.capacity), stream>>>(OneJob<PairIO>{io});
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     if (cudaMemcpyAsync(output, &io.state->result, sizeof(*output), cudaMemcpyDeviceToHost, stream) != cudaSuccess)

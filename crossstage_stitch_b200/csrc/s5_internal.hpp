@@ -17,5 +17,6 @@ Status check_and_build(const Keypoints& a, const Keypoints& b, const Matches& m,
 int plan_search(int count, int hpw);
 int search_smem_bytes(int match_capacity);
 bool enable_search_smem_once(const void* fn);
+bool enable_finish_smem_once(const void* fn);
 
 }  // namespace stitch::b200::s5k

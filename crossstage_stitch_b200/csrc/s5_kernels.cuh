@@ -75,7 +75,6 @@ constexpr int kSearchWarps = kSearchThreads / 32;
 constexpr int kMaxSearchBlocks = 2 * kSmCount;
 constexpr int kStagePoints = 4096;  // matched points staged in shared memory per search block
 constexpr int kFinishThreads = 256;
-constexpr int kFinishChunk = 256;
 
 // Inputs of one pair, as the caller passed them.
 struct PairIO {
@@ -234,157 +233,12 @@ __device__ __forceinline__ bool nondegenerate(const Pt* p) {
     return true;
 }
 
-// Entry `col` of the two design rows of one normalised correspondence
-// (x, y) -> (u, v): row 0 = {x, y, 1, 0, 0, 0, -u x, -u y, u},
-// row 1 = {0, 0, 0, x, y, 1, -v x, -v y, v}.
-__device__ __forceinline__ double design(int row, int col, double x, double y, double u, double v) {
-    if (row == 0) {
-        switch (col) {
-            case 0: return x; case 1: return y; case 2: return 1.0;
-            case 3: case 4: case 5: return 0.0;
-            case 6: return -u * x; case 7: return -u * y; default: return u;
-        }
-    }
-    switch (col) {
-        case 0: case 1: case 2: return 0.0;
-        case 3: return x; case 4: return y; case 5: return 1.0;
-        case 6: return -v * x; case 7: return -v * y; default: return v;
-    }
-}
-
-// Gauss-Jordan with partial pivoting on the 8x9 normal equations, h33 = 1,
-// then denormalisation and scaling; m is destroyed.
-__device__ __forceinline__ bool solve_normalised(double (*m)[9], double cax, double cay, double cbx,
-                                                 double cby, double sa, double sb, double* out) {
-    double max_entry = 0.0;
-    for (int i = 0; i < 8; ++i)
-        if (fabs(m[i][i]) > max_entry) max_entry = fabs(m[i][i]);
-    for (int c = 0; c < 8; ++c) {
-        int piv = c;
-        for (int r = c + 1; r < 8; ++r)
-            if (fabs(m[r][c]) > fabs(m[piv][c])) piv = r;
-        if (!fin(m[piv][c]) || fabs(m[piv][c]) <= 1e-12 * max_entry) return false;
-        for (int jx = c; jx < 9; ++jx) {
-            const double t = m[c][jx]; m[c][jx] = m[piv][jx]; m[piv][jx] = t;
-        }
-        const double div = m[c][c];
-        for (int jx = c; jx < 9; ++jx) m[c][jx] /= div;
-        for (int r = 0; r < 8; ++r) {
-            if (r == c) continue;
-            const double f = m[r][c];
-            for (int jx = c; jx < 9; ++jx) m[r][jx] -= f * m[c][jx];
-        }
-    }
-    double h[9];
-    for (int i = 0; i < 8; ++i) h[i] = m[i][8];
-    h[8] = 1.0;
-    const double den_a[9] = {1.0 / sa, 0, cax, 0, 1.0 / sa, cay, 0, 0, 1};
-    const double nrm_b[9] = {sb, 0, -sb * cbx, 0, sb, -sb * cby, 0, 0, 1};
-    double tmp[9];
-    mat3_mul(den_a, h, tmp);
-    mat3_mul(tmp, nrm_b, out);
-    return h_normalize(out);
-}
-
-// Gauss-Jordan of solve_normalised, run by all 32 lanes of a warp on M in
-// shared memory (warp-private). Every entry goes through the serial
-// solver's exact sequence of operations, so the model is bit-identical;
-// lanes only split the independent per-entry work. Returns the same
-// validity on every lane, and every lane holds the model in out.
-__device__ inline bool warp_solve(double (*M)[9], double cax, double cay, double cbx, double cby, double sa,
-                                  double sb, double* out) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    double max_entry = 0.0;
-    for (int i = 0; i < 8; ++i)
-        if (fabs(M[i][i]) > max_entry) max_entry = fabs(M[i][i]);
-    for (int c = 0; c < 8; ++c) {
-        int piv = c;
-        for (int r = c + 1; r < 8; ++r)
-            if (fabs(M[r][c]) > fabs(M[piv][c])) piv = r;
-        const double pv = M[piv][c];
-        if (!fin(pv) || fabs(pv) <= 1e-12 * max_entry) return false;
-        __syncwarp();
-        if (lane >= c && lane < 9) {
-            const double t = M[c][lane];
-            M[c][lane] = M[piv][lane];
-            M[piv][lane] = t;
-        }
-        __syncwarp();
-        const double div = M[c][c];
-        __syncwarp();
-        if (lane >= c && lane < 9) M[c][lane] /= div;
-        __syncwarp();
-        // entries (r, jx), r != c, jx >= c: M[r][jx] -= f_r * M[c][jx] with
-        // f_r = M[r][c] read before any entry of row r changes
-        double f[3], pr[3];
-        int rr[3], jj[3];
-        bool own[3];
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int e = lane + 32 * s;
-            rr[s] = e / 9;
-            jj[s] = e % 9;
-            own[s] = e < 72 && rr[s] != c && jj[s] >= c;
-            f[s] = own[s] ? M[rr[s]][c] : 0.0;
-            pr[s] = own[s] ? M[c][jj[s]] : 0.0;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int s = 0; s < 3; ++s)
-            if (own[s]) M[rr[s]][jj[s]] -= f[s] * pr[s];
-        __syncwarp();
-    }
-    double h[9];
-    for (int i = 0; i < 8; ++i) h[i] = M[i][8];
-    h[8] = 1.0;
-    __syncwarp();
-    const double den_a[9] = {1.0 / sa, 0, cax, 0, 1.0 / sa, cay, 0, 0, 1};
-    const double nrm_b[9] = {sb, 0, -sb * cbx, 0, sb, -sb * cby, 0, 0, 1};
-    double tmp[9];
-    mat3_mul(den_a, h, tmp);
-    mat3_mul(tmp, nrm_b, out);
-    return h_normalize(out);
-}
-
-// Minimal 4-point model computed by a whole warp (all lanes pass the same
-// points): normalisation on every lane, the 72 normal-matrix entries split
-// over the lanes (each summed over the 4 points in order), then
-// warp_solve. Bit-identical to fit4.
-__device__ inline bool warp_fit4(const Pt* p, double (*M)[9], double* out) {
-    const int lane = threadIdx.x & 31;
-    double cax = 0, cay = 0, cbx = 0, cby = 0;
-    for (int i = 0; i < 4; ++i) { cax += p[i].ax; cay += p[i].ay; cbx += p[i].bx; cby += p[i].by; }
-    cax /= 4; cay /= 4; cbx /= 4; cby /= 4;
-    double va = 0.0, vb = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        va += (p[i].ax - cax) * (p[i].ax - cax) + (p[i].ay - cay) * (p[i].ay - cay);
-        vb += (p[i].bx - cbx) * (p[i].bx - cbx) + (p[i].by - cby) * (p[i].by - cby);
-    }
-    if (!(va > 0.0) || !(vb > 0.0) || !fin(va) || !fin(vb)) return false;
-    const double sa = sqrt(2.0 * 4 / va);
-    const double sb = sqrt(2.0 * 4 / vb);
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        const int e = lane + 32 * s;
-        if (e >= 72) continue;
-        const int r = e / 9, c = e % 9;
-        double acc = 0.0;
-        for (int i = 0; i < 4; ++i) {
-            const double x = (p[i].bx - cbx) * sb, y = (p[i].by - cby) * sb;
-            const double u = (p[i].ax - cax) * sa, v = (p[i].ay - cay) * sa;
-            acc += design(0, r, x, y, u, v) * design(0, c, x, y, u, v) +
-                   design(1, r, x, y, u, v) * design(1, c, x, y, u, v);
-        }
-        M[r][c] = acc;
-    }
-    return warp_solve(M, cax, cay, cbx, cby, sa, sb, out);
-}
-
-// Minimal 4-point model on one thread with the 8x9 system in registers:
-// every loop is unrolled and the pivot row swap is a predicated select per
-// entry, so no entry is indexed at run time. Same operations, in the same
-// order per entry, as fit4; bit-identical results.
+// Minimal 4-point model on one thread: the normalised normal equations of the
+// design rows {x, y, 1, 0, 0, 0, -u x, -u y, u} and {0, 0, 0, x, y, 1, -v x,
+// -v y, v}, Gauss-Jordan with partial pivoting, h33 = 1, denormalisation and
+// scaling. The 8x9 system stays in registers: every loop is unrolled and the
+// pivot row swap is a predicated select per entry, so no entry is indexed at
+// run time. Operations per entry are the reference's, in its order.
 __device__ __forceinline__ bool fit4_regs(const Pt* p, double* out) {
     double cax = 0, cay = 0, cbx = 0, cby = 0;
 #pragma unroll
@@ -469,33 +323,6 @@ __device__ __forceinline__ bool fit4_regs(const Pt* p, double* out) {
     mat3_mul(den_a, h, tmp);
     mat3_mul(tmp, nrm_b, out);
     return h_normalize(out);
-}
-
-// Minimal 4-point model (one thread).
-__device__ inline bool fit4(const Pt* p, double* out) {
-    double cax = 0, cay = 0, cbx = 0, cby = 0;
-    for (int i = 0; i < 4; ++i) { cax += p[i].ax; cay += p[i].ay; cbx += p[i].bx; cby += p[i].by; }
-    cax /= 4; cay /= 4; cbx /= 4; cby /= 4;
-    double va = 0.0, vb = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        va += (p[i].ax - cax) * (p[i].ax - cax) + (p[i].ay - cay) * (p[i].ay - cay);
-        vb += (p[i].bx - cbx) * (p[i].bx - cbx) + (p[i].by - cby) * (p[i].by - cby);
-    }
-    if (!(va > 0.0) || !(vb > 0.0) || !fin(va) || !fin(vb)) return false;
-    const double sa = sqrt(2.0 * 4 / va);
-    const double sb = sqrt(2.0 * 4 / vb);
-    double m[8][9];
-    for (int r = 0; r < 8; ++r)
-        for (int c = 0; c < 9; ++c) m[r][c] = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        const double x = (p[i].bx - cbx) * sb, y = (p[i].by - cby) * sb;
-        const double u = (p[i].ax - cax) * sa, v = (p[i].ay - cay) * sa;
-        const double r0[9] = {x, y, 1, 0, 0, 0, -u * x, -u * y, u};
-        const double r1[9] = {0, 0, 0, x, y, 1, -v * x, -v * y, v};
-        for (int r = 0; r < 8; ++r)
-            for (int c = 0; c < 9; ++c) m[r][c] += r0[r] * r0[c] + r1[r] * r1[c];
-    }
-    return solve_normalised(m, cax, cay, cbx, cby, sa, sb, out);
 }
 
 __device__ __forceinline__ bool valid_domain(const double* h, int width, int height) {
@@ -798,136 +625,371 @@ __global__ __launch_bounds__(kSearchThreads, 3) void search_kernel(const __grid_
 
 // ---------------------------------------------------------------- finish
 
-// Sum over i < nm of f(i) in index order (one dependent chain, as the
-// reference's single-thread loop), with the terms computed by the block.
-template <class F>
-__device__ double ordered_sum(int nm, double* buf /*kFinishChunk shared*/, F term) {
-    __shared__ double total;
-    if (threadIdx.x == 0) total = 0.0;
-    for (int base = 0; base < nm; base += kFinishChunk) {
-        const int n = min(kFinishChunk, nm - base);
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) buf[i] = term(base + i);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = total;
-#pragma unroll 8
-            for (int i = 0; i < n; ++i) t += buf[i];
-            total = t;
-        }
-    }
-    __syncthreads();
-    const double r = total;
-    __syncthreads();
-    return r;
+// The finish kernel is bound by its serial FP64 sums: the reference adds
+// every loss, centroid, spread and normal-matrix sum in index order on one
+// thread, and bit-identical sums need that order. What is left to choose is
+// how few such passes run one after another and what a pass waits for:
+// - the points are gathered once into shared memory (kFinishStage of them);
+// - the producer warps compute a chunk of terms while the lanes of warp 0, one per
+//   sum, add the chunk before it, read two doubles at a time and a group of
+//   eight ahead of the adds (chain_sums);
+// - the sums that need the same pass share it: a model's loss, its inlier
+//   residual sum and its inliers' centroid (6 lanes), the two spreads, and
+//   the 28 distinct sums of the 72 normal-matrix entries;
+// - the refit passes run over the list of kept points only: a dropped point
+//   adds +0.0, which leaves a sum started at +0.0 bit for bit unchanged.
+// Per-pair finish at 512x512, 310 matches: 49 -> 27 us; 8000 matches,
+// half of them inliers: 641 -> 156 us (seven passes over all points before).
+// Chunks are as long as shared memory allows (a chunk costs a barrier and the
+// latency of its first loads, about 200 cycles, against 8 cycles per add).
+constexpr int kFinishStage = 8192;  // matched points held in shared memory
+constexpr int kFinishProducers = kFinishThreads - 32;
+constexpr int kEvalChunk = 448;     // points per chunk of the loss and spread passes
+constexpr int kMatrixChunk = 112;   // and of the normal-matrix pass
+constexpr int kEvalSums = 6;        // loss, inlier residuals, centroid of the inliers
+constexpr int kMatrixSums = 28;
+// a sum's terms of a chunk: one row, padded by 16 bytes so that the rows of
+// eight lanes reading 16 bytes each lie in different banks
+__host__ __device__ constexpr int kTermRow(int chunk) { return chunk + 2; }
+constexpr int kTermWords = kMatrixSums * kTermRow(kMatrixChunk);
+static_assert(kEvalSums * kTermRow(kEvalChunk) <= kTermWords, "term buffer");
+
+// Bytes of dynamic shared memory for a match capacity: two chunks of terms,
+// the points, the kept list and two sets of keep flags.
+__host__ __device__ inline int finish_smem_bytes(int match_capacity) {
+    const int n = match_capacity < 1 ? 1 : (match_capacity < kFinishStage ? match_capacity : kFinishStage);
+    return 2 * kTermWords * static_cast<int>(sizeof(double)) +
+           (n + 7) / 8 * 8 * static_cast<int>(sizeof(float4) + sizeof(std::uint16_t) + 2);
 }
 
-// Least-squares refit over the points with keep[i] != 0: the centroid,
-// scale and normal-matrix sums each run in index order as in the reference;
-// the 72 matrix entries are accumulated by 72 threads side by side.
-__device__ inline bool block_fit(const PairIO& j, int nm, const std::uint8_t* keep, double* out, double (*dv)[10],
-                          std::uint8_t* ckeep /*kFinishChunk shared*/) {
-    __shared__ double sums[6];
-    __shared__ int kept;
+struct FinishShared {
+    float4* pts;
+    std::uint16_t* list;
+    std::uint8_t* keep[2];  // inliers of the current model and of the candidate
+    double (*terms)[kTermWords];  // two chunks
+};
+
+// kSums sums over i < n of the terms produce(i, part, out) writes at out[c *
+// kTermRow(kChunk)], c < kSums: sum c in index order on lane c of warp 0
+// (acc, carried in and out), with the terms computed one chunk ahead by the
+// other warps. The last chunk is filled up to a multiple of 16 with +0.0.
+// Every thread of the block calls it; it ends with a barrier. A point's terms
+// are computed in kParts parts by as many threads.
+template <int kChunk, int kSums, int kParts, class F>
+__device__ __forceinline__ void chain_sums(int n, double (*terms)[kTermWords], double& acc, F produce) {
+    static_assert(kChunk % 16 == 0 && kChunk * kParts % kFinishProducers == 0, "producers");
+    const int t = threadIdx.x;
+    const int steps = (n + kChunk - 1) / kChunk;
+#pragma unroll 1
+    for (int step = 0; step <= steps; ++step) {
+        if (t >= 32) {
+            if (step < steps) {
+#pragma unroll 1
+                for (int w = t - 32; w < kChunk * kParts; w += kFinishProducers) {
+                    const int x = w % kChunk, part = w / kChunk;
+                    const int i = step * kChunk + x;
+                    double* out = terms[step & 1] + x;
+                    if (i < n) {
+                        produce(i, part, out);
+                    } else if (part == 0 && i < (n + 15) / 16 * 16) {
+#pragma unroll 1
+                        for (int c = 0; c < kSums; ++c) out[c * kTermRow(kChunk)] = 0.0;
+                    }
+                }
+            }
+        } else if (t < kSums && step > 0) {
+            const int left = min(kChunk, n - (step - 1) * kChunk);
+            const double2* row = reinterpret_cast<const double2*>(terms[(step - 1) & 1] + t * kTermRow(kChunk));
+            double a = acc;
+            double2 q0 = row[0], q1 = row[1], q2 = row[2], q3 = row[3];
+#pragma unroll 1
+            for (int i = 0; i < left; i += 16) {  // reads up to 8 terms past the last 16, without adding them
+                const double2* r = row + i / 2;
+                const double2 p0 = r[4], p1 = r[5], p2 = r[6], p3 = r[7];
+                a += q0.x; a += q0.y; a += q1.x; a += q1.y;
+                a += q2.x; a += q2.y; a += q3.x; a += q3.y;
+                q0 = r[8]; q1 = r[9]; q2 = r[10]; q3 = r[11];
+                a += p0.x; a += p0.y; a += p1.x; a += p1.y;
+                a += p2.x; a += p2.y; a += p3.x; a += p3.y;
+            }
+            acc = a;
+        }
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ Pt finish_point(const PairIO& j, const FinishShared& sh, int i) {
+    if (i < kFinishStage) {
+        const float4 q = sh.pts[i];
+        return Pt{q.x, q.y, q.z, q.w};
+    }
+    return gather(j, i);
+}
+
+// Serial loss, inlier residual sum and inlier centroid sums of model h, into
+// sums[kEvalSums], and its inlier count into *kept; the inliers' flags go to
+// keep, or to j.mask when there are more points than shared memory holds.
+__device__ __forceinline__ void evaluate(const PairIO& j, const FinishShared& sh, int nm, double thr2,
+                                         const double* hs, double* sums, int* kept, std::uint8_t* keep) {
+    double h[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) h[e] = hs[e];
+    constexpr int kRow = kTermRow(kEvalChunk);
+    const bool staged = nm <= kFinishStage;
+    double acc = 0.0;
+    int mine = 0;
+    if (threadIdx.x == 0) *kept = 0;
+    chain_sums<kEvalChunk, kEvalSums, 1>(nm, sh.terms, acc, [&](int i, int, double* out) {
+        const Pt p = finish_point(j, sh, i);
+        const double r = residual2(h, p);
+        const bool in = r <= thr2;
+        mine += in;
+        if (staged) keep[i] = in;
+        else j.mask[i] = in;
+        out[0] = r < thr2 ? r : thr2;
+        out[kRow] = in ? r : 0.0;
+        out[2 * kRow] = in ? p.ax : 0.0;
+        out[3 * kRow] = in ? p.ay : 0.0;
+        out[4 * kRow] = in ? p.bx : 0.0;
+        out[5 * kRow] = in ? p.by : 0.0;
+    });
+    if (threadIdx.x < kEvalSums) sums[threadIdx.x] = acc;
+    if (mine) atomicAdd(kept, mine);
+    __syncthreads();
+}
+
+// The kept points' indices, in order, into sh.list (block-wide scan).
+__device__ __forceinline__ void list_kept(const FinishShared& sh, const std::uint8_t* keep, int nm) {
+    __shared__ int warp_total[kFinishThreads / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int seg = (nm + kFinishThreads - 1) / kFinishThreads;
+    const int lo = min(nm, t * seg), hi = min(nm, lo + seg);
+    int n = 0;
+    for (int i = lo; i < hi; ++i) n += keep[i];
+    int run = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
+    }
+    if (lane == 31) warp_total[warp] = run;
+    __syncthreads();
+    int at = run - n;
+    for (int w = 0; w < warp; ++w) at += warp_total[w];
+    for (int i = lo; i < hi; ++i)
+        if (keep[i]) sh.list[at++] = static_cast<std::uint16_t>(i);
+    __syncthreads();
+}
+
+// 3x3 matrices with entry e (row-major) on lane e, lanes 9 and up a copy of
+// entry 8: mat3_mul and h_normalize, each entry by the same operations.
+__device__ __forceinline__ double warp_mat3(double a, double b) {
+    const int lane = threadIdx.x & 31, e = lane < 9 ? lane : 8, r = 3 * (e / 3), c = e % 3;
+    const double a0 = __shfl_sync(0xffffffffu, a, r), a1 = __shfl_sync(0xffffffffu, a, r + 1),
+                 a2 = __shfl_sync(0xffffffffu, a, r + 2);
+    const double b0 = __shfl_sync(0xffffffffu, b, c), b1 = __shfl_sync(0xffffffffu, b, c + 3),
+                 b2 = __shfl_sync(0xffffffffu, b, c + 6);
+    return a0 * b0 + a1 * b1 + a2 * b2;
+}
+
+// The nine entries, on every lane.
+__device__ __forceinline__ void warp_spread(double x, double* out) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) out[i] = __shfl_sync(0xffffffffu, x, i);
+}
+
+__device__ __forceinline__ bool warp_normalize(double& x) {
+    double scale = fabs(x);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, scale, o);
+        if (v > scale) scale = v;
+    }
+    scale = __shfl_sync(0xffffffffu, scale, 0);  // the largest of lanes 0..15: every entry
+    if (!__all_sync(0xffffffffu, fin(x)) || !(scale > 0.0)) return false;
+    x /= scale;
+    double h[9];
+    warp_spread(x, h);
+    const double det = h[0] * (h[4] * h[8] - h[5] * h[7]) - h[1] * (h[3] * h[8] - h[5] * h[6]) +
+                       h[2] * (h[3] * h[7] - h[4] * h[6]);
+    return fin(det) && fabs(det) > 1e-15;
+}
+
+// fit4_regs' Gauss-Jordan by one warp on M in shared memory (destroyed): each
+// entry takes the serial solver's operations, the lanes split the independent
+// ones, and columns left of the pivot, which are not read again, are left
+// alone. Same validity and model on every lane. The loop over the columns
+// stays a loop: the code runs once per launch, and unrolled its instruction
+// fetches took longer than the arithmetic.
+__device__ inline bool warp_solve(double (*M)[9], double cax, double cay, double cbx, double cby, double sa,
+                                  double sb, double* out) {
+    const int lane = threadIdx.x & 31, row = lane & 7, col = lane < 9 ? lane : 8;
+    double max_entry = fabs(M[row][row]);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, max_entry, o);
+        if (v > max_entry) max_entry = v;
+    }
+    bool solvable = true;
+#pragma unroll 1
+    for (int c = 0; c < 8; ++c) {
+        // the first of the largest entries at or below the diagonal. (A NaN
+        // may be picked or passed over here; its row stays NaN until it is the
+        // pivot row, so the system is rejected either way.)
+        double pv = M[row][c];
+        double best = row >= c ? fabs(pv) : -1.0;
+        int piv = row;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, best, o), w = __shfl_xor_sync(0xffffffffu, pv, o);
+            const int r = __shfl_xor_sync(0xffffffffu, piv, o);
+            if (v > best || (v == best && r < piv)) { best = v; pv = w; piv = r; }
+        }
+        piv = __shfl_sync(0xffffffffu, piv, 0);
+        pv = __shfl_sync(0xffffffffu, pv, 0);
+        if (piv < c) {  // only NaN entries are left
+            piv = c;
+            pv = M[c][c];
+        }
+        solvable = solvable && fin(pv) && !(fabs(pv) <= 1e-12 * max_entry);
+        const double a = M[c][col], b = M[piv][col];
+        const double scaled = b / pv;
+        __syncwarp();
+        if (lane >= c && lane < 9) {
+            M[piv][lane] = a;
+            M[c][lane] = scaled;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            const int e = lane + 32 * s, r = e / 9, jx = e % 9;
+            if (e < 72 && r != c && jx > c) M[r][jx] -= M[r][c] * M[c][jx];
+        }
+        __syncwarp();
+    }
+    double x = col < 8 ? M[col][8] : 1.0;  // entry `col` of the normalised model
+    const double isa = 1.0 / sa;
+    const double den_a = col == 0 || col == 4 ? isa : col == 2 ? cax : col == 5 ? cay : col == 8 ? 1.0 : 0.0;
+    const double nrm_b = col == 0 || col == 4 ? sb : col == 2 ? -sb * cbx : col == 5 ? -sb * cby : col == 8 ? 1.0 : 0.0;
+    x = warp_mat3(warp_mat3(den_a, x), nrm_b);
+    const bool ok = warp_normalize(x);
+    warp_spread(x, out);
+    return solvable && ok;
+}
+
+// Least-squares refit over the kept points (sums and keep: evaluate()'s, of
+// the model that kept them), into out (shared memory); false, on every
+// thread, when there is no model or its domain test fails. The few divisions
+// and square roots run side by side on the lanes of a warp: one after the
+// other, on one thread, they took as long as a pass over 300 points.
+__device__ inline bool block_fit(const PairIO& j, const FinishShared& sh, const std::uint8_t* keep, int nm, int kept,
+                                 const double* sums, int bw, int bh, double* out) {
+    __shared__ double centre[4], spread[2], scale[2], total[kMatrixSums];
     __shared__ double m[8][9];
     __shared__ int ok;
     const int t = threadIdx.x;
-    if (t < 6) sums[t] = 0.0;
-    if (t == 6) kept = 0;
-    if (t < 72) m[t / 9][t % 9] = 0.0;
-    // Each sum below starts at +0.0 and runs in index order on one thread
-    // over terms the block computed beforehand; a dropped point contributes
-    // +0.0, which leaves such a sum bit-identical to skipping the point
-    // (round-to-nearest never turns a sum that starts at +0.0 into -0.0).
-    // pass 1: centroids
-    int mine = 0;
-    for (int base = 0; base < nm; base += kFinishChunk) {
-        const int n = min(kFinishChunk, nm - base);
-        __syncthreads();
-        for (int i = t; i < n; i += blockDim.x) {
-            const Pt p = gather(j, base + i);
-            const bool k = keep[base + i] != 0;
-            mine += k ? 1 : 0;
-            dv[i][0] = k ? p.ax : 0.0;
-            dv[i][1] = k ? p.ay : 0.0;
-            dv[i][2] = k ? p.bx : 0.0;
-            dv[i][3] = k ? p.by : 0.0;
+    if (kept < 4) return false;
+    const bool listed = nm <= kFinishStage;
+    const int items = listed ? kept : nm;
+    if (t < 4) centre[t] = sums[2 + t] / kept;
+    if (listed) list_kept(sh, keep, nm);
+    else __syncthreads();
+    const double cax = centre[0], cay = centre[1], cbx = centre[2], cby = centre[3];
+    const auto point = [&](int i, Pt& p) {  // whether item i is kept
+        if (listed) {
+            const float4 q = sh.pts[sh.list[i]];
+            p = Pt{q.x, q.y, q.z, q.w};
+            return true;
+        }
+        p = gather(j, i);
+        return j.mask[i] != 0;
+    };
+    // spreads
+    {
+        constexpr int kRow = kTermRow(kEvalChunk);
+        double acc = 0.0;
+        chain_sums<kEvalChunk, 2, 1>(items, sh.terms, acc, [&](int i, int, double* o) {
+            Pt p;
+            const bool k = point(i, p);
+            o[0] = k ? (p.ax - cax) * (p.ax - cax) + (p.ay - cay) * (p.ay - cay) : 0.0;
+            o[kRow] = k ? (p.bx - cbx) * (p.bx - cbx) + (p.by - cby) * (p.by - cby) : 0.0;
+        });
+        if (t < 2) {
+            spread[t] = acc;
+            scale[t] = sqrt(2.0 * kept / acc);
         }
         __syncthreads();
-        if (t < 4) {
-            double a = sums[t];
-#pragma unroll 8
-            for (int i = 0; i < n; ++i) a += dv[i][t];
-            sums[t] = a;
-        }
     }
-    if (mine) atomicAdd(&kept, mine);
-    __syncthreads();
-    const int count = kept;
-    if (count < 4) return false;
-    const double cax = sums[0] / count, cay = sums[1] / count, cbx = sums[2] / count, cby = sums[3] / count;
-    // pass 2: spreads
-    for (int base = 0; base < nm; base += kFinishChunk) {
-        const int n = min(kFinishChunk, nm - base);
-        __syncthreads();
-        for (int i = t; i < n; i += blockDim.x) {
-            const Pt p = gather(j, base + i);
-            const bool k = keep[base + i] != 0;
-            dv[i][0] = k ? (p.ax - cax) * (p.ax - cax) + (p.ay - cay) * (p.ay - cay) : 0.0;
-            dv[i][1] = k ? (p.bx - cbx) * (p.bx - cbx) + (p.by - cby) * (p.by - cby) : 0.0;
-        }
-        __syncthreads();
-        if (t == 0 || t == 32) {
-            const int col = t ? 1 : 0;
-            double a = sums[4 + col];
-#pragma unroll 8
-            for (int i = 0; i < n; ++i) a += dv[i][col];
-            sums[4 + col] = a;
-        }
-    }
-    __syncthreads();
-    const double va = sums[4], vb = sums[5];
+    const double va = spread[0], vb = spread[1];
     if (!(va > 0.0) || !(vb > 0.0) || !fin(va) || !fin(vb)) return false;
-    const double sa = sqrt(2.0 * count / va);
-    const double sb = sqrt(2.0 * count / vb);
-    // pass 3: normal matrix, entry (r, c) on thread 9r + c. Each point's ten
-    // design values are computed once (by the point's thread) into dv; a
-    // matrix thread reads its four factors by index:
-    // dv = {x, y, 1, 0, u, v, -u x, -u y, -v x, -v y},
-    // row 0 = dv[{0,1,2,3,3,3,6,7,4}], row 1 = dv[{3,3,3,0,1,2,8,9,5}].
-    constexpr unsigned char kRow0[9] = {0, 1, 2, 3, 3, 3, 6, 7, 4};
-    constexpr unsigned char kRow1[9] = {3, 3, 3, 0, 1, 2, 8, 9, 5};
-    const int r = t / 9, c = t % 9;
-    const int i0r = t < 72 ? kRow0[r] : 0, i0c = t < 72 ? kRow0[c] : 0;
-    const int i1r = t < 72 ? kRow1[r] : 0, i1c = t < 72 ? kRow1[c] : 0;
-    for (int base = 0; base < nm; base += kFinishChunk) {
-        const int n = min(kFinishChunk, nm - base);
-        __syncthreads();
-        for (int i = t; i < n; i += blockDim.x) {
-            const Pt p = gather(j, base + i);
-            ckeep[i] = keep[base + i];
+    const double sa = scale[0], sb = scale[1];
+    // normal matrix of the design rows {x, y, 1, 0, 0, 0, -ux, -uy, u} and
+    // {0, 0, 0, x, y, 1, -vx, -vy, v}. A product with a structural 0 adds
+    // +-0, a no-op; the blocks (0..2, 0..2) and (3..5, 3..5) are equal, the
+    // matrix is symmetric (products commute) and the entry of the two 1s is
+    // the count. What is left are kMatrixSums sums, in two parts: the x, y
+    // block with the u rows (14 sums), and the v rows with rows 6 and 7 (14).
+    {
+        constexpr int kRow = kTermRow(kMatrixChunk);
+        double acc = 0.0;
+        chain_sums<kMatrixChunk, kMatrixSums, 2>(items, sh.terms, acc, [&](int i, int part, double* o) {
+            Pt p;
+            const bool k = point(i, p);
             const double x = (p.bx - cbx) * sb, y = (p.by - cby) * sb;
             const double u = (p.ax - cax) * sa, v = (p.ay - cay) * sa;
-            double* d = dv[i];
-            d[0] = x; d[1] = y; d[2] = 1.0; d[3] = 0.0; d[4] = u; d[5] = v;
-            d[6] = -u * x; d[7] = -u * y; d[8] = -v * x; d[9] = -v * y;
-        }
-        __syncthreads();
-        if (t < 72) {
-            double acc = m[r][c];
-#pragma unroll 4
-            for (int i = 0; i < n; ++i) {
-                const double* d = dv[i];
-                const double term = d[i0r] * d[i0c] + d[i1r] * d[i1c];
-                acc += ckeep[i] ? term : 0.0;
+            const double w = part == 0 ? u : v;
+            const double wx = -w * x, wy = -w * y;
+            double* q = o + (part == 0 ? 10 : 19) * kRow;
+            q[0] = k ? x * wx : 0.0;
+            q[kRow] = k ? x * wy : 0.0;
+            q[2 * kRow] = k ? x * w : 0.0;
+            q[3 * kRow] = k ? y * wx : 0.0;
+            q[4 * kRow] = k ? y * wy : 0.0;
+            q[5 * kRow] = k ? y * w : 0.0;
+            q[6 * kRow] = k ? wx : 0.0;
+            q[7 * kRow] = k ? wy : 0.0;
+            q[8 * kRow] = k ? w : 0.0;
+            if (part == 0) {
+                o[0] = k ? x * x : 0.0;
+                o[kRow] = k ? x * y : 0.0;
+                o[2 * kRow] = k ? x : 0.0;
+                o[3 * kRow] = k ? y * y : 0.0;
+                o[4 * kRow] = k ? y : 0.0;
+            } else {
+                const double ux = -u * x, uy = -u * y;
+                o[5 * kRow] = k ? ux * ux + wx * wx : 0.0;
+                o[6 * kRow] = k ? ux * uy + wx * wy : 0.0;
+                o[7 * kRow] = k ? ux * u + wx * v : 0.0;
+                o[8 * kRow] = k ? uy * uy + wy * wy : 0.0;
+                o[9 * kRow] = k ? uy * u + wy * v : 0.0;
             }
-            m[r][c] = acc;
-        }
+        });
+        if (t < kMatrixSums) total[t] = acc;
+        __syncthreads();
+    }
+    if (t < 72) {
+        // sum of each entry: kMatrixSums is 0, kMatrixSums + 1 the count
+        constexpr unsigned char kZ = kMatrixSums, kN = kMatrixSums + 1;
+        constexpr unsigned char kSum[72] = {0,  1,  2,  kZ, kZ, kZ, 10, 11, 12,   // x
+                                            1,  3,  4,  kZ, kZ, kZ, 13, 14, 15,   // y
+                                            2,  4,  kN, kZ, kZ, kZ, 16, 17, 18,   // 1
+                                            kZ, kZ, kZ, 0,  1,  2,  19, 20, 21,   // x
+                                            kZ, kZ, kZ, 1,  3,  4,  22, 23, 24,   // y
+                                            kZ, kZ, kZ, 2,  4,  kN, 25, 26, 27,   // 1
+                                            10, 13, 16, 19, 22, 25, 5,  6,  7,    // -ux, -vx
+                                            11, 14, 17, 20, 23, 26, 6,  8,  9};   // -uy, -vy
+        const int e = kSum[t];
+        m[t / 9][t % 9] = e == kZ ? 0.0 : e == kN ? static_cast<double>(kept) : total[e];
     }
     __syncthreads();
     if (t < 32) {
-        const bool solved = warp_solve(m, cax, cay, cbx, cby, sa, sb, out);
-        if (t == 0) ok = solved;
+        double h[9];
+        const bool solved = warp_solve(m, cax, cay, cbx, cby, sa, sb, h) && valid_domain(h, bw, bh);
+        if (t == 0) {
+            ok = solved;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) out[i] = h[i];
+        }
     }
     __syncthreads();
     return ok;
@@ -937,166 +999,190 @@ __device__ inline bool block_fit(const PairIO& j, int nm, const std::uint8_t* ke
 // winner, refine, and build the mask and the result.
 template <class Src>
 __global__ __launch_bounds__(kFinishThreads, 1) void finish_kernel(const __grid_constant__ Src src) {
-    __shared__ int red_src[kFinishThreads];
-    __shared__ double buf[kFinishChunk];
-    __shared__ std::uint8_t ckeep[kFinishChunk];
-    __shared__ double dv[kFinishChunk][10];
-    __shared__ Model model, cand;
+    extern __shared__ float4 finish_smem[];  // terms, points, kept list, keep flags
+    __shared__ double model[2][9], loss;  // current model and candidate; loss of the current one
     __shared__ HomographyResult res;
-    __shared__ int cand_ok, inl;
+    __shared__ double sums[2][kEvalSums];
+    __shared__ int keep_mask, kept[2];
     __shared__ double mins[4][kFinishThreads / 32];
     PairIO j;
     int local;
     if (!src.find(blockIdx.x, &j, &local)) return;
     State* s = j.state;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const double nanv = __longlong_as_double(0x7ff8000000000000ll);
-    // 1. raw winner: index of the best block result (-1: none)
-    int src_i = -1;
-    for (int i = t; i < j.search_blocks; i += kFinishThreads)
-        if (src_i < 0 ? j.block_best[i].valid != 0 : better(j.block_best[i], j.block_best[src_i])) src_i = i;
-    red_src[t] = src_i;
-    __syncthreads();
-    for (int o = kFinishThreads / 2; o > 0; o >>= 1) {
-        if (t < o) {
-            const int other = red_src[t + o], mine = red_src[t];
-            if (other >= 0 && (mine < 0 || better(j.block_best[other], j.block_best[mine]))) red_src[t] = other;
-        }
-        __syncthreads();
-    }
     const int status0 = s->status;
-    if (t == 0) {
-        if (status0 == static_cast<int>(Status::OK) && red_src[0] >= 0 &&
-            better(j.block_best[red_src[0]], s->best))
-            s->best = j.block_best[red_src[0]];
-        HomographyResult r{};
-        for (int i = 0; i < 9; ++i) r.H[i] = r.H_s[i] = nanv;
-        r.reproj_residual = nanv;
-        r.num_matches = (s->nm >= 0 && s->nm <= j.m.capacity) ? s->nm : 0;
-        r.status = static_cast<Status>(status0);
-        if (status0 == static_cast<int>(Status::OK) && !s->best.valid) r.status = Status::DEGENERATE;
-        res = r;
-        model = s->best;
+    const bool go = status0 == static_cast<int>(Status::OK);
+    const int cap = min(j.m.capacity, kFinishStage);
+    FinishShared sh;
+    const int room = (max(cap, 1) + 7) / 8 * 8;
+    sh.terms = reinterpret_cast<double (*)[kTermWords]>(finish_smem);
+    sh.pts = finish_smem + 2 * kTermWords * sizeof(double) / sizeof(float4);
+    sh.list = reinterpret_cast<std::uint16_t*>(sh.pts + room);
+    sh.keep[0] = reinterpret_cast<std::uint8_t*>(sh.list + room);
+    sh.keep[1] = sh.keep[0] + room;
+    if (warp == 0) {
+        // 1. raw winner: the best block result, if it beats the saved one
+        Model b;  // only loss, hypothesis and valid are used
+        b.loss = 0.0;
+        b.hypothesis = 0;
+        b.valid = 0;
+        int at = -1;
+#pragma unroll 4
+        for (int i = lane; i < j.search_blocks; i += 32) {
+            Model c;
+            c.loss = j.block_best[i].loss;
+            c.hypothesis = j.block_best[i].hypothesis;
+            c.valid = j.block_best[i].valid;
+            if (better(c, b)) { b.loss = c.loss; b.hypothesis = c.hypothesis; b.valid = c.valid; at = i; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            Model c;
+            c.loss = __shfl_xor_sync(0xffffffffu, b.loss, o);
+            c.hypothesis = __shfl_xor_sync(0xffffffffu, b.hypothesis, o);
+            c.valid = __shfl_xor_sync(0xffffffffu, b.valid, o);
+            const int other = __shfl_xor_sync(0xffffffffu, at, o);
+            if (better(c, b)) { b.loss = c.loss; b.hypothesis = c.hypothesis; b.valid = c.valid; at = other; }
+        }
+        at = __shfl_sync(0xffffffffu, at, 0);
+        const bool take = go && at >= 0 && better(b, s->best);
+        const bool any = take || s->best.valid;
+        const double x = lane < 9 ? (take ? j.block_best[at].h[lane] : s->best.h[lane]) : 0.0;
+        __syncwarp();
+        if (take && lane < 9) s->best.h[lane] = x;
+        if (take && lane == 0) {
+            s->best.loss = b.loss;
+            s->best.hypothesis = b.hypothesis;
+            s->best.valid = b.valid;
+        }
+        static_assert(sizeof(HomographyResult) % 8 == 0 && sizeof(HomographyResult) / 8 <= 32, "result words");
+        if (lane < sizeof(HomographyResult) / 8) reinterpret_cast<std::uint64_t*>(&res)[lane] = 0;  // padding too
+        __syncwarp();
+        if (lane < 9) {
+            model[0][lane] = x;
+            res.H[lane] = res.H_s[lane] = nanv;
+        }
+        if (lane == 0) {
+            res.num_matches = (s->nm >= 0 && s->nm <= j.m.capacity) ? s->nm : 0;
+            res.reproj_residual = nanv;
+            res.status = go && !any ? Status::DEGENERATE : static_cast<Status>(status0);
+        }
+    } else if (go) {
+        const int staged = min(s->nm, kFinishStage);
+#pragma unroll 4
+        for (int i = t - 32; i < staged; i += kFinishThreads - 32) {
+            const int ia = j.m.idx_a[i], ib = j.m.idx_b[i];
+            sh.pts[i] = make_float4(j.a.x[ia], j.a.y[ia], j.b.x[ib], j.b.y[ib]);
+        }
     }
-    for (int i = t; i < j.m.capacity; i += kFinishThreads) j.mask[i] = 0;
     __syncthreads();
+    bool fill = true;  // whether the mask is still to be cleared
     if (res.status == Status::OK) {
         const int nm = s->nm;
         const double thr2 = j.c.threshold * j.c.threshold;
         const int bw = s->scale_b.work_w, bh = s->scale_b.work_h;
-        {
-            double h[9];
-            for (int e = 0; e < 9; ++e) h[e] = model.h[e];
-            const double loss = ordered_sum(nm, buf, [&](int i) {
-                const double r = residual2(h, gather(j, i));
-                return r < thr2 ? r : thr2;
-            });
-            if (t == 0) model.loss = loss;
-        }
-        __syncthreads();
-        for (int step = 0; step < j.c.refinement_steps; ++step) {
-            double h[9];
-            for (int e = 0; e < 9; ++e) h[e] = model.h[e];
-            // inliers of the current model, kept in the mask buffer
-            for (int i = t; i < nm; i += kFinishThreads) j.mask[i] = residual2(h, gather(j, i)) <= thr2;
-            __syncthreads();
-            double ch[9];
-            const bool fitted = block_fit(j, nm, j.mask, ch, dv, ckeep);
-            if (t == 0) {
-                cand_ok = fitted && valid_domain(ch, bw, bh);
-                for (int e = 0; e < 9; ++e) cand.h[e] = ch[e];
-            }
-            __syncthreads();
-            if (!cand_ok) break;
-            double hc[9];
-            for (int e = 0; e < 9; ++e) hc[e] = cand.h[e];
-            const double closs = ordered_sum(nm, buf, [&](int i) {
-                const double r = residual2(hc, gather(j, i));
-                return r < thr2 ? r : thr2;
-            });
-            const bool take = fin(closs) && closs < model.loss;
+        // One loop, so that the code of a pass is fetched once: the raw model,
+        // then each refit, accepted on a strictly lower serial loss.
+        int cur = 0, trial = 0;
+#pragma unroll 1
+        for (int step = 0;; ++step) {
+            evaluate(j, sh, nm, thr2, model[trial], sums[trial], &kept[trial], sh.keep[trial]);
+            const double now = sums[trial][0];
+            const bool take = step == 0 || (fin(now) && now < loss);
             __syncthreads();
             if (!take) break;
-            if (t == 0) {
-                for (int e = 0; e < 9; ++e) model.h[e] = cand.h[e];
-                model.loss = closs;
-            }
-            __syncthreads();
+            cur = trial;
+            if (t == 0) loss = now;
+            if (step >= j.c.refinement_steps) break;
+            trial = cur ^ 1;
+            if (!block_fit(j, sh, sh.keep[cur], nm, kept[cur], sums[cur], bw, bh, model[trial])) break;
         }
-        // mask, inlier count, residual sum (index order), inlier extent
-        double h[9];
-        for (int e = 0; e < 9; ++e) h[e] = model.h[e];
-        if (t == 0) inl = 0;
-        __syncthreads();
+        // mask and inlier extent of the final model, and the result
         double mnx = DBL_MAX, mny = DBL_MAX, mxx = -DBL_MAX, mxy = -DBL_MAX;
-        int cnt = 0;
-        for (int i = t; i < j.m.capacity; i += kFinishThreads) {
-            std::uint8_t in = 0;
-            if (i < nm) {
+        if (nm <= kFinishStage) {
+            for (int i = t; i < nm; i += kFinishThreads)
+                if (sh.keep[cur][i]) {
+                    const float4 q = sh.pts[i];
+                    mnx = fmin(mnx, static_cast<double>(q.x)); mxx = fmax(mxx, static_cast<double>(q.x));
+                    mny = fmin(mny, static_cast<double>(q.y)); mxy = fmax(mxy, static_cast<double>(q.y));
+                }
+        } else {
+            double h[9];
+            for (int e = 0; e < 9; ++e) h[e] = model[cur][e];
+            for (int i = t; i < nm; i += kFinishThreads) {
                 const Pt q = gather(j, i);
-                if (residual2(h, q) <= thr2) {
-                    in = 1;
-                    ++cnt;
+                const bool in = residual2(h, q) <= thr2;
+                j.mask[i] = in;
+                if (in) {
                     mnx = fmin(mnx, q.ax); mxx = fmax(mxx, q.ax);
                     mny = fmin(mny, q.ay); mxy = fmax(mxy, q.ay);
                 }
             }
-            j.mask[i] = in;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
             mnx = fmin(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
             mny = fmin(mny, __shfl_xor_sync(0xffffffffu, mny, o));
             mxx = fmax(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
             mxy = fmax(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
         }
-        if ((t & 31) == 0) {
-            atomicAdd(&inl, cnt);
-            mins[0][t >> 5] = mnx; mins[1][t >> 5] = mny; mins[2][t >> 5] = mxx; mins[3][t >> 5] = mxy;
+        if (lane == 0) {
+            mins[0][warp] = mnx; mins[1][warp] = mny; mins[2][warp] = mxx; mins[3][warp] = mxy;
         }
-        const double sum = ordered_sum(nm, buf, [&](int i) {
-            const double r = residual2(h, gather(j, i));
-            return r <= thr2 ? r : 0.0;
-        });
-        if (t == 0) {
+        __syncthreads();
+        if (warp == 0) {  // one lane per entry of the matrices
+            const int inliers = kept[cur], e = lane < 9 ? lane : 8;
             double a = DBL_MAX, bb = DBL_MAX, c = -DBL_MAX, d = -DBL_MAX;
             for (int w = 0; w < kFinishThreads / 32; ++w) {
                 a = fmin(a, mins[0][w]); bb = fmin(bb, mins[1][w]);
                 c = fmax(c, mins[2][w]); d = fmax(d, mins[3][w]);
             }
-            HomographyResult r = res;
-            r.num_inliers = inl;
-            if (r.num_inliers < 4) {
-                r.status = Status::DEGENERATE;
-                r.num_inliers = 0;
-                cand_ok = 0;  // clear the mask below
-            } else {
-                r.inlier_ratio = static_cast<double>(r.num_inliers) / nm;
-                r.reproj_residual = sqrt(sum / r.num_inliers);
-                const double w = fmax(1.0, static_cast<double>(s->scale_a.work_w - 1));
-                const double hh = fmax(1.0, static_cast<double>(s->scale_a.work_h - 1));
-                r.inlier_coverage = fmin(1.0, (c - a) / w) * fmin(1.0, (d - bb) / hh);
-                for (int e = 0; e < 9; ++e) r.H_s[e] = h[e];
-                double tmp[9];
-                mat3_mul(j.inverse_a, h, tmp);
-                mat3_mul(tmp, j.d_b, r.H);
-                cand_ok = 1;
-                if (!h_normalize(r.H) || !valid_domain(r.H, s->scale_b.orig_w, s->scale_b.orig_h)) {
-                    r.status = Status::DEGENERATE;
-                    r.num_inliers = 0;
-                    r.inlier_ratio = r.inlier_coverage = 0.0;
-                    r.reproj_residual = nanv;
-                    for (int e = 0; e < 9; ++e) r.H[e] = r.H_s[e] = nanv;
-                    cand_ok = 0;
-                }
+            const double hs = model[cur][e];
+            double ia = j.inverse_a[0], db = j.d_b[0];  // selects: a run-time index would put the job in local memory
+#pragma unroll
+            for (int i = 1; i < 9; ++i) {
+                ia = e == i ? j.inverse_a[i] : ia;
+                db = e == i ? j.d_b[i] : db;
             }
-            res = r;
+            double H = warp_mat3(warp_mat3(ia, hs), db);
+            bool ok = warp_normalize(H);
+            double hh[9];
+            warp_spread(H, hh);
+            ok = ok && valid_domain(hh, s->scale_b.orig_w, s->scale_b.orig_h) && inliers >= 4;
+            // four divisions, one per lane
+            const double w = fmax(1.0, static_cast<double>(s->scale_a.work_w - 1));
+            const double ht = fmax(1.0, static_cast<double>(s->scale_a.work_h - 1));
+            const double num = lane == 0 ? static_cast<double>(inliers) : lane == 1 ? sums[cur][1] : lane == 2 ? c - a : d - bb;
+            const double den = lane == 0 ? nm : lane == 1 ? inliers : lane == 2 ? w : ht;
+            const double q = num / den;
+            const double cover_x = __shfl_sync(0xffffffffu, q, 2), cover_y = __shfl_sync(0xffffffffu, q, 3);
+            if (ok && lane < 9) {
+                res.H[lane] = H;
+                res.H_s[lane] = hs;
+            }
+            if (ok && lane == 0) {
+                res.num_inliers = inliers;
+                res.inlier_ratio = q;
+                res.inlier_coverage = fmin(1.0, cover_x) * fmin(1.0, cover_y);
+            }
+            if (ok && lane == 1) res.reproj_residual = sqrt(q);
+            if (lane == 0) {
+                if (!ok) res.status = Status::DEGENERATE;
+                keep_mask = ok;
+            }
         }
         __syncthreads();
-        if (!cand_ok)
-            for (int i = t; i < j.m.capacity; i += kFinishThreads) j.mask[i] = 0;
+        if (keep_mask) {
+            fill = false;
+            if (nm <= kFinishStage)
+                for (int i = t; i < j.m.capacity; i += kFinishThreads) j.mask[i] = i < nm ? sh.keep[cur][i] : 0;
+            else
+                for (int i = nm + t; i < j.m.capacity; i += kFinishThreads) j.mask[i] = 0;
+        }
     }
+    if (fill)
+        for (int i = t; i < j.m.capacity; i += kFinishThreads) j.mask[i] = 0;
     if (t == 0) {
         s->evaluated = j.c.hypotheses;
         s->result = res;
