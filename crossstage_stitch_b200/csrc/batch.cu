@@ -21,6 +21,7 @@
 #include <iterator>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "batch.hpp"
 
@@ -65,8 +66,11 @@ void set_attributes_once() {
         cudaFuncSetAttribute(s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              s2s3::kSortCap * static_cast<int>(sizeof(std::uint64_t)));
-        s5k::enable_search_smem_once(
-            reinterpret_cast<const void*>(s5k::search_kernel<s5k::JobTable<SearchJob>, true>));
+        using Src = s5k::JobTable<SearchJob>;
+        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 32>), true);
+        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 64>), true);
+        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 128>), true);
+        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 256>), true);
         s5k::enable_finish_smem_once(reinterpret_cast<const void*>(s5k::finish_kernel<s5k::JobTable<PairIO>>));
     });
 }
@@ -213,22 +217,27 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     }
     sort_smem = s2s3::sort_smem_bytes(max_cand);
     rank_fallback = max_cand > s2s3::kSortCap;
-    search_smem = s5k::search_smem_bytes(max_cap_m);
+    search_smem = s5k::search_smem_bytes(max_cap_m, true);
     finish_smem = s5k::finish_smem_bytes(max_cap_m);
     // S4: one train partition per block unless the batch is too small to fill the GPU
     n_knn = 0;
     for (int i = 0; i < n; ++i) n_knn += pairs[i].s4.cross_check ? 2 : 1;
     const int want_splits = knn_want_splits();
     knn_blocks = merge_blocks = 0;
-    // S5: hypotheses per warp round, as large as still fills about two waves
+    // S5: hypotheses per warp (8 warps a block), as many as still fill a wave
+    // of four blocks per SM: fewer blocks gather the matches fewer times and
+    // score fewer models exactly before the first bounds are known, but 32 (a
+    // whole block's thread per hypothesis) leaves too few blocks to balance.
+    // 64 pairs x 2000 hypotheses, search without the fit: 66 us at 16, 70 at
+    // 8, 80 at 4, 88 at 32.
     long long rounds_at = 0;
-    hpw = 32;
+    hpw = 4;
     for (int h : {32, 16, 8, 4}) {
-        if (tuning.search_hpw && h != tuning.search_hpw) continue;
+        if (tuning.search_hpw ? h != tuning.search_hpw : h == 32) continue;
         hpw = h;
         rounds_at = 0;
         for (int i = 0; i < n; ++i) rounds_at += s5k::plan_search(pairs[i].s5.hypotheses, h);
-        if (tuning.search_hpw || rounds_at >= 2 * kSmCount) break;
+        if (tuning.search_hpw || rounds_at >= 4 * kSmCount) break;
     }
     search_blocks = static_cast<int>(rounds_at);
     // block totals of every detect, describe and resize kind, for the block
@@ -698,18 +707,28 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
     const PairSrc pairsrc = with_map(PairSrc{reinterpret_cast<const PairIO*>(T + offsets[kPairJobs]),
                                              reinterpret_cast<const int*>(T + offsets[kPairPrefix]), n},
                                      kMapPair);
-    if (go(n)) s5k::prepare_kernel<PairSrc><<<n, 256, 0, s>>>(pairsrc);
+    if (go(n)) s5k::prepare_kernel<PairSrc><<<n, s5k::kPrepareThreads, 0, s>>>(pairsrc);
     mark();
     if (go(fit_blocks))
         s5k::fit_kernel<SearchSrc><<<fit_blocks, s5k::kFitThreads, 0, s>>>(
             with_map(SearchSrc{reinterpret_cast<const SearchJob*>(T + offsets[kSearchJobs]),
                                reinterpret_cast<const int*>(T + offsets[kFitPrefix]), n},
                      kMapFit));
-    if (go(search_blocks))
-        s5k::search_kernel<SearchSrc, true><<<search_blocks, s5k::kSearchThreads, search_smem, s>>>(
-            with_map(SearchSrc{reinterpret_cast<const SearchJob*>(T + offsets[kSearchJobs]),
-                               reinterpret_cast<const int*>(T + offsets[kSearchPrefix]), n},
-                     kMapSearch));
+    if (go(search_blocks)) {
+        const SearchSrc ss = with_map(SearchSrc{reinterpret_cast<const SearchJob*>(T + offsets[kSearchJobs]),
+                                                reinterpret_cast<const int*>(T + offsets[kSearchPrefix]), n},
+                                      kMapSearch);
+        const auto search = [&](auto group) {
+            s5k::search_kernel<SearchSrc, true, decltype(group)::value>
+                <<<search_blocks, s5k::kSearchThreads, search_smem, s>>>(ss);
+        };
+        switch (hpw) {
+            case 4: search(std::integral_constant<int, 32>{}); break;
+            case 8: search(std::integral_constant<int, 64>{}); break;
+            case 16: search(std::integral_constant<int, 128>{}); break;
+            default: search(std::integral_constant<int, 256>{});
+        }
+    }
     mark();
     if (go(n)) s5k::finish_kernel<PairSrc><<<n, s5k::kFinishThreads, finish_smem, s>>>(pairsrc);
     mark();

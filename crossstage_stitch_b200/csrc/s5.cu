@@ -86,8 +86,9 @@ int plan_search(int count, int hpw) {
     return std::min(kMaxSearchBlocks, ceil_div(rounds, kSearchWarps));
 }
 
-int search_smem_bytes(int match_capacity) {
-    return std::min(std::max(match_capacity, 1), kStagePoints) * static_cast<int>(sizeof(float4));
+int search_smem_bytes(int match_capacity, bool prefit) {
+    const int n = std::min(std::max(match_capacity, 1), prefit ? kStagePoints : kStagePointsFused);
+    return (n + (n & 1)) * static_cast<int>(sizeof(float4));  // staged two by two
 }
 
 bool enable_finish_smem_once(const void* fn) {
@@ -95,9 +96,9 @@ bool enable_finish_smem_once(const void* fn) {
            cudaSuccess;
 }
 
-bool enable_search_smem_once(const void* fn) {
+bool enable_search_smem_once(const void* fn, bool prefit) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kStagePoints * static_cast<int>(sizeof(float4))) == cudaSuccess;
+                                search_smem_bytes(INT_MAX, prefit)) == cudaSuccess;
 }
 
 }  // namespace stitch::b200::s5k
@@ -106,6 +107,19 @@ namespace stitch::s5 {
 
 using namespace ::stitch::b200;
 using namespace ::stitch::b200::s5k;
+
+namespace {
+
+template <int kGroup> void launch_search(const SearchJob& sj, int match_capacity, cudaStream_t stream) {
+    using Src = OneJob<SearchJob>;
+    static const bool smem_ok =
+        enable_search_smem_once(reinterpret_cast<const void*>(search_kernel<Src, false, kGroup>), false);
+    (void)smem_ok;
+    search_kernel<Src, false, kGroup>
+        <<<sj.io.search_blocks, kSearchThreads, search_smem_bytes(match_capacity, false), stream>>>(Src{sj});
+}
+
+}  // namespace
 
 Status s5_workspace_bytes(const Config& c, std::size_t* bytes) {
     if (!bytes || !valid_config(c)) return Status::INVALID_ARGUMENT;
@@ -120,21 +134,23 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
     const Status chk = check_and_build(a, b, matches, scale_a, scale_b, config, inlier_mask, output, workspace,
                                        workspace_bytes, &io);
     if (chk != Status::OK) return chk;
-    constexpr int kHpw = 8;
     const int count = config.hypotheses - config.previous_hypotheses;
-    io.hpw = kHpw;
-    io.search_blocks = plan_search(count, kHpw);
-    prepare_kernel<OneJob<PairIO>><<<1, 256, 0, stream>>>(OneJob<PairIO>{io});
+    // Hypotheses per block (8 * hpw) as few as keep the blocks, one per SM, in
+    // one wave: a block's fit (one thread per hypothesis) takes about as long
+    // for 8 models as for 64.
+    io.hpw = count <= 8 * kSmCount ? 1 : count <= 16 * kSmCount ? 2 : count <= 32 * kSmCount ? 4 : 8;
+    io.search_blocks = plan_search(count, io.hpw);
+    prepare_kernel<OneJob<PairIO>><<<1, kPrepareThreads, 0, stream>>>(OneJob<PairIO>{io});
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     if (io.search_blocks > 0) {
-        using Src = OneJob<SearchJob>;
-        static const bool smem_ok =
-            enable_search_smem_once(reinterpret_cast<const void*>(search_kernel<Src, false>));
-        (void)smem_ok;
-        SearchJob sj{io, config.previous_hypotheses, count, nullptr};
-        search_kernel<Src, false>
-            <<<io.search_blocks, kSearchThreads, search_smem_bytes(matches.capacity), stream>>>(Src{sj});
+        const SearchJob sj{io, config.previous_hypotheses, count, nullptr};
+        switch (io.hpw) {
+            case 1: launch_search<8>(sj, matches.capacity, stream); break;
+            case 2: launch_search<16>(sj, matches.capacity, stream); break;
+            case 4: launch_search<32>(sj, matches.capacity, stream); break;
+            default: launch_search<64>(sj, matches.capacity, stream);
+        }
         note_launches(1);
         if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     }

@@ -13,10 +13,12 @@ bool valid_config(const ::stitch::s5::Config& c);
 Status check_and_build(const Keypoints& a, const Keypoints& b, const Matches& m, const ScaleInfo& sa,
                        const ScaleInfo& sb, const ::stitch::s5::Config& c, std::uint8_t* mask,
                        const void* output, void* ws, std::size_t bytes, PairIO* io);
-// Search blocks for `count` hypotheses at `hpw` hypotheses per warp round.
+// Search blocks for `count` hypotheses at `hpw` hypotheses per warp, 8 warps a block.
 int plan_search(int count, int hpw);
-int search_smem_bytes(int match_capacity);
-bool enable_search_smem_once(const void* fn);
+// Dynamic shared memory of a search block, with or without the models fitted
+// beforehand.
+int search_smem_bytes(int match_capacity, bool prefit);
+bool enable_search_smem_once(const void* fn, bool prefit);
 bool enable_finish_smem_once(const void* fn);
 
 }  // namespace stitch::b200::s5k

@@ -16,12 +16,13 @@
 //   inlier mask r^2 <= tau^2, telemetry, H = D_A^-1 H_s D_B
 //                             src/s5/s5.cu:139-212
 //
-// Layout of the work: a warp owns HPW consecutive hypotheses; lanes
-// 0..HPW-1 each draw one sample and test it for degeneracy, then the whole
-// warp fits each usable sample (the 8x9 system in shared memory, entries split
-// over the lanes) and scores it. Lane l of the warp plays the reference's
-// virtual lanes l, l+32, l+64 and l+96, so both the per-lane sums and the
-// reduction tree are the reference's, operation for operation.
+// Layout of the work: a block of the search owns 8 * HPW consecutive
+// hypotheses. Their models (fitted one per thread, in this kernel or by
+// fit_kernel) are first bounded from below and above in FP32, all of them over
+// all matches; the few whose lower bound does not exceed the smallest loss
+// known to the pair are then scored exactly, by 128 threads that play the
+// reference's 128 virtual lanes, so that the per-lane sums and the reduction
+// tree are the reference's, operation for operation.
 #pragma once
 
 #include <cfloat>
@@ -62,10 +63,12 @@ struct State {
     std::uint64_t seed, generation;
     ScaleInfo scale_a, scale_b;
     int status;
-    // bits of the smallest loss of a fully scored model of this search (or
-    // of the previous winner), +inf when none: a pruning bound shared by
-    // every warp of the pair (nonnegative doubles order like their bits)
+    // bits of the smallest upper bound of a loss of this search (a model's
+    // FP32 upper bound, its exact loss, or the previous winner's), +inf when
+    // none: a pruning bound shared by every block of the pair (nonnegative
+    // doubles order like their bits)
     unsigned long long bound;
+    float coord_max[4];  // largest |ax|, |ay|, |bx|, |by| of the matches
 };
 
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;  // +inf
@@ -73,7 +76,11 @@ constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;  // +inf
 constexpr int kSearchThreads = 256;
 constexpr int kSearchWarps = kSearchThreads / 32;
 constexpr int kMaxSearchBlocks = 2 * kSmCount;
-constexpr int kStagePoints = 4096;  // matched points staged in shared memory per search block
+// matched points staged in shared memory per search block: the batched form
+// keeps several blocks per SM, the per-pair form has one or two
+constexpr int kStagePoints = 2048;
+constexpr int kStagePointsFused = 8192;
+constexpr int kPrepareThreads = 1024;
 constexpr int kFinishThreads = 256;
 
 // Inputs of one pair, as the caller passed them.
@@ -179,11 +186,15 @@ __device__ __forceinline__ std::uint64_t splitmix64(std::uint64_t v) {
 
 // Four distinct indices in [0, n): draw k = counter seed ^ (4h + k) mod
 // (n - k), stepped past the earlier draws in ascending order.
-__device__ __forceinline__ void sample_four(int n, std::uint64_t seed, int h, int* s) {
+__device__ __forceinline__ int sample_draw(int n, std::uint64_t seed, int h, int k) {
+    return static_cast<int>(splitmix64(seed ^ (static_cast<std::uint64_t>(h) * 4 + k)) %
+                            static_cast<std::uint64_t>(n - k));
+}
+
+__device__ __forceinline__ void distinct_draws(int* s) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        int v = static_cast<int>(splitmix64(seed ^ (static_cast<std::uint64_t>(h) * 4 + k)) %
-                                 static_cast<std::uint64_t>(n - k));
+    for (int k = 1; k < 4; ++k) {
+        int v = s[k];
         // earlier draws in ascending order
         int lo[3] = {s[0], s[1], s[2]};
         if (k >= 2 && lo[0] > lo[1]) { const int t = lo[0]; lo[0] = lo[1]; lo[1] = t; }
@@ -198,47 +209,73 @@ __device__ __forceinline__ void sample_four(int n, std::uint64_t seed, int h, in
     }
 }
 
-__device__ __forceinline__ double coord(const Pt& p, int image, int axis) {
-    return image ? (axis ? p.by : p.bx) : (axis ? p.ay : p.ax);
+// No three of the four points (xy of one image) nearly collinear.
+__device__ __forceinline__ bool nondegenerate(const double (&p)[4][2]) {
+    double scale = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < i; ++j) {
+            const double dx = p[i][0] - p[j][0], dy = p[i][1] - p[j][1];
+            const double d = dx * dx + dy * dy;
+            if (d > scale) scale = d;
+        }
+    bool ok = scale > 0.0 && fin(scale);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = i + 1; j < 4; ++j)
+#pragma unroll
+            for (int k = j + 1; k < 4; ++k) {
+                const double x1 = p[j][0] - p[i][0], y1 = p[j][1] - p[i][1];
+                const double x2 = p[k][0] - p[i][0], y2 = p[k][1] - p[i][1];
+                ok = ok && !(fabs(x1 * y2 - y1 * x2) <= 1e-8 * scale);
+            }
+    return ok;
 }
 
-// No three of the four points (in either image) nearly collinear.
-__device__ __forceinline__ bool nondegenerate(const Pt* p) {
+// Gauss-Jordan step of column C on the 8x9 system of fit4_regs: every index is
+// a compile-time constant, and the pivot row swap is a predicated select per
+// entry, so the system stays in registers.
+template <int C> __device__ __forceinline__ void eliminate(double (&m)[8][9], double max_entry, bool& solvable) {
+    constexpr auto idle = [](int r) { return C < 3 && r >= 3 && r < 6; };
+    int piv = C;
+    double best = fabs(m[C][C]), pv = m[C][C];
 #pragma unroll
-    for (int image = 0; image < 2; ++image) {
-        double scale = 0.0;
+    for (int r = C + 1; r < 8; ++r)
+        if (!idle(r) && fabs(m[r][C]) > best) { best = fabs(m[r][C]); piv = r; pv = m[r][C]; }
+    solvable = solvable && fin(pv) && !(fabs(pv) <= 1e-12 * max_entry);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+    for (int r = C + 1; r < 8; ++r)
 #pragma unroll
-            for (int j = 0; j < i; ++j) {
-                const double dx = coord(p[i], image, 0) - coord(p[j], image, 0);
-                const double dy = coord(p[i], image, 1) - coord(p[j], image, 1);
-                const double d = dx * dx + dy * dy;
-                if (d > scale) scale = d;
+        for (int jx = C; jx < 9; ++jx)
+            if (!idle(r)) {
+                const double a = m[C][jx], b = m[r][jx];
+                m[C][jx] = r == piv ? b : a;
+                m[r][jx] = r == piv ? a : b;
             }
-        if (!(scale > 0.0) || !fin(scale)) return false;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+    for (int jx = C + 1; jx < 9; ++jx) m[C][jx] /= pv;
 #pragma unroll
-            for (int j = i + 1; j < 4; ++j)
+    for (int r = 0; r < 8; ++r)
 #pragma unroll
-                for (int k = j + 1; k < 4; ++k) {
-                    const double x1 = coord(p[j], image, 0) - coord(p[i], image, 0);
-                    const double y1 = coord(p[j], image, 1) - coord(p[i], image, 1);
-                    const double x2 = coord(p[k], image, 0) - coord(p[i], image, 0);
-                    const double y2 = coord(p[k], image, 1) - coord(p[i], image, 1);
-                    if (fabs(x1 * y2 - y1 * x2) <= 1e-8 * scale) return false;
-                }
-    }
-    return true;
+        for (int jx = C + 1; jx < 9; ++jx)
+            if (r != C && !idle(r)) m[r][jx] -= m[r][C] * m[C][jx];
 }
 
 // Minimal 4-point model on one thread: the normalised normal equations of the
 // design rows {x, y, 1, 0, 0, 0, -u x, -u y, u} and {0, 0, 0, x, y, 1, -v x,
 // -v y, v}, Gauss-Jordan with partial pivoting, h33 = 1, denormalisation and
-// scaling. The 8x9 system stays in registers: every loop is unrolled and the
-// pivot row swap is a predicated select per entry, so no entry is indexed at
-// run time. Operations per entry are the reference's, in its order.
+// scaling, every value by the reference's operations in its order. Work whose
+// result is known beforehand is left out:
+// - products with a structural 0 add +-0 to a sum started at +0.0, the matrix
+//   is symmetric (products commute) and its (0..2) and (3..5) blocks are equal,
+//   so 27 sums and a count stand for the 72 entries;
+// - rows 3..5 hold +0.0 in columns 0..2: they are never the pivot there (a
+//   pivot of 0 is rejected) and subtracting 0 times a row changes nothing;
+// - the pivot column itself is not read again.
+// FP64 operations per model about 2700 -> 1450; fit_kernel of 64 pairs x 2000
+// hypotheses 63 -> 55 us, and 46 us at three blocks per SM (168 registers).
 __device__ __forceinline__ bool fit4_regs(const Pt* p, double* out) {
     double cax = 0, cay = 0, cbx = 0, cby = 0;
 #pragma unroll
@@ -253,65 +290,68 @@ __device__ __forceinline__ bool fit4_regs(const Pt* p, double* out) {
     if (!(va > 0.0) || !(vb > 0.0) || !fin(va) || !fin(vb)) return false;
     const double sa = sqrt(2.0 * 4 / va);
     const double sb = sqrt(2.0 * 4 / vb);
+    double xx = 0, xy = 0, x1 = 0, yy = 0, y1 = 0;    // x, y block
+    double xu[3] = {}, yu[3] = {}, ou[3] = {};        // x, y, 1 times -ux, -uy, u
+    double xv[3] = {}, yv[3] = {}, ov[3] = {};        // and -vx, -vy, v
+    double s66 = 0, s67 = 0, s68 = 0, s77 = 0, s78 = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double x = (p[i].bx - cbx) * sb, y = (p[i].by - cby) * sb;
+        const double u = (p[i].ax - cax) * sa, v = (p[i].ay - cay) * sa;
+        const double du[3] = {-u * x, -u * y, u}, dv[3] = {-v * x, -v * y, v};
+        xx += x * x; xy += x * y; x1 += x; yy += y * y; y1 += y;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            xu[c] += x * du[c]; yu[c] += y * du[c]; ou[c] += du[c];
+            xv[c] += x * dv[c]; yv[c] += y * dv[c]; ov[c] += dv[c];
+        }
+        s66 += du[0] * du[0] + dv[0] * dv[0];
+        s67 += du[0] * du[1] + dv[0] * dv[1];
+        s68 += du[0] * du[2] + dv[0] * dv[2];
+        s77 += du[1] * du[1] + dv[1] * dv[1];
+        s78 += du[1] * du[2] + dv[1] * dv[2];
+    }
     double m[8][9];
 #pragma unroll
     for (int r = 0; r < 8; ++r)
 #pragma unroll
         for (int c = 0; c < 9; ++c) m[r][c] = 0.0;
+    m[0][0] = m[3][3] = xx;
+    m[0][1] = m[1][0] = m[3][4] = m[4][3] = xy;
+    m[0][2] = m[2][0] = m[3][5] = m[5][3] = x1;
+    m[1][1] = m[4][4] = yy;
+    m[1][2] = m[2][1] = m[4][5] = m[5][4] = y1;
+    m[2][2] = m[5][5] = 4.0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const double x = (p[i].bx - cbx) * sb, y = (p[i].by - cby) * sb;
-        const double u = (p[i].ax - cax) * sa, v = (p[i].ay - cay) * sa;
-        const double r0[9] = {x, y, 1, 0, 0, 0, -u * x, -u * y, u};
-        const double r1[9] = {0, 0, 0, x, y, 1, -v * x, -v * y, v};
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int c = 0; c < 9; ++c) m[r][c] += r0[r] * r0[c] + r1[r] * r1[c];
+    for (int c = 0; c < 3; ++c) {
+        m[0][6 + c] = xu[c]; m[1][6 + c] = yu[c]; m[2][6 + c] = ou[c];
+        m[3][6 + c] = xv[c]; m[4][6 + c] = yv[c]; m[5][6 + c] = ov[c];
     }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        m[6 + c][0] = xu[c]; m[6 + c][1] = yu[c]; m[6 + c][2] = ou[c];
+        m[6 + c][3] = xv[c]; m[6 + c][4] = yv[c]; m[6 + c][5] = ov[c];
+    }
+    m[6][6] = s66;
+    m[6][7] = m[7][6] = s67;
+    m[6][8] = s68;
+    m[7][7] = s77;
+    m[7][8] = s78;
     double max_entry = 0.0;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         if (fabs(m[i][i]) > max_entry) max_entry = fabs(m[i][i]);
-    // A failed pivot makes the model invalid; the loop still runs to the
-    // end (an early exit would stop full unrolling) and the values computed
-    // after a failure are discarded.
+    // A failed pivot makes the model invalid; the steps after it still run
+    // and their values are discarded.
     bool solvable = true;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        int piv = c;
-        double best = fabs(m[c][c]);
-        double pv = m[c][c];
-#pragma unroll
-        for (int r = c + 1; r < 8; ++r)
-            if (fabs(m[r][c]) > best) { best = fabs(m[r][c]); piv = r; pv = m[r][c]; }
-        solvable = solvable && fin(pv) && !(fabs(pv) <= 1e-12 * max_entry);
-        // (loops run over all columns with a compile-time skip of jx < c, a
-        // form that keeps every entry in a register after unrolling)
-#pragma unroll
-        for (int r = c + 1; r < 8; ++r) {
-            const bool sw = r == piv;
-#pragma unroll
-            for (int jx = 0; jx < 9; ++jx) {
-                if (jx < c) continue;
-                const double a = m[c][jx], b = m[r][jx];
-                m[c][jx] = sw ? b : a;
-                m[r][jx] = sw ? a : b;
-            }
-        }
-        const double div = m[c][c];
-#pragma unroll
-        for (int jx = 0; jx < 9; ++jx)
-            if (jx >= c) m[c][jx] /= div;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            if (r == c) continue;
-            const double f = m[r][c];
-#pragma unroll
-            for (int jx = 0; jx < 9; ++jx)
-                if (jx >= c) m[r][jx] -= f * m[c][jx];
-        }
-    }
+    eliminate<0>(m, max_entry, solvable);
+    eliminate<1>(m, max_entry, solvable);
+    eliminate<2>(m, max_entry, solvable);
+    eliminate<3>(m, max_entry, solvable);
+    eliminate<4>(m, max_entry, solvable);
+    eliminate<5>(m, max_entry, solvable);
+    eliminate<6>(m, max_entry, solvable);
+    eliminate<7>(m, max_entry, solvable);
     if (!solvable) return false;
     double h[9];
 #pragma unroll
@@ -343,13 +383,162 @@ __device__ __forceinline__ Pt gather(const PairIO& j, int i) {
               static_cast<double>(j.b.y[ib])};
 }
 
-// Match i of the pair: from the staged float4 copy when it is staged.
-__device__ __forceinline__ Pt point_at(const PairIO& j, const float4* pts, int i) {
-    if (i < kStagePoints) {
-        const float4 q = pts[i];
-        return Pt{q.x, q.y, q.z, q.w};
+__device__ __forceinline__ double octet(double v, int src) { return __shfl_sync(0xffffffffu, v, src, 8); }
+
+// Hypothesis h by eight lanes (every lane of the warp calls, each eight with
+// their own h): the sample, the degeneracy test, the 4-point fit and the
+// domain test. The fit solves the normalised normal equations of the design
+// rows {x, y, 1, 0, 0, 0, -u x, -u y, u} and {0, 0, 0, x, y, 1, -v x, -v y, v}
+// by Gauss-Jordan with partial pivoting, h33 = 1, then denormalises and
+// scales, as fit4_regs does. Lane r owns row r of the 8x9 system; every entry goes through the
+// reference's operations in its order (products with a structural 0 only add
+// +-0 to a sum started at +0.0 and are left out). True, with the model on all
+// eight lanes, when the hypothesis is usable.
+//
+// For the per-pair call, whose hypotheses leave most of the chip idle: a
+// thread per hypothesis (fit4_regs) takes 18,000 cycles, most of them its 45
+// divisions, each a branchy sequence of about 125 cycles, one after the other;
+// here a pivot row's divisions run side by side. Per-pair search at 512x512,
+// 2000 hypotheses: 25 -> 15 us. It issues more instructions per hypothesis,
+// so the batched form, which fills the chip, keeps fit4_regs (64 pairs x 2000
+// hypotheses: 132 us with eight lanes).
+__device__ __forceinline__ bool fit_octet(const PairIO& j, int nm, int h, int bw, int bh, double* out) {
+    const int k8 = threadIdx.x & 7;
+    // the sample: lane k < 4 draws and gathers point k
+    int idx[4];
+    {
+        const int mine = sample_draw(nm, j.c.seed, h, k8 & 3);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) idx[k] = __shfl_sync(0xffffffffu, mine, k, 8);
+        distinct_draws(idx);
     }
-    return gather(j, i);
+    Pt p[4];
+    {
+        int i = idx[0];
+#pragma unroll
+        for (int k = 1; k < 4; ++k) i = (k8 & 3) == k ? idx[k] : i;
+        const int ia = j.m.idx_a[i], ib = j.m.idx_b[i];
+        const float ax = j.a.x[ia], ay = j.a.y[ia], bx = j.b.x[ib], by = j.b.y[ib];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            p[k] = Pt{__shfl_sync(0xffffffffu, ax, k, 8), __shfl_sync(0xffffffffu, ay, k, 8),
+                      __shfl_sync(0xffffffffu, bx, k, 8), __shfl_sync(0xffffffffu, by, k, 8)};
+    }
+    // image A on the even lanes, B on the odd ones: degeneracy, centroid, scale
+    double q[4][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        q[k][0] = k8 & 1 ? p[k].bx : p[k].ax;
+        q[k][1] = k8 & 1 ? p[k].by : p[k].ay;
+    }
+    bool ok = nondegenerate(q);
+    double cx = 0, cy = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { cx += q[k][0]; cy += q[k][1]; }
+    cx /= 4; cy /= 4;
+    double var = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) var += (q[k][0] - cx) * (q[k][0] - cx) + (q[k][1] - cy) * (q[k][1] - cy);
+    ok = ok && var > 0.0 && fin(var);
+    const double scale = sqrt(2.0 * 4 / var);
+    const double inv = 1.0 / scale;
+    const double cax = octet(cx, 0), cay = octet(cy, 0), sa = octet(scale, 0), isa = octet(inv, 0);
+    const double cbx = octet(cx, 1), cby = octet(cy, 1), sb = octet(scale, 1);
+    {
+        const unsigned int votes = __ballot_sync(0xffffffffu, ok) >> (threadIdx.x & 24);
+        ok = (votes & 3u) == 3u;
+    }
+    // row k8 of the normal equations
+    double m[9];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) m[c] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double x = (p[k].bx - cbx) * sb, y = (p[k].by - cby) * sb;
+        const double u = (p[k].ax - cax) * sa, v = (p[k].ay - cay) * sa;
+        const double ux = -u * x, uy = -u * y, vx = -v * x, vy = -v * y;
+        const double r0 = k8 == 0 ? x : k8 == 1 ? y : k8 == 2 ? 1.0 : k8 == 6 ? ux : k8 == 7 ? uy : 0.0;
+        const double r1 = k8 == 3 ? x : k8 == 4 ? y : k8 == 5 ? 1.0 : k8 == 6 ? vx : k8 == 7 ? vy : 0.0;
+        m[0] += r0 * x;
+        m[1] += r0 * y;
+        m[2] += r0;
+        m[3] += r1 * x;
+        m[4] += r1 * y;
+        m[5] += r1;
+        m[6] += r0 * ux + r1 * vx;
+        m[7] += r0 * uy + r1 * vy;
+        m[8] += r0 * u + r1 * v;
+    }
+    double max_entry = fabs(m[0]);
+#pragma unroll
+    for (int c = 1; c < 8; ++c) max_entry = k8 == c ? fabs(m[c]) : max_entry;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, max_entry, o);
+        if (v > max_entry) max_entry = v;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        // pivot: the first of the largest entries at or below the diagonal. (A
+        // NaN may be picked or passed over; its row stays NaN until it is the
+        // pivot row, so the system is rejected either way.)
+        double best = k8 >= c ? fabs(m[c]) : -1.0;
+        int piv = k8;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, best, o);
+            const int r = __shfl_xor_sync(0xffffffffu, piv, o);
+            if (v > best || (v == best && r < piv)) { best = v; piv = r; }
+        }
+        piv = max(__shfl_sync(0xffffffffu, piv, 0, 8), c);  // below c only when NaN entries alone are left
+        const double pv = octet(m[c], piv);
+        ok = ok && fin(pv) && !(fabs(pv) <= 1e-12 * max_entry);
+        // the pivot row divided by the pivot: column c + 1 + k on lane k
+        double num = 1.0;
+#pragma unroll
+        for (int jx = c + 1; jx < 9; ++jx) {
+            const double v = octet(m[jx], piv);
+            num = k8 == jx - c - 1 ? v : num;
+        }
+        const double quo = num / pv;
+        // row c moves to the pivot row's place
+        const double fc = octet(m[c], c);
+        const double f = k8 == piv ? fc : m[c];
+#pragma unroll
+        for (int jx = c + 1; jx < 9; ++jx) {
+            const double old = octet(m[jx], c);
+            const double v = octet(quo, jx - c - 1);
+            const double e = k8 == piv ? old : m[jx];
+            m[jx] = k8 == c ? v : e - f * v;
+        }
+    }
+    double n[9];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) n[i] = octet(m[8], i);
+    n[8] = 1.0;
+    const double den_a[9] = {isa, 0, cax, 0, isa, cay, 0, 0, 1};
+    const double nrm_b[9] = {sb, 0, -sb * cbx, 0, sb, -sb * cby, 0, 0, 1};
+    double tmp[9];
+    mat3_mul(den_a, n, tmp);
+    mat3_mul(tmp, nrm_b, n);
+    // scaled to the largest magnitude: entry k on lane k, entry 8 on every lane
+    double top = 0.0;
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        finite = finite && fin(n[i]);
+        if (fabs(n[i]) > top) top = fabs(n[i]);
+    }
+    double e = n[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) e = k8 == i ? n[i] : e;
+    e /= top;
+    out[8] = n[8] / top;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = octet(e, i);
+    const double det = out[0] * (out[4] * out[8] - out[5] * out[7]) - out[1] * (out[3] * out[8] - out[5] * out[6]) +
+                       out[2] * (out[3] * out[7] - out[4] * out[6]);
+    return ok && finite && top > 0.0 && fin(det) && fabs(det) > 1e-15 && valid_domain(out, bw, bh);
 }
 
 __device__ __forceinline__ bool same_scale(const ScaleInfo& a, const ScaleInfo& b) {
@@ -366,8 +555,9 @@ __device__ __forceinline__ bool same_scale(const ScaleInfo& a, const ScaleInfo& 
 // Restart or validate an extension, then check counts, indices and
 // coordinates of every match. One block per pair.
 template <class Src>
-__global__ __launch_bounds__(256) void prepare_kernel(const __grid_constant__ Src src) {
+__global__ __launch_bounds__(kPrepareThreads) void prepare_kernel(const __grid_constant__ Src src) {
     __shared__ int go, bad;
+    __shared__ unsigned int top[4];
     PairIO j;
     int local;
     if (!src.find(blockIdx.x, &j, &local)) return;
@@ -405,16 +595,29 @@ __global__ __launch_bounds__(256) void prepare_kernel(const __grid_constant__ Sr
         go = g;
         bad = 0;
     }
+    if (threadIdx.x < 4) top[threadIdx.x] = 0;
     __syncthreads();
     if (!go) return;
     const int na = s->na, nb = s->nb, nm = s->nm;
-    for (int i = threadIdx.x; i < nm; i += blockDim.x) {
+    unsigned int mx[4] = {0, 0, 0, 0};  // |x| of a float orders like its bits
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nm; i += kPrepareThreads) {
         const int ia = j.m.idx_a[i], ib = j.m.idx_b[i];
         if (ia < 0 || ia >= na || ib < 0 || ib >= nb) { bad = 1; continue; }
-        const Pt q = gather(j, i);
-        if (!fin(q.ax) || !fin(q.ay) || !fin(q.bx) || !fin(q.by)) bad = 1;
+        const float q[4] = {j.a.x[ia], j.a.y[ia], j.b.x[ib], j.b.y[ib]};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (!fin(q[c])) bad = 1;
+            mx[c] = max(mx[c], __float_as_uint(fabsf(q[c])));
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const unsigned int w = __reduce_max_sync(0xffffffffu, mx[c]);
+        if ((threadIdx.x & 31) == 0) atomicMax(&top[c], w);
     }
     __syncthreads();
+    if (threadIdx.x < 4) s->coord_max[threadIdx.x] = __uint_as_float(top[threadIdx.x]);
     if (threadIdx.x == 0) {
         if (bad) s->status = static_cast<int>(Status::INVALID_ARGUMENT);
         else if (nm < 4) s->status = static_cast<int>(Status::NOT_ENOUGH_POINTS);
@@ -432,12 +635,12 @@ struct SearchJob {
 constexpr int kFitThreads = 128;
 
 // One thread per hypothesis h in [first, first + count): the counter-based
-// sample, the degeneracy test, the 4-point fit and the domain test, the same
-// functions the search runs in place, into prefit[h - first] (valid = 0 for
-// a rejected sample). A thread owns the whole 8x9 system, so this kernel
-// runs with all the registers it needs, apart from the scoring.
+// sample, the degeneracy test, the 4-point fit and the domain test into
+// prefit[h - first] (valid = 0 for a rejected sample). A thread owns the
+// whole 8x9 system, so this kernel runs with all the registers it needs,
+// apart from the scoring.
 template <class Src>
-__global__ __launch_bounds__(kFitThreads) void fit_kernel(const __grid_constant__ Src src) {
+__global__ __launch_bounds__(kFitThreads, 3) void fit_kernel(const __grid_constant__ Src src) {
     SearchJob sj;
     int block;
     if (!src.find(blockIdx.x, &sj, &block)) return;
@@ -449,178 +652,351 @@ __global__ __launch_bounds__(kFitThreads) void fit_kernel(const __grid_constant_
     m.hypothesis = h;
     m.valid = 0;
     if (s->status == static_cast<int>(Status::OK)) {
-        const int nm = s->nm;
-        int idx[4] = {0, 0, 0, 0};
-        sample_four(nm, j.c.seed, h, idx);
-        Pt f[4];
+        int idx[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) f[k] = gather(j, idx[k]);
-        m.valid = nondegenerate(f) && fit4_regs(f, m.h) && valid_domain(m.h, s->scale_b.work_w, s->scale_b.work_h);
+        for (int k = 0; k < 4; ++k) idx[k] = sample_draw(s->nm, j.c.seed, h, k);
+        distinct_draws(idx);
+        Pt f[4];
+        double qa[4][2], qb[4][2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            f[k] = gather(j, idx[k]);
+            qa[k][0] = f[k].ax; qa[k][1] = f[k].ay;
+            qb[k][0] = f[k].bx; qb[k][1] = f[k].by;
+        }
+        m.valid = nondegenerate(qa) && nondegenerate(qb) && fit4_regs(f, m.h) &&
+                  valid_domain(m.h, s->scale_b.work_w, s->scale_b.work_h);
     }
     sj.prefit[h - sj.first] = m;
 }
 
-// Block b of a pair walks warp rounds b*8 + w, b*8 + w + 8*blocks, ...; a
-// round is HPW consecutive hypotheses. The block's best model goes to
-// block_best[b].
-// Three blocks per SM: the register-resident 4-point fit then spills to
-// L1-backed local memory, but it is a small share of the work, and the
-// scoring loop gains the occupancy (1 block: 0.62 ms, 3 blocks: 0.43 ms for
-// 64 pairs x 2000 hypotheses x ~530 matches).
-constexpr int kPruneEvery = 128;  // points between the pruning checks of a model (multiple of 128)
+// FP32 bounds of a model's loss L = sum of min(r^2, tau^2), r = |H b - a|.
+// With u = 2^-24, the coordinate bounds Ax, Ay, Bx, By of the pair and the
+// FP32 evaluation of X, Y, Z (two FMAs on rounded entries each), 1/Z (one
+// approximate reciprocal, relative error 2u) and d = X (1/Z) - ax (one FMA):
+//   |Z' - Z| <= EZ = 4u (|h6| Bx + |h7| By + |h8|) + 2e-15, likewise EX, EY,
+//   e = |r' - r| <= c0 + c1 |1/Z'|, W = 4 tau + Ax + Ay,
+//   c0 = 2.2u W + 4u tau,  c1 = 1.5 (W EZ + EX + EY),
+// for points with both |d'| <= 2 tau and c0 + c1 |1/Z'| <= tau / 2. There
+// min(r, tau)^2 changes by at most 2 tau e. Where c0 + c1 |1/Z'| > tau / 2 the
+// bound used is 2 tau * tau / 2, which no change of min(r, tau)^2 exceeds; and
+// with it <= tau / 2, |d'| > 2 tau implies that both r and r' exceed tau, so
+// the term is tau^2 either way. (The 2e-15 covers |Z| < 1e-15, which the exact
+// residual calls unreachable: then c1 |1/Z'| > tau / 2.) So
+//   |L - L'| <= 2 tau (c0 n + c1 sum min(|1/Z'|, cap)) + 6u tau^2 n,
+//   cap = (tau / 2 - c0) / c1,
+// with 6u tau^2 for the rounding of each squared term, plus the FP32
+// summation's relative error. Used only where no FP32 operation can overflow.
+struct Bounds {
+    double c0, c1;
+    float cap;
+};
 
-// kPrefit: the models come from fit_kernel (sj.prefit) and the kernel only
-// scores (batched form: 0.387 -> 0.367 ms per step with the fit kernel
-// included; 4 and 5 blocks per SM spill in the scoring loop and are slower).
-template <class Src, bool kPrefit>
-__global__ __launch_bounds__(kSearchThreads, 3) void search_kernel(const __grid_constant__ Src src) {
-    extern __shared__ float4 pts[];
-    __shared__ Model warp_best[kSearchWarps];
+__device__ __forceinline__ bool bounds_apply(const State* s, int nm, double tau) {
+    const float* c = s->coord_max;
+    return tau >= 1e-6 && tau <= 1e6 && nm <= (1 << 20) && fmaxf(fmaxf(c[0], c[1]), fmaxf(c[2], c[3])) <= 1048576.0f;
+}
+
+__device__ __forceinline__ Bounds model_bounds(const double* h, const State* s, double tau) {
+    constexpr double u = 1.0 / 16777216.0;
+    const double w = 4.0 * tau + s->coord_max[0] + s->coord_max[1];
+    const double bx = s->coord_max[2], by = s->coord_max[3];
+    const double ex = 4.0 * u * (fabs(h[0]) * bx + fabs(h[1]) * by + fabs(h[2])) + 1e-30;
+    const double ey = 4.0 * u * (fabs(h[3]) * bx + fabs(h[4]) * by + fabs(h[5])) + 1e-30;
+    const double ez = 4.0 * u * (fabs(h[6]) * bx + fabs(h[7]) * by + fabs(h[8])) + 2e-15;
+    Bounds b;
+    b.c0 = 1.05 * (2.2 * u * w + 4.0 * u * tau);
+    b.c1 = 1.05 * 1.5 * (w * ez + ex + ey);
+    const double cap = (0.5 * tau - b.c0) / b.c1;
+    b.cap = cap > 0.0 ? static_cast<float>(fmin(cap, 1e30)) : 0.0f;
+    return b;
+}
+
+__device__ __forceinline__ float approx_rcp(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Two FP32 operations per instruction (each rounded as the scalar one).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void f2_split(F2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+
+// Matches in shared memory, two by two: {bx0, bx1, by0, by1, -ax0, -ax1, -ay0,
+// -ay1}, the operands of the packed FP32 bounds.
+__device__ __forceinline__ void put_match(float* pts, int i, float ax, float ay, float bx, float by) {
+    float* q = pts + 8 * (i >> 1) + (i & 1);
+    q[0] = bx;
+    q[2] = by;
+    q[4] = -ax;
+    q[6] = -ay;
+}
+
+__device__ __forceinline__ Pt get_match(const float* pts, int i) {
+    const float* q = pts + 8 * (i >> 1) + (i & 1);
+    return Pt{-q[4], -q[6], q[0], q[2]};
+}
+
+// Block b of a pair takes the groups b, b + blocks, ... of kGroup consecutive
+// hypotheses; its best model goes to block_best[b].
+// Why bounds first: with about 90 % inliers nearly every model used to be
+// scored in FP64 over a fifth to all of the matches before it could be
+// dropped, two FP64 divisions per match (36 issue slots each). The FP32 bounds
+// take 10 instructions per match (two matches per FMA), read a match once for
+// 32 models (a broadcast), and are within about 0.1 % of the loss, so that only the models
+// that close to the best are left for FP64: usually one per block.
+// Of 64 pairs x 2000 models 155 are scored in FP64 at 512x512; the batched
+// search without the fit went 188 -> 64 us, the per-pair search 52 -> 15 us
+// (2000 hypotheses, 310 matches) and 331 -> 95 us (8000, 8000).
+// Layout: 256 / kGroup threads share a model, each over every (256 / kGroup)th
+// pair of matches. kPrefit: the models come from fit_kernel (batched form);
+// else the block fits them here (per-pair form, whose workspace has no room
+// for them).
+template <class Src, bool kPrefit, int kGroup>
+__global__ __launch_bounds__(kSearchThreads, kPrefit ? 4 : 2) void search_kernel(const __grid_constant__ Src src) {
+    constexpr int kSlices = kSearchThreads / kGroup;
+    constexpr int kStage = kPrefit ? kStagePoints : kStagePointsFused;
+    extern __shared__ float4 pts4[];
+    float* const pts = reinterpret_cast<float*>(pts4);
+    __shared__ double mh[kGroup][9], low[kGroup];  // models and the lower bounds of their losses
+    __shared__ float part[kSlices][2][kGroup], caps[kGroup];
+    __shared__ double red[2][128];
+    __shared__ Model best;
+    __shared__ int chosen[2];
     SearchJob sj;
     int block;
     if (!src.find(blockIdx.x, &sj, &block)) return;
     const PairIO& j = sj.io;
-    const State* s = j.state;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // the warp's best model so far lives in shared memory, written by lane 0
-    // (registers stay with the scoring loop)
-    Model& best = warp_best[warp];
-    if (lane == 0) best.valid = 0;
-    __syncwarp();
+    State* s = j.state;
+    const int t = threadIdx.x, lane = t & 31;
+    if (t == 0) best.valid = 0;
     const bool ok = s->status == static_cast<int>(Status::OK);
     const int nm = ok ? s->nm : 0;
-    const int staged = min(nm, kStagePoints);
-    for (int i = threadIdx.x; i < staged; i += kSearchThreads) {
-        const int ia = j.m.idx_a[i], ib = j.m.idx_b[i];
-        pts[i] = make_float4(j.a.x[ia], j.a.y[ia], j.b.x[ib], j.b.y[ib]);
-    }
-    __syncthreads();
-    if (ok) {
-        const double thr2 = j.c.threshold * j.c.threshold;
-        const int bw = s->scale_b.work_w, bh = s->scale_b.work_h;
-        const std::uint64_t seed = j.c.seed;
-        const int hpw = j.hpw;
-        const int rounds = (sj.count + hpw - 1) / hpw;
-        const int stride = j.search_blocks * kSearchWarps;
-        for (int round = block * kSearchWarps + warp; round < rounds; round += stride) {
-            const int h0 = sj.first + round * hpw;
-            const int hend = min(sj.first + sj.count, h0 + hpw);
-            // lanes 0..hpw-1 build one model each (system in registers)
-            double hm[9];
-            int valid = 0;
-            if (kPrefit) {
-                valid = lane < hend - h0 ? sj.prefit[h0 + lane - sj.first].valid : 0;
-            } else if (lane < hend - h0) {
-                int idx[4] = {0, 0, 0, 0};
-                sample_four(nm, seed, h0 + lane, idx);
-                Pt f[4];
+    const double tau = j.c.threshold, thr2 = tau * tau;
+    const bool bounded = ok && bounds_apply(s, nm, tau);
+    const auto stage = [&](int base) {
+        const int n = min(kStage, nm - base);
+#pragma unroll 4
+        for (int i = t; i < n; i += kSearchThreads) {
+            const int ia = j.m.idx_a[base + i], ib = j.m.idx_b[base + i];
+            put_match(pts, i, j.a.x[ia], j.a.y[ia], j.b.x[ib], j.b.y[ib]);
+        }
+    };
+    if (ok) stage(0);
+    const int groups = ok ? (sj.count + kGroup - 1) / kGroup : 0;
+    for (int group = block; group < groups; group += j.search_blocks) {
+        const int h0 = sj.first + group * kGroup;
+        // 1. models
+        int valid = 0;
+        if (kPrefit) {
+            if (t < kGroup && h0 + t < sj.first + sj.count) {
+                const Model& m = sj.prefit[h0 + t - sj.first];
+                valid = m.valid;
+                if (valid)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (idx[k] < kStagePoints) {
-                        const float4 q = pts[idx[k]];
-                        f[k] = Pt{q.x, q.y, q.z, q.w};
-                    } else {
-                        f[k] = gather(j, idx[k]);
-                    }
-                }
-                valid = nondegenerate(f) && fit4_regs(f, hm) && valid_domain(hm, bw, bh);
+                    for (int e = 0; e < 9; ++e) mh[t][e] = m.h[e];
             }
-            // then the whole warp scores the valid models one by one
-            for (int k = 0; k < hend - h0; ++k) {
-                if (!__shfl_sync(0xffffffffu, valid, k)) continue;
+        } else {
+            for (int g = t >> 3; g - (lane >> 3) < kGroup; g += kSearchThreads / 8) {  // warp-uniform
+                const int hyp = min(h0 + g, sj.first + sj.count - 1);
                 double h[9];
-                if (kPrefit) {
-                    const Model& mk = sj.prefit[h0 + k - sj.first];  // the same address on every lane
+                const bool fit = fit_octet(j, nm, hyp, s->scale_b.work_w, s->scale_b.work_h, h);
+                if (g < kGroup) {
+                    if ((t & 7) == 0) {
 #pragma unroll
-                    for (int e = 0; e < 9; ++e) h[e] = mk.h[e];
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 9; ++e) h[e] = __shfl_sync(0xffffffffu, hm[e], k);
-                }
-                // Exact pruning against the smallest loss of a fully scored
-                // model so far (this warp's best, or the pair's bound that
-                // every warp publishes to): every term is >= 0 and a
-                // correctly rounded sum of nonnegative values is nondecreasing
-                // in each operand, so the tree sum of the partial accumulators
-                // never exceeds the final loss. Once it is above that loss the
-                // model cannot win (ties need equal losses).
-                const double shared_bound =
-                    __longlong_as_double(static_cast<long long>(*reinterpret_cast<volatile unsigned long long*>(&j.state->bound)));
-                const double bound = best.valid && best.loss < shared_bound ? best.loss : shared_bound;
-                const bool prune = bound <= DBL_MAX;
-                // Lane l accumulates the points l, l+32, l+64, l+96 (virtual
-                // lanes, slots 0..3) and every 128 after them in order: four
-                // points per step, four independent FP64 chains. A point past
-                // nm adds +0.0, which leaves a sum of nonnegative terms
-                // (started at +0.0) bit for bit unchanged.
-                double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-                bool lost = false;
-                for (int base = 0; base < nm; base += 128) {  // warp-uniform trip count
-                    const int i0 = base + lane, i1 = i0 + 32, i2 = i0 + 64, i3 = i0 + 96;
-                    if (base + 128 <= nm) {  // every slot of the step holds a point
-                        const Pt p0 = point_at(j, pts, i0), p1 = point_at(j, pts, i1);
-                        const Pt p2 = point_at(j, pts, i2), p3 = point_at(j, pts, i3);
-                        const double r0 = residual2(h, p0), r1 = residual2(h, p1);
-                        const double r2 = residual2(h, p2), r3 = residual2(h, p3);
-                        acc0 += r0 < thr2 ? r0 : thr2;
-                        acc1 += r1 < thr2 ? r1 : thr2;
-                        acc2 += r2 < thr2 ? r2 : thr2;
-                        acc3 += r3 < thr2 ? r3 : thr2;
-                    } else {
-                        // the last, partial step: a virtual lane past nm adds
-                        // +0.0, a no-op on a sum of nonnegative terms, so the
-                        // chains with no point left (warp-uniform) are skipped
-                        const double r0 = residual2(h, point_at(j, pts, min(i0, nm - 1)));
-                        acc0 += i0 < nm ? (r0 < thr2 ? r0 : thr2) : 0.0;
-                        if (base + 32 < nm) {
-                            const double r1 = residual2(h, point_at(j, pts, min(i1, nm - 1)));
-                            acc1 += i1 < nm ? (r1 < thr2 ? r1 : thr2) : 0.0;
-                        }
-                        if (base + 64 < nm) {
-                            const double r2 = residual2(h, point_at(j, pts, min(i2, nm - 1)));
-                            acc2 += i2 < nm ? (r2 < thr2 ? r2 : thr2) : 0.0;
-                        }
-                        if (base + 96 < nm) {
-                            const double r3 = residual2(h, point_at(j, pts, min(i3, nm - 1)));
-                            acc3 += i3 < nm ? (r3 < thr2 ? r3 : thr2) : 0.0;
-                        }
-                    }
-                    if (prune && (base & (kPruneEvery - 1)) == kPruneEvery - 128 && base + 128 < nm) {
-                        double part = (acc0 + acc2) + (acc1 + acc3);
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-                        if (__shfl_sync(0xffffffffu, part > bound ? 1 : 0, 0)) {
-                            lost = true;
-                            break;
-                        }
+                        for (int e = 0; e < 9; ++e) mh[g][e] = h[e];
+                        low[g] = fit && h0 + g < sj.first + sj.count ? 1.0 : 0.0;
                     }
                 }
-                if (lost) continue;
-                // virtual lanes l, l+32, l+64, l+96: strides 64 and 32 of the tree
-                double v = (acc0 + acc2) + (acc1 + acc3);
+            }
+            __syncthreads();
+            if (t < kGroup) valid = low[t] != 0.0;
+        }
+        Bounds bd{};
+        if (t < kGroup) {
+            if (valid) {
+                double h[9];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                if (lane == 0) {
+                for (int e = 0; e < 9; ++e) h[e] = mh[t][e];
+                bd = model_bounds(h, s, tau);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 9; ++e) mh[t][e] = 0.0;
+            }
+            caps[t] = bd.cap;
+        }
+        __syncthreads();
+        // 2. FP32 bounds
+        double lo = 0.0;
+        if (bounded) {
+            const int m = t % kGroup, slice = t / kGroup;
+            float h[9];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) h[e] = static_cast<float>(mh[m][e]);
+            const float cap = caps[m], top = static_cast<float>(thr2);
+            F2 hh[9];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) hh[e] = f2(h[e], h[e]);
+            F2 sums = f2(0.0f, 0.0f), invs = sums;
+            float sum = 0.0f, inv = 0.0f;
+            for (int base = 0; base < nm; base += kStage) {
+                if (nm > kStage) {
+                    __syncthreads();
+                    stage(base);
+                    __syncthreads();
+                }
+                const int n = min(kStage, nm - base);
+                const ulonglong2* const two = reinterpret_cast<const ulonglong2*>(pts);
+#pragma unroll 4
+                for (int i = slice; i < n / 2; i += kSlices) {
+                    const ulonglong2 b = two[2 * i], a = two[2 * i + 1];
+                    const F2 z = f2_fma(hh[6], b.x, f2_fma(hh[7], b.y, hh[8]));
+                    const F2 x = f2_fma(hh[0], b.x, f2_fma(hh[1], b.y, hh[2]));
+                    const F2 y = f2_fma(hh[3], b.x, f2_fma(hh[4], b.y, hh[5]));
+                    float z0, z1;
+                    f2_split(z, z0, z1);
+                    const float r0 = approx_rcp(z0), r1 = approx_rcp(z1);
+                    const F2 r = f2(r0, r1);
+                    const F2 dx = f2_fma(x, r, a.x), dy = f2_fma(y, r, a.y);
+                    float d0, d1;
+                    f2_split(f2_fma(dx, dx, f2_mul(dy, dy)), d0, d1);
+                    // a NaN counts as top, within its error
+                    sums = f2_add(sums, f2(fminf(d0, top), fminf(d1, top)));
+                    invs = f2_add(invs, f2(fminf(fabsf(r0), cap), fminf(fabsf(r1), cap)));
+                }
+                if ((n & 1) && slice == 0) {
+                    const Pt q = get_match(pts, n - 1);
+                    const float bx = static_cast<float>(q.bx), by = static_cast<float>(q.by);
+                    const float r = approx_rcp(__fmaf_rn(h[6], bx, __fmaf_rn(h[7], by, h[8])));
+                    const float dx = __fmaf_rn(__fmaf_rn(h[0], bx, __fmaf_rn(h[1], by, h[2])), r, -static_cast<float>(q.ax));
+                    const float dy = __fmaf_rn(__fmaf_rn(h[3], bx, __fmaf_rn(h[4], by, h[5])), r, -static_cast<float>(q.ay));
+                    sum += fminf(__fmaf_rn(dx, dx, dy * dy), top);
+                    inv += fminf(fabsf(r), cap);
+                }
+            }
+            {
+                float lo0, hi0;
+                f2_split(sums, lo0, hi0);
+                sum += lo0 + hi0;
+                f2_split(invs, lo0, hi0);
+                inv += lo0 + hi0;
+            }
+            part[slice][0][m] = sum;
+            part[slice][1][m] = inv;
+            __syncthreads();
+            if (t < kGroup) {
+                double total = 0.0, reach = 0.0;
+#pragma unroll
+                for (int v = 0; v < kSlices; ++v) {
+                    total += part[v][0][t];
+                    reach += part[v][1][t];
+                }
+                const double rel = 1.2e-7 * (nm / kSlices + 16);  // FP32 summation of nonnegative terms
+                const double err = 1.01 * (2.0 * tau * (bd.c0 * nm + bd.c1 * reach * (1.0 + rel)) + 3.6e-7 * thr2 * nm);
+                lo = total * (1.0 - rel) - err;
+                double hi = valid ? total * (1.0 + rel) + err : DBL_MAX;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    if (kGroup < 32 && o >= kGroup) continue;
+                    const double v = __shfl_xor_sync(kGroup < 32 ? (1u << kGroup) - 1u : 0xffffffffu, hi, o);
+                    hi = v < hi ? v : hi;
+                }
+                if ((t & 31) == 0 && hi < DBL_MAX)
+                    atomicMin(&s->bound, static_cast<unsigned long long>(__double_as_longlong(hi)));
+            }
+        }
+        if (t < kGroup) low[t] = valid ? lo : __longlong_as_double(static_cast<long long>(kInfBits));
+        __syncthreads();
+        // 3. exact losses of the models that may still win, the two lowest
+        // bounds at a time. A model whose lower bound exceeds another valid
+        // model's loss or upper bound loses to it (ties need equal losses).
+        for (;;) {
+            if (t < 32) {
+                const double bound = __longlong_as_double(
+                    static_cast<long long>(*reinterpret_cast<volatile unsigned long long*>(&s->bound)));
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    double v = DBL_MAX;
+                    int at = -1;
+                    for (int m = lane; m < kGroup; m += 32)
+                        if (low[m] <= bound && low[m] < v) { v = low[m]; at = m; }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const double w = __shfl_xor_sync(0xffffffffu, v, o);
+                        const int x = __shfl_xor_sync(0xffffffffu, at, o);
+                        if (x >= 0 && (at < 0 || w < v || (w == v && x < at))) { v = w; at = x; }
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        chosen[half] = at;
+                        if (at >= 0) low[at] = __longlong_as_double(static_cast<long long>(kInfBits));
+                    }
+                    __syncwarp();
+                }
+            }
+            __syncthreads();
+            if (chosen[0] < 0) break;
+            const int half = t >> 7, v = t & 127, m = chosen[half];
+            if (m >= 0) {
+                double h[9];
+#pragma unroll
+                for (int e = 0; e < 9; ++e) h[e] = mh[m][e];
+                double acc = 0.0;
+#pragma unroll 2
+                for (int i = v; i < nm; i += 128) {
+                    const double r = residual2(h, nm <= kStage ? get_match(pts, i) : gather(j, i));
+                    acc += r < thr2 ? r : thr2;
+                }
+                red[half][v] = acc;
+            }
+            __syncthreads();
+            if (v < 32 && m >= 0) {  // strides 64 and 32 of the tree, then 16 ... 1
+                double a = (red[half][v] + red[half][v + 64]) + (red[half][v + 32] + red[half][v + 96]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+                if (v == 0) red[half][0] = a;
+            }
+            __syncthreads();
+            if (t == 0) {
+                for (int k = 0; k < 2 && chosen[k] >= 0; ++k) {
                     Model cand;
-#pragma unroll
-                    for (int e = 0; e < 9; ++e) cand.h[e] = h[e];
-                    cand.loss = v;
-                    cand.hypothesis = h0 + k;
-                    cand.valid = fin(v);
-                    if (better(cand, best)) best = cand;
-                    if (cand.valid) atomicMin(&j.state->bound, static_cast<unsigned long long>(__double_as_longlong(v)));
+                    cand.loss = red[k][0];
+                    cand.hypothesis = h0 + chosen[k];
+                    cand.valid = fin(cand.loss);
+                    if (!better(cand, best)) continue;
+                    for (int e = 0; e < 9; ++e) best.h[e] = mh[chosen[k]][e];
+                    best.loss = cand.loss;
+                    best.hypothesis = cand.hypothesis;
+                    best.valid = 1;
+                    atomicMin(&s->bound, static_cast<unsigned long long>(__double_as_longlong(cand.loss)));
                 }
-                __syncwarp();
             }
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        Model b = warp_best[0];
-        for (int w = 1; w < kSearchWarps; ++w)
-            if (better(warp_best[w], b)) b = warp_best[w];
-        j.block_best[block] = b;
-    }
+    if (t == 0) j.block_best[block] = best;
 }
 
 // ---------------------------------------------------------------- finish

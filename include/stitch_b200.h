@@ -325,9 +325,10 @@ int stitch_batch_create(int n_pairs, const stitch_pair_desc* pairs, stitch_batch
  * persistent FAST grid, 1..7 (default 7); blur_ctas_per_sm: the same for the
  * on-demand blur, 1..6 (default 6); matcher: 1 + an S4 matcher kind (0..4,
  * as for stitch_s4_set_matcher), or 0 for the creating thread's choice;
- * search_hpw: MSAC hypotheses per warp round, 4, 8, 16 or 32 (default: the
- * largest that still fills about two waves); resize_tile_h: pyramid rows per
- * resize block, 16, 32 or 64 (default 64). */
+ * search_hpw: MSAC hypotheses per warp (a block has 8 warps), 4, 8, 16 or 32
+ * (default: the largest up to 16 that still fills a wave of four blocks per
+ * SM); resize_tile_h: pyramid rows per resize block, 16, 32 or 64 (default
+ * 64). */
 typedef struct stitch_batch_tuning {
     int fast_ctas_per_sm;
     int blur_ctas_per_sm;

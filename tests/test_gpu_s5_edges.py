@@ -31,3 +31,16 @@ def check(n, frac, R, refine, seed, tau=3.0, scale=1.0):
 @pytest.mark.parametrize("n", [15, 16, 17, 112, 113, 447, 449, 465, 897, 8192, 8193, 8300])
 def test_match_counts(cuda, n):
     check(n, 0.0 if n < 20 else 0.3, 64, 2, seed=n)
+
+
+@pytest.mark.parametrize("R", [1, 7, 9, 1184, 1185, 2369, 4737, 9600])
+def test_hypothesis_counts(cuda, R):
+    """8, 16, 32 and 64 hypotheses per block, partial groups, several groups per block."""
+    check(97, 0.4, R, 1, seed=R)
+
+
+@pytest.mark.parametrize("tau,scale", [(1e-7, 1.0), (0.05, 1.0), (2e6, 1.0), (3.0, 3000.0), (500.0, 1e-3), (1e-3, 1e-6)])
+def test_bounds_range(cuda, tau, scale):
+    """Thresholds and coordinates inside and outside the range of the FP32
+    bounds, and thresholds that every or no match meets."""
+    check(301, 0.3, 700, 1, seed=77, tau=tau, scale=scale)
