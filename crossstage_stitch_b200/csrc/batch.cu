@@ -199,6 +199,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     }
     // 4. launch shapes (block counts are final once stage_tables has run)
     int max_cand = 0, max_cap_m = 1;
+    long long keypoints = 0;
     for (int i = 0; i < n; ++i) {
         const auto& q = pairs[i];
         for (int s = 0; s < 2; ++s) {
@@ -214,9 +215,11 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
             }
         }
         max_cap_m = std::max(max_cap_m, q.s2.max_keypoints);
+        keypoints += 2ll * q.s2.max_keypoints;
     }
     sort_smem = s2s3::sort_smem_bytes(max_cand);
     rank_fallback = max_cand > s2s3::kSortCap;
+    desc_keys = s2s3::desc_keys(keypoints);
     search_smem = s5k::search_smem_bytes(max_cap_m, true);
     finish_smem = s5k::finish_smem_bytes(max_cap_m);
     // S4: one train partition per block unless the batch is too small to fill the GPU
@@ -267,6 +270,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
                 }
             }
         }
+    rank = s2s3::rank_pays(det_total[s2s3::kHarrisKind], det_total[s2s3::kSortKind], max_cand);
     std::size_t map_entries = 0;
     for (int kind = 0; kind < s2s3::kDetectKinds; ++kind) {
         det_first[kind] = map_entries;
@@ -373,7 +377,7 @@ void Plan::job_blocks(int i, int s, int l, int (&db)[s2s3::kDetectKinds], int (&
     const auto& o = off[i];
     if (o.pyramid[s]) {
         s2s3::pyramid_detect_blocks(o.pyr[s], l, db);
-        s2s3::pyramid_describe_blocks(o.pyr[s], l, sb);
+        s2s3::pyramid_describe_blocks(o.pyr[s], l, desc_keys, sb);
         return;
     }
     const stitch_image_view& im = s ? q.image_b : q.image_a;
@@ -384,7 +388,7 @@ void Plan::job_blocks(int i, int s, int l, int (&db)[s2s3::kDetectKinds], int (&
     db[s2s3::kHarrisKind] = active ? ceil_div(o.det[s].candidates, s2s3::kHarrisThreads) : 0;
     db[s2s3::kSortKind] = active ? 1 : 0;
     sb[s2s3::kBlurKind] = 0;  // on demand: blur_tiles_kernel takes the flagged tiles from a list
-    sb[s2s3::kDescKind] = k > 0 ? ceil_div(k, s2s3::kDescKeys) : 0;
+    sb[s2s3::kDescKind] = k > 0 ? ceil_div(k, desc_keys) : 0;
 }
 
 Status Plan::stage_tables(void* ws) {
@@ -648,26 +652,31 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
     mark();
     if (go(det_blocks[s2s3::kSelectKind])) {
         s2s3::select_kernel<DetSrc><<<det_blocks[s2s3::kSelectKind], 256, 0, s>>>(det);
-        s2s3::ties_kernel<DetSrc><<<det_blocks[s2s3::kSortKind], s2s3::kTieThreads, 0, s>>>(det);
-        ++launches;
     }
     mark();
     if (go(det_blocks[s2s3::kHarrisKind]))
         s2s3::harris_kernel<DetSrc><<<det_blocks[s2s3::kHarrisKind], s2s3::kHarrisThreads, 0, s>>>(det);
     mark();
-    if (go(det_blocks[s2s3::kSortKind]))
-        s2s3::sort_topk_kernel<DetSrc><<<det_blocks[s2s3::kSortKind], s2s3::kSortThreads, sort_smem, s>>>(det);
-    if (rank_fallback && go(det_blocks[s2s3::kHarrisKind]))
-        s2s3::rank_topk_kernel<DetSrc><<<det_blocks[s2s3::kHarrisKind], s2s3::kHarrisThreads, 0, s>>>(det);
+    if (rank) {
+        if (go(det_blocks[s2s3::kHarrisKind]))
+            s2s3::rank_topk_kernel<DetSrc>
+                <<<det_blocks[s2s3::kHarrisKind] * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, 0);
+    } else {
+        if (go(det_blocks[s2s3::kSortKind]))
+            s2s3::sort_topk_kernel<DetSrc><<<det_blocks[s2s3::kSortKind], s2s3::kSortThreads, sort_smem, s>>>(det);
+        if (rank_fallback && go(det_blocks[s2s3::kHarrisKind]))
+            s2s3::rank_topk_kernel<DetSrc>
+                <<<det_blocks[s2s3::kHarrisKind] * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, s2s3::kSortCap);
+    }
     mark();
     if (go(tiles > 0 && blur_total > 0 ? 1 : 0))
-        s2s3::blur_tiles_kernel<DesSrc>
+        s2s3::blur_tiles_kernel<DesSrc, true>
             <<<static_cast<int>(std::min<std::size_t>(
                    blur_total, kSmCount * (tuning.blur_ctas_per_sm ? tuning.blur_ctas_per_sm : s2s3::kBlurCtasPerSm))),
-               256, 0, s>>>(des, at<uint2>(ws, blur_list), q + 1);
+               256, 0, s>>>(des, at<uint2>(ws, blur_list), q + 1, 0);
     mark();
     if (go(des_blocks[s2s3::kDescKind]))
-        s2s3::describe_kernel<DesSrc><<<des_blocks[s2s3::kDescKind], s2s3::kDescWarps * 32, 0, s>>>(des);
+        s2s3::describe_kernel<DesSrc><<<des_blocks[s2s3::kDescKind], s2s3::kDescWarps * 32, 0, s>>>(des, desc_keys);
     mark();
 
     // S4/S5 job tables, with their block maps when the plan has them

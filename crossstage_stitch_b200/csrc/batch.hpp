@@ -55,7 +55,9 @@ public:
     int knn_blocks = 0, merge_blocks = 0, n_knn = 0;
     int search_blocks = 0, fit_blocks = 0;
     int sort_smem = 0, search_smem = 0, finish_smem = 0;
-    bool rank_fallback = false;
+    bool rank_fallback = false;  // a job has more candidates than the sort takes
+    bool rank = false;           // every job's candidates are ranked, not sorted
+    int desc_keys = 0;           // keypoints per describe block
     int hpw = 8;
     // binary matcher of this plan's S4 launches (s4k::kMatcherPopc or
     // kMatcherTensor): the building thread's choice, or stitch_batch_set_matcher's

@@ -157,10 +157,10 @@ void pyramid_detect_blocks(const PyramidLayout& l, int i, int (&blocks)[kDetectK
     blocks[kSortKind] = active ? 1 : 0;
 }
 
-void pyramid_describe_blocks(const PyramidLayout& l, int i, int (&blocks)[kDescribeKinds]) {
+void pyramid_describe_blocks(const PyramidLayout& l, int i, int keys, int (&blocks)[kDescribeKinds]) {
     const bool active = i < l.plan.levels && l.plan.budget[i] > 0;
     blocks[kBlurKind] = 0;  // on demand: blur_tiles_kernel takes the flagged tiles from a list
-    blocks[kDescKind] = active ? ceil_div(l.plan.budget[i], kDescKeys) : 0;
+    blocks[kDescKind] = active ? ceil_div(l.plan.budget[i], keys) : 0;
 }
 
 namespace {
@@ -228,35 +228,34 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
     DesSrc des{};
     det.n = des.n = n;
     int max_cand = 0;
+    const int keys = desc_keys(c.max_keypoints);
     for (int i = 0; i < n; ++i) {
         det.jobs[i] = jobs.detect[i];
         des.jobs[i] = jobs.describe[i];
         int db[kDetectKinds], sb[kDescribeKinds];
         pyramid_detect_blocks(l, i, db);
-        pyramid_describe_blocks(l, i, sb);
+        pyramid_describe_blocks(l, i, keys, sb);
         for (int k = 0; k < kDetectKinds; ++k) det.first[k][i + 1] = det.first[k][i] + db[k];
         for (int k = 0; k < kDescribeKinds; ++k) des.first[k][i + 1] = des.first[k][i] + sb[k];
-        if (db[kSortKind]) max_cand = max_cand > l.det[i].candidates ? max_cand : l.det[i].candidates;
+        if (db[kSortKind]) max_cand = std::max(max_cand, l.det[i].candidates);
     }
     auto blocks = [&](int kind) { return det.first[kind][n]; };
     if (blocks(kFastKind)) {
         fast_kernel<DetSrc><<<std::min(blocks(kFastKind), kSmCount * kFastCtasPerSm), kFastThreads, 0, stream>>>(
             det, queue, blocks(kFastKind));
         select_kernel<DetSrc><<<blocks(kSelectKind), 256, 0, stream>>>(det);
-        ties_kernel<DetSrc><<<blocks(kSortKind), kTieThreads, 0, stream>>>(det);
         harris_kernel<DetSrc><<<blocks(kHarrisKind), kHarrisThreads, 0, stream>>>(det);
-        sort_topk_kernel<DetSrc><<<blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream>>>(det);
-        launches += 5;
-        if (max_cand > kSortCap) {
-            rank_topk_kernel<DetSrc><<<blocks(kHarrisKind), kHarrisThreads, 0, stream>>>(det);
-            ++launches;
-        }
-        blur_tiles_kernel<DesSrc><<<std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), 256, 0, stream>>>(
-            des, at_offset<uint2>(ws, l.blur_list), queue + 1);
+        if (max_cand > kSortCap || rank_pays(blocks(kHarrisKind), blocks(kSortKind), max_cand))
+            rank_topk_kernel<DetSrc><<<blocks(kHarrisKind) * kRankPer, kRankThreads, 0, stream>>>(det, 0);
+        else
+            sort_topk_kernel<DetSrc><<<blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream>>>(det);
+        launches += 4;
+        blur_tiles_kernel<DesSrc, true><<<std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), 256, 0, stream>>>(
+            des, at_offset<uint2>(ws, l.blur_list), queue + 1, 0);
         ++launches;
     }
     if (des.first[kDescKind][n]) {
-        describe_kernel<DesSrc><<<des.first[kDescKind][n], kDescWarps * 32, 0, stream>>>(des);
+        describe_kernel<DesSrc><<<des.first[kDescKind][n], kDescWarps * 32, 0, stream>>>(des, keys);
         ++launches;
     }
     note_launches(launches);

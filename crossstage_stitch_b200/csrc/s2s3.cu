@@ -46,6 +46,8 @@ bool detect_layout(int w, int h, int k, DetectLayout* out) {
     l.params = lay.take(1, sizeof(SelectParams));
     l.keys = lay.take(static_cast<std::size_t>(l.candidates), sizeof(std::uint64_t));
     l.maxima = lay.take(std::max<std::size_t>(cells, 1), sizeof(std::uint64_t));
+    l.max_ties = static_cast<int>(std::min<std::size_t>(cells, kTieCap));
+    l.ties = lay.take(static_cast<std::size_t>(std::max(l.max_ties, 1)), sizeof(std::uint32_t));
     if (!lay.ok) return false;
     l.total = lay.cursor;
     *out = l;
@@ -78,6 +80,8 @@ DetectJob make_detect_job(const ImageView& im, const s2::Config& c, const Keypoi
     j.harris_k = c.harris_k;
     j.maxima = at_offset<std::uint64_t>(ws, l.maxima);
     j.max_maxima = l.max_maxima;
+    j.ties = at_offset<std::uint32_t>(ws, l.ties);
+    j.max_ties = l.max_ties;
     j.hist = at_offset<std::uint32_t>(ws, l.hist);
     j.params = at_offset<SelectParams>(ws, l.params);
     j.keys = at_offset<std::uint64_t>(ws, l.keys);
@@ -148,15 +152,15 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
     fast_kernel<Src><<<fast_grid, kFastThreads, 0, stream>>>(src, src.job.counters() + kTileQueue, l.tiles);
     if (!record(e_fast, stream)) return Status::CUDA_ERROR;
     select_kernel<Src><<<l.select_blocks, 256, 0, stream>>>(src);
-    ties_kernel<Src><<<1, kTieThreads, 0, stream>>>(src);
     if (!record(e_select, stream)) return Status::CUDA_ERROR;
     const int harris_blocks = ceil_div(l.candidates, kHarrisThreads);
     harris_kernel<Src><<<harris_blocks, kHarrisThreads, 0, stream>>>(src);
     if (!record(e_harris, stream)) return Status::CUDA_ERROR;
-    sort_topk_kernel<Src><<<1, kSortThreads, sort_smem_bytes(l.candidates), stream>>>(src);
-    if (l.candidates > kSortCap)
-        rank_topk_kernel<Src><<<harris_blocks, kHarrisThreads, 0, stream>>>(src);
-    note_launches(l.candidates > kSortCap ? 7 : 6);
+    if (l.candidates > kSortCap || rank_pays(harris_blocks, 1, l.candidates))
+        rank_topk_kernel<Src><<<harris_blocks * kRankPer, kRankThreads, 0, stream>>>(src, 0);
+    else
+        sort_topk_kernel<Src><<<1, kSortThreads, sort_smem_bytes(l.candidates), stream>>>(src);
+    note_launches(4);
     return launch_status();
 }
 
@@ -174,9 +178,10 @@ Status describe(const ImageView& image, const Keypoints& kp, const Descriptors& 
     if (kp.capacity == 0) return record(e_blur, stream) ? Status::OK : Status::CUDA_ERROR;
     using Src = OneJob<DescribeJob>;
     const Src src{make_describe_job(image, kp, out, ws, l)};
-    blur_kernel<Src><<<l.tiles, 256, 0, stream>>>(src);
+    blur_tiles_kernel<Src, false><<<std::min(l.tiles, kSmCount * kBlurCtasPerSm), 256, 0, stream>>>(src, nullptr, nullptr, l.tiles);
     if (!record(e_blur, stream)) return Status::CUDA_ERROR;
-    describe_kernel<Src><<<ceil_div(kp.capacity, kDescKeys), kDescWarps * 32, 0, stream>>>(src);
+    const int keys = desc_keys(kp.capacity);
+    describe_kernel<Src><<<ceil_div(kp.capacity, keys), kDescWarps * 32, 0, stream>>>(src, keys);
     note_launches(2);
     return launch_status();
 }

@@ -10,8 +10,8 @@ namespace stitch::b200::s2s3 {
 // histogram bins and then the kDetectCounters counters, zeroed together
 // (hist_bytes) before each run.
 struct DetectLayout {
-    std::size_t maxima, hist, params, keys, total;
-    int max_maxima, candidates, tiles_x, tiles, select_blocks;
+    std::size_t maxima, hist, params, keys, ties, total;
+    int max_maxima, max_ties, candidates, tiles_x, tiles, select_blocks;
     static constexpr std::size_t hist_bytes = kHistWords * sizeof(std::uint32_t);
 };
 
@@ -32,6 +32,18 @@ DetectJob make_detect_job(const ImageView& im, const s2::Config& c, const Keypoi
                           const DetectLayout& l);
 DescribeJob make_describe_job(const ImageView& im, const Keypoints& kp, const Descriptors& out, void* ws,
                               const DescribeLayout& l);
+// Whether rank_topk_kernel orders a launch's jobs faster than
+// sort_topk_kernel. Measured, a rank block costs about 9.5 ns (a block has
+// some microseconds of latency, 592 run at once), and so does a key of the
+// largest job, padded to a power of two, per wave of sort blocks (one per job,
+// two per SM). K = 2000 at 8 layers: 4 pairs 20 us either way, 8 pairs 31
+// ranked, 21 sorted, 64 pairs 170 and 62; single level: 8 pairs 25 and 49;
+// K = 8000 at 8 layers, 2 pairs: 29 and 49.
+inline bool rank_pays(long long harris_blocks, int jobs, int max_candidates) {
+    long long keys = 1024;
+    while (keys < max_candidates) keys *= 2;
+    return harris_blocks * kRankPer <= keys * ceil_div(jobs, 2 * kSmCount);
+}
 // Dynamic shared memory of sort_topk_kernel for `candidates` keys.
 int sort_smem_bytes(int candidates);
 
@@ -100,7 +112,8 @@ void make_pyramid_jobs(const ImageView& im, const s2::Config& c, const Keypoints
 
 // Block count of each detect/describe kind for layer i (0 when inactive).
 void pyramid_detect_blocks(const PyramidLayout& l, int layer, int (&blocks)[kDetectKinds]);
-void pyramid_describe_blocks(const PyramidLayout& l, int layer, int (&blocks)[kDescribeKinds]);
+// `keys`: keypoints per describe block (desc_keys).
+void pyramid_describe_blocks(const PyramidLayout& l, int layer, int keys, int (&blocks)[kDescribeKinds]);
 
 Status pyramid_workspace_bytes(int w, int h, const s2::Config& c, int levels, float scale_factor,
                                std::size_t* bytes);

@@ -31,7 +31,12 @@ struct SelectParams {
 };
 
 // Per-job counters of the detect kernels, after the 256 histogram bins.
-enum DetectCounter { kListed = 0, kAboveWritten = 1, kTiesWritten = 2, kTileQueue = 3, kDetectCounters = 4 };
+enum DetectCounter {
+    kListed, kAboveWritten, kTiesWritten, kTileQueue,
+    kTiesListed,   // maxima at the threshold listed in `ties`
+    kSelectDone,   // select blocks that have finished
+    kDetectCounters
+};
 constexpr int kHistWords = 256 + kDetectCounters;  // one job's histogram and counters
 
 struct alignas(16) DetectJob {  // 16-byte multiple: copied into shared memory in 16-byte chunks
@@ -46,6 +51,8 @@ struct alignas(16) DetectJob {  // 16-byte multiple: copied into shared memory i
                                    // all zeroed before the FAST launch
     SelectParams* params;
     std::uint64_t* keys;           // [candidates]
+    std::uint32_t* ties;           // raster indices of the maxima at the selection threshold
+    int max_ties;                  // capacity of `ties`
     // output
     float* x;
     float* y;
@@ -189,19 +196,34 @@ constexpr int kSelectPx = 65536;   // image pixels per select block (a job's max
                                    // by ceil(W * H / kSelectPx) blocks)
 constexpr int kFastThreads = 256;
 constexpr int kFastCtasPerSm = 7;  // resident FAST blocks per SM (shared memory); the persistent grid is 148 x this
-constexpr int kTieThreads = 1024;
+constexpr int kTieCap = 16384;      // tie list entries; more ties are picked from the maxima list itself
+constexpr int kTieRank = 1024;      // ties ranked against each other in shared memory
 // Largest offset of a rotated rBRIEF sample from its keypoint: the pattern's
 // coordinates lie within a radius of 18.39 px (|x|, |y| <= 13), so a rotated
 // coordinate rounds to at most 18.
 constexpr int kSampleRadius = 18;
-constexpr int kHarrisThreads = 256;
+constexpr int kHarrisThreads = 128;  // candidates of a harris (and rank) block: small blocks spread one image's few
+                                     // thousand candidates over the chip
+constexpr int kRankKeys = 32;        // keys a rank block ranks: small blocks, so that one image's largest layer
+                                     // spreads over the chip
+constexpr int kRankThreads = 512;
+constexpr int kRankPer = kHarrisThreads / kRankKeys;  // rank blocks per harris block
+constexpr int kRankTile = 1024;      // keys staged at a time
 constexpr int kSortCap = 16384;    // candidates sorted in shared memory by one block
 constexpr int kSortThreads = 1024;
 constexpr int kSortChunk = 64;      // keys a warp sorts in registers (2 per lane)
 constexpr int kBlurTileW = 64, kBlurTileH = 64;
 constexpr int kDescWarps = 8;
-constexpr int kDescRounds = 4;                        // keypoints per warp of a describe block
-constexpr int kDescKeys = kDescWarps * kDescRounds;  // keypoints per describe block
+// Keypoints per warp of a describe block: one while all blocks are resident
+// at once (a warp's rounds run one after the other, 2.5 us each), more when
+// there are more keypoints than that, so that a block's tables are shared.
+// 512x512, K = 1000: 20 us at 4, 14 us at 1; 4K, K = 8000: 24 and 18 us.
+constexpr int kDescMaxRounds = 4;
+constexpr int kDescResident = 148 * 8;  // describe blocks on the chip
+__host__ __device__ inline int desc_keys(long long keypoints) {
+    const long long one = kDescWarps * static_cast<long long>(kDescResident);
+    return kDescWarps * (keypoints <= one ? 1 : keypoints <= 2 * one ? 2 : kDescMaxRounds);
+}
 constexpr int kEdge = 31;
 constexpr int kResizeTileW = 128, kResizeTileH = 64;  // tallest tile; a job's tile_h may be smaller
 constexpr int kMaxLevels = 16;
@@ -297,15 +319,38 @@ __device__ __forceinline__ float2 byte_pair(std::uint32_t wa, std::uint32_t wb, 
     return __fadd2_rn(biased, make_float2(-8388608.0f, -8388608.0f));
 }
 
-// A blur tap in both lanes of a packed pair. The sm_100 packed FP32 add and
-// multiply round each lane exactly as __fadd_rn / __fmul_rn do, so two rows
-// (or two columns) of the blur run in one instruction stream.
+// A blur tap in both lanes of a packed pair: two rows (or two columns) of the
+// blur in one instruction stream.
 __device__ __forceinline__ float2 tap_pair(int t) { return make_float2(blur_tap(t), blur_tap(t)); }
 
-// Rounds a blur sum half-to-even after clamping to [0, 255] (clamping the
-// float first gives the same byte for every finite sum).
-__device__ __forceinline__ std::uint32_t blur_byte(float acc) {
-    return static_cast<std::uint32_t>(__float2int_rn(fminf(fmaxf(acc, 0.0f), 255.0f)));
+// Tap t of a pair of sums. Packed: the sm_100 packed FP32 multiply and add,
+// which ptxas may join into one fused operation per lane. Scalar: every
+// product and sum rounded on its own, as the reference does.
+template <bool kPacked> __device__ __forceinline__ float2 first_tap(float2 v) {
+    return kPacked ? __fmul2_rn(tap_pair(0), v)
+                   : make_float2(__fmul_rn(blur_tap(0), v.x), __fmul_rn(blur_tap(0), v.y));
+}
+template <bool kPacked> __device__ __forceinline__ float2 next_tap(float2 sum, int t, float2 v) {
+    return kPacked ? __fadd2_rn(sum, __fmul2_rn(tap_pair(t), v))
+                   : make_float2(__fadd_rn(sum.x, __fmul_rn(blur_tap(t), v.x)),
+                                 __fadd_rn(sum.y, __fmul_rn(blur_tap(t), v.y)));
+}
+
+// Rounds two blur sums half-to-even to integers, in the low mantissa bits:
+// adding 1.5 * 2^23 rounds a float below 2^22 to an integer the way
+// __float2int_rn does, on the FP32 pipe (the conversion instruction runs at a
+// sixteenth of its rate). No clamp: the taps are positive and rounding is
+// monotone, so a sum lies between 0 and that of an all-255 window, which is
+// below 255.5 (tests/test_gpu_detect_edges.py checks that window).
+__device__ __forceinline__ float2 round_pair(float2 v) {
+    return __fadd2_rn(v, make_float2(12582912.0f, 12582912.0f));
+}
+
+// Low bytes of four rounded sums (round_pair), first in the low byte.
+__device__ __forceinline__ std::uint32_t pack_bytes(float2 a, float2 b) {
+    const std::uint32_t lo = __byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040);
+    const std::uint32_t hi = __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
 }
 
 // Asynchronous 16-byte copy, global to shared memory (both 16-byte aligned).
@@ -629,18 +674,101 @@ __device__ __forceinline__ SelectParams select_params(const std::uint32_t* hist,
     return *out;
 }
 
+// The first `p.ties` maxima at the threshold score in raster order, when they
+// cannot all be kept (the reference's raster-order scatter of the first ties,
+// src/s2_s3/s2.cu:182-235), by the 256 threads of one block, into keys[above,
+// selected). The listed ties are walked, or the maxima list when the ties
+// outgrew their list (then an entry counts only with the threshold's score).
+// A few ties are ranked against each other; more go through a
+// most-significant-digit radix select of the p.ties-th smallest raster index.
+__device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams& p, std::uint32_t listed) {
+    __shared__ __align__(16) std::uint32_t buf[kTieRank];  // staged ties, or the 256 radix bins
+    __shared__ std::uint32_t pick[2];        // digit, maxima before it
+    std::uint32_t* ctr = j.counters();
+    const std::uint32_t T = p.threshold, total = j.hist[T];
+    const int t = threadIdx.x;
+    if (total <= kTieRank && total <= static_cast<std::uint32_t>(j.max_ties)) {
+        const int n = static_cast<int>(total), padded = (n + 3) / 4 * 4;
+        for (int i = t; i < padded; i += 256) buf[i] = i < n ? __ldcg(j.ties + i) : 0xffffffffu;
+        __syncthreads();
+        for (int i = t; i < n; i += 256) {
+            const std::uint32_t px = buf[i];
+            std::uint32_t rank = 0;
+            for (int k = 0; k < padded; k += 4) {
+                const uint4 q = *reinterpret_cast<const uint4*>(buf + k);
+                rank += (q.x < px) + (q.y < px) + (q.z < px) + (q.w < px);
+            }
+            if (rank < p.ties) j.keys[p.above + rank] = px;
+        }
+        return;
+    }
+    const bool own = total <= static_cast<std::uint32_t>(j.max_ties);
+    const std::uint32_t n = own ? total : listed;
+    const auto entry = [&](std::uint32_t i, std::uint32_t& px) {  // whether entry i is a tie
+        if (own) {
+            px = __ldcg(j.ties + i);
+            return true;
+        }
+        const std::uint64_t e = j.maxima[i];
+        px = static_cast<std::uint32_t>(e);
+        return static_cast<std::uint32_t>(e >> 32) == T;
+    };
+    std::uint32_t prefix = 0, need = p.ties;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+        const std::uint32_t high = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+        buf[t] = 0;
+        __syncthreads();
+#pragma unroll 4
+        for (std::uint32_t i = t; i < n; i += 256) {
+            std::uint32_t px;
+            if (entry(i, px) && (px & high) == prefix) atomicAdd(&buf[(px >> shift) & 255u], 1u);
+        }
+        __syncthreads();
+        if (t == 0) {
+            std::uint32_t run = 0, d = 0;
+            while (d < 255 && run + buf[d] < need) run += buf[d++];
+            pick[0] = d;
+            pick[1] = run;
+        }
+        __syncthreads();
+        prefix |= pick[0] << shift;
+        need -= pick[1];
+        __syncthreads();
+    }
+    const int lane = t & 31;
+    const unsigned below = (1u << lane) - 1u;
+    for (std::uint32_t i0 = 0; i0 < n; i0 += 256) {  // block-uniform
+        const std::uint32_t i = i0 + t;
+        std::uint32_t px = 0;
+        const bool keep = i < n && entry(i, px) && px <= prefix;
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        std::uint32_t b = 0;
+        if (lane == 0 && m) b = atomicAdd(&ctr[kTiesWritten], static_cast<std::uint32_t>(__popc(m)));
+        b = __shfl_sync(0xffffffffu, b, 0) + __popc(m & below);
+        if (keep && b < p.ties) j.keys[p.above + b] = px;
+    }
+}
+
 // Pre-selection over a job's maxima list: every block of the job derives the
 // same threshold from the histogram; block 0 publishes the parameters and
 // the keypoint count min(selected, K). The maxima above the threshold go to
 // keys[0, above), and when every maximum at the threshold is kept (selected
 // below the cap, or the cap falls exactly on a score boundary) those go to
-// keys[above, selected); otherwise the tie kernel picks them. The order
-// inside each range is not the raster order: the keys are sorted later by
-// (response, raster index), which no order of equal sets changes.
+// keys[above, selected); otherwise they are listed, and the job's last block
+// to finish picks the first of them in raster order. The order inside each
+// range is not the raster order: the keys are sorted later by (response,
+// raster index), which no order of equal sets changes.
+//
+// Latency-bound. The ties used to be picked by a kernel of one block per job
+// that walked the whole maxima list five times (512x512, 8 layers: 15 us; 4K:
+// 60 us); the list of the ties alone is some hundred entries, and picking
+// them in the last block saves a launch. Select and ties together, 512x512:
+// 18.5 -> 7 us, 4K: 67 -> 23 us.
 template <class Src>
 __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src src) {
     __shared__ std::uint32_t suffix[257];
     __shared__ SelectParams sp;
+    __shared__ bool last;
     DetectJob j;
     int local;
     if (!src.find(blockIdx.x, kSelectKind, &j, &local)) return;
@@ -654,6 +782,8 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
     const std::uint32_t n = min(ctr[kListed], static_cast<std::uint32_t>(j.max_maxima));
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
+    // ties go behind the keys above the threshold, or to their list
+    std::uint32_t* const tie_count = &ctr[all_ties ? kTiesWritten : kTiesListed];
     const std::uint32_t stride = static_cast<std::uint32_t>(j.select_blocks) * 256u;
     for (std::uint32_t i0 = static_cast<std::uint32_t>(local) * 256u; i0 < n; i0 += stride) {  // block-uniform
         const std::uint32_t i = i0 + threadIdx.x;
@@ -664,79 +794,29 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
             const auto score = static_cast<std::uint32_t>(e >> 32);
             px = static_cast<std::uint32_t>(e);
             above = score > p.threshold;
-            tie = all_ties && score == p.threshold;
+            tie = score == p.threshold;
         }
         const unsigned ma = __ballot_sync(0xffffffffu, above), mt = __ballot_sync(0xffffffffu, tie);
         std::uint32_t ba = 0, bt = 0;
         if (lane == 0) {
             if (ma) ba = atomicAdd(&ctr[kAboveWritten], static_cast<std::uint32_t>(__popc(ma)));
-            if (mt) bt = atomicAdd(&ctr[kTiesWritten], static_cast<std::uint32_t>(__popc(mt)));
+            if (mt) bt = atomicAdd(tie_count, static_cast<std::uint32_t>(__popc(mt)));
         }
         ba = __shfl_sync(0xffffffffu, ba, 0) + __popc(ma & below);
         bt = __shfl_sync(0xffffffffu, bt, 0) + __popc(mt & below);
         if (above && ba < p.above) j.keys[ba] = px;  // always true when list and histogram agree
-        if (tie && bt < p.ties) j.keys[p.above + bt] = px;
+        if (tie && all_ties && bt < p.ties) j.keys[p.above + bt] = px;
+        if (tie && !all_ties && bt < static_cast<std::uint32_t>(j.max_ties)) j.ties[bt] = px;
     }
-}
-
-// The first `ties` maxima at the threshold score in raster order, when the
-// select kernel could not take every tie: a most-significant-digit radix
-// select over their raster indices (unique) finds the ties-th smallest, P,
-// and every tie at or below P goes to keys[above, selected). One block per
-// job; the reference's equivalent is the raster-order scatter of the first
-// ties (src/s2_s3/s2.cu:182-235).
-template <class Src>
-__global__ __launch_bounds__(kTieThreads) void ties_kernel(const __grid_constant__ Src src) {
-    __shared__ std::uint32_t bins[256];
-    __shared__ std::uint32_t pick[2];  // digit, maxima before it
-    DetectJob j;
-    int local;
-    if (!src.find(blockIdx.x, kSortKind, &j, &local)) return;
-    const SelectParams p = *j.params;
-    if (p.selected == 0 || p.ties == j.hist[p.threshold]) return;  // nothing to pick, or all written
-    std::uint32_t* ctr = j.counters();
-    const std::uint32_t n = min(ctr[kListed], static_cast<std::uint32_t>(j.max_maxima));
-    const std::uint32_t T = p.threshold;
-    std::uint32_t prefix = 0, need = p.ties;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        const std::uint32_t high = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
-        for (int b = threadIdx.x; b < 256; b += kTieThreads) bins[b] = 0;
-        __syncthreads();
-        for (std::uint32_t i = threadIdx.x; i < n; i += kTieThreads) {
-            const std::uint64_t e = j.maxima[i];
-            const auto px = static_cast<std::uint32_t>(e);
-            if (static_cast<std::uint32_t>(e >> 32) == T && (px & high) == prefix)
-                atomicAdd(&bins[(px >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            std::uint32_t run = 0, d = 0;
-            while (d < 255 && run + bins[d] < need) run += bins[d++];
-            pick[0] = d;
-            pick[1] = run;
-        }
-        __syncthreads();
-        prefix |= pick[0] << shift;
-        need -= pick[1];
-        __syncthreads();
-    }
-    const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    for (std::uint32_t i0 = 0; i0 < n; i0 += kTieThreads) {  // block-uniform
-        const std::uint32_t i = i0 + threadIdx.x;
-        bool keep = false;
-        std::uint32_t px = 0;
-        if (i < n) {
-            const std::uint64_t e = j.maxima[i];
-            px = static_cast<std::uint32_t>(e);
-            keep = static_cast<std::uint32_t>(e >> 32) == T && px <= prefix;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        std::uint32_t b = 0;
-        if (lane == 0 && m) b = atomicAdd(&ctr[kTiesWritten], static_cast<std::uint32_t>(__popc(m)));
-        b = __shfl_sync(0xffffffffu, b, 0) + __popc(m & below);
-        if (keep && b < p.ties) j.keys[p.above + b] = px;
-    }
+    if (all_ties || p.selected == 0) return;
+    __threadfence();  // this block's list entries, before it counts as done
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd(&ctr[kSelectDone], 1u) == static_cast<std::uint32_t>(j.select_blocks) - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    pick_ties(j, p, n);
 }
 
 // ------------------------------------------------------------- Harris
@@ -755,27 +835,57 @@ constexpr float kHarrisScale4 = 0x1.bb9da2p-52f;
 
 // Harris response over the 7x7 window of 3x3 Sobel gradients centred on
 // (x, y): integer sums, then det - k * trace^2 in float32 with every product
-// and sum rounded separately.
-__device__ __forceinline__ float harris_response(const std::uint8_t* img, int pitch, int x, int y, float k) {
-    int p[9][9];
-    const std::uint8_t* base = img + static_cast<std::size_t>(y - 4) * pitch + (x - 4);
+// and sum rounded separately. The gradients are separable: ix is the
+// horizontal difference of the columns' 1-2-1 sums, iy the vertical
+// difference of the rows' 1-2-1 sums. With 4-byte aligned rows (words) a
+// row's nine bytes come from three word loads, else from nine byte loads: the
+// lanes of a warp look at scattered patches, so the loads are what the kernel
+// takes its time for (64 pairs at 512x512: 37 -> 20 us; one image: 9 -> 6 us).
+__device__ __forceinline__ float harris_response(const std::uint8_t* img, int pitch, int x, int y, float k, bool words) {
+    const int x0 = x - 4, off = words ? x0 & 3 : 0;
+    const std::uint8_t* base = img + static_cast<std::size_t>(y - 4) * pitch + (x0 - off);
+    std::uint32_t raw[9][3];  // bytes 0..8 of each row
+    if (words) {
 #pragma unroll
-    for (int r = 0; r < 9; ++r)
+        for (int r = 0; r < 9; ++r)
 #pragma unroll
-        for (int c = 0; c < 9; ++c) p[r][c] = base[static_cast<std::size_t>(r) * pitch + c];
+            for (int w = 0; w < 3; ++w)
+                raw[r][w] = __ldg(reinterpret_cast<const unsigned int*>(base + static_cast<std::size_t>(r) * pitch) + w);
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+            raw[r][0] = __funnelshift_r(raw[r][0], raw[r][1], 8 * off);
+            raw[r][1] = __funnelshift_r(raw[r][1], raw[r][2], 8 * off);
+            raw[r][2] >>= 8 * off;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+            const std::uint8_t* q = base + static_cast<std::size_t>(r) * pitch;
+            raw[r][0] = q[0] | q[1] << 8 | q[2] << 16 | static_cast<std::uint32_t>(q[3]) << 24;
+            raw[r][1] = q[4] | q[5] << 8 | q[6] << 16 | static_cast<std::uint32_t>(q[7]) << 24;
+            raw[r][2] = q[8];
+        }
+    }
+    int p[3][9], h[3][7];  // the last three rows: bytes, 1-2-1 sums
     int a = 0, b = 0, cc = 0;
 #pragma unroll
-    for (int i = 1; i < 8; ++i)
+    for (int r = 0; r < 9; ++r) {
 #pragma unroll
-        for (int jx = 1; jx < 8; ++jx) {
-            const int ix = (p[i][jx + 1] - p[i][jx - 1]) * 2 + (p[i - 1][jx + 1] - p[i - 1][jx - 1]) +
-                           (p[i + 1][jx + 1] - p[i + 1][jx - 1]);
-            const int iy = (p[i + 1][jx] - p[i - 1][jx]) * 2 + (p[i + 1][jx - 1] - p[i - 1][jx - 1]) +
-                           (p[i + 1][jx + 1] - p[i - 1][jx + 1]);
+        for (int c = 0; c < 9; ++c) p[r % 3][c] = static_cast<int>((raw[r][c / 4] >> (8 * (c % 4))) & 0xffu);
+#pragma unroll
+        for (int c = 0; c < 7; ++c) h[r % 3][c] = p[r % 3][c] + 2 * p[r % 3][c + 1] + p[r % 3][c + 2];
+        if (r < 2) continue;
+        int v[9];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) v[c] = p[(r + 1) % 3][c] + 2 * p[(r + 2) % 3][c] + p[r % 3][c];
+#pragma unroll
+        for (int c = 0; c < 7; ++c) {
+            const int ix = v[c + 2] - v[c], iy = h[r % 3][c] - h[(r + 1) % 3][c];
             a += ix * ix;
             b += iy * iy;
             cc += ix * iy;
         }
+    }
     const float fa = static_cast<float>(a), fb = static_cast<float>(b), fc = static_cast<float>(cc);
     const float trace = __fadd_rn(fa, fb);
     const float det = __fsub_rn(__fmul_rn(fa, fb), __fmul_rn(fc, fc));
@@ -798,7 +908,8 @@ __global__ __launch_bounds__(kHarrisThreads) void harris_kernel(const __grid_con
     const auto px = static_cast<std::uint32_t>(j.keys[slot]);
     const int x = static_cast<int>(px % static_cast<std::uint32_t>(j.width));
     const int y = static_cast<int>(px / static_cast<std::uint32_t>(j.width));
-    const float r = harris_response(j.image, j.pitch, x, y, j.harris_k);
+    const bool words = ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 3) == 0;
+    const float r = harris_response(j.image, j.pitch, x, y, j.harris_k, words);
     j.keys[slot] = (static_cast<std::uint64_t>(order_bits(r)) << 32) | (0xffffffffu - px);
 }
 
@@ -828,7 +939,7 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
     if (j.blur_marks) mark_blur_tiles(j, static_cast<int>(x), static_cast<int>(y));
 }
 
-// One block per image: bitonic sort (descending) of up to kSortCap keys in
+// One block per job: bitonic sort (descending) of up to kSortCap keys in
 // shared memory, then the first min(K, selected) become the keypoints.
 template <class Src>
 __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_constant__ Src src) {
@@ -892,30 +1003,47 @@ __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_co
     for (int i = threadIdx.x; i < limit; i += kSortThreads) write_keypoint(j, i, sk[i]);
 }
 
-// Fallback for images with more than kSortCap pre-selected points: the rank
-// of a key is the number of larger keys (keys are unique). Launched over the
-// same blocks as the Harris kernel.
+// Top-K by counting: the rank of a key is the number of larger keys (keys are
+// unique). A block ranks kRankKeys keys, one per lane; its 16 warps share the
+// comparisons with every key of the job, staged kRankTile at a time. Jobs with
+// at most `above` keys are left to the sort. Counting n keys costs n^2
+// comparisons, but spread over the whole chip, where the sort has one block
+// per job: one 512x512 image, 8 layers: 12 -> 6 us; 4K, K = 8000: 46 -> 14 us.
+// rank_pays draws the line between the two.
 template <class Src>
-__global__ __launch_bounds__(kHarrisThreads) void rank_topk_kernel(const __grid_constant__ Src src) {
-    __shared__ std::uint64_t tile[kHarrisThreads];
+__global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_constant__ Src src, int above) {
+    __shared__ __align__(16) std::uint64_t tile[kRankTile];
+    __shared__ int part[kRankThreads / 32][kRankKeys];
+    static_assert(kRankKeys == 32, "one key per lane");
     DetectJob j;
     int local;
-    if (!src.find(blockIdx.x, kHarrisKind, &j, &local)) return;
+    if (!src.find(blockIdx.x / kRankPer, kHarrisKind, &j, &local)) return;
+    const int first = (local * kRankPer + static_cast<int>(blockIdx.x % kRankPer)) * kRankKeys;
     const int n = static_cast<int>(j.params->selected);
-    if (n <= kSortCap) return;
-    const int slot = local * kHarrisThreads + static_cast<int>(threadIdx.x);
-    if (local * kHarrisThreads >= n) return;  // block-uniform
-    const std::uint64_t key = slot < n ? j.keys[slot] : 0ull;
+    if (n <= above || first >= n) return;  // block-uniform
+    const int t = threadIdx.x, k = t % kRankKeys, slice = t / kRankKeys;
+    const int slot = first + k;
+    const std::uint64_t key = slot < n ? j.keys[slot] : ~0ull;
     int rank = 0;
-    for (int b0 = 0; b0 < n; b0 += kHarrisThreads) {
-        const int q = b0 + static_cast<int>(threadIdx.x);
-        tile[threadIdx.x] = q < n ? j.keys[q] : 0ull;
+    for (int b0 = 0; b0 < n; b0 += kRankTile) {
+        if (b0) __syncthreads();
+#pragma unroll
+        for (int i = t; i < kRankTile; i += kRankThreads) tile[i] = b0 + i < n ? j.keys[b0 + i] : 0ull;
         __syncthreads();
-        const int m = min(kHarrisThreads, n - b0);
-        for (int i = 0; i < m; ++i) rank += tile[i] > key;
-        __syncthreads();
+        const int m = min(kRankTile, (n - b0 + 1) / 2 * 2);  // keys past n are 0, never larger
+#pragma unroll 4
+        for (int i = 2 * slice; i < m; i += 2 * (kRankThreads / 32)) {
+            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(tile + i);
+            rank += (q.x > key) + (q.y > key);
+        }
     }
-    if (slot < n && rank < j.max_keypoints) write_keypoint(j, rank, key);
+    part[slice][k] = rank;
+    __syncthreads();
+    if (slice == 0 && slot < n) {
+#pragma unroll
+        for (int v = 1; v < kRankThreads / 32; ++v) rank += part[v][k];
+        if (rank < j.max_keypoints) write_keypoint(j, rank, key);
+    }
 }
 
 // ------------------------------------------------------ pyramid layers
@@ -1088,58 +1216,15 @@ __global__ __launch_bounds__(256, 5) void resize_kernel(const __grid_constant__ 
 
 // ------------------------------------------------------------- S3 blur
 
-// One block = one 64x64 tile: rows pass into a float tile with a 3-row halo,
-// then the columns pass; per output the taps are summed first to last with
-// each product and sum rounded separately, then rounded half-to-even and
-// clamped to [0, 255].
-template <class Src>
-__global__ __launch_bounds__(256) void blur_kernel(const __grid_constant__ Src src) {
-    __shared__ std::uint8_t in[kBlurTileH + 6][kBlurTileW + 6];
-    __shared__ float rows[kBlurTileH + 6][kBlurTileW];
-    DescribeJob j;
-    int local;
-    if (!src.find(blockIdx.x, kBlurKind, &j, &local)) return;
-    const int W = j.width, H = j.height;
-    const int y0 = (local / j.tiles_x) * kBlurTileH;
-    const int x0 = (local % j.tiles_x) * kBlurTileW;
-    for (int i = threadIdx.x; i < (kBlurTileH + 6) * (kBlurTileW + 6); i += 256) {
-        const int r = i / (kBlurTileW + 6), c = i - r * (kBlurTileW + 6);
-        const int gy = reflect101(y0 - 3 + r, H), gx = reflect101(x0 - 3 + c, W);
-        in[r][c] = j.image[static_cast<std::size_t>(gy) * j.pitch + gx];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < (kBlurTileH + 6) * kBlurTileW; i += 256) {
-        const int r = i / kBlurTileW, c = i - r * kBlurTileW;
-        float acc = 0.0f;
-#pragma unroll
-        for (int t = 0; t < 7; ++t) acc = __fadd_rn(acc, __fmul_rn(blur_tap(t), static_cast<float>(in[r][c + t])));
-        rows[r][c] = acc;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kBlurTileH * kBlurTileW; i += 256) {
-        const int r = i / kBlurTileW, c = i - r * kBlurTileW;
-        const int gy = y0 + r, gx = x0 + c;
-        if (gx >= W || gy >= H) continue;
-        float acc = 0.0f;
-#pragma unroll
-        for (int t = 0; t < 7; ++t) acc = __fadd_rn(acc, __fmul_rn(blur_tap(t), rows[r + t][c]));
-        // Clamping the float to [0, 255] before rounding half-to-even gives
-        // the same byte as rounding then clamping the integer, for every
-        // finite acc, and keeps signed integer min/max out of this kernel.
-        j.blurred[static_cast<std::size_t>(gy) * j.blur_pitch + gx] =
-            static_cast<std::uint8_t>(__float2int_rn(fminf(fmaxf(acc, 0.0f), 255.0f)));
-    }
-}
-
-// The S3 blur of the 64x64 tiles listed by the keypoint writers (on-demand
-// blur of the pyramid and batched paths): the same bytes as blur_kernel
-// (per output the taps summed first to last, each product and sum rounded on
-// its own, then rounded half-to-even and clamped), with both passes on the
-// sm_100 packed FP32x2 add and multiply (two rows, or two columns, per
-// instruction, each lane rounded as the scalar op). Persistent: block b takes
-// list entries b, b + gridDim.x, ... (the list is complete when the kernel
-// starts). A tile is staged with its reflect-101 halo: 16-byte loads for
-// interior tiles of 16-byte aligned images, reflected byte loads otherwise.
+// The S3 blur of 64x64 tiles: those listed by the keypoint writers (on-demand
+// blur of the pyramid and batched paths, kPacked), or, without a list, the
+// first all_tiles tiles of job 0 (the per-image S3 call, scalar). Per output
+// the taps are summed first to last, then rounded half-to-even. Persistent:
+// block b takes list entries b, b + gridDim.x, ... (the list is complete when
+// the kernel starts). A tile is staged with its reflect-101 halo: 16-byte
+// copies for 16-byte aligned images, reflected byte loads otherwise. The
+// per-image call used to have a kernel with byte-wise loads of its own
+// (640x480: 14 -> 5 us).
 constexpr int kBlurInH = kBlurTileH + 8;  // staged rows of a blur tile: rows y0-4 .. y0+kBlurTileH+3 (halo 3, rounded to 4)
 
 // Origin of blur tile `tile` of job j.
@@ -1200,18 +1285,19 @@ __device__ __forceinline__ void blur_fix_columns(int x0, int W, std::uint8_t (*i
 }
 
 constexpr int kBlurCtasPerSm = 6;  // resident blur blocks per SM; the persistent grid is 148 x this
-template <class Src>
+template <class Src, bool kPacked>
 __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const __grid_constant__ Src src, const uint2* list,
-                                                            const std::uint32_t* count) {
+                                                            const std::uint32_t* count, int all_tiles) {
     __shared__ __align__(16) std::uint8_t in2[2][kBlurInH][kInStride];  // rows y0-4 .., columns x0-16 ..
     __shared__ __align__(16) float rows[kBlurTileH + 6][kBlurTileW];
     __shared__ std::size_t row_at[kBlurInH];
     __shared__ int col_at[kInStride];
     const int tid = threadIdx.x;
-    const int n = static_cast<int>(*count);
+    const int n = list ? static_cast<int>(*count) : all_tiles;
+    const auto tile_at = [&](int i) { return list ? list[i] : make_uint2(0u, static_cast<unsigned>(i)); };
     // tiles of aligned images are copied asynchronously, the next one while this one is blurred
     auto prefetch = [&](int i, std::uint8_t (*dst)[kInStride]) {
-        const uint2 e = list[i];
+        const uint2 e = tile_at(i);
         const DescribeJob jn = src.at(static_cast<int>(e.x));
         if (!aligned16(jn)) return;
         int x0, y0;
@@ -1222,7 +1308,7 @@ __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const _
     if (static_cast<int>(blockIdx.x) < n) prefetch(blockIdx.x, in2[0]);
     for (int i = blockIdx.x; i < n; i += gridDim.x, buf ^= 1) {
         std::uint8_t (*in)[kInStride] = in2[buf];
-        const uint2 e = list[i];
+        const uint2 e = tile_at(i);
         const DescribeJob j = src.at(static_cast<int>(e.x));
         const int W = j.width, H = j.height;
         int x0, y0;
@@ -1267,8 +1353,8 @@ __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const _
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int t = m - 1 - k;
-                    if (t == 0) out[k] = __fmul2_rn(tap_pair(0), xm);
-                    else if (t > 0 && t < 7) out[k] = __fadd2_rn(out[k], __fmul2_rn(tap_pair(t), xm));
+                    if (t == 0) out[k] = first_tap<kPacked>(xm);
+                    else if (t > 0 && t < 7) out[k] = next_tap<kPacked>(out[k], t, xm);
                 }
             }
             *reinterpret_cast<float4*>(&rows[rr][4 * q]) = make_float4(out[0].x, out[1].x, out[2].x, out[3].x);
@@ -1287,11 +1373,11 @@ __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const _
                 for (int o = 0; o < 2; ++o) {
                     const int t = r - o;
                     if (t == 0) {
-                        lo[o] = __fmul2_rn(tap_pair(0), vl);
-                        hi[o] = __fmul2_rn(tap_pair(0), vh);
+                        lo[o] = first_tap<kPacked>(vl);
+                        hi[o] = first_tap<kPacked>(vh);
                     } else if (t > 0 && t < 7) {
-                        lo[o] = __fadd2_rn(lo[o], __fmul2_rn(tap_pair(t), vl));
-                        hi[o] = __fadd2_rn(hi[o], __fmul2_rn(tap_pair(t), vh));
+                        lo[o] = next_tap<kPacked>(lo[o], t, vl);
+                        hi[o] = next_tap<kPacked>(hi[o], t, vh);
                     }
                 }
             }
@@ -1299,8 +1385,7 @@ __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const _
             for (int o = 0; o < 2; ++o) {
                 const int gy = y0 + 2 * pr + o, gx = x0 + 4 * q;
                 if (gy >= H || gx >= W) continue;
-                const std::uint32_t packed = blur_byte(lo[o].x) | (blur_byte(lo[o].y) << 8) |
-                                             (blur_byte(hi[o].x) << 16) | (blur_byte(hi[o].y) << 24);
+                const std::uint32_t packed = pack_bytes(round_pair(lo[o]), round_pair(hi[o]));
                 std::uint8_t* dst = j.blurred + static_cast<std::size_t>(gy) * j.blur_pitch + gx;
                 if (gx + 3 < W && (reinterpret_cast<std::uintptr_t>(dst) & 3) == 0) {
                     *reinterpret_cast<std::uint32_t*>(dst) = packed;
@@ -1338,23 +1423,29 @@ __device__ __forceinline__ int disc_half_width(int v) {
 // k of word w is column u = 4w + k - a - 15 of row v = row - 15; inside the
 // disc its weights are u (for m10) and v (for m01) as signed bytes, outside 0.
 constexpr int kDiscSlots = 288;  // 9 rounds of 32 lanes over the 279 slots
-__device__ __forceinline__ uint2 disc_weights(int a, int slot) {
-    const int row = slot / 9, word = slot - 9 * row;
-    const int v = row - 15, av = v < 0 ? -v : v;
-    std::uint32_t wu = 0, wv = 0;
-    if (row < 31) {
-        const int hw = disc_half_width(av);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int u = 4 * word + k - a - 15;
-            if ((u < 0 ? -u : u) <= hw) {
-                wu |= (static_cast<std::uint32_t>(u) & 0xffu) << (8 * k);
-                wv |= (static_cast<std::uint32_t>(v) & 0xffu) << (8 * k);
+struct alignas(16) DiscTable {
+    uint2 w[4][kDiscSlots];  // [a][slot]: weights for m10, for m01
+};
+constexpr DiscTable disc_table() {
+    constexpr int half[16] = {15, 15, 15, 15, 14, 14, 14, 13, 13, 12, 11, 10, 9, 8, 6, 3};
+    DiscTable t{};
+    for (int a = 0; a < 4; ++a)
+        for (int slot = 0; slot < 279; ++slot) {
+            const int v = slot / 9 - 15, word = slot % 9;
+            unsigned int wu = 0, wv = 0;
+            for (int k = 0; k < 4; ++k) {
+                const int u = 4 * word + k - a - 15;
+                if ((u < 0 ? -u : u) <= half[v < 0 ? -v : v]) {
+                    wu |= (static_cast<unsigned int>(u) & 0xffu) << (8 * k);
+                    wv |= (static_cast<unsigned int>(v) & 0xffu) << (8 * k);
+                }
             }
+            t.w[a][slot].x = wu;
+            t.w[a][slot].y = wv;
         }
-    }
-    return make_uint2(wu, wv);
+    return t;
 }
+__device__ const DiscTable kDiscTable = disc_table();
 
 // acc + sum of the four unsigned bytes of `bytes` times the four signed bytes of `w`
 __device__ __forceinline__ int dot4_us(std::uint32_t bytes, std::uint32_t w, int acc) {
@@ -1381,15 +1472,20 @@ __device__ __forceinline__ float fast_atan2_deg(float y, float x) {
     return a;
 }
 
-__device__ __forceinline__ int rotated_sample(const std::uint8_t* centre, int stride, float fx, float fy,
-                                              float a, float b) {
-    const int ix = __float2int_rn(__fsub_rn(__fmul_rn(fx, a), __fmul_rn(fy, b)));
-    const int iy = __float2int_rn(__fadd_rn(__fmul_rn(fx, b), __fmul_rn(fy, a)));
-    return centre[iy * stride + ix];
+// The blurred byte at the pattern point rotated by (a, b) = (cos, sin),
+// rounded half-to-even by adding 1.5 * 2^23 (as in round_pair): the float's
+// bits are kRoundBits + the integer, and `bias`, -kRoundBits * (stride + 1)
+// modulo 2^32, takes the offset out of row * stride + column.
+constexpr std::uint32_t kRoundBits = 0x4B400000u;
+__device__ __forceinline__ int rotated_sample(const std::uint8_t* centre, std::uint32_t stride, std::uint32_t bias,
+                                              float fx, float fy, float a, float b) {
+    const float cx = __fadd_rn(__fsub_rn(__fmul_rn(fx, a), __fmul_rn(fy, b)), 12582912.0f);
+    const float cy = __fadd_rn(__fadd_rn(__fmul_rn(fx, b), __fmul_rn(fy, a)), 12582912.0f);
+    return centre[static_cast<int>(__float_as_uint(cy) * stride + __float_as_uint(cx) + bias)];
 }
 
-// One warp per keypoint, kDescRounds keypoints per warp (the block stages
-// the pattern once for its kDescKeys keypoints): intensity-centroid moments
+// One warp per keypoint, keys / kDescWarps keypoints per warp (the block
+// stages the pattern and the disc weights once for its `keys` keypoints): intensity-centroid moments
 // over the radius-15 disc of the unblurred image (lane l sums column l - 15),
 // the angle on lane 0 (float fastAtan2, cos/sin evaluated in double then
 // rounded to float), then lane l packs pattern pairs 8l..8l+7 of the blurred
@@ -1397,9 +1493,9 @@ __device__ __forceinline__ int rotated_sample(const std::uint8_t* centre, int st
 // 8 blocks per SM (32 registers): the kernel waits on scattered patch loads,
 // so resident warps matter more than the few registers it spills.
 template <class Src>
-__global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __grid_constant__ Src src) {
+__global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __grid_constant__ Src src, int keys) {
     __shared__ float4 pat[8][32];  // pat[k][l] = pair 8l + k as floats (x0, y0, x1, y1)
-    __shared__ uint2 disc_w[4][kDiscSlots];  // disc_weights(a, slot)
+    __shared__ DiscTable disc;
     DescribeJob j;
     int local;
     if (!src.find(blockIdx.x, kDescKind, &j, &local)) return;
@@ -1410,7 +1506,7 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
         if (local == 0 && threadIdx.x == 0) atomicAdd(j.out_count, count);
         for (int m = 0; m < j.level; ++m) base += j.level_counts[m];
     }
-    if (local * kDescKeys >= count) return;
+    if (local * keys >= count) return;
     {
         const int p = threadIdx.x;  // 256 threads, one pattern pair each
         const int4 q = kOrbPattern[p];
@@ -1420,15 +1516,14 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
     // word loads of the disc need 4-byte aligned rows (block-uniform)
     const bool words = ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 3) == 0;
     if (words)
-        for (int e = threadIdx.x; e < 4 * kDiscSlots; e += kDescWarps * 32)
-            disc_w[e / kDiscSlots][e % kDiscSlots] = disc_weights(e / kDiscSlots, e % kDiscSlots);
+        for (int e = threadIdx.x; e < static_cast<int>(sizeof(DiscTable) / 16); e += kDescWarps * 32)
+            reinterpret_cast<uint4*>(&disc)[e] = __ldg(reinterpret_cast<const uint4*>(&kDiscTable) + e);
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int u = lane - 15, au = u < 0 ? -u : u;
     const int pitch = j.pitch, blur_pitch = j.blur_pitch;
-    for (int r = 0; r < kDescRounds; ++r) {
-        const int index = local * kDescKeys + r * kDescWarps + (threadIdx.x >> 5);
-        if (index >= count) break;
+    const std::uint32_t bias = 0u - kRoundBits * (static_cast<std::uint32_t>(blur_pitch) + 1u);
+    for (int index = local * keys + (threadIdx.x >> 5); index < min(count, (local + 1) * keys); index += kDescWarps) {
         std::uint8_t* row = j.out + static_cast<std::size_t>(base + index) * j.row_stride;
         const float fx = j.x[index], fy = j.y[index];
         const int x = __float2int_rn(fx);
@@ -1457,7 +1552,7 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
                     const int row = (slot * 57) >> 9, word = slot - 9 * row;  // slot / 9 for slot < 288
                     const std::uint32_t d =
                         __ldg(reinterpret_cast<const unsigned int*>(top + static_cast<std::size_t>(row) * pitch + 4 * word));
-                    const uint2 w = disc_w[a][slot];
+                    const uint2 w = disc.w[a][slot];
                     m10 = dot4_us(d, w.x, m10);
                     m01 = dot4_us(d, w.y, m01);
                 }
@@ -1474,11 +1569,8 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
                 }
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            m10 += __shfl_xor_sync(0xffffffffu, m10, o);
-            m01 += __shfl_xor_sync(0xffffffffu, m01, o);
-        }
+        m10 = __reduce_add_sync(0xffffffffu, m10);
+        m01 = __reduce_add_sync(0xffffffffu, m01);
         float a = 0.0f, b = 0.0f;
         if (lane == 0) {
             const float angle = __fmul_rn(fast_atan2_deg(static_cast<float>(m01), static_cast<float>(m10)),
@@ -1498,8 +1590,8 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const float4 q = pat[k][lane];
-            const int t0 = rotated_sample(smooth, blur_pitch, q.x, q.y, a, b);
-            const int t1 = rotated_sample(smooth, blur_pitch, q.z, q.w, a, b);
+            const int t0 = rotated_sample(smooth, blur_pitch, bias, q.x, q.y, a, b);
+            const int t1 = rotated_sample(smooth, blur_pitch, bias, q.z, q.w, a, b);
             value |= (t0 < t1) << k;
         }
         row[lane] = static_cast<std::uint8_t>(value);

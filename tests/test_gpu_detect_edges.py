@@ -1,0 +1,73 @@
+"""S2/S3 where the selection, the rank sort, the Harris loads, the describe
+rounds and the blur change path, bit for bit against the oracle: tie counts
+around the ranked and the listed ties, candidate counts around the rank
+kernel's blocks and tiles, aligned and odd pitches, saturated windows."""
+import numpy as np
+import pytest
+
+from oracle import s2s3
+from tests import gpu_util as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ours(cuda):
+    return G.Lib("ours")
+
+
+def check(ours, gray, thr, k):
+    kp, desc, blurred, (st2, st3, n) = G.detect_describe(ours, gray, thr, k)
+    want_kp, want_desc = s2s3.detect_and_describe(gray, thr, k)
+    assert (st2, st3) == (0, 0) and n == want_kp.shape[0]
+    assert np.array_equal(kp, want_kp) and np.array_equal(desc, want_desc)
+    return n
+
+
+def dots(w, h, step):
+    """Equal isolated dots: every one a maximum of the same score."""
+    g = np.full((h, w), 60, np.uint8)
+    g[::step, ::step] = 200
+    return g
+
+
+@pytest.mark.parametrize("w,h,step,k", [(120, 120, 5, 10),       # some ties, ranked
+                                        (222, 222, 5, 100),      # 1024 ties, the last that are ranked
+                                        (227, 222, 5, 100),      # one column more: radix select of the tie list
+                                        (400, 397, 5, 700),
+                                        (701, 703, 5, 3000),     # 16384 ties and a little more: the maxima list
+                                        (640, 640, 4, 8192)])
+def test_ties(ours, w, h, step, k):
+    assert check(ours, dots(w, h, step), 20, k) == k
+
+
+@pytest.mark.parametrize("k", [1, 63, 64, 65, 511, 512, 513, 1025, 6200])
+def test_candidate_counts(ours, k):
+    rng = np.random.default_rng(k)
+    check(ours, rng.integers(0, 256, (331, 350), dtype=np.uint8), 15, k)
+
+
+@pytest.mark.parametrize("k", [9472, 9473, 18945])
+def test_describe_rounds(ours, k):
+    rng = np.random.default_rng(5)
+    check(ours, rng.integers(0, 256, (900, 901), dtype=np.uint8), 10, k)
+
+
+@pytest.mark.parametrize("pad", [0, 1, 2, 4, 16])
+def test_pitches(ours, pad, monkeypatch):
+    """Word and byte loads of the Harris window and the orientation disc."""
+    monkeypatch.setattr(G, "pitched", lambda gray: pitched(gray, pad))
+    rng = np.random.default_rng(9)
+    check(ours, rng.integers(0, 256, (200, 256), dtype=np.uint8), 20, 400)
+
+
+pitched = G.pitched
+
+
+def test_saturated_blur(ours):
+    """The largest blur sums: an all-255 image and its edges against black."""
+    g = np.full((150, 170), 255, np.uint8)
+    g[70:, 90:] = 0
+    g[20:30, 20:30] = 0
+    _, _, blurred, _ = G.detect_describe(ours, g, 20, 50)
+    assert np.array_equal(blurred, s2s3.blur(g)) and blurred.max() == 255
