@@ -220,8 +220,8 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
     make_pyramid_jobs(image, c, out, desc, ws, l, sh, &jobs);
     int launches = 0;
     for (int i = 1; i < n; ++i) {
-        resize_kernel<OneJob<ResizeJob>, kSingleResizeTileH>
-            <<<l.resize_tiles[i], 256, 0, stream>>>(OneJob<ResizeJob>{jobs.resize[i]}, 0);
+        launch_chained(resize_kernel<OneJob<ResizeJob>, kSingleResizeTileH>, l.resize_tiles[i], 256, 0, stream,
+                       OneJob<ResizeJob>{jobs.resize[i]}, 0);
         ++launches;
     }
     DetSrc det{};
@@ -241,21 +241,21 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
     }
     auto blocks = [&](int kind) { return det.first[kind][n]; };
     if (blocks(kFastKind)) {
-        fast_kernel<DetSrc><<<std::min(blocks(kFastKind), kSmCount * kFastCtasPerSm), kFastThreads, 0, stream>>>(
+        launch_chained(fast_kernel<DetSrc>, std::min(blocks(kFastKind), kSmCount * kFastCtasPerSm), kFastThreads, 0, stream,
             det, queue, blocks(kFastKind));
-        select_kernel<DetSrc><<<blocks(kSelectKind), 256, 0, stream>>>(det);
-        harris_kernel<DetSrc><<<blocks(kHarrisKind), kHarrisThreads, 0, stream>>>(det);
+        launch_chained(select_kernel<DetSrc>, blocks(kSelectKind), 256, 0, stream, det);
+        launch_chained(harris_kernel<DetSrc>, blocks(kHarrisKind), kHarrisThreads, 0, stream, det);
         if (max_cand > kSortCap || rank_pays(blocks(kHarrisKind), blocks(kSortKind), max_cand))
-            rank_topk_kernel<DetSrc><<<blocks(kHarrisKind) * kRankPer, kRankThreads, 0, stream>>>(det, 0);
+            launch_chained(rank_topk_kernel<DetSrc>, blocks(kHarrisKind) * kRankPer, kRankThreads, 0, stream, det, 0);
         else
-            sort_topk_kernel<DetSrc><<<blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream>>>(det);
+            launch_chained(sort_topk_kernel<DetSrc>, blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream, det);
         launches += 4;
-        blur_tiles_kernel<DesSrc, true><<<std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), 256, 0, stream>>>(
+        launch_chained(blur_tiles_kernel<DesSrc, true>, std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), 256, 0, stream,
             des, at_offset<uint2>(ws, l.blur_list), queue + 1, 0);
         ++launches;
     }
     if (des.first[kDescKind][n]) {
-        describe_kernel<DesSrc><<<des.first[kDescKind][n], kDescWarps * 32, 0, stream>>>(des, keys);
+        launch_chained(describe_kernel<DesSrc>, des.first[kDescKind][n], kDescWarps * 32, 0, stream, des, keys);
         ++launches;
     }
     note_launches(launches);

@@ -149,17 +149,17 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
     if (cudaMemsetAsync(src.job.hist, 0, DetectLayout::hist_bytes, stream) != cudaSuccess)
         return Status::CUDA_ERROR;
     const int fast_grid = std::min(l.tiles, kSmCount * kFastCtasPerSm);
-    fast_kernel<Src><<<fast_grid, kFastThreads, 0, stream>>>(src, src.job.counters() + kTileQueue, l.tiles);
+    launch_chained(fast_kernel<Src>, fast_grid, kFastThreads, 0, stream, src, src.job.counters() + kTileQueue, l.tiles);
     if (!record(e_fast, stream)) return Status::CUDA_ERROR;
-    select_kernel<Src><<<l.select_blocks, 256, 0, stream>>>(src);
+    launch_chained(select_kernel<Src>, l.select_blocks, 256, 0, stream, src);
     if (!record(e_select, stream)) return Status::CUDA_ERROR;
     const int harris_blocks = ceil_div(l.candidates, kHarrisThreads);
-    harris_kernel<Src><<<harris_blocks, kHarrisThreads, 0, stream>>>(src);
+    launch_chained(harris_kernel<Src>, harris_blocks, kHarrisThreads, 0, stream, src);
     if (!record(e_harris, stream)) return Status::CUDA_ERROR;
     if (l.candidates > kSortCap || rank_pays(harris_blocks, 1, l.candidates))
-        rank_topk_kernel<Src><<<harris_blocks * kRankPer, kRankThreads, 0, stream>>>(src, 0);
+        launch_chained(rank_topk_kernel<Src>, harris_blocks * kRankPer, kRankThreads, 0, stream, src, 0);
     else
-        sort_topk_kernel<Src><<<1, kSortThreads, sort_smem_bytes(l.candidates), stream>>>(src);
+        launch_chained(sort_topk_kernel<Src>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src);
     note_launches(4);
     return launch_status();
 }
@@ -178,10 +178,10 @@ Status describe(const ImageView& image, const Keypoints& kp, const Descriptors& 
     if (kp.capacity == 0) return record(e_blur, stream) ? Status::OK : Status::CUDA_ERROR;
     using Src = OneJob<DescribeJob>;
     const Src src{make_describe_job(image, kp, out, ws, l)};
-    blur_tiles_kernel<Src, false><<<std::min(l.tiles, kSmCount * kBlurCtasPerSm), 256, 0, stream>>>(src, nullptr, nullptr, l.tiles);
+    launch_chained(blur_tiles_kernel<Src, false>, std::min(l.tiles, kSmCount * kBlurCtasPerSm), 256, 0, stream, src, nullptr, nullptr, l.tiles);
     if (!record(e_blur, stream)) return Status::CUDA_ERROR;
     const int keys = desc_keys(kp.capacity);
-    describe_kernel<Src><<<ceil_div(kp.capacity, keys), kDescWarps * 32, 0, stream>>>(src, keys);
+    launch_chained(describe_kernel<Src>, ceil_div(kp.capacity, keys), kDescWarps * 32, 0, stream, src, keys);
     note_launches(2);
     return launch_status();
 }

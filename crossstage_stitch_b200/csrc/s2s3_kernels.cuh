@@ -430,6 +430,7 @@ __device__ __forceinline__ void stage_fast_tile(const DetectJob& j, int local, s
 template <class Src>
 __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(const __grid_constant__ Src src,
                                                                           std::uint32_t* queue, int total) {
+    wait_for_previous();
     static_assert(sizeof(DetectJob) % 16 == 0, "jobs are copied in 16-byte chunks");
     __shared__ __align__(16) std::uint8_t in[2][kFastInH][kInStride];
     __shared__ __align__(16) std::uint8_t sc[kFastScH][kScStride];
@@ -766,6 +767,7 @@ __device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams
 // 18.5 -> 7 us, 4K: 67 -> 23 us.
 template <class Src>
 __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     __shared__ std::uint32_t suffix[257];
     __shared__ SelectParams sp;
     __shared__ bool last;
@@ -898,6 +900,7 @@ __device__ __forceinline__ float harris_response(const std::uint8_t* img, int pi
 // equal responses prefer the smaller raster index.
 template <class Src>
 __global__ __launch_bounds__(kHarrisThreads) void harris_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     DetectJob j;
     int local;
     if (!src.find(blockIdx.x, kHarrisKind, &j, &local)) return;
@@ -943,6 +946,7 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
 // shared memory, then the first min(K, selected) become the keypoints.
 template <class Src>
 __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     extern __shared__ std::uint64_t sk[];
     DetectJob j;
     int local;
@@ -1012,6 +1016,7 @@ __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_co
 // rank_pays draws the line between the two.
 template <class Src>
 __global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_constant__ Src src, int above) {
+    wait_for_previous();
     __shared__ __align__(16) std::uint64_t tile[kRankTile];
     __shared__ int part[kRankThreads / 32][kRankKeys];
     static_assert(kRankKeys == 32, "one key per lane");
@@ -1101,7 +1106,10 @@ __global__ __launch_bounds__(256, 5) void resize_kernel(const __grid_constant__ 
     __shared__ __align__(16) std::uint8_t raw[kRows][kRawStride];
     ResizeJob j;
     int local;
-    if (!src.find(blockIdx.x, kind, &j, &local)) return;
+    if (!src.find(blockIdx.x, kind, &j, &local)) {
+        wait_for_previous();
+        return;
+    }
     const int y0 = (local / j.tiles_x) * kTileH;
     const int x0 = (local % j.tiles_x) * kResizeTileW;
     const int t = threadIdx.x;
@@ -1109,6 +1117,7 @@ __global__ __launch_bounds__(256, 5) void resize_kernel(const __grid_constant__ 
     if (t < kResizeTileW) xtap[t] = linear_exact_tap(min(x0 + t, j.width - 1), j.src_width, j.scale_x);
     else if (t < kResizeTileW + kTileH)
         ytap[t - kResizeTileW] = linear_exact_tap(min(y0 + t - kResizeTileW, j.height - 1), j.src_height, j.scale_y);
+    wait_for_previous();  // what stands above depends on the job alone
     __syncthreads();
     // 2. source window: rows ry0 .. ry1, 16-byte chunks from column rx0
     const int ry0 = ytap[0].x, ry1 = min(ytap[kTileH - 1].x + 1, j.src_height - 1);
@@ -1288,6 +1297,7 @@ constexpr int kBlurCtasPerSm = 6;  // resident blur blocks per SM; the persisten
 template <class Src, bool kPacked>
 __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const __grid_constant__ Src src, const uint2* list,
                                                             const std::uint32_t* count, int all_tiles) {
+    wait_for_previous();
     __shared__ __align__(16) std::uint8_t in2[2][kBlurInH][kInStride];  // rows y0-4 .., columns x0-16 ..
     __shared__ __align__(16) float rows[kBlurTileH + 6][kBlurTileW];
     __shared__ std::size_t row_at[kBlurInH];
@@ -1498,15 +1508,10 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
     __shared__ DiscTable disc;
     DescribeJob j;
     int local;
-    if (!src.find(blockIdx.x, kDescKind, &j, &local)) return;
-    // The grid covers the capacity; blocks past the keypoint count leave now.
-    const int count = min(*j.count, j.capacity);
-    int base = 0;  // first output row of this layer
-    if (j.level_counts) {
-        if (local == 0 && threadIdx.x == 0) atomicAdd(j.out_count, count);
-        for (int m = 0; m < j.level; ++m) base += j.level_counts[m];
+    if (!src.find(blockIdx.x, kDescKind, &j, &local)) {
+        wait_for_previous();
+        return;
     }
-    if (local * keys >= count) return;
     {
         const int p = threadIdx.x;  // 256 threads, one pattern pair each
         const int4 q = kOrbPattern[p];
@@ -1518,6 +1523,15 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
     if (words)
         for (int e = threadIdx.x; e < static_cast<int>(sizeof(DiscTable) / 16); e += kDescWarps * 32)
             reinterpret_cast<uint4*>(&disc)[e] = __ldg(reinterpret_cast<const uint4*>(&kDiscTable) + e);
+    wait_for_previous();  // what stands above depends on the job and on constants alone
+    // The grid covers the capacity; blocks past the keypoint count leave now.
+    const int count = min(*j.count, j.capacity);
+    int base = 0;  // first output row of this layer
+    if (j.level_counts) {
+        if (local == 0 && threadIdx.x == 0) atomicAdd(j.out_count, count);
+        for (int m = 0; m < j.level; ++m) base += j.level_counts[m];
+    }
+    if (local * keys >= count) return;
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int u = lane - 15, au = u < 0 ? -u : u;

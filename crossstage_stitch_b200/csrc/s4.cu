@@ -141,11 +141,11 @@ Status launch_direction(const Keypoints& qk, const Descriptors& qd, const Keypoi
             const int tc_splits = ceil_div(std::max(tk.capacity, 1), tc_rows);
             const Src tc{make_knn_job(qk, qd, tk, td, q_tiles, tc_splits, tc_rows, partial, out)};
             if (!launch_tc(matcher(), q_tiles * tc_splits, tc, stream)) return Status::CUDA_ERROR;
-            if (tc_splits > 1) knn_merge_kernel<Src><<<ceil_div(qk.capacity, 256), 256, 0, stream>>>(tc);
+            if (tc_splits > 1) launch_chained(knn_merge_kernel<Src>, ceil_div(qk.capacity, 256), 256, 0, stream, tc);
             note_launches(tc_splits > 1 ? 2 : 1);
         } else {
-            knn_popc_kernel<Src, 1><<<q_tiles * splits, kQueryThreads, 0, stream>>>(src);
-            if (splits > 1) knn_merge_kernel<Src><<<ceil_div(qk.capacity, 256), 256, 0, stream>>>(src);
+            launch_chained(knn_popc_kernel<Src, 1>, q_tiles * splits, kQueryThreads, 0, stream, src);
+            if (splits > 1) launch_chained(knn_merge_kernel<Src>, ceil_div(qk.capacity, 256), 256, 0, stream, src);
             note_launches(splits > 1 ? 2 : 1);
         }
     } else {
@@ -153,9 +153,9 @@ Status launch_direction(const Keypoints& qk, const Descriptors& qd, const Keypoi
         const Side t{static_cast<const std::uint8_t*>(td.data), td.row_stride_bytes, tk.capacity, tk.d_count};
         const int blocks = std::min(ceil_div(qk.capacity, 8), 65535);
         if (qd.type == DescriptorType::FLOAT32)
-            knn_generic_kernel<true><<<blocks, 256, 0, stream>>>(q, t, qd.dim, out);
+            launch_chained(knn_generic_kernel<true>, blocks, 256, 0, stream, q, t, qd.dim, out);
         else
-            knn_generic_kernel<false><<<blocks, 256, 0, stream>>>(q, t, qd.dim, out);
+            launch_chained(knn_generic_kernel<false>, blocks, 256, 0, stream, q, t, qd.dim, out);
         note_launches(1);
     }
     return launch_status();
@@ -227,13 +227,13 @@ Status s4_match(const Keypoints& a, const Descriptors& da, const Keypoints& b, c
     aj.ratio = aj.l2 ? config.ratio_threshold * config.ratio_threshold : config.ratio_threshold;
     aj.out = output;
     if (a.capacity <= 1024) {
-        accept_kernel<OneJob<AcceptJob>><<<1, 1024, 0, stream>>>(OneJob<AcceptJob>{aj});
+        launch_chained(accept_kernel<OneJob<AcceptJob>>, 1, 1024, 0, stream, OneJob<AcceptJob>{aj});
         note_launches(1);
     } else {  // many blocks: counts per 1024 queries, then offsets and the compaction
         const int blocks = ceil_div(a.capacity, 1024);
         int* counts = at_offset<int>(workspace, l.accept_counts);
-        accept_count_kernel<OneJob<AcceptJob>><<<blocks, 1024, 0, stream>>>(OneJob<AcceptJob>{aj}, counts);
-        accept_scatter_kernel<OneJob<AcceptJob>><<<blocks, 1024, 0, stream>>>(OneJob<AcceptJob>{aj}, counts);
+        launch_chained(accept_count_kernel<OneJob<AcceptJob>>, blocks, 1024, 0, stream, OneJob<AcceptJob>{aj}, counts);
+        launch_chained(accept_scatter_kernel<OneJob<AcceptJob>>, blocks, 1024, 0, stream, OneJob<AcceptJob>{aj}, counts);
         note_launches(2);
     }
     return launch_status();

@@ -3,6 +3,8 @@
 
 #include <mutex>
 
+#include <type_traits>
+
 #include "s4_kernels.cuh"
 
 namespace stitch::b200::s4k {
@@ -59,25 +61,19 @@ template <class Src> bool enable_pipe_smem() {
     });
     return ok[dev];
 }
+// Launches the tensor-core matcher: chained (launch_chained) for the per-pair
+// call, plainly in the batched chain.
 template <class Src> bool launch_tc(int kind, int blocks, const Src& src, cudaStream_t s) {
-    if (kind == kMatcherTensorPipe) {
-        if (!enable_pipe_smem<Src>()) return false;
-        knn_tc_pipe_kernel<Src><<<blocks, kPipeThreads, kPipeSmem, s>>>(src);
+    const auto go = [&](auto kernel, int threads, int smem) {
+        if constexpr (std::is_same_v<Src, OneJob<KnnJob>>) launch_chained(kernel, blocks, threads, smem, s, src);
+        else kernel<<<blocks, threads, smem, s>>>(src);
         return true;
-    }
+    };
+    if (kind == kMatcherTensorPipe) return enable_pipe_smem<Src>() && go(knn_tc_pipe_kernel<Src>, kPipeThreads, kPipeSmem);
     switch (tc_rows(kind)) {
-        case 64:
-            if (!enable_tc_smem<Src, 64>()) return false;
-            knn_tc_kernel<Src, 64><<<blocks, kQueryThreads, TcShape<64>::smem, s>>>(src);
-            return true;
-        case 128:
-            if (!enable_tc_smem<Src, 128>()) return false;
-            knn_tc_kernel<Src, 128><<<blocks, kQueryThreads, TcShape<128>::smem, s>>>(src);
-            return true;
-        default:
-            if (!enable_tc_smem<Src, 256>()) return false;
-            knn_tc_kernel<Src, 256><<<blocks, kQueryThreads, TcShape<256>::smem, s>>>(src);
-            return true;
+        case 64: return enable_tc_smem<Src, 64>() && go(knn_tc_kernel<Src, 64>, kQueryThreads, TcShape<64>::smem);
+        case 128: return enable_tc_smem<Src, 128>() && go(knn_tc_kernel<Src, 128>, kQueryThreads, TcShape<128>::smem);
+        default: return enable_tc_smem<Src, 256>() && go(knn_tc_kernel<Src, 256>, kQueryThreads, TcShape<256>::smem);
     }
 }
 constexpr int tc_blocks_per_sm(int kind) {

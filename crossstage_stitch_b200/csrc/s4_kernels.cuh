@@ -117,6 +117,7 @@ __device__ __forceinline__ void keep2(std::uint32_t& k1, std::uint32_t& k2, std:
 // from shared memory serves kQ queries.
 template <class Src, int kQ>
 __global__ __launch_bounds__(kQueryThreads) void knn_popc_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     __shared__ uint4 stage[kTrainStage * 2];
     KnnJob j;
     int local;
@@ -315,6 +316,7 @@ __device__ __forceinline__ void fold_stage(std::uint32_t (&p1)[4], std::uint32_t
 
 template <class Src, int kRowsB>
 __global__ __launch_bounds__(kQueryThreads, 1) void knn_tc_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     using Shape = TcShape<kRowsB>;
     constexpr int kTcRowsB = Shape::rows_b;
     constexpr int kTcBytesB = Shape::bytes_b;
@@ -486,6 +488,7 @@ __device__ __forceinline__ bool bar_wait(std::uint64_t* bar, std::uint32_t parit
 
 template <class Src>
 __global__ __launch_bounds__(kPipeThreads, 1) void knn_tc_pipe_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     extern __shared__ std::uint8_t dyn[];
     KnnJob j;
     int local;
@@ -640,6 +643,7 @@ __global__ __launch_bounds__(kPipeThreads, 1) void knn_tc_pipe_kernel(const __gr
 // Thread per query: the two smallest keys over all train partitions.
 template <class Src>
 __global__ __launch_bounds__(256) void knn_merge_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     KnnJob j;
     int local;
     if (!src.find(blockIdx.x, &j, &local)) return;
@@ -678,6 +682,7 @@ __device__ __forceinline__ void push(Top2& t, double d, int i) {
 // train rows round-robin, then the lane top-2s are merged across the warp.
 template <bool kFloat>
 __global__ __launch_bounds__(256) void knn_generic_kernel(Side query, Side train, int dim, Top2* out) {
+    wait_for_previous();
     const int lane = threadIdx.x & 31;
     const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
     const int nq = *query.count, nt = *train.count;
@@ -750,6 +755,7 @@ __device__ __forceinline__ void write_match(const AcceptJob& j, int at, int q, c
 // the accepted queries among b * 1024 .. b * 1024 + 1023 ...
 template <class Src>
 __global__ __launch_bounds__(1024) void accept_count_kernel(const __grid_constant__ Src src, int* counts) {
+    wait_for_previous();
     AcceptJob j;
     int local;
     if (!src.find(0, &j, &local)) return;
@@ -763,6 +769,7 @@ __global__ __launch_bounds__(1024) void accept_count_kernel(const __grid_constan
 // blocks, in query order; the last block writes the match count.
 template <class Src>
 __global__ __launch_bounds__(1024) void accept_scatter_kernel(const __grid_constant__ Src src, const int* counts) {
+    wait_for_previous();
     __shared__ int warp_sum[32];
     __shared__ int offset;
     AcceptJob j;
@@ -795,6 +802,7 @@ __global__ __launch_bounds__(1024) void accept_scatter_kernel(const __grid_const
 // compaction in query order; writes the match count.
 template <class Src>
 __global__ __launch_bounds__(1024) void accept_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     __shared__ int warp_sum[32];
     AcceptJob j;
     int local;

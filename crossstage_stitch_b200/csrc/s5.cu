@@ -115,8 +115,7 @@ template <int kGroup> void launch_search(const SearchJob& sj, int match_capacity
     static const bool smem_ok =
         enable_search_smem_once(reinterpret_cast<const void*>(search_kernel<Src, false, kGroup>), false);
     (void)smem_ok;
-    search_kernel<Src, false, kGroup>
-        <<<sj.io.search_blocks, kSearchThreads, search_smem_bytes(match_capacity, false), stream>>>(Src{sj});
+    launch_chained(search_kernel<Src, false, kGroup>, sj.io.search_blocks, kSearchThreads, search_smem_bytes(match_capacity, false), stream, Src{sj});
 }
 
 }  // namespace
@@ -140,7 +139,7 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
     // for 8 models as for 64.
     io.hpw = count <= 8 * kSmCount ? 1 : count <= 16 * kSmCount ? 2 : count <= 32 * kSmCount ? 4 : 8;
     io.search_blocks = plan_search(count, io.hpw);
-    prepare_kernel<OneJob<PairIO>><<<1, kPrepareThreads, 0, stream>>>(OneJob<PairIO>{io});
+    launch_chained(prepare_kernel<OneJob<PairIO>>, 1, kPrepareThreads, 0, stream, OneJob<PairIO>{io});
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     if (io.search_blocks > 0) {
@@ -157,8 +156,7 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
     static const bool finish_ok =
         enable_finish_smem_once(reinterpret_cast<const void*>(finish_kernel<OneJob<PairIO>>));
     (void)finish_ok;
-    finish_kernel<OneJob<PairIO>>
-        <<<1, kFinishThreads, finish_smem_bytes(matches.capacity), stream>>>(OneJob<PairIO>{io});
+    launch_chained(finish_kernel<OneJob<PairIO>>, 1, kFinishThreads, finish_smem_bytes(matches.capacity), stream, OneJob<PairIO>{io});
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     if (cudaMemcpyAsync(output, &io.state->result, sizeof(*output), cudaMemcpyDeviceToHost, stream) != cudaSuccess)

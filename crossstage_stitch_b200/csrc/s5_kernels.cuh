@@ -556,6 +556,7 @@ __device__ __forceinline__ bool same_scale(const ScaleInfo& a, const ScaleInfo& 
 // coordinates of every match. One block per pair.
 template <class Src>
 __global__ __launch_bounds__(kPrepareThreads) void prepare_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     __shared__ int go, bad;
     __shared__ unsigned int top[4];
     PairIO j;
@@ -641,6 +642,7 @@ constexpr int kFitThreads = 128;
 // apart from the scoring.
 template <class Src>
 __global__ __launch_bounds__(kFitThreads, 3) void fit_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     SearchJob sj;
     int block;
     if (!src.find(blockIdx.x, &sj, &block)) return;
@@ -776,6 +778,7 @@ __device__ __forceinline__ Pt get_match(const float* pts, int i) {
 // for them).
 template <class Src, bool kPrefit, int kGroup>
 __global__ __launch_bounds__(kSearchThreads, kPrefit ? 4 : 2) void search_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     constexpr int kSlices = kSearchThreads / kGroup;
     constexpr int kStage = kPrefit ? kStagePoints : kStagePointsFused;
     extern __shared__ float4 pts4[];
@@ -1375,6 +1378,7 @@ __device__ inline bool block_fit(const PairIO& j, const FinishShared& sh, const 
 // winner, refine, and build the mask and the result.
 template <class Src>
 __global__ __launch_bounds__(kFinishThreads, 1) void finish_kernel(const __grid_constant__ Src src) {
+    wait_for_previous();
     extern __shared__ float4 finish_smem[];  // terms, points, kept list, keep flags
     __shared__ double model[2][9], loss;  // current model and candidate; loss of the current one
     __shared__ HomographyResult res;
