@@ -20,12 +20,16 @@ void note_launches(int n);
 
 // Launches of the per-image and per-pair calls: a kernel may be scheduled while
 // the one before it on the stream still runs, and holds at
-// wait_for_previous(), the first statement of every kernel launched this way,
-// until that one has completed and its writes are visible. Every kernel waits
-// (whatever its blocks do afterwards), so "the one before" has itself waited
-// for all earlier work. These calls are chains of short dependent kernels, in
-// which the launch latency is a large part: 512x512 pair, 30 launches, 233 ->
-// 200 us. The batched chain launches plainly (its kernels are long).
+// wait_for_previous(), the first statement of every kernel launched this way
+// that touches memory, until that one has completed and its writes are
+// visible. Every kernel waits (whatever its blocks do afterwards), so "the one
+// before" has itself waited for all earlier work. A kernel lets the next one
+// be scheduled only once it has been released itself: let go before the wait,
+// several waiting kernels pile up on the chip and the blocks of the working
+// ones are placed unevenly (512x512 pair 219 us that way, 184 this way). These
+// calls are chains of some thirty short dependent kernels, in which the launch
+// latency is a large part: VGA single-level pair 133 -> 100 us, 512x512 at 8
+// layers 233 -> 184 us. The batched chain launches plainly.
 template <class... P, class... A>
 inline void launch_chained(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg{};
@@ -42,7 +46,7 @@ inline void launch_chained(void (*kernel)(P...), int grid, int block, int smem, 
 }
 
 __device__ __forceinline__ void wait_for_previous() {
-    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
 
 inline Status launch_status() {
