@@ -6,9 +6,9 @@ Function names and argument meaning follow the reference's C++ stage API
 src/s5/s5.hpp:23-39); every call goes through the C ABI of libstitch_b200.so
 and returns the Status code. PairRunner reproduces the reference harness's
 fixed-config pair run (harness/pipeline_runner.cu:335-416): buffers are
-allocated once for the largest image and K, then each pair runs
-S2(A), S2(B), S3(A), S3(B), S4, S5 on one stream and synchronises once
-(with pyramid levels > 1, S2+S3 of each image is one pyramid call).
+allocated once for the largest image and K, then each pair runs S2 and S3 of
+both images, S4 and S5 and synchronises once (with pyramid levels > 1, S2+S3
+of each image is one pyramid call).
 """
 from __future__ import annotations
 
@@ -137,8 +137,13 @@ def workspace(nbytes: int, device) -> torch.Tensor:
 
 
 class PairRunner:
-    """The plain per-pair form: the drop-in stages called one pair at a time
-    on one stream, exactly as the reference harness calls them."""
+    """The plain per-pair form: the drop-in stages called one pair at a time,
+    as the reference harness calls them. Image B's S2 and S3 run on a stream of
+    the runner beside image A's on the caller's, between an event of the
+    caller's stream and one the caller's stream waits for: to the caller all
+    work is on their stream. One image leaves most of the chip idle (512x512
+    pair 176 -> XXX us). With another stage library everything stays on the
+    caller's stream."""
 
     def __init__(self, max_w: int, max_h: int, max_k: int, max_r: int = 8192, device: str | int = "cuda",
                  cross_check: bool = False, stage_lib=None):
@@ -161,7 +166,7 @@ class PairRunner:
         self.ws2 = [workspace(self.s2_bytes, self.device) for _ in range(2)]
         check("s3_workspace_bytes", L.stitch_s3_workspace_bytes(max_w, max_h, ref(b)))
         self.s3_bytes = b.value
-        self.ws3 = workspace(self.s3_bytes, self.device)
+        self.ws3 = [workspace(self.s3_bytes, self.device) for _ in range(2)]
         c4 = S4Config()
         c4.ratio_threshold = 0.8
         c4.cross_check = 1 if cross_check else 0
@@ -173,18 +178,31 @@ class PairRunner:
         self.ws5 = workspace(self.s5_bytes, self.device)
         self.pinned = torch.zeros(C.sizeof(HomographyResult), dtype=torch.uint8, pin_memory=True)
         self.result = HomographyResult.from_address(self.pinned.data_ptr())
-        self.wsp: dict[tuple[int, float], tuple[torch.Tensor, int]] = {}
+        self.wsp: dict[tuple[int, float], tuple[list[torch.Tensor], int]] = {}
+        # image B's stream, and the events that order it against the caller's
+        self.side = torch.cuda.Stream(self.device) if stage_lib is None else None
+        self.ready, self.done = torch.cuda.Event(), torch.cuda.Event()
+        self.scales: dict[tuple[int, int], ScaleInfo] = {}
 
-    def pyramid_workspace(self, knobs: Knobs) -> tuple[torch.Tensor, int]:
-        """Workspace of the pyramid S2/S3 call for the largest image and K at
-        these levels (allocated on first use)."""
-        key = (knobs.levels, float(np.float32(knobs.scale_factor)))
+    def pyramid_workspace(self, knobs: Knobs, image: int = 0) -> tuple[torch.Tensor, int]:
+        """Workspace of image `image`'s pyramid S2/S3 call for the largest image
+        and K at these levels (allocated on first use)."""
+        key = (knobs.levels, knobs.scale_factor)
         if key not in self.wsp:
             b = C.c_size_t()
             check("pyramid_workspace_bytes", self.L.stitch_pyramid_workspace_bytes(
                 self.max_w, self.max_h, ref(S2Config(20, self.max_k, 0.04)), ref(knobs.pyramid()), ref(b)))
-            self.wsp[key] = (workspace(b.value, self.device), b.value)
-        return self.wsp[key]
+            count = 1 if self.side is None else 2
+            self.wsp[key] = ([workspace(b.value, self.device) for _ in range(count)], b.value)
+        ws, nbytes = self.wsp[key]
+        return ws[image if self.side is not None else 0], nbytes
+
+    def identity_scale(self, w: int, h: int) -> ScaleInfo:
+        if (w, h) not in self.scales:
+            if len(self.scales) >= 64:
+                self.scales.clear()
+            self.scales[w, h] = make_scale_info(w, h, 1.0)
+        return self.scales[w, h]
 
     def matches_view(self, capacity: int) -> Matches:
         return Matches(self.idx_a.data_ptr(), self.idx_b.data_ptr(), self.dist.data_ptr(), capacity,
@@ -196,36 +214,43 @@ class PairRunner:
         """Enqueues S2..S5 (no sync) for the pair in self.img[0/1], or in
         `images` (two device uint8 tensors) when given."""
         L = self.L
-        s = stream_handle(stream)
+        main = stream if stream is not None else torch.cuda.current_stream(self.device)
+        s = C.c_void_p(main.cuda_stream)
         k = knobs.max_keypoints
         dims = ((wa, ha), (wb, hb))
         imgs = self.img if images is None else images
-        c2 = knobs.s2()
-        if knobs.levels > 1:
-            wsp, nbytes = self.pyramid_workspace(knobs)
-            for i in range(2):
-                iv = image_view(imgs[i], *dims[i])
-                check("pyramid_detect_describe", L.stitch_pyramid_detect_describe(
-                    ref(iv), ref(c2), ref(knobs.pyramid()), ref(self.feat[i].keypoints(k)),
-                    ref(self.feat[i].descriptors()), ptr(wsp), nbytes, s))
-        else:
-            for i in range(2):
-                iv = image_view(imgs[i], *dims[i])
-                check("s2_detect", L.stitch_s2_detect(ref(iv), ref(c2), ref(self.feat[i].keypoints(k)),
-                                                      ptr(self.ws2[i]), self.s2_bytes, s))
-            for i in range(2):
-                iv = image_view(imgs[i], *dims[i])
-                check("s3_describe", L.stitch_s3_describe(ref(iv), ref(self.feat[i].keypoints(k)),
-                                                          ref(self.feat[i].descriptors()), ptr(self.ws3),
-                                                          self.s3_bytes, s))
-        ka, kb = self.feat[0].keypoints(k), self.feat[1].keypoints(k)
-        da, db = self.feat[0].descriptors(), self.feat[1].descriptors()
+        c2, pyr = knobs.s2(), knobs.pyramid()
+        kps = [f.keypoints(k) for f in self.feat]
+        descs = [f.descriptors() for f in self.feat]
+        views = [image_view(imgs[i], *dims[i]) for i in range(2)]
+        streams = [s, s]
+        if self.side is not None:
+            self.ready.record(main)
+            self.side.wait_event(self.ready)
+            streams[1] = C.c_void_p(self.side.cuda_stream)
+        try:
+            if knobs.levels > 1:
+                for i in range(2):
+                    wsp, nbytes = self.pyramid_workspace(knobs, i)
+                    check("pyramid_detect_describe", L.stitch_pyramid_detect_describe(
+                        ref(views[i]), ref(c2), ref(pyr), ref(kps[i]), ref(descs[i]), ptr(wsp), nbytes, streams[i]))
+            else:
+                for i in range(2):
+                    check("s2_detect", L.stitch_s2_detect(ref(views[i]), ref(c2), ref(kps[i]), ptr(self.ws2[i]),
+                                                          self.s2_bytes, streams[i]))
+                for i in range(2):
+                    check("s3_describe", L.stitch_s3_describe(ref(views[i]), ref(kps[i]), ref(descs[i]),
+                                                              ptr(self.ws3[i]), self.s3_bytes, streams[i]))
+        finally:  # after a failed call too: the caller's stream stays behind the side stream
+            if self.side is not None:
+                self.done.record(self.side)
+                main.wait_event(self.done)
         m = self.matches_view(k)
-        check("s4_match", L.stitch_s4_match(ref(ka), ref(da), ref(kb), ref(db), ref(knobs.s4()), ref(m),
-                                            ptr(self.ws4), self.s4_bytes, s))
-        sa = scale_a if scale_a is not None else make_scale_info(wa, ha, 1.0)
-        sb = scale_b if scale_b is not None else make_scale_info(wb, hb, 1.0)
-        check("s5_estimate", L.stitch_s5_estimate(ref(ka), ref(kb), ref(m), ref(sa), ref(sb), ref(knobs.s5()),
+        check("s4_match", L.stitch_s4_match(ref(kps[0]), ref(descs[0]), ref(kps[1]), ref(descs[1]), ref(knobs.s4()),
+                                            ref(m), ptr(self.ws4), self.s4_bytes, s))
+        sa = scale_a if scale_a is not None else self.identity_scale(wa, ha)
+        sb = scale_b if scale_b is not None else self.identity_scale(wb, hb)
+        check("s5_estimate", L.stitch_s5_estimate(ref(kps[0]), ref(kps[1]), ref(m), ref(sa), ref(sb), ref(knobs.s5()),
                                                   ptr(self.mask), C.c_void_p(self.pinned.data_ptr()),
                                                   ptr(self.ws5), self.s5_bytes, s))
 
