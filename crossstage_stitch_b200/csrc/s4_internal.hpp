@@ -71,9 +71,9 @@ template <class Src> bool launch_tc(int kind, int blocks, const Src& src, cudaSt
     };
     if (kind == kMatcherTensorPipe) return enable_pipe_smem<Src>() && go(knn_tc_pipe_kernel<Src>, kPipeThreads, kPipeSmem);
     switch (tc_rows(kind)) {
-        case 64: return enable_tc_smem<Src, 64>() && go(knn_tc_kernel<Src, 64>, kQueryThreads, TcShape<64>::smem);
-        case 128: return enable_tc_smem<Src, 128>() && go(knn_tc_kernel<Src, 128>, kQueryThreads, TcShape<128>::smem);
-        default: return enable_tc_smem<Src, 256>() && go(knn_tc_kernel<Src, 256>, kQueryThreads, TcShape<256>::smem);
+        case 64: return enable_tc_smem<Src, 64>() && go(knn_tc_kernel<Src, 64>, kTcThreads, TcShape<64>::smem);
+        case 128: return enable_tc_smem<Src, 128>() && go(knn_tc_kernel<Src, 128>, kTcThreads, TcShape<128>::smem);
+        default: return enable_tc_smem<Src, 256>() && go(knn_tc_kernel<Src, 256>, kTcThreads, TcShape<256>::smem);
     }
 }
 constexpr int tc_blocks_per_sm(int kind) {

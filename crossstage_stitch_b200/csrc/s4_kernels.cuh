@@ -178,24 +178,36 @@ __global__ __launch_bounds__(kQueryThreads) void knn_popc_kernel(const __grid_co
 
 // ------------------------------------------------- tensor-core matcher
 //
-// Exact Hamming distance on the 5th-generation tensor cores: every
-// descriptor bit b becomes the int8 value +1 (b = 1) or -1 (b = 0), so for
-// two 256-bit descriptors dot = 256 - 2 * Hamming, and tcgen05.mma
-// kind::i8 (int32 accumulation, exact) gives dot for a 128-query x
-// 256-train tile in TMEM. The block walks the same train partition as the
-// popc kernel; each query's thread reads its row of dot products back with
-// tcgen05.ld and keeps the two smallest (distance << 23 | train index)
-// keys, so results equal knn_popc_kernel's bit for bit.
+// Exact Hamming distance on the 5th-generation tensor cores. In
+// knn_tc_kernel every query bit b becomes the int8 value 1 - 2b and every
+// train bit the int8 value b, so for two 256-bit descriptors
+// Hamming = popcount(query) + dot, and tcgen05.mma kind::i8 (int32
+// accumulation, exact) gives dot for a 128-query tile against a stage of train
+// rows in TMEM. The block walks the same train partition as the popc kernel;
+// each query's thread reads its row of dot products back with tcgen05.ld and
+// keeps the two smallest (distance << 23 | train index) keys, so results equal
+// knn_popc_kernel's bit for bit. The order of the 256 products is free, as
+// long as both sides share it: byte k of expanded word i of a descriptor word
+// is its bit 8k + i, one shift and one mask per four bytes.
 //
-// Shared memory holds the expanded queries (128 rows x 256 bytes) and one
-// train stage (kRowsB rows x 256 bytes: 256, 128 or 64) in the K-major
-// 128-byte-swizzle layout tcgen05 reads: per 128-byte K block, 8-row groups
-// of 1024 bytes, 16-byte chunk c of row r stored at chunk c ^ (r % 8). A
-// narrower stage halves the shared memory and TMEM of a block, so more
-// blocks share an SM and one block's staging and epilogue overlap another's
-// MMA (2, 3 or 4 blocks per SM).
+// Shared memory holds the expanded queries (128 rows x 256 bytes) and two half
+// stages of train rows (kRowsB / 2 rows x 256 bytes each; kRowsB 256, 128 or
+// 64) in the K-major 128-byte-swizzle layout tcgen05 reads: per 128-byte K
+// block, 8-row groups of 1024 bytes, 16-byte chunk c of row r stored at chunk
+// c ^ (r % 8). While the MMAs of one half run, the other half is expanded (its
+// rows fetched a half ahead), and while its MMAs run the first half's dot
+// products are folded into the keys. A narrower stage halves the shared memory
+// and TMEM of a block, so more blocks share an SM (2, 3 or 4 blocks per SM).
+//
+// What bounds it: the latency of a half's chain (barrier, keys, next
+// expansion) at 16 warps per SM; the tensor pipe is busy a quarter of the
+// time. Before, both sides were +-1 (six instructions per four bytes instead
+// of two), one thread kept a query's keys, and a stage's fetch, expansion,
+// MMAs and keys ran one after the other: s4_match 8192 x 8192 47 -> 35 us,
+// 64 pairs of 2000 x 2000 119 -> 84 us. Narrower stages: 107 and 168 us.
 constexpr int kTcRowsA = kQueryThreads;       // 128 queries (MMA M)
 constexpr int kTcBytesA = kTcRowsA * 256;
+constexpr int kTcThreads = 2 * kTcRowsA;      // two threads per query, each for half of a half stage's columns
 template <int kRowsB> struct TcShape {
     static_assert(kRowsB == 64 || kRowsB == 128 || kRowsB == 256, "MMA N and TMEM columns");
     static constexpr int rows_b = kRowsB;                                  // MMA N, TMEM columns
@@ -206,6 +218,8 @@ template <int kRowsB> struct TcShape {
     // K-major, N = kRowsB, M = 128
     static constexpr std::uint32_t idesc =
         (2u << 4) | (1u << 7) | (1u << 10) | ((kRowsB >> 3) << 17) | ((kTcRowsA >> 4) << 24);
+    static constexpr std::uint32_t idesc_half =  // N = kRowsB / 2
+        (2u << 4) | (1u << 7) | (1u << 10) | ((kRowsB >> 4) << 17) | ((kTcRowsA >> 4) << 24);
     static_assert(blocks_per_sm * kRowsB <= 512, "TMEM columns of the resident blocks");
 };
 constexpr long long kTcWaitLimit = 1ll << 26;  // mbarrier polls before giving up
@@ -223,6 +237,49 @@ __device__ __forceinline__ std::uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ std::uint32_t pm_one4(std::uint32_t n) {
     const std::uint32_t spread = (n * 0x00204081u) & 0x01010101u;
     return 0x01010101u | ((spread ^ 0x01010101u) * 0xFEu);
+}
+
+// kWords consecutive words of a descriptor row from `src` (16-byte aligned
+// row), zeros when src is null.
+template <int kWords> struct Words {
+    std::uint32_t w[kWords];
+};
+template <int kWords> __device__ __forceinline__ Words<kWords> load_words(const std::uint8_t* src) {
+    Words<kWords> r{};
+    if (src) {
+        if constexpr (kWords >= 4) {
+#pragma unroll
+            for (int i = 0; i < kWords / 4; ++i) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + i);
+                r.w[4 * i] = v.x; r.w[4 * i + 1] = v.y; r.w[4 * i + 2] = v.z; r.w[4 * i + 3] = v.w;
+            }
+        } else if constexpr (kWords == 2) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+            r.w[0] = v.x; r.w[1] = v.y;
+        } else {
+            r.w[0] = __ldg(reinterpret_cast<const std::uint32_t*>(src));
+        }
+    }
+    return r;
+}
+
+// Writes the expanded words first .. first + kWords - 1 of row `row` of a tile
+// of `rows` rows into the swizzled layout: bytes b, or 1 - 2b for the query
+// side (kSigned).
+template <bool kSigned, int kWords>
+__device__ __forceinline__ void stage_bits(std::uint8_t* tile, int rows, int row, int first, const std::uint32_t* w) {
+    std::uint8_t* base = tile + (row >> 3) * 1024 + (row & 7) * 128;
+#pragma unroll
+    for (int h = 0; h < 2 * kWords; ++h) {  // half a descriptor word -> one 16-byte chunk
+        std::uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = (w[h >> 1] >> (4 * (h & 1) + i)) & 0x01010101u;
+            if (kSigned) v[i] = 0x01010101u ^ (v[i] * 0xFEu);
+        }
+        const int at = 2 * first + h, kb = at >> 3, c = at & 7;
+        *reinterpret_cast<uint4*>(base + kb * rows * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
 }
 
 // Writes descriptor row `row` (32 bytes at src; zeros when src is null) of
@@ -257,176 +314,252 @@ __device__ __forceinline__ std::uint64_t sw128_desc(std::uint32_t addr) {
 
 // Packed top-2 of one stage's columns: in each 32-bit word the low 16-bit
 // lane holds a key of an even column and the high lane one of the next odd
-// column, key16 = (distance << 7) | (column - first) / 2 with distance =
-// (256 - dot) / 2 <= 256 (so key16 <= 32895; 0xffff is empty). Within a
-// lane, smaller key16 is exactly (smaller distance, then smaller column), so
-// one min/max.u16x2 updates two candidates. The even and odd lanes are
-// folded into the 32-bit (distance << 23 | train index) chains when the
-// stage ends (fold_stage), which keeps the top-2 exact.
-__device__ __forceinline__ void keep2x2(std::uint32_t& a1, std::uint32_t& a2, std::uint32_t x) {
-    a2 = __vminu2(a2, __vmaxu2(a1, x));
-    a1 = __vminu2(a1, x);
+// column, key16 = (distance << 7) | (column - first) / 2 with distance <= 256
+// (so key16 <= 32895; 0xffff is empty). Within a lane, smaller key16 is
+// exactly (smaller distance, then smaller column), so one min/max.u16x2
+// updates two candidates. The even and odd lanes are folded into the 32-bit
+// (distance << 23 | train index) chains when the stage ends (fold_stage),
+// which keeps the top-2 exact.
+// Four packed words into a (smallest, second) chain: two sorted pairs, merged,
+// then merged into the chain (10 min/max, where one word at a time takes 12).
+__device__ __forceinline__ void keep4x2(std::uint32_t& a1, std::uint32_t& a2, const std::uint32_t (&x)[4]) {
+    const std::uint32_t l0 = __vminu2(x[0], x[1]), h0 = __vmaxu2(x[0], x[1]);
+    const std::uint32_t l1 = __vminu2(x[2], x[3]), h1 = __vmaxu2(x[2], x[3]);
+    const std::uint32_t lo = __vminu2(l0, l1), hi = __vimin3_u16x2(h0, h1, __vmaxu2(l0, l1));
+    a2 = __vimin3_u16x2(a2, hi, __vmaxu2(a1, lo));
+    a1 = __vminu2(a1, lo);
 }
 
-// 32 dot products v of columns first + c .. first + c + 31 (c even) into
-// the packed chains; columns at or past `limit` (train rows past the end)
-// are left out.
-__device__ __forceinline__ void stage_keys32(const std::uint32_t (&v)[32], int c, int first, int limit,
+// 32 dot products v of train rows row .. row + 31 (row of v[0]) into the packed
+// chains, as pairs pair, pair + 1, ... of the thread's chain; rows at or past
+// `limit` (train rows past the end) are left out. A key's distance is
+// (bias + kScale * dot) / 128 per lane (modulo 2^32, where the true keys fit
+// their lanes): kScale -64 and bias 256 * 64 for +-1 on both sides, 128 and
+// popcount(query) * 128 for knn_tc_kernel.
+template <int kScale>
+__device__ __forceinline__ void stage_keys32(const std::uint32_t (&v)[32], int pair, int row, int limit, std::uint32_t bias,
                                              std::uint32_t (&p1)[4], std::uint32_t (&p2)[4]) {
-    const std::uint32_t m0 = static_cast<std::uint32_t>(c >> 1);
-    constexpr std::uint32_t kBias = (256u << 6) + (256u << 22);  // (256 - v) << 6 per lane, as one add
-    if (first + c + 32 <= limit) {
+    constexpr std::uint32_t lo = static_cast<std::uint32_t>(kScale), hi = static_cast<std::uint32_t>(kScale) << 16;
+    const std::uint32_t b0 = (bias + static_cast<std::uint32_t>(pair)) * 0x00010001u;
+    const bool whole = row + 32 <= limit;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const std::uint32_t m = m0 + static_cast<std::uint32_t>(i);
-            const std::uint32_t x = (kBias + (m | (m << 16))) - (v[2 * i] << 6) - (v[2 * i + 1] << 22);
-            keep2x2(p1[i & 3], p2[i & 3], x);
+    for (int g = 0; g < 4; ++g) {
+        std::uint32_t x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = 4 * g + u;
+            x[u] = v[2 * i] * lo + (v[2 * i + 1] * hi + (b0 + i * 0x00010001u));
         }
-    } else {
+        if (!whole) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const std::uint32_t m = m0 + static_cast<std::uint32_t>(i);
-            std::uint32_t x = (kBias + (m | (m << 16))) - (v[2 * i] << 6) - (v[2 * i + 1] << 22);
-            if (first + c + 2 * i >= limit) x |= 0x0000ffffu;
-            if (first + c + 2 * i + 1 >= limit) x |= 0xffff0000u;
-            keep2x2(p1[i & 3], p2[i & 3], x);
-        }
-    }
-}
-
-// The packed chains of a stage whose first column is train row `first`
-// into the 32-bit key chains; the packed chains are emptied.
-__device__ __forceinline__ void fold_stage(std::uint32_t (&p1)[4], std::uint32_t (&p2)[4], std::uint32_t first,
-                                           std::uint32_t (&k1)[4], std::uint32_t (&k2)[4]) {
-#pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const std::uint32_t w = r ? p2[ch] : p1[ch];
-#pragma unroll
-            for (int lane = 0; lane < 2; ++lane) {
-                const std::uint32_t key = (w >> (16 * lane)) & 0xffffu;
-                if (key != 0xffffu)
-                    keep2(k1[ch], k2[ch], ((key >> 7) << 23) + first + 2 * (key & 127u) + static_cast<std::uint32_t>(lane));
+            for (int u = 0; u < 4; ++u) {
+                const int i = 4 * g + u;
+                if (row + 2 * i >= limit) x[u] |= 0x0000ffffu;
+                if (row + 2 * i + 1 >= limit) x[u] |= 0xffff0000u;
             }
         }
-        p1[ch] = p2[ch] = 0xffffffffu;
+        keep4x2(p1[g], p2[g], x);
     }
+}
+
+// 32 columns of this warp's TMEM lanes from `addr`.
+__device__ __forceinline__ void tmem_load32(std::uint32_t addr, std::uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+        "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
+        "[%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+          "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
+          "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
+          "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The packed chains, of rows from `first` on, into the 32-bit keys; the chains
+// are emptied. Pair p of the chains holds the rows first + p / kPairs * kStep +
+// 2 * (p % kPairs) and the next: within a lane smaller keys are earlier rows,
+// so the four chains merge in packed form and four keys are left to decode.
+template <int kPairs, int kStep>
+__device__ __forceinline__ void fold_stage(std::uint32_t (&p1)[4], std::uint32_t (&p2)[4], std::uint32_t first,
+                                           std::uint32_t& k1, std::uint32_t& k2) {
+    std::uint32_t a1 = p1[0], a2 = p2[0];
+#pragma unroll
+    for (int ch = 1; ch < 4; ++ch) {
+        a2 = __vimin3_u16x2(a2, p2[ch], __vmaxu2(a1, p1[ch]));
+        a1 = __vminu2(a1, p1[ch]);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const std::uint32_t w = r ? a2 : a1;
+#pragma unroll
+        for (int lane = 0; lane < 2; ++lane) {
+            const std::uint32_t key = (w >> (16 * lane)) & 0xffffu, p = key & 127u;
+            if (key != 0xffffu)
+                keep2(k1, k2, ((key >> 7) << 23) + first + p / kPairs * kStep + 2 * (p % kPairs) + static_cast<std::uint32_t>(lane));
+        }
+    }
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) p1[ch] = p2[ch] = 0xffffffffu;
+}
+
+// Bounded wait for the completion of an mbarrier phase; the same on every
+// lane of the warp.
+__device__ __forceinline__ bool tc_wait(std::uint64_t* bar, std::uint32_t parity) {
+    std::uint32_t done = 0;
+    for (long long it = 0; it < kTcWaitLimit && !done; ++it) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    }
+    return __all_sync(0xffffffffu, done);
 }
 
 template <class Src, int kRowsB>
-__global__ __launch_bounds__(kQueryThreads, 1) void knn_tc_kernel(const __grid_constant__ Src src) {
+__global__ __launch_bounds__(kTcThreads, 2) void knn_tc_kernel(const __grid_constant__ Src src) {
     wait_for_previous();
     using Shape = TcShape<kRowsB>;
-    constexpr int kTcRowsB = Shape::rows_b;
-    constexpr int kTcBytesB = Shape::bytes_b;
+    constexpr int kHalf = kRowsB / 2;               // train rows per half stage (MMA N)
+    constexpr int kHalfBytes = kHalf * 256;
+    constexpr int kWords = 8 * kHalf / kTcThreads;  // descriptor words a thread expands of a half stage
+    constexpr int kSpan = kHalf / 2 < 32 ? 32 : kHalf / 2;  // columns of a half stage per thread
+    constexpr int kPairs = kSpan / 2, kFold = 128 / kPairs;  // key pairs per half; halves until the 7-bit pairs run out
     extern __shared__ std::uint8_t dyn[];
     KnnJob j;
     int local;
     if (!src.find(blockIdx.x, &j, &local)) return;
     std::uint8_t* tileA = reinterpret_cast<std::uint8_t*>((reinterpret_cast<std::uintptr_t>(dyn) + 1023) & ~std::uintptr_t(1023));
-    std::uint8_t* tileB = tileA + kTcBytesA;
-    auto* bar = reinterpret_cast<std::uint64_t*>(tileB + kTcBytesB);
-    auto* tmem_slot = reinterpret_cast<std::uint32_t*>(bar + 1);
-    auto* stop = reinterpret_cast<int*>(tmem_slot + 1);
+    std::uint8_t* tileB = tileA + kTcBytesA;        // two halves
+    auto* bar = reinterpret_cast<std::uint64_t*>(tileB + 2 * kHalfBytes);  // one per half
+    auto* tmem_slot = reinterpret_cast<std::uint32_t*>(bar + 2);
+    auto* stop = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5;
+    const int qrow = tid % kTcRowsA, side = tid / kTcRowsA;  // TMEM lane, column half
     const int qt = local % j.q_tiles, split = local / j.q_tiles;
     int nq, nt;
     const bool ok = counts_valid(j, &nq, &nt);
     const int t0 = split * j.rows_per_split;
     const int t1 = ok ? min(nt, t0 + j.rows_per_split) : t0;
-    const int q = qt * kTcRowsA + tid;
+    const int halves = t1 > t0 ? (t1 - t0 + kHalf - 1) / kHalf : 0;
+    const int q = qt * kTcRowsA + qrow;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(kTcRowsB));
+                     "r"(kRowsB));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar + 1)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *stop = 0;
     }
-    stage_pm_row(tileA, kTcRowsA, tid,
-                 ok && q < nq ? j.query.rows + static_cast<std::size_t>(q) * j.query.stride : nullptr);
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const std::uint32_t tmem = *tmem_slot;
-    // four independent (smallest, second) key pairs, merged at the end: keys
-    // are distinct (they carry the train index), so the merge is exact
-    std::uint32_t k1[4] = {kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey};
-    std::uint32_t k2[4] = {kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey};
-    std::uint32_t phase = 0;
-    std::uint32_t p1[4] = {~0u, ~0u, ~0u, ~0u}, p2[4] = {~0u, ~0u, ~0u, ~0u};  // packed chains of a stage
-    for (int base = t0; base < t1; base += kTcRowsB) {
-        for (int r = tid; r < kTcRowsB; r += kQueryThreads)
-            stage_pm_row(tileB, kTcRowsB, r,
-                         base + r < t1 ? j.train.rows + static_cast<std::size_t>(base + r) * j.train.stride : nullptr);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const std::uint32_t a0 = smem_u32(tileA), b0 = smem_u32(tileB);
+    const int brow = tid % kHalf, bword = tid / kHalf * kWords;  // this thread's share of a half stage
+    const auto train_words = [&](int s) {
+        const int r = t0 + s * kHalf + brow;
+        return load_words<kWords>(r < t1 ? j.train.rows + static_cast<std::size_t>(r) * j.train.stride + 4 * bword : nullptr);
+    };
+    Words<kWords> ahead = train_words(0);
+    std::uint32_t bias = 0;  // popcount(query) << 7
+    {
+        const Words<8> d = load_words<8>(ok && q < nq ? j.query.rows + static_cast<std::size_t>(q) * j.query.stride : nullptr);
+        std::uint32_t own[4];
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {  // K = 256 in slices of 32 bytes
-                const std::uint32_t koff = (s & 3) * 32;  // within the 128-byte swizzle atom
-                const std::uint64_t da = sw128_desc(a0 + (s >> 2) * kTcRowsA * 128 + koff);
-                const std::uint64_t db = sw128_desc(b0 + (s >> 2) * kTcRowsB * 128 + koff);
+        for (int i = 0; i < 8; ++i) bias += static_cast<std::uint32_t>(__popc(d.w[i])) << 7;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) own[i] = side ? d.w[4 + i] : d.w[i];
+        stage_bits<true, 4>(tileA, kTcRowsA, qrow, 4 * side, own);
+    }
+    // half stage s, already fetched in `ahead`, into its buffer, and its MMAs
+    // into its accumulator; false when the block has stopped
+    std::uint32_t tmem = 0;
+    const auto issue = [&](int s) {
+        std::uint8_t* const half = tileB + (s & 1) * kHalfBytes;
+        stage_bits<false, kWords>(half, kHalf, brow, bword, ahead.w);
+        if (s + 1 < halves) ahead = train_words(s + 1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        tmem = *tmem_slot;
+        if (*stop) return false;
+        if (tid == 0) {
+            const std::uint32_t a0 = smem_u32(tileA), b0 = smem_u32(half);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {  // K = 256 in slices of 32 bytes
+                const std::uint32_t koff = (k & 3) * 32;  // within the 128-byte swizzle atom
+                const std::uint64_t da = sw128_desc(a0 + (k >> 2) * kTcRowsA * 128 + koff);
+                const std::uint64_t db = sw128_desc(b0 + (k >> 2) * kHalf * 128 + koff);
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                    "l"(da), "l"(db), "r"(Shape::idesc), "r"(s));
+                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
+                        tmem + static_cast<std::uint32_t>((s & 1) * kHalf)),
+                    "l"(da), "l"(db), "r"(Shape::idesc_half), "r"(k));
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(bar))
+                             smem_u32(bar + (s & 1)))
                          : "memory");
         }
-        // bounded wait for the MMA chain of this stage
-        std::uint32_t done = 0;
-        for (long long it = 0; it < kTcWaitLimit && !done; ++it) {
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}\n"
-                : "=r"(done)
-                : "r"(smem_u32(bar)), "r"(phase)
-                : "memory");
-        }
-        if (!done) *stop = 1;
-        __syncthreads();
-        if (*stop) break;
-        phase ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        // this thread's query row: 256 dot products in 8 loads of 32 columns
-#pragma unroll 1
-        for (int c = 0; c < kTcRowsB; c += 32) {
-            std::uint32_t v[32];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
-                "[%32];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                  "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                  "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                  "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(tmem + (static_cast<std::uint32_t>(warp * 32) << 16) + static_cast<std::uint32_t>(c)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            stage_keys32(v, c, base, t1, p1, p2);
-        }
-        fold_stage(p1, p2, static_cast<std::uint32_t>(base), k1, k2);
+        return true;
+    };
+    std::uint32_t k1 = kEmptyKey, k2 = kEmptyKey;  // smallest and second key
+    std::uint32_t p1[4] = {~0u, ~0u, ~0u, ~0u}, p2[4] = {~0u, ~0u, ~0u, ~0u};  // packed chains
+    // Buffer and accumulator s % 2 are free for half stage s + 2 once every
+    // thread has folded half s: it does so before it stages s + 2, and the
+    // barrier of issue(s + 2) comes before its MMAs.
+    bool running = true;
+    int issued = 0;
+    if (halves > 0) issue(0), issued = 1;
+    else {
         asm volatile("tcgen05.fence::before_thread_sync;");
-        __syncthreads();  // TMEM and the train stage are free for the next stage
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        tmem = *tmem_slot;
     }
+    for (int s = 0; s < halves && running; ++s) {
+        if (s + 1 < halves) {
+            running = issue(s + 1);
+            if (!running) break;
+            issued = s + 2;
+        }
+        if (!tc_wait(bar + (s & 1), static_cast<std::uint32_t>(s >> 1) & 1u)) {
+            *stop = 1;  // the other warps see it at the next barrier
+            continue;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        // this thread's query row: its columns of the half, 32 at a time
+#pragma unroll 1
+        for (int c = side * kSpan; c < min(kHalf, (side + 1) * kSpan); c += 32) {
+            std::uint32_t v[32];
+            tmem_load32(tmem + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) +
+                            static_cast<std::uint32_t>((s & 1) * kHalf + c), v);
+            stage_keys32<128>(v, s % kFold * kPairs + (c - side * kSpan) / 2, t0 + s * kHalf + c, t1, bias, p1, p2);
+        }
+        if (s % kFold == kFold - 1 || s + 1 == halves)
+            fold_stage<kPairs, kHalf>(p1, p2, static_cast<std::uint32_t>(t0 + s / kFold * kFold * kHalf + side * kSpan), k1, k2);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
     const bool failed = *stop != 0;
-    if (failed && tid == 0) atomicExch(&g_tc_error, 1);
-#pragma unroll
-    for (int u = 1; u < 4; ++u) {
-        keep2(k1[0], k2[0], k1[u]);
-        keep2(k1[0], k2[0], k2[u]);
+    if (failed) {
+        if (tid == 0) atomicExch(&g_tc_error, 1);
+        // MMAs still in flight read shared memory and write TMEM: wait (bounded) for the last two
+        for (int s = max(issued - 2, 0); s < issued; ++s) tc_wait(bar + (s & 1), static_cast<std::uint32_t>(s >> 1) & 1u);
     }
-    if (!failed && q < j.query.capacity) {
+    auto* const other = reinterpret_cast<uint2*>(tileB);  // the second threads' keys (every MMA is complete)
+    if (side) other[qrow] = make_uint2(k1, k2);
+    __syncthreads();
+    if (!side) {
+        const uint2 o = other[qrow];
+        keep2(k1, k2, o.x);
+        keep2(k1, k2, o.y);
+    }
+    if (!failed && !side && q < j.query.capacity) {
         const bool active = ok && q < nq;
-        const std::uint32_t a1 = active ? k1[0] : kEmptyKey, a2 = active ? k2[0] : kEmptyKey;
+        const std::uint32_t a1 = active ? k1 : kEmptyKey, a2 = active ? k2 : kEmptyKey;
         if (j.splits == 1) {
             j.top2[q] = top2_from_keys(a1, a2);
         } else {
@@ -434,13 +567,13 @@ __global__ __launch_bounds__(kQueryThreads, 1) void knn_tc_kernel(const __grid_c
         }
     }
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcRowsB));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kRowsB));
 }
 
 // ------------------------------------------------ pipelined tensor cores
 //
-// The same exact top-2 search as knn_tc_kernel, with the three kinds of work
-// of a stage overlapped instead of run one after the other. Warp roles:
+// The same exact top-2 search as knn_tc_kernel, with +-1 on both sides (dot =
+// 256 - 2 * Hamming) and the three kinds of work of a stage overlapped instead of run one after the other. Warp roles:
 //   warps 0-7   epilogue: warp w reads TMEM lane quarter w % 4 (its 32
 //               queries) and column half w / 4 of an accumulator, keeping
 //               four top-2 key chains per thread;
@@ -528,8 +661,7 @@ __global__ __launch_bounds__(kPipeThreads, 1) void knn_tc_pipe_kernel(const __gr
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const std::uint32_t tmem = *tmem_slot;
-    std::uint32_t k1[4] = {kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey};
-    std::uint32_t k2[4] = {kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey};
+    std::uint32_t k1 = kEmptyKey, k2 = kEmptyKey;
     const int qrow = 32 * (warp & 3) + lane;  // epilogue: the query of this thread
     if (warp < kPipeEpiWarps) {
         const int half = warp >> 2;
@@ -543,23 +675,13 @@ __global__ __launch_bounds__(kPipeThreads, 1) void knn_tc_pipe_kernel(const __gr
 #pragma unroll 1
             for (int c = 0; c < kPipeStage / 2; c += 32) {
                 std::uint32_t v[32];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                    "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
-                    "[%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                      "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                      "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                      "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(tmem + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) +
-                          static_cast<std::uint32_t>(b * kPipeStage + half * (kPipeStage / 2) + c)));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                stage_keys32(v, c, base, t1, p1, p2);
+                tmem_load32(tmem + (static_cast<std::uint32_t>((warp & 3) * 32) << 16) +
+                                static_cast<std::uint32_t>(b * kPipeStage + half * (kPipeStage / 2) + c), v);
+                stage_keys32<-64>(v, c / 2, base + c, t1, 256u * 64u, p1, p2);
             }
             asm volatile("tcgen05.fence::before_thread_sync;");
             bar_arrive(&freeb[b]);
-            fold_stage(p1, p2, static_cast<std::uint32_t>(base), k1, k2);
+            fold_stage<128, 0>(p1, p2, static_cast<std::uint32_t>(base), k1, k2);
         }
     } else if (warp < kPipeEpiWarps + kPipeProdWarps) {
         const int p = tid - kPipeEpiWarps * 32;  // 0 .. 127
@@ -604,23 +726,18 @@ __global__ __launch_bounds__(kPipeThreads, 1) void knn_tc_pipe_kernel(const __gr
     __syncthreads();
     const bool failed = *stop != 0;
     if (warp < kPipeEpiWarps) {
-#pragma unroll
-        for (int u = 1; u < 4; ++u) {
-            keep2(k1[0], k2[0], k1[u]);
-            keep2(k1[0], k2[0], k2[u]);
-        }
-        if (warp >= 4) xchg[qrow] = make_uint2(k1[0], k2[0]);
+        if (warp >= 4) xchg[qrow] = make_uint2(k1, k2);
     }
     __syncthreads();
     if (failed && tid == 0) atomicExch(&g_tc_error, 1);
     if (!failed && warp < 4) {
         const uint2 o = xchg[qrow];
-        keep2(k1[0], k2[0], o.x);
-        keep2(k1[0], k2[0], o.y);
+        keep2(k1, k2, o.x);
+        keep2(k1, k2, o.y);
         const int q = qt * kTcRowsA + qrow;
         if (q < j.query.capacity) {
             const bool active = ok && q < nq;
-            const std::uint32_t a1 = active ? k1[0] : kEmptyKey, a2 = active ? k2[0] : kEmptyKey;
+            const std::uint32_t a1 = active ? k1 : kEmptyKey, a2 = active ? k2 : kEmptyKey;
             if (j.splits == 1) {
                 j.top2[q] = top2_from_keys(a1, a2);
             } else {
