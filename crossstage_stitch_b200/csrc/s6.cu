@@ -24,6 +24,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "quotient.cuh"
 #include "stitch_b200.h"
 
 namespace stitch::b200::s6k {
@@ -163,57 +164,63 @@ bool overlap(const Span& a, const Span& b) { return a.first < b.last && b.first 
 // ------------------------------------------------------------------ device
 
 // Snaps a sample coordinate within max(tolerance, 16 eps max(1, |x|)) of an
-// integer onto it; inside the pixel-centre grid [0, n - 1]?
-__device__ __forceinline__ bool centre_coord(double& x, int n, double tol) {
+// integer onto it; then its floor (as an integer and a double), and whether it
+// lies inside the pixel-centre grid [0, n - 1]. tol_rules: tolerance >= 16 eps
+// max(1, n + 1), so that it is the larger wherever the answer can be yes.
+__device__ __forceinline__ bool centre_coord(double& x, int n, double tol, bool tol_rules, int& xi, double& fl) {
     if (!isfinite(x)) return false;
-    const double near = nearbyint(x);
-    const double roundoff = __dmul_rn(16 * 2.2204460492503131e-16, fmax(1.0, fabs(x)));
-    if (fabs(__dsub_rn(x, near)) <= fmax(tol, roundoff)) x = near;
-    return x >= 0 && x <= n - 1.0;
+    const double near = nearbyint(x), off = fabs(__dsub_rn(x, near));
+    double bound = tol;
+    if (!tol_rules) bound = fmax(tol, __dmul_rn(16 * 2.2204460492503131e-16, fmax(1.0, fabs(x))));
+    if (off <= bound) x = near;
+    fl = floor(x);
+    xi = __double2int_rd(x);  // saturates
+    return xi >= 0 && (xi < n - 1 || (xi == n - 1 && x == fl));
 }
 
-// Distance-to-edge score min((x + .5) / w, (w - .5 - x) / w, (y + .5) / h,
-// (h - .5 - y) / h) with two divisions: correctly rounded division by a
-// positive number preserves order, so the smaller of two quotients over the
-// same w is the quotient of the smaller numerator (both numerators >= 0.5).
-__device__ __forceinline__ double edge_score(double x, double y, double w, double h) {
-    return fmin(__ddiv_rn(fmin(__dadd_rn(x, 0.5), __dsub_rn(__dsub_rn(w, 0.5), x)), w),
-                __ddiv_rn(fmin(__dadd_rn(y, 0.5), __dsub_rn(__dsub_rn(h, 0.5), y)), h));
+// One axis of the distance-to-edge score: the smaller of (x + .5) / n and
+// (n - .5 - x) / n. Correctly rounded division by a positive number preserves
+// order, so it is the quotient of the smaller numerator (both >= 0.5 inside).
+__device__ __forceinline__ double edge_numerator(double x, double n) {
+    return fmin(__dadd_rn(x, 0.5), __dsub_rn(__dsub_rn(n, 0.5), x));
 }
 
-// General bilinear sample of the pixel-centre grid at (x, y).
-__device__ __forceinline__ bool sample(const ImageView& im, double x, double y, float* rgb, double& score,
-                                       double tol) {
-    if (!centre_coord(x, im.width, tol) || !centre_coord(y, im.height, tol)) return false;
-    const int x0 = static_cast<int>(floor(x)), y0 = static_cast<int>(floor(y));
+// General bilinear sample of the pixel-centre grid at (x, y); inv_w, inv_h:
+// 1 / width and 1 / height, correctly rounded; value: the bytes as doubles (a
+// table in shared memory: a conversion or an FP64 add each otherwise).
+__device__ __forceinline__ bool sample(const ImageView& im, double x, double y, double inv_w, double inv_h,
+                                       const double* value, float* rgb, double& score, double tol, bool tol_rules) {
+    int x0, y0;
+    double fx, fy;
+    if (!centre_coord(x, im.width, tol, tol_rules, x0, fx) || !centre_coord(y, im.height, tol, tol_rules, y0, fy)) return false;
     const int x1 = x0 < im.width - 1 ? x0 + 1 : x0;
     const int y1 = y0 < im.height - 1 ? y0 + 1 : y0;
-    const double ax = __dsub_rn(x, x0), ay = __dsub_rn(y, y0);
+    const double ax = __dsub_rn(x, fx), ay = __dsub_rn(y, fy);
     const double bx = __dsub_rn(1.0, ax), by = __dsub_rn(1.0, ay);
     const std::uint8_t* r0 = im.data + static_cast<std::size_t>(y0) * im.pitch_bytes;
     const std::uint8_t* r1 = im.data + static_cast<std::size_t>(y1) * im.pitch_bytes;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const double v0 = __dadd_rn(__dmul_rn(bx, r0[3 * x0 + c]), __dmul_rn(ax, r0[3 * x1 + c]));
-        const double v1 = __dadd_rn(__dmul_rn(bx, r1[3 * x0 + c]), __dmul_rn(ax, r1[3 * x1 + c]));
-        rgb[c] = static_cast<float>(__ddiv_rn(__dadd_rn(__dmul_rn(by, v0), __dmul_rn(ay, v1)), 255.0));
+        const double v0 = __dadd_rn(__dmul_rn(bx, value[r0[3 * x0 + c]]), __dmul_rn(ax, value[r0[3 * x1 + c]]));
+        const double v1 = __dadd_rn(__dmul_rn(bx, value[r1[3 * x0 + c]]), __dmul_rn(ax, value[r1[3 * x1 + c]]));
+        rgb[c] = static_cast<float>(over255(__dadd_rn(__dmul_rn(by, v0), __dmul_rn(ay, v1))));
     }
-    score = edge_score(x, y, im.width, im.height);
+    const double w = im.width, h = im.height;
+    score = fmin(quotient(edge_numerator(x, w), w, inv_w), quotient(edge_numerator(y, h), h, inv_h));
     return true;
 }
 
-// The same sample at integer (x, y), which is where A is sampled: no snap
-// moves it, both bilinear weights are exactly 0, so each channel is the byte
-// p itself and the colour is (float)(p / 255.0), read from `unit`.
-__device__ __forceinline__ bool sample_at_pixel(const ImageView& im, int x, int y, const float* unit, float* rgb,
-                                                double& score) {
-    if (x < 0 || x >= im.width || y < 0 || y >= im.height) return false;
-    const std::uint8_t* px = im.data + static_cast<std::size_t>(y) * im.pitch_bytes + 3 * x;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) rgb[c] = unit[px[c]];
-    score = edge_score(x, y, im.width, im.height);
-    return true;
+// (float)(p / 255.0) of every byte: the colour of A, which is sampled at
+// integer positions (no snap moves them and both bilinear weights are 0).
+struct UnitTable {
+    float v[256];
+};
+constexpr UnitTable unit_table() {
+    UnitTable t{};
+    for (int i = 0; i < 256; ++i) t.v[i] = static_cast<float>(static_cast<double>(i) / 255.0);
+    return t;
 }
+__device__ const UnitTable kUnit = unit_table();
 
 __device__ __forceinline__ std::uint8_t quantize(float c) {
     return static_cast<std::uint8_t>(floorf(__fadd_rn(fminf(255.0f, fmaxf(0.0f, __fmul_rn(255.0f, c))), 0.5f)));
@@ -223,18 +230,36 @@ struct FeatherArgs {
     ImageView a, b, out, mask;
     s6::Geometry g;
     unsigned long long* stats;  // {union, overlap} or null
+    double inv_wb, inv_hb;      // 1 / B's width and height
+    int tol_rules;              // see centre_coord
 };
 
 constexpr int kS6BlockX = 32, kS6BlockY = 8;
 
+// Bound by issue slots (75 % of them used), before by FP64: 12 correctly
+// rounded divisions per overlap pixel were most of it. A's edge scores are
+// those of the block's columns and rows (40 divisions per block), the
+// divisions by 255 and by B's size are corrected products, and the two
+// quotients of the projection and the three of the blend share one reciprocal
+// each: 2 divisions per pixel are left. 1080p pair: 61 -> 42 us. (Four rows
+// per thread, with the tables built a quarter as often: 42 us too.)
 __global__ __launch_bounds__(kS6BlockX * kS6BlockY) void feather_kernel(const __grid_constant__ FeatherArgs p) {
     __shared__ unsigned long long sums[2];
     __shared__ float unit[256];
+    __shared__ double edge_x[kS6BlockX], edge_y[kS6BlockY], value[256];
     static_assert(kS6BlockX * kS6BlockY == 256, "one byte value per thread");
     const s6::Geometry& g = p.g;
     const int x = blockIdx.x * kS6BlockX + threadIdx.x, y = blockIdx.y * kS6BlockY + threadIdx.y;
     const int t = threadIdx.y * kS6BlockX + threadIdx.x;
-    unit[t] = static_cast<float>(__ddiv_rn(static_cast<double>(t), 255.0));
+    unit[t] = __ldg(&kUnit.v[t]);
+    value[t] = t;
+    if (t < kS6BlockX) {
+        const double w = p.a.width;
+        edge_x[t] = __ddiv_rn(edge_numerator(x + g.origin_x, w), w);
+    } else if (t < kS6BlockX + kS6BlockY) {
+        const double h = p.a.height;
+        edge_y[t - kS6BlockX] = __ddiv_rn(edge_numerator(static_cast<int>(blockIdx.y) * kS6BlockY + (t - kS6BlockX) + g.origin_y, h), h);
+    }
     if (t < 2) sums[t] = 0;
     __syncthreads();
     bool ma = false, mb = false;
@@ -243,22 +268,38 @@ __global__ __launch_bounds__(kS6BlockX * kS6BlockY) void feather_kernel(const __
         const double xa = ia, ya = ja;
         float ra[3] = {}, rb[3] = {};
         double sa = 0, sb = 0;
-        ma = sample_at_pixel(p.a, ia, ja, unit, ra, sa);
+        ma = ia >= 0 && ia < p.a.width && ja >= 0 && ja < p.a.height;
+        if (ma) {
+            const std::uint8_t* px = p.a.data + static_cast<std::size_t>(ja) * p.a.pitch_bytes + 3 * ia;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) ra[c] = unit[px[c]];
+            sa = fmin(edge_x[threadIdx.x], edge_y[threadIdx.y]);
+        }
         const double* m = g.inverse;
         const double den = __dadd_rn(__dadd_rn(__dmul_rn(m[6], xa), __dmul_rn(m[7], ya)), m[8]);
         const double den_scale = __dadd_rn(__dadd_rn(fabs(__dmul_rn(m[6], xa)), fabs(__dmul_rn(m[7], ya))), fabs(m[8]));
         if (isfinite(den) && den_scale > 0 && fabs(den) > __dmul_rn(g.denominator_tolerance, den_scale)) {
-            const double xb = __ddiv_rn(__dadd_rn(__dadd_rn(__dmul_rn(m[0], xa), __dmul_rn(m[1], ya)), m[2]), den);
-            const double yb = __ddiv_rn(__dadd_rn(__dadd_rn(__dmul_rn(m[3], xa), __dmul_rn(m[4], ya)), m[5]), den);
-            mb = sample(p.b, xb, yb, rb, sb, g.snap_tolerance);
+            const double nx = __dadd_rn(__dadd_rn(__dmul_rn(m[0], xa), __dmul_rn(m[1], ya)), m[2]);
+            const double ny = __dadd_rn(__dadd_rn(__dmul_rn(m[3], xa), __dmul_rn(m[4], ya)), m[5]);
+            double xb, yb;
+            if (quotient_range(nx, den) && quotient_range(ny, den)) {
+                const double inv = __drcp_rn(den);
+                xb = quotient(nx, den, inv);
+                yb = quotient(ny, den, inv);
+            } else {
+                xb = __ddiv_rn(nx, den);
+                yb = __ddiv_rn(ny, den);
+            }
+            mb = sample(p.b, xb, yb, p.inv_wb, p.inv_hb, value, rb, sb, g.snap_tolerance, p.tol_rules != 0);
         }
         p.mask.data[static_cast<std::size_t>(y) * p.mask.pitch_bytes + x] = ma || mb ? 1 : 0;
         std::uint8_t* o = p.out.data + static_cast<std::size_t>(y) * p.out.pitch_bytes + 3 * x;
-        const double sw = __dadd_rn(sa, sb);
+        // scores lie in [0.5 / size, 1] and colours are 0 or above 1e-30: no underflow in the blend
+        const double sw = __dadd_rn(sa, sb), inv = ma && mb ? __drcp_rn(sw) : 0.0;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float col = ma && mb ? static_cast<float>(__ddiv_rn(
-                                             __dadd_rn(__dmul_rn(sa, ra[c]), __dmul_rn(sb, rb[c])), sw))
+            const float col = ma && mb ? static_cast<float>(quotient(
+                                             __dadd_rn(__dmul_rn(sa, ra[c]), __dmul_rn(sb, rb[c])), sw, inv))
                                        : (ma ? ra[c] : rb[c]);
             o[c] = quantize(col);
         }
@@ -406,7 +447,8 @@ Status render(const ImageView& a, const ImageView& b, const Geometry& g, BlendMo
     }
     if (statistics && cudaMemsetAsync(statistics, 0, sizeof(RenderStatistics), stream) != cudaSuccess)
         return Status::CUDA_ERROR;
-    FeatherArgs args{a, b, output, mask, g, reinterpret_cast<unsigned long long*>(statistics)};
+    FeatherArgs args{a, b, output, mask, g, reinterpret_cast<unsigned long long*>(statistics), 1.0 / b.width, 1.0 / b.height,
+                     g.snap_tolerance >= 16 * 2.2204460492503131e-16 * (std::max(b.width, b.height) + 1.0)};
     const dim3 block(kS6BlockX, kS6BlockY);
     const dim3 grid(b200::ceil_div(g.width, kS6BlockX), b200::ceil_div(g.height, kS6BlockY));
     if (grid.y > 65535) return Status::INVALID_ARGUMENT;
