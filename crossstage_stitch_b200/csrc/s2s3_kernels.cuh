@@ -214,15 +214,16 @@ constexpr int kSortThreads = 1024;
 constexpr int kSortChunk = 64;      // keys a warp sorts in registers (2 per lane)
 constexpr int kBlurTileW = 64, kBlurTileH = 64;
 constexpr int kDescWarps = 8;
-// Keypoints per warp of a describe block: one while all blocks are resident
-// at once (a warp's rounds run one after the other, 2.5 us each), more when
-// there are more keypoints than that, so that a block's tables are shared.
-// 512x512, K = 1000: 20 us at 4, 14 us at 1; 4K, K = 8000: 24 and 18 us.
-constexpr int kDescMaxRounds = 4;
-constexpr int kDescResident = 148 * 8;  // describe blocks on the chip
+// Keypoints per warp of a describe block: as many as leave the chip's block
+// slots filled, up to 8, so that a block's tables and a warp's angle pass are
+// shared by more. 512x512, K = 1000, one image: 20 us at 4, 14 us at 1; 64
+// pairs, K = 2000: 174 us at 4, 166 at 8, 174 at 16.
+constexpr int kDescMaxRounds = 8;
+constexpr int kDescCtasPerSm = 5;
 __host__ __device__ inline int desc_keys(long long keypoints) {
-    const long long one = kDescWarps * static_cast<long long>(kDescResident);
-    return kDescWarps * (keypoints <= one ? 1 : keypoints <= 2 * one ? 2 : kDescMaxRounds);
+    int rounds = kDescMaxRounds;
+    while (rounds > 1 && keypoints < static_cast<long long>(kDescWarps) * rounds * 148 * kDescCtasPerSm) rounds /= 2;
+    return kDescWarps * rounds;
 }
 constexpr int kEdge = 31;
 constexpr int kResizeTileW = 128, kResizeTileH = 64;  // tallest tile; a job's tile_h may be smaller
@@ -1494,16 +1495,20 @@ __device__ __forceinline__ int rotated_sample(const std::uint8_t* centre, std::u
     return centre[static_cast<int>(__float_as_uint(cy) * stride + __float_as_uint(cx) + bias)];
 }
 
-// One warp per keypoint, keys / kDescWarps keypoints per warp (the block
-// stages the pattern and the disc weights once for its `keys` keypoints): intensity-centroid moments
-// over the radius-15 disc of the unblurred image (lane l sums column l - 15),
-// the angle on lane 0 (float fastAtan2, cos/sin evaluated in double then
-// rounded to float), then lane l packs pattern pairs 8l..8l+7 of the blurred
-// image into descriptor byte l.
-// 8 blocks per SM (32 registers): the kernel waits on scattered patch loads,
-// so resident warps matter more than the few registers it spills.
+// A warp describes keys / kDescWarps keypoints (the block stages the pattern
+// and the disc weights once): first the intensity-centroid moments over the
+// radius-15 disc of the unblurred image of each (kept on lane r for the r-th),
+// then all their angles at once, one per lane (float fastAtan2, cos/sin
+// evaluated in double then rounded to float), then, two keypoints per pass over
+// the pattern, lane l packs pattern pairs 8l..8l+7 of the blurred image into
+// descriptor byte l. An angle takes about 130 instructions, a quarter of a
+// keypoint's when each is computed alone; a pattern entry is 4 of the shared
+// memory wavefronts that bound the kernel.
+// 5 blocks per SM (48 registers): at 8 the two-keypoint pass spills (194 us for
+// 64 pairs of 512x512, K = 2000), at 6 and 4 it takes 172 and 178; one keypoint
+// at a time from moments to samples took 192, this 166.
 template <class Src>
-__global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __grid_constant__ Src src, int keys) {
+__global__ __launch_bounds__(kDescWarps * 32, kDescCtasPerSm) void describe_kernel(const __grid_constant__ Src src, int keys) {
     __shared__ float4 pat[8][32];  // pat[k][l] = pair 8l + k as floats (x0, y0, x1, y1)
     __shared__ DiscTable disc;
     DescribeJob j;
@@ -1534,31 +1539,36 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
     if (local * keys >= count) return;
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int u = lane - 15, au = u < 0 ? -u : u;
     const int pitch = j.pitch, blur_pitch = j.blur_pitch;
-    const std::uint32_t bias = 0u - kRoundBits * (static_cast<std::uint32_t>(blur_pitch) + 1u);
-    for (int index = local * keys + (threadIdx.x >> 5); index < min(count, (local + 1) * keys); index += kDescWarps) {
-        std::uint8_t* row = j.out + static_cast<std::size_t>(base + index) * j.row_stride;
+    const int first = local * keys + (threadIdx.x >> 5);  // the warp's r-th keypoint is first + r * kDescWarps
+    const int rounds = min(keys / kDescWarps, (count - first + kDescWarps - 1) / kDescWarps);
+    if (rounds <= 0) return;
+    // keypoint r on lane r: position (x = -1: too near the edge), moments, then cos and sin
+    int x = -1, y = 0;
+    if (lane < rounds) {
+        const int index = first + lane * kDescWarps;
         const float fx = j.x[index], fy = j.y[index];
-        const int x = __float2int_rn(fx);
-        const int y = __float2int_rn(fy);
-        if (j.level_counts && lane == 0) {
+        x = __float2int_rn(fx);
+        y = __float2int_rn(fy);
+        if (j.level_counts) {
             j.out_x[base + index] = __fmul_rn(fx, j.scale);
             j.out_y[base + index] = __fmul_rn(fy, j.scale);
             if (j.out_response) j.out_response[base + index] = j.response[index];
         }
-        if (x < kEdge || x >= j.width - kEdge || y < kEdge || y >= j.height - kEdge) {
-            row[lane] = 0;
-            continue;
-        }
+        if (x < kEdge || x >= j.width - kEdge || y < kEdge || y >= j.height - kEdge) x = -1;
+    }
+    int m10 = 0, m01 = 0;
+    for (int r = 0; r < rounds; ++r) {
+        const int cx = __shfl_sync(0xffffffffu, x, r), cy = __shfl_sync(0xffffffffu, y, r);
+        if (cx < 0) continue;
         // Moments as exact integer sums over the disc. With aligned rows each
         // lane takes slots lane, lane + 32, ... of the disc's words (four
         // pixels per load, weighted by two byte dot products); otherwise lane
         // l owns column u = l - 15 and walks the 31 rows.
-        int m10 = 0, m01 = 0;
+        int s10 = 0, s01 = 0;
         if (words) {
-            const int xs = x - 15, a = xs & 3;
-            const std::uint8_t* top = j.image + static_cast<std::size_t>(y - 15) * pitch + (xs - a);
+            const int xs = cx - 15, a = xs & 3;
+            const std::uint8_t* top = j.image + static_cast<std::size_t>(cy - 15) * pitch + (xs - a);
 #pragma unroll
             for (int k = 0; k < kDiscSlots / 32; ++k) {
                 const int slot = 32 * k + lane;
@@ -1567,48 +1577,79 @@ __global__ __launch_bounds__(kDescWarps * 32, 8) void describe_kernel(const __gr
                     const std::uint32_t d =
                         __ldg(reinterpret_cast<const unsigned int*>(top + static_cast<std::size_t>(row) * pitch + 4 * word));
                     const uint2 w = disc.w[a][slot];
-                    m10 = dot4_us(d, w.x, m10);
-                    m01 = dot4_us(d, w.y, m01);
+                    s10 = dot4_us(d, w.x, s10);
+                    s01 = dot4_us(d, w.y, s01);
                 }
             }
         } else {
-            const std::uint8_t* centre = j.image + static_cast<std::size_t>(y) * pitch + x;
+            const int u = lane - 15, au = u < 0 ? -u : u;
+            const std::uint8_t* centre = j.image + static_cast<std::size_t>(cy) * pitch + cx;
 #pragma unroll
             for (int v = -15; v <= 15; ++v) {
                 const int av = v < 0 ? -v : v;
                 if (lane < 31 && au <= disc_half_width(av)) {
                     const int val = centre[v * pitch + u];
-                    m10 += u * val;
-                    m01 += v * val;
+                    s10 += u * val;
+                    s01 += v * val;
                 }
             }
         }
-        m10 = __reduce_add_sync(0xffffffffu, m10);
-        m01 = __reduce_add_sync(0xffffffffu, m01);
-        float a = 0.0f, b = 0.0f;
-        if (lane == 0) {
-            const float angle = __fmul_rn(fast_atan2_deg(static_cast<float>(m01), static_cast<float>(m10)),
-                                          0x1.1df46ap-6f);
-            // one sincos for both: it equals cos() and sin() bit for bit on every
-            // float in [0, 6.2832] (all the angles this can produce; checked
-            // exhaustively by tests/test_gpu_sincos.py)
-            double sd, cd;
-            sincos(static_cast<double>(angle), &sd, &cd);
-            a = static_cast<float>(cd);
-            b = static_cast<float>(sd);
+        s10 = __reduce_add_sync(0xffffffffu, s10);
+        s01 = __reduce_add_sync(0xffffffffu, s01);
+        if (lane == r) {
+            m10 = s10;
+            m01 = s01;
         }
-        a = __shfl_sync(0xffffffffu, a, 0);
-        b = __shfl_sync(0xffffffffu, b, 0);
-        const std::uint8_t* smooth = j.blurred + static_cast<std::size_t>(y) * blur_pitch + x;
-        int value = 0;
+    }
+    float a = 0.0f, b = 0.0f;
+    if (lane < rounds) {
+        const float angle = __fmul_rn(fast_atan2_deg(static_cast<float>(m01), static_cast<float>(m10)), 0x1.1df46ap-6f);
+        // one sincos for both: it equals cos() and sin() bit for bit on every
+        // float in [0, 6.2832] (all the angles this can produce; checked
+        // exhaustively by tests/test_gpu_sincos.py)
+        double sd, cd;
+        sincos(static_cast<double>(angle), &sd, &cd);
+        a = static_cast<float>(cd);
+        b = static_cast<float>(sd);
+    }
+    const std::uint32_t bias = 0u - kRoundBits * (static_cast<std::uint32_t>(blur_pitch) + 1u);
+    const auto centre_of = [&](int r, float& ca, float& cb) {  // the blurred centre; a null edge keypoint
+        const int cx = __shfl_sync(0xffffffffu, x, r), cy = __shfl_sync(0xffffffffu, y, r);
+        ca = __shfl_sync(0xffffffffu, a, r);
+        cb = __shfl_sync(0xffffffffu, b, r);
+        return cx < 0 ? nullptr : j.blurred + static_cast<std::size_t>(cy) * blur_pitch + cx;
+    };
+    const auto write = [&](int r, int value) {
+        j.out[static_cast<std::size_t>(base + first + r * kDescWarps) * j.row_stride + lane] = static_cast<std::uint8_t>(value);
+    };
+    for (int r = 0; r < rounds; r += 2) {
+        float a0, b0, a1 = 0.0f, b1 = 0.0f;
+        const std::uint8_t* const c0 = centre_of(r, a0, b0);
+        const std::uint8_t* const c1 = r + 1 < rounds ? centre_of(r + 1, a1, b1) : nullptr;
+        int v0 = 0, v1 = 0;
+        if (c0 && c1) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float4 q = pat[k][lane];
-            const int t0 = rotated_sample(smooth, blur_pitch, bias, q.x, q.y, a, b);
-            const int t1 = rotated_sample(smooth, blur_pitch, bias, q.z, q.w, a, b);
-            value |= (t0 < t1) << k;
+            for (int k = 0; k < 8; ++k) {
+                const float4 q = pat[k][lane];
+                v0 |= (rotated_sample(c0, blur_pitch, bias, q.x, q.y, a0, b0) <
+                       rotated_sample(c0, blur_pitch, bias, q.z, q.w, a0, b0)) << k;
+                v1 |= (rotated_sample(c1, blur_pitch, bias, q.x, q.y, a1, b1) <
+                       rotated_sample(c1, blur_pitch, bias, q.z, q.w, a1, b1)) << k;
+            }
+        } else if (c0 || c1) {
+            const std::uint8_t* const c = c0 ? c0 : c1;
+            const float ca = c0 ? a0 : a1, cb = c0 ? b0 : b1;
+            int v = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float4 q = pat[k][lane];
+                v |= (rotated_sample(c, blur_pitch, bias, q.x, q.y, ca, cb) <
+                      rotated_sample(c, blur_pitch, bias, q.z, q.w, ca, cb)) << k;
+            }
+            (c0 ? v0 : v1) = v;
         }
-        row[lane] = static_cast<std::uint8_t>(value);
+        write(r, v0);
+        if (r + 1 < rounds) write(r + 1, v1);
     }
 }
 

@@ -47,7 +47,7 @@ def test_candidate_counts(ours, k):
     check(ours, rng.integers(0, 256, (331, 350), dtype=np.uint8), 15, k)
 
 
-@pytest.mark.parametrize("k", [9472, 9473, 18945])
+@pytest.mark.parametrize("k", [5919, 9472, 9473, 11839, 11840, 18945, 23680])
 def test_describe_rounds(ours, k):
     rng = np.random.default_rng(5)
     check(ours, rng.integers(0, 256, (900, 901), dtype=np.uint8), 10, k)
