@@ -286,31 +286,61 @@ __device__ __forceinline__ int fast_score(const std::uint8_t* p, int stride, int
     return score > thr ? score - 1 : 0;
 }
 
-// Compass test of two pixels in 16-bit lanes (values 0..255), a necessary
-// condition for a FAST-9 corner: every 9-pixel arc of the circle holds one of
-// the compass pixels s0, s8 (3 below, 3 above) and one of s4, s12 (3 right,
-// 3 left), so an arc brighter than v + t needs
-// min(max(s0, s8), max(s4, s12)) >= v + t + 1 and one darker than v - t needs
-// max(min(s0, s8), min(s4, s12)) <= v - t - 1. x >= y per lane is the top bit
-// of (x | 0x8000) - y, with no borrow between lanes for x, y < 0x8000.
-// thr1 = (t + 1) in both lanes. Returns 0x8000 per passing lane.
-__device__ __forceinline__ std::uint32_t compass_pass2(std::uint32_t v, std::uint32_t s0, std::uint32_t s4,
-                                                       std::uint32_t s8, std::uint32_t s12, std::uint32_t thr1) {
-    const std::uint32_t hi = __vminu2(__vmaxu2(s0, s8), __vmaxu2(s4, s12));
-    const std::uint32_t lo = __vmaxu2(__vminu2(s0, s8), __vminu2(s4, s12));
-    constexpr std::uint32_t kTop = 0x80008000u;
-    const std::uint32_t bright = ((hi | kTop) - (v + thr1)) & kTop;  // min(...) >= v + t + 1
-    const std::uint32_t dark = ((v | kTop) - (lo + thr1)) & kTop;    // v >= max(...) + t + 1
-    return bright | dark;
+// Compass test of four pixels, a necessary condition for a FAST-9 corner: every
+// 9-pixel arc of the circle holds one of the compass pixels s0, s8 (3 below, 3
+// above) and one of s4, s12 (3 right, 3 left), so an arc brighter than v + t
+// needs hi = min(max(s0, s8), max(s4, s12)) >= v + t + 1 and one darker than v -
+// t needs lo = max(min(s0, s8), min(s4, s12)) <= v - t - 1.
+// Two pixels per word, their bytes in the high bytes of the 16-bit lanes: the
+// minima and maxima of such lanes are right in the high byte whatever the low
+// bytes hold, so the odd pixels' words are taken as loaded, the even pixels'
+// shifted left by 8, and only hi, lo and v are masked. In the masked lanes
+// hi + 0x8000 - v - (t + 1) and v + 0x8000 - lo - (t + 1) have their top bit
+// set exactly when the test passes, with no borrow between lanes.
+// The kernel is bound by the ALU pipe and by issue slots: the sums are
+// multiply-adds, which run on the FMA pipe (`one` and `minus` are 1 and -1
+// where the compiler cannot see them). FAST of 64 pairs at 512x512 with 8
+// layers: 252 -> 240 us with this test, 221 with eight pixels per thread (the
+// list bookkeeping once per eight), 217 with the staging's chunk per thread
+// fixed; 30 mixed pairs: 1300, 1227, 1143, 1120 us.
+struct Compass {
+    std::uint32_t one, minus, top;  // top = 0x80008000 - (t + 1) in both lanes
+};
+
+__device__ __forceinline__ std::uint32_t mad32(std::uint32_t a, std::uint32_t b, std::uint32_t c) {
+    std::uint32_t d;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
 }
 
-// Shared-memory tile of the FAST kernel: rows of kInStride bytes holding
-// image columns x0-16 .. x0+79; the halo-4 column c (image x0-4+c) is at byte
-// c + kInOff. Scores: rows of kScStride bytes, position (r, c) = image
-// (y0-1+r, x0-1+c).
-constexpr int kInStride = 96, kInOff = 12;
-constexpr int kScStride = 68;
-constexpr int kScGroups = kScStride / 4;  // groups of 4 positions per score row
+// Top bits of the lanes whose pixel passes; s0 .. s12 and v with the pixels in
+// the high bytes, v with clear low bytes shifted down (masked).
+__device__ __forceinline__ std::uint32_t compass_lanes(std::uint32_t v, std::uint32_t s0, std::uint32_t s4,
+                                                       std::uint32_t s8, std::uint32_t s12, const Compass& k) {
+    const std::uint32_t hi = __byte_perm(__vminu2(__vmaxu2(s0, s8), __vmaxu2(s4, s12)), 0, 0x4341);
+    const std::uint32_t lo = __byte_perm(__vmaxu2(__vminu2(s0, s8), __vminu2(s4, s12)), 0, 0x4341);
+    return mad32(hi, k.one, mad32(v, k.minus, k.top)) | mad32(lo, k.minus, mad32(v, k.one, k.top));
+}
+
+// Survivor bits 0 .. 3 of the four pixels of word v, with the words left and
+// right of it and those three rows below and above; other bits are undefined.
+__device__ __forceinline__ unsigned compass_bits(std::uint32_t l, std::uint32_t v, std::uint32_t r, std::uint32_t s0,
+                                                 std::uint32_t s8, const Compass& k) {
+    const std::uint32_t odd = compass_lanes(__byte_perm(v, 0, 0x4341), s0, __funnelshift_r(v, r, 24), s8,
+                                            __funnelshift_r(l, v, 8), k);
+    const std::uint32_t even = compass_lanes(v & 0x00ff00ffu, mad32(s0, 256u, 0u), __funnelshift_r(v, r, 16),
+                                             mad32(s8, 256u, 0u), l, k);
+    // bits 14, 15 (pixels 0, 1) and 30, 31 (pixels 2, 3), then together
+    const std::uint32_t m = (((even >> 1) & 0x40004000u) | (odd & 0x80008000u)) >> 14;
+    return m | (m >> 14);
+}
+
+constexpr int kInStride = 96;
+// Score rows hold columns x0-4 .. x0+67 of a tile at x0: words aligned with the
+// staged bytes (score column c is staged byte kInOff + c). The tile and its
+// 1-pixel ring are columns kScRing .. kScRing + kFastScW - 1.
+constexpr int kInOff = 12, kScStride = 72, kScRing = 3;
+constexpr int kScGroups = kScStride / 8;  // groups of 8 positions per score row
 
 // Bytes k of wa and wb as a float pair (rows r, r + 1 of one column), each
 // exact: the float 2^23 + b (byte b placed in the low mantissa) minus 2^23.
@@ -392,17 +422,21 @@ __device__ __forceinline__ void stage_fast_tile(const DetectJob& j, int local, s
     const int y0 = org.y, x0 = org.x;
     const bool vec = ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 15) == 0;
     if (vec) {
-        constexpr int kChunks = kInStride / 16;  // 6 per row
-        for (int i = tid; i < kFastInH * kChunks; i += kFastThreads) {
-            const int r = i / kChunks, q = i - r * kChunks;
-            const int gy = min(max(y0 - 4 + r, 0), H - 1);
-            const int cx = x0 - 16 + 16 * q;
-            const int limit = gy == H - 1 ? W : j.pitch;  // bytes of the row that may be read
-            const std::uint8_t* row = j.image + static_cast<std::size_t>(gy) * j.pitch;
-            if (cx >= 0 && cx + 16 <= limit) {
-                cp_async16(&in[r][16 * q], row + cx);
-            } else if (cx >= 0 && cx < W) {
-                for (int b = 0; b < 16 && cx + b < W; ++b) in[r][16 * q + b] = row[cx + b];
+        // thread (r, q): chunk q of rows r, r + 42
+        constexpr int kChunks = kInStride / 16, kRows = kFastThreads / kChunks;  // 6, 42
+        const int r0 = tid / kChunks, q = tid - r0 * kChunks, cx = x0 - 16 + 16 * q;
+        if (r0 < kRows && cx >= 0 && cx < W) {
+            const std::uint8_t* const column = j.image + cx;
+#pragma unroll
+            for (int r = r0; r < kFastInH; r += kRows) {
+                const int gy = min(max(y0 - 4 + r, 0), H - 1);
+                const std::uint8_t* from = column + static_cast<std::size_t>(gy) * j.pitch;
+                // bytes of the row that may be read: the pitch, the width on the last row
+                if (cx + 16 <= (gy == H - 1 ? W : j.pitch)) {
+                    cp_async16(&in[r][16 * q], from);
+                } else {
+                    for (int b = 0; b < 16 && cx + b < W; ++b) in[r][16 * q + b] = from[b];
+                }
             }
         }
     } else {
@@ -419,7 +453,7 @@ __device__ __forceinline__ void stage_fast_tile(const DetectJob& j, int local, s
 // t of `total` is looked up through the source's kFastKind entries), while
 // the next tile's bytes are copied into the other half of a double buffer.
 // The jobs of the current and the next tile sit in shared memory. Per tile:
-//   1. the compass test on the tile plus a 1-pixel ring, 4 positions per
+//   1. the compass test on the tile plus a 1-pixel ring, 8 positions per
 //      thread in 16-bit lanes; groups with a survivor are listed;
 //   2. the groups are expanded into one list of survivor positions, scored
 //      on full warps (every other position scores 0);
@@ -435,7 +469,7 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
     static_assert(sizeof(DetectJob) % 16 == 0, "jobs are copied in 16-byte chunks");
     __shared__ __align__(16) std::uint8_t in[2][kFastInH][kInStride];
     __shared__ __align__(16) std::uint8_t sc[kFastScH][kScStride];
-    __shared__ std::uint16_t cand[kFastScH * kScGroups];
+    __shared__ std::uint32_t cand[kFastScH * kScGroups];
     __shared__ std::uint16_t pos[kFastScH * kFastScW];  // survivor positions r * kScStride + c
     __shared__ std::uint32_t hist[256];
     __shared__ DetectJob jobs[2];  // jobs of the tiles in in[0] and in[1] (kept here, not in registers)
@@ -448,6 +482,8 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
     // the current one is copied into shared memory asynchronously while the
     // current tile is tested, and the queue index and map entry of the tile
     // after that are fetched a tile ahead, so no thread waits on the lookup.
+    std::uint32_t one = 1u, minus = ~0u;
+    asm("" : "+r"(one), "+r"(minus));  // see Compass
     const std::uint32_t* map = fast_map(src);
     if (map) total = min(total, fast_map_tiles(src));
     hist[tid] = 0;
@@ -494,46 +530,34 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
                 next = t;
             }
         }
-        // 1. compass test: thread (q, rb) takes positions 4q .. 4q+3 of rows rb,
-        // rb + 15, rb + 30, ...; groups with a survivor are listed as
-        // (group << 4 | survivor bits)
-        const std::uint32_t thr1 = static_cast<std::uint32_t>(j.threshold + 1) * 0x00010001u;
+        // 1. compass test: thread (q, rb) takes positions 8q .. 8q+7 of rows rb,
+        // rb + 28, rb + 56; groups with a survivor are listed as
+        // (group << 8 | survivor bits)
+        const Compass compass{one, minus, 0x80008000u - static_cast<std::uint32_t>(j.threshold + 1) * 0x00010001u};
         {
-            constexpr int kRowSets = 256 / kScGroups;  // 15
-            const int q = tid % kScGroups, rb = tid / kScGroups, c = 4 * q;
+            constexpr int kRowSets = 256 / kScGroups;  // 28
+            const int q = tid % kScGroups, rb = tid / kScGroups, c = 8 * q;
             unsigned colmask = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int gx = x0 - 1 + c + k;
-                if (c + k < kFastScW && gx >= 3 && gx < W - 3) colmask |= 1u << k;
+            for (int k = 0; k < 8; ++k) {
+                const int gx = x0 - 1 - kScRing + c + k;
+                if (c + k >= kScRing && c + k < kScRing + kFastScW && gx >= 3 && gx < W - 3) colmask |= 1u << k;
             }
             for (int it = 0; it < (kFastScH + kRowSets - 1) / kRowSets; ++it) {  // same trip count everywhere
                 const int r = rb + it * kRowSets;
                 unsigned bits = 0;
                 if (rb < kRowSets && r < kFastScH) {
-                    *reinterpret_cast<std::uint32_t*>(&sc[r][c]) = 0u;
+                    *reinterpret_cast<uint2*>(&sc[r][c]) = make_uint2(0u, 0u);
                     const int gy = y0 - 1 + r;
                     if (colmask && gy >= 3 && gy < H - 3) {
-                        const int w = q + 3;  // word holding halo columns c .. c+3 (bytes c+12 .. c+15)
-                        const auto* mid = reinterpret_cast<const std::uint32_t*>(&cur[r + 3][0]);
-                        const auto* bot = reinterpret_cast<const std::uint32_t*>(&cur[r + 6][0]);
-                        const auto* top = reinterpret_cast<const std::uint32_t*>(&cur[r][0]);
-                        const std::uint32_t a0 = mid[w], a1 = mid[w + 1], a2 = mid[w + 2];
-                        const std::uint32_t v = __funnelshift_r(a0, a1, 24);   // centres, halo columns c+3 .. c+6
-                        const std::uint32_t s12 = a0;                          // 3 left
-                        const std::uint32_t s4 = __funnelshift_r(a1, a2, 16);  // 3 right
-                        const std::uint32_t s0 = __funnelshift_r(bot[w], bot[w + 1], 24);  // 3 down
-                        const std::uint32_t s8 = __funnelshift_r(top[w], top[w + 1], 24);  // 3 up
-                        const std::uint32_t plo =
-                            compass_pass2(__byte_perm(v, 0, 0x4140), __byte_perm(s0, 0, 0x4140),
-                                          __byte_perm(s4, 0, 0x4140), __byte_perm(s8, 0, 0x4140),
-                                          __byte_perm(s12, 0, 0x4140), thr1);
-                        const std::uint32_t phi =
-                            compass_pass2(__byte_perm(v, 0, 0x4342), __byte_perm(s0, 0, 0x4342),
-                                          __byte_perm(s4, 0, 0x4342), __byte_perm(s8, 0, 0x4342),
-                                          __byte_perm(s12, 0, 0x4342), thr1);
-                        bits = (((plo >> 15) & 1u) | ((plo >> 30) & 2u) | ((phi >> 13) & 4u) | ((phi >> 28) & 8u)) &
-                               colmask;
+                        const int w = 2 * q + kInOff / 4;  // the first centres' word
+                        const auto* mid = reinterpret_cast<const std::uint32_t*>(&cur[r + 3][0]) + w;
+                        const auto* bot = reinterpret_cast<const std::uint32_t*>(&cur[r + 6][0]) + w;
+                        const auto* top = reinterpret_cast<const std::uint32_t*>(&cur[r][0]) + w;
+                        const std::uint32_t m0 = mid[-1], m1 = mid[0], m2 = mid[1], m3 = mid[2];
+                        const unsigned b0 = compass_bits(m0, m1, m2, bot[0], top[0], compass);
+                        const unsigned b1 = compass_bits(m1, m2, m3, bot[1], top[1], compass);
+                        bits = ((b0 & 0xfu) | (b1 << 4)) & colmask;
                     }
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, bits != 0);
@@ -541,8 +565,7 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
                 if (lane == 0 && m) base = atomicAdd(&n_cand, __popc(m));
                 base = __shfl_sync(0xffffffffu, base, 0);
                 if (bits)
-                    cand[base + __popc(m & ((1u << lane) - 1u))] =
-                        static_cast<std::uint16_t>(((r * kScGroups + q) << 4) | bits);
+                    cand[base + __popc(m & ((1u << lane) - 1u))] = (static_cast<unsigned>(r * kScGroups + q) << 8) | bits;
             }
         }
         if (tid == 0 && map) cp_async_wait_all();  // the next tile's job
@@ -562,9 +585,9 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
             unsigned bits = 0;
             int pos0 = 0;
             if (i < nc) {
-                const int e = cand[i];
-                const int grp = e >> 4, r = grp / kScGroups, c0 = 4 * (grp - r * kScGroups);
-                bits = e & 0xfu;
+                const int e = static_cast<int>(cand[i]);
+                const int grp = e >> 8, r = grp / kScGroups, c0 = 8 * (grp - r * kScGroups);
+                bits = e & 0xffu;
                 pos0 = r * kScStride + c0;
             }
             const int cnt = __popc(bits);
@@ -585,7 +608,7 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
         for (int k = tid; k < np; k += kFastThreads) {
             const int e = pos[k];
             const int r = e / kScStride, c = e - r * kScStride;
-            sc[r][c] = static_cast<std::uint8_t>(fast_score(&cur[r + 3][c + 3 + kInOff], kInStride, j.threshold));
+            sc[r][c] = static_cast<std::uint8_t>(fast_score(&cur[r + 3][c + kInOff], kInStride, j.threshold));
         }
         __syncthreads();
         // 3. strict 3x3 maxima inside the 31-pixel edge margin: only listed
@@ -600,8 +623,8 @@ __global__ __launch_bounds__(kFastThreads, kFastCtasPerSm) void fast_kernel(cons
             if (k < np) {
                 const int e = pos[k];
                 const int r = e / kScStride, c = e - r * kScStride;
-                const int gy = y0 - 1 + r, gx = x0 - 1 + c;
-                if (r >= 1 && r <= kFastTileH && c >= 1 && c <= kFastTileW && gy >= kEdge && gy < H - kEdge &&
+                const int gy = y0 - 1 + r, gx = x0 - 1 - kScRing + c;
+                if (r >= 1 && r <= kFastTileH && c >= kScRing + 1 && c <= kScRing + kFastTileW && gy >= kEdge && gy < H - kEdge &&
                     gx >= kEdge && gx < W - kEdge) {
                     const unsigned s0 = sc[r][c];
                     if (s0 && s0 > sc[r - 1][c - 1] && s0 > sc[r - 1][c] && s0 > sc[r - 1][c + 1] &&
