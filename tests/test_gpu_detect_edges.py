@@ -1,12 +1,13 @@
 """S2/S3 where the selection, the rank sort, the Harris loads, the describe
-rounds and the blur change path, bit for bit against the oracle: tie counts
+rounds, the blur, FAST and the resize change path, bit for bit against the oracle: tie counts
 around the ranked and the listed ties, candidate counts around the rank
 kernel's blocks and tiles, aligned and odd pitches, saturated windows."""
 import numpy as np
 import pytest
 
-from oracle import s2s3
+from oracle import pyramid, s2s3
 from tests import gpu_util as G
+from tests.test_gpu_pyramid import run_pyramid
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +72,17 @@ def test_saturated_blur(ours):
     g[20:30, 20:30] = 0
     _, _, blurred, _ = G.detect_describe(ours, g, 20, 50)
     assert np.array_equal(blurred, s2s3.blur(g)) and blurred.max() == 255
+
+
+@pytest.mark.parametrize("w,h,factor", [(134, 134, 1.0001), (135, 147, 1.2), (154, 160, 1.2), (155, 163, 1.2),
+                                        (257, 199, 1.44), (263, 258, 1.05), (390, 141, 1.2)])
+@pytest.mark.parametrize("aligned", [True, False], ids=["pitch16", "pitch-odd"])
+def test_layer_edges(ours, w, h, factor, aligned):
+    """FAST groups of eight and resize bands at the edges of their tiles
+    (64 pixels from the rim of 3, 128 columns, 16 rows), on noise, where every
+    pixel of a layer decides about corners: positions, scores and order."""
+    rng = np.random.default_rng(w * 1000 + h)
+    gray = rng.integers(0, 256, (h, w), dtype=np.uint8)
+    st, kp, _ = run_pyramid(gray, 12, 3000, 3, factor, pad=(-w) % 16 + 16 if aligned else None)
+    assert st == 0
+    assert np.array_equal(kp, pyramid.detect_and_describe(gray, 12, 3000, 3, factor)[0])
