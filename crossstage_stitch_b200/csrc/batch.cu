@@ -673,7 +673,7 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
         s2s3::blur_tiles_kernel<DesSrc, true>
             <<<static_cast<int>(std::min<std::size_t>(
                    blur_total, kSmCount * (tuning.blur_ctas_per_sm ? tuning.blur_ctas_per_sm : s2s3::kBlurCtasPerSm))),
-               256, 0, s>>>(des, at<uint2>(ws, blur_list), q + 1, 0);
+               s2s3::kBlurThreads, 0, s>>>(des, at<uint2>(ws, blur_list), q + 1, 0);
     mark();
     if (go(des_blocks[s2s3::kDescKind]))
         s2s3::describe_kernel<DesSrc><<<des_blocks[s2s3::kDescKind], s2s3::kDescWarps * 32, 0, s>>>(des, desc_keys);
@@ -781,7 +781,7 @@ int stitch_batch_create_tuned(int n_pairs, const stitch_pair_desc* pairs, const 
     if (tuning) {
         const auto& t = *tuning;
         const bool ok = t.fast_ctas_per_sm >= 0 && t.fast_ctas_per_sm <= stitch::b200::s2s3::kFastCtasPerSm &&
-                        t.blur_ctas_per_sm >= 0 && t.blur_ctas_per_sm <= stitch::b200::s2s3::kBlurCtasPerSm &&
+                        t.blur_ctas_per_sm >= 0 && t.blur_ctas_per_sm <= stitch::b200::s2s3::kBlurMaxCtasPerSm &&
                         (t.matcher == 0 || stitch::b200::s4k::valid_matcher(t.matcher - 1)) &&
                         (t.search_hpw == 0 || t.search_hpw == 4 || t.search_hpw == 8 || t.search_hpw == 16 ||
                          t.search_hpw == 32) &&

@@ -250,7 +250,7 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
         else
             launch_chained(sort_topk_kernel<DetSrc>, blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream, det);
         launches += 4;
-        launch_chained(blur_tiles_kernel<DesSrc, true>, std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), 256, 0, stream,
+        launch_chained(blur_tiles_kernel<DesSrc, true>, std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), kBlurThreads, 0, stream,
             des, at_offset<uint2>(ws, l.blur_list), queue + 1, 0);
         ++launches;
     }

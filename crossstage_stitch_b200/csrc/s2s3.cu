@@ -178,7 +178,7 @@ Status describe(const ImageView& image, const Keypoints& kp, const Descriptors& 
     if (kp.capacity == 0) return record(e_blur, stream) ? Status::OK : Status::CUDA_ERROR;
     using Src = OneJob<DescribeJob>;
     const Src src{make_describe_job(image, kp, out, ws, l)};
-    launch_chained(blur_tiles_kernel<Src, false>, std::min(l.tiles, kSmCount * kBlurCtasPerSm), 256, 0, stream, src, nullptr, nullptr, l.tiles);
+    launch_chained(blur_tiles_kernel<Src, false>, std::min(l.tiles, kSmCount * kBlurCtasPerSm), kBlurThreads, 0, stream, src, nullptr, nullptr, l.tiles);
     if (!record(e_blur, stream)) return Status::CUDA_ERROR;
     const int keys = desc_keys(kp.capacity);
     launch_chained(describe_kernel<Src>, ceil_div(kp.capacity, keys), kDescWarps * 32, 0, stream, src, keys);

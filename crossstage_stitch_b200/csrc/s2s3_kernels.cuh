@@ -354,15 +354,18 @@ __device__ __forceinline__ float2 byte_pair(std::uint32_t wa, std::uint32_t wb, 
 // blur in one instruction stream.
 __device__ __forceinline__ float2 tap_pair(int t) { return make_float2(blur_tap(t), blur_tap(t)); }
 
-// Tap t of a pair of sums. Packed: the sm_100 packed FP32 multiply and add,
-// which ptxas may join into one fused operation per lane. Scalar: every
-// product and sum rounded on its own, as the reference does.
-template <bool kPacked> __device__ __forceinline__ float2 first_tap(float2 v) {
-    return kPacked ? __fmul2_rn(tap_pair(0), v)
-                   : make_float2(__fmul_rn(blur_tap(0), v.x), __fmul_rn(blur_tap(0), v.y));
+// Taps 0 and 1, then tap t, of a pair of sums. Packed: one rounding less per
+// tap, in the order that the pyramid and batched paths have always had (the
+// compiler joined their packed products and sums so; written out, the bytes no
+// longer depend on it). Scalar: every product and sum rounded on its own, as
+// the reference does. On noise 3 pixels of a million differ by one.
+template <bool kPacked> __device__ __forceinline__ float2 first_taps(float2 v0, float2 v1) {
+    return kPacked ? __ffma2_rn(tap_pair(0), v0, __fmul2_rn(tap_pair(1), v1))
+                   : make_float2(__fadd_rn(__fmul_rn(blur_tap(0), v0.x), __fmul_rn(blur_tap(1), v1.x)),
+                                 __fadd_rn(__fmul_rn(blur_tap(0), v0.y), __fmul_rn(blur_tap(1), v1.y)));
 }
 template <bool kPacked> __device__ __forceinline__ float2 next_tap(float2 sum, int t, float2 v) {
-    return kPacked ? __fadd2_rn(sum, __fmul2_rn(tap_pair(t), v))
+    return kPacked ? __ffma2_rn(tap_pair(t), v, sum)
                    : make_float2(__fadd_rn(sum.x, __fmul_rn(blur_tap(t), v.x)),
                                  __fadd_rn(sum.y, __fmul_rn(blur_tap(t), v.y)));
 }
@@ -1269,17 +1272,47 @@ __global__ __launch_bounds__(256, 6) void resize_kernel(const __grid_constant__ 
 // copies for 16-byte aligned images, reflected byte loads otherwise. The
 // per-image call used to have a kernel with byte-wise loads of its own
 // (640x480: 14 -> 5 us).
+// Bound by issue slots and shared-memory wavefronts alike (66 and 64 % busy; the
+// packed sums alone would take 45 %). 128 images of 512x512 with 8 layers: 160 us
+// with the job, the origin and the halo made by every thread and 2x4 outputs
+// per item of either pass; 143 with the descriptions, 8x2 and 4x4 items; 133
+// with 5 blocks per SM instead of 6 (spills at 40 registers); 129 with the
+// swizzled rows, the list read ahead and one row item per thread. 4 blocks: 127.
+// 30 mixed pairs: 411 -> 330 us.
+// One thread for each item of the rows pass (35 row pairs x 8 groups of 8
+// columns = 280); the columns pass has 256, and the ninth warp makes the next
+// but one tile's description beside it.
+constexpr int kBlurThreads = 288;
 constexpr int kBlurInH = kBlurTileH + 8;  // staged rows of a blur tile: rows y0-4 .. y0+kBlurTileH+3 (halo 3, rounded to 4)
 
-// Origin of blur tile `tile` of job j.
-__device__ __forceinline__ void blur_tile_origin(const DescribeJob& j, unsigned tile, int* x0, int* y0) {
-    const int tiles_x = (j.width + kBlurTileW - 1) / kBlurTileW;
-    *y0 = (static_cast<int>(tile) / tiles_x) * kBlurTileH;
-    *x0 = (static_cast<int>(tile) % tiles_x) * kBlurTileW;
-}
+// What the threads of a block need of a tile, in shared memory: one thread
+// reads the list, the job and makes the origin, a tile ahead of the staging.
+struct BlurTile {
+    const std::uint8_t* image;
+    std::uint8_t* blurred;  // the tile's first pixel
+    int width, height, pitch, blur_pitch;
+    int x0, y0;
+    bool aligned;  // 16-byte copies and word-wise halo columns
+    bool whole;    // 64x64 pixels inside the image, stored as words
+};
 
-__device__ __forceinline__ bool aligned16(const DescribeJob& j) {
-    return ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 15) == 0;
+template <class Src>
+__device__ __forceinline__ void blur_tile_at(const Src& src, uint2 e, BlurTile* t) {
+    const DescribeJob j = src.at(static_cast<int>(e.x));
+    const int tiles_x = (j.width + kBlurTileW - 1) / kBlurTileW;
+    const int y0 = (static_cast<int>(e.y) / tiles_x) * kBlurTileH, x0 = (static_cast<int>(e.y) % tiles_x) * kBlurTileW;
+    t->image = j.image;
+    t->blurred = j.blurred + static_cast<std::size_t>(y0) * j.blur_pitch + x0;
+    t->width = j.width;
+    t->height = j.height;
+    t->pitch = j.pitch;
+    t->blur_pitch = j.blur_pitch;
+    t->x0 = x0;
+    t->y0 = y0;
+    // three columns are mirrored about the first and the last one
+    t->aligned = ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 15) == 0 && j.width >= 4;
+    t->whole = x0 + kBlurTileW <= j.width && y0 + kBlurTileH <= j.height &&
+               ((reinterpret_cast<std::uintptr_t>(j.blurred) | static_cast<std::uintptr_t>(j.blur_pitch)) & 3) == 0;
 }
 
 // Asynchronous staging of a blur tile of a 16-byte aligned image: row r of
@@ -1288,19 +1321,19 @@ __device__ __forceinline__ bool aligned16(const DescribeJob& j) {
 // (inside the width on the last image row) are 16-byte copies, a chunk
 // straddling the end of the last row is copied byte by byte; the reflected
 // halo columns are filled by blur_fix_columns once the copies are complete.
-__device__ __forceinline__ void blur_stage_async(const DescribeJob& j, int x0, int y0, std::uint8_t (*in)[kInStride]) {
-    const int tid = threadIdx.x;
-    constexpr int kChunks = kInStride / 16;
-    for (int i = tid; i < kBlurInH * kChunks; i += 256) {
-        const int r = i / kChunks, q = i - r * kChunks;
-        const int gy = reflect101(y0 - 4 + r, j.height);
-        const int cx = x0 - 16 + 16 * q;
-        const int limit = gy == j.height - 1 ? j.width : j.pitch;
-        const std::uint8_t* row = j.image + static_cast<std::size_t>(gy) * j.pitch;
-        if (cx >= 0 && cx + 16 <= limit) {
-            cp_async16(&in[r][16 * q], row + cx);
-        } else if (cx >= 0 && cx < j.width) {
-            for (int b = 0; b < 16 && cx + b < j.width; ++b) in[r][16 * q + b] = row[cx + b];
+// A thread has the same chunk of rows r and r + 48 in every tile.
+__device__ __forceinline__ void blur_stage_async(const BlurTile& t, std::uint8_t (*in)[kInStride]) {
+    constexpr int kChunks = kInStride / 16, kRows = kBlurThreads / kChunks;  // 6, 48
+    const int r0 = static_cast<int>(threadIdx.x) / kChunks, q = static_cast<int>(threadIdx.x) - r0 * kChunks;
+    const int cx = t.x0 - 16 + 16 * q;
+    if (cx < 0 || cx >= t.width) return;
+    for (int r = r0; r < kBlurInH; r += kRows) {
+        const int gy = reflect101(t.y0 - 4 + r, t.height);
+        const std::uint8_t* p = t.image + static_cast<std::size_t>(gy) * t.pitch + cx;
+        if (cx + 16 <= (gy == t.height - 1 ? t.width : t.pitch)) {
+            cp_async16(&in[r][16 * q], p);
+        } else {
+            for (int b = 0; b < 16 && cx + b < t.width; ++b) in[r][16 * q + b] = p[b];
         }
     }
 }
@@ -1308,63 +1341,64 @@ __device__ __forceinline__ void blur_stage_async(const DescribeJob& j, int x0, i
 // Whether the 7x7 blur of the tile at x0 reads columns outside the image.
 __device__ __forceinline__ bool blur_needs_columns(int x0, int W) { return x0 < 3 || x0 + kBlurTileW + 3 > W; }
 
-// Reflect-101 halo columns of a staged tile: column -k is column k, column
-// W - 1 + k is column W - 1 - k (k = 1..3), copied inside `in`.
+// Reflect-101 halo columns of a staged tile of an image of 4 columns or more:
+// column -k is column k, column W - 1 + k is column W - 1 - k (k = 1..3),
+// copied inside `in` (sources are interior columns, never written here).
 __device__ __forceinline__ void blur_fix_columns(int x0, int W, std::uint8_t (*in)[kInStride]) {
-    for (int i = threadIdx.x; i < kBlurInH * 6; i += 256) {  // sources are interior columns, never written here
-        const int r = i / 6, k = i % 6;
-        const int off = x0 - 16;  // column of byte 0
-        int dst, srcc;
-        if (k < 3) {  // left edge
-            dst = -(k + 1);
-            srcc = k + 1;
-        } else {      // right edge
-            dst = W - 1 + (k - 2);
-            srcc = W - 1 - (k - 2);
-        }
-        const int db = dst - off, sb = srcc - off;
-        if (db >= 0 && db < kInStride && sb >= 0 && sb < kInStride && dst >= x0 - 3 && dst <= x0 + kBlurTileW + 2)
-            in[r][db] = in[r][sb];
+    const int tid = threadIdx.x;
+    static_assert(kBlurInH <= 128, "a side per half of the block");
+    if (tid < kBlurInH) {
+        auto* w = reinterpret_cast<std::uint32_t*>(in[tid]);
+        if (x0 < 3) w[3] = __byte_perm(w[4], 0u, 0x1230);  // bytes 13..15 are bytes 19..17
+    } else if (tid >= 128 && tid < 128 + kBlurInH && x0 + kBlurTileW + 3 > W) {
+        std::uint8_t* b = &in[tid - 128][16 + W - x0];  // column W
+        const std::uint8_t c0 = b[-2], c1 = b[-3], c2 = b[-4];
+        b[0] = c0;
+        b[1] = c1;
+        b[2] = c2;
     }
 }
 
-constexpr int kBlurCtasPerSm = 6;  // resident blur blocks per SM; the persistent grid is 148 x this
+// Where the four sums of columns 4c .. 4c+3 of a row stand: a thread of the
+// rows pass writes 2q and 2q+1, one of the columns pass reads one, and eight
+// lanes in turn meet no bank twice.
+__device__ __forceinline__ int blur_quad(int c) { return c ^ (c >> 3); }
+
+constexpr int kBlurCtasPerSm = 5;     // resident blur blocks per SM; the persistent grid is 148 x this
+constexpr int kBlurMaxCtasPerSm = 6;  // the largest grid a tuning may ask for
 template <class Src, bool kPacked>
-__global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const __grid_constant__ Src src, const uint2* list,
+__global__ __launch_bounds__(kBlurThreads, kBlurCtasPerSm) void blur_tiles_kernel(const __grid_constant__ Src src, const uint2* list,
                                                             const std::uint32_t* count, int all_tiles) {
     wait_for_previous();
     __shared__ __align__(16) std::uint8_t in2[2][kBlurInH][kInStride];  // rows y0-4 .., columns x0-16 ..
     __shared__ __align__(16) float rows[kBlurTileH + 6][kBlurTileW];
+    __shared__ BlurTile info[3];
     __shared__ std::size_t row_at[kBlurInH];
     __shared__ int col_at[kInStride];
     const int tid = threadIdx.x;
     const int n = list ? static_cast<int>(*count) : all_tiles;
+    const int grid = gridDim.x;
     const auto tile_at = [&](int i) { return list ? list[i] : make_uint2(0u, static_cast<unsigned>(i)); };
+    if (static_cast<int>(blockIdx.x) >= n) return;
+    if (tid == 0) blur_tile_at(src, tile_at(blockIdx.x), &info[0]);
+    if (tid == 32 && static_cast<int>(blockIdx.x) + grid < n) blur_tile_at(src, tile_at(blockIdx.x + grid), &info[1]);
+    __syncthreads();
     // tiles of aligned images are copied asynchronously, the next one while this one is blurred
-    auto prefetch = [&](int i, std::uint8_t (*dst)[kInStride]) {
-        const uint2 e = tile_at(i);
-        const DescribeJob jn = src.at(static_cast<int>(e.x));
-        if (!aligned16(jn)) return;
-        int x0, y0;
-        blur_tile_origin(jn, e.y, &x0, &y0);
-        blur_stage_async(jn, x0, y0, dst);
-    };
-    int buf = 0;
-    if (static_cast<int>(blockIdx.x) < n) prefetch(blockIdx.x, in2[0]);
-    for (int i = blockIdx.x; i < n; i += gridDim.x, buf ^= 1) {
+    if (info[0].aligned) blur_stage_async(info[0], in2[0]);
+    const auto entry_at = [&](int i) { return i < n ? tile_at(i) : make_uint2(0u, 0u); };
+    uint2 ahead = entry_at(blockIdx.x + 2 * grid);
+    int buf = 0, slot = 0;
+    for (int i = blockIdx.x; i < n; i += grid, buf ^= 1) {
         std::uint8_t (*in)[kInStride] = in2[buf];
-        const uint2 e = tile_at(i);
-        const DescribeJob j = src.at(static_cast<int>(e.x));
-        const int W = j.width, H = j.height;
-        int x0, y0;
-        blur_tile_origin(j, e.y, &x0, &y0);
-        if (!aligned16(j)) {  // unaligned image: reflected byte loads
-            if (tid < kBlurInH) row_at[tid] = static_cast<std::size_t>(reflect101(y0 - 4 + tid, H)) * j.pitch;
-            else if (tid < kBlurInH + kInStride) col_at[tid - kBlurInH] = reflect101(x0 - 16 + (tid - kBlurInH), W);
+        const BlurTile& t = info[slot];
+        const int next = slot == 2 ? 0 : slot + 1, after = next == 2 ? 0 : next + 1;
+        if (!t.aligned) {  // unaligned image: reflected byte loads
+            if (tid < kBlurInH) row_at[tid] = static_cast<std::size_t>(reflect101(t.y0 - 4 + tid, t.height)) * t.pitch;
+            else if (tid < kBlurInH + kInStride) col_at[tid - kBlurInH] = reflect101(t.x0 - 16 + (tid - kBlurInH), t.width);
             __syncthreads();
-            for (int k = tid; k < kBlurInH * (kInStride / 4); k += 256) {
+            for (int k = tid; k < kBlurInH * (kInStride / 4); k += kBlurThreads) {
                 const int r = k / (kInStride / 4), b = 4 * (k - r * (kInStride / 4));
-                const std::uint8_t* row = j.image + row_at[r];
+                const std::uint8_t* row = t.image + row_at[r];
                 *reinterpret_cast<std::uint32_t*>(&in[r][b]) =
                     static_cast<std::uint32_t>(row[col_at[b]]) | (static_cast<std::uint32_t>(row[col_at[b + 1]]) << 8) |
                     (static_cast<std::uint32_t>(row[col_at[b + 2]]) << 16) |
@@ -1372,76 +1406,91 @@ __global__ __launch_bounds__(256, kBlurCtasPerSm) void blur_tiles_kernel(const _
             }
         }
         cp_async_wait_all();
-        __syncthreads();
-        if (aligned16(j) && blur_needs_columns(x0, W)) {
-            blur_fix_columns(x0, W, in);
+        __syncthreads();  // also: everyone is done with the tile before
+        if (t.aligned && blur_needs_columns(t.x0, t.width)) {
+            blur_fix_columns(t.x0, t.width, in);
             __syncthreads();
         }
-        if (i + static_cast<int>(gridDim.x) < n) prefetch(i + gridDim.x, in2[buf ^ 1]);
-        // rows pass: image rows y0-3 .. y0+34, two rows x 4 outputs per item
-        static_assert((kBlurTileH + 6) % 2 == 0, "rows pass takes row pairs");
-        for (int g = tid; g < (kBlurTileH + 6) / 2 * (kBlurTileW / 4); g += 256) {
-            const int rp = g / (kBlurTileW / 4), q = g - rp * (kBlurTileW / 4), rr = 2 * rp;
-            const auto* ra = reinterpret_cast<const std::uint32_t*>(&in[rr + 1][0]);
-            const auto* rb = reinterpret_cast<const std::uint32_t*>(&in[rr + 2][0]);
-            const std::uint32_t a0 = ra[q + 3], a1 = ra[q + 4], a2 = ra[q + 5];  // bytes 4q+12 .. 4q+23
-            const std::uint32_t b0 = rb[q + 3], b1 = rb[q + 4], b2 = rb[q + 5];
-            // output 4q+k reads halo columns 4q+k+1 .. 4q+k+7, tap t on column
-            // 4q+k+1+t; lane x holds row rr, lane y row rr + 1. The columns
+        if (i + grid < n && info[next].aligned) blur_stage_async(info[next], in2[buf ^ 1]);
+        const int out_rows = min(kBlurTileH, t.height - t.y0);
+        // rows pass: image rows y0-3 .., two rows x 8 outputs per item
+        static_assert((kBlurTileH + 6) % 2 == 0 && (kBlurTileH + 6) / 2 * (kBlurTileW / 8) <= kBlurThreads,
+                      "rows pass takes row pairs, one item per thread");
+        if (tid < (out_rows + 7) / 2 * (kBlurTileW / 8)) {
+            const int rr = 2 * (tid / (kBlurTileW / 8)), q = tid % (kBlurTileW / 8);
+            const auto* ra = reinterpret_cast<const std::uint32_t*>(&in[rr + 1][0]) + 2 * q + 3;  // bytes 8q+12 .. 8q+27
+            const auto* rb = reinterpret_cast<const std::uint32_t*>(&in[rr + 2][0]) + 2 * q + 3;
+            const uint2 a12 = *reinterpret_cast<const uint2*>(ra + 1), b12 = *reinterpret_cast<const uint2*>(rb + 1);
+            const std::uint32_t wa[4] = {ra[0], a12.x, a12.y, ra[3]}, wb[4] = {rb[0], b12.x, b12.y, rb[3]};
+            // output 8q+k reads halo columns 8q+k+1 .. 8q+k+7, tap t on column
+            // 8q+k+1+t; lane x holds row rr, lane y row rr + 1. The columns
             // stream in once and every output adds its taps in order (0 + a
             // nonnegative product is the product).
-            float2 out[4];
+            float2 out[8], before;
 #pragma unroll
-            for (int m = 1; m <= 10; ++m) {
-                const std::uint32_t wa = m < 4 ? a0 : m < 8 ? a1 : a2, wb = m < 4 ? b0 : m < 8 ? b1 : b2;
-                const float2 xm = byte_pair(wa, wb, m & 3);
+            for (int m = 1; m <= 14; ++m) {
+                const float2 xm = byte_pair(wa[m >> 2], wb[m >> 2], m & 3);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int t = m - 1 - k;
-                    if (t == 0) out[k] = first_tap<kPacked>(xm);
-                    else if (t > 0 && t < 7) out[k] = next_tap<kPacked>(out[k], t, xm);
+                for (int k = 0; k < 8; ++k) {
+                    const int tap = m - 1 - k;
+                    if (tap == 1) out[k] = first_taps<kPacked>(before, xm);
+                    else if (tap > 1 && tap < 7) out[k] = next_tap<kPacked>(out[k], tap, xm);
                 }
+                before = xm;
             }
-            *reinterpret_cast<float4*>(&rows[rr][4 * q]) = make_float4(out[0].x, out[1].x, out[2].x, out[3].x);
-            *reinterpret_cast<float4*>(&rows[rr + 1][4 * q]) = make_float4(out[0].y, out[1].y, out[2].y, out[3].y);
+            auto* o = reinterpret_cast<float4*>(&rows[rr][0]) + blur_quad(2 * q);
+            auto* o1 = reinterpret_cast<float4*>(&rows[rr][0]) + blur_quad(2 * q + 1);
+            constexpr int kNextRow = kBlurTileW / 4;
+            o[0] = make_float4(out[0].x, out[1].x, out[2].x, out[3].x);
+            o1[0] = make_float4(out[4].x, out[5].x, out[6].x, out[7].x);
+            o[kNextRow] = make_float4(out[0].y, out[1].y, out[2].y, out[3].y);
+            o1[kNextRow] = make_float4(out[4].y, out[5].y, out[6].y, out[7].y);
         }
         __syncthreads();
-        // columns pass: rows 2p, 2p+1 and columns 4q .. 4q+3 per thread and step
-        for (int pr = tid / (kBlurTileW / 4), q = tid % (kBlurTileW / 4); pr < kBlurTileH / 2;
-             pr += 256 / (kBlurTileW / 4)) {
-            float2 lo[2], hi[2];
+        // columns pass: a thread has rows 4p .. 4p+3 and columns 4q .. 4q+3
+        static_assert(kBlurTileH / 4 * (kBlurTileW / 4) == 256, "columns pass: one 4x4 block per thread");
+        const int row = 4 * (tid / (kBlurTileW / 4)), col = 4 * (tid % (kBlurTileW / 4));
+        if (tid >= 256) {
+            if (tid == kBlurThreads - 1 && i + 2 * grid < n) {
+                blur_tile_at(src, ahead, &info[after]);
+                ahead = entry_at(i + 3 * grid);
+            }
+        } else if (row < out_rows) {
+            const auto* quads = reinterpret_cast<const float4*>(&rows[row][0]) + blur_quad(col / 4);
+            float2 lo[4], hi[4], bl, bh;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const float4 v = *reinterpret_cast<const float4*>(&rows[2 * pr + r][4 * q]);
+            for (int r = 0; r < 10; ++r) {
+                const float4 v = quads[r * (kBlurTileW / 4)];
                 const float2 vl = make_float2(v.x, v.y), vh = make_float2(v.z, v.w);
 #pragma unroll
-                for (int o = 0; o < 2; ++o) {
-                    const int t = r - o;
-                    if (t == 0) {
-                        lo[o] = first_tap<kPacked>(vl);
-                        hi[o] = first_tap<kPacked>(vh);
-                    } else if (t > 0 && t < 7) {
-                        lo[o] = next_tap<kPacked>(lo[o], t, vl);
-                        hi[o] = next_tap<kPacked>(hi[o], t, vh);
+                for (int o = 0; o < 4; ++o) {
+                    const int tap = r - o;
+                    if (tap == 1) {
+                        lo[o] = first_taps<kPacked>(bl, vl);
+                        hi[o] = first_taps<kPacked>(bh, vh);
+                    } else if (tap > 1 && tap < 7) {
+                        lo[o] = next_tap<kPacked>(lo[o], tap, vl);
+                        hi[o] = next_tap<kPacked>(hi[o], tap, vh);
                     }
                 }
+                bl = vl;
+                bh = vh;
             }
+            std::uint8_t* dst = t.blurred + static_cast<std::size_t>(row) * t.blur_pitch + col;
+            const int nx = t.whole ? 4 : t.width - t.x0 - col;
 #pragma unroll
-            for (int o = 0; o < 2; ++o) {
-                const int gy = y0 + 2 * pr + o, gx = x0 + 4 * q;
-                if (gy >= H || gx >= W) continue;
+            for (int o = 0; o < 4; ++o, dst += t.blur_pitch) {
                 const std::uint32_t packed = pack_bytes(round_pair(lo[o]), round_pair(hi[o]));
-                std::uint8_t* dst = j.blurred + static_cast<std::size_t>(gy) * j.blur_pitch + gx;
-                if (gx + 3 < W && (reinterpret_cast<std::uintptr_t>(dst) & 3) == 0) {
+                if (t.whole || (nx >= 4 && row + o < out_rows && (reinterpret_cast<std::uintptr_t>(dst) & 3) == 0)) {
                     *reinterpret_cast<std::uint32_t*>(dst) = packed;
-                } else {
+                } else if (row + o < out_rows) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        if (gx + k < W) dst[k] = static_cast<std::uint8_t>(packed >> (8 * k));
+                        if (k < nx) dst[k] = static_cast<std::uint8_t>(packed >> (8 * k));
                 }
             }
         }
-        __syncthreads();  // before the next tile's staging
+        slot = next;
     }
 }
 

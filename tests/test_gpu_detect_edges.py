@@ -86,3 +86,14 @@ def test_layer_edges(ours, w, h, factor, aligned):
     st, kp, _ = run_pyramid(gray, 12, 3000, 3, factor, pad=(-w) % 16 + 16 if aligned else None)
     assert st == 0
     assert np.array_equal(kp, pyramid.detect_and_describe(gray, 12, 3000, 3, factor)[0])
+
+
+@pytest.mark.parametrize("w,h", [(4, 40), (5, 9), (17, 64), (63, 65), (64, 64), (65, 67), (67, 128), (128, 131), (200, 61)])
+@pytest.mark.parametrize("pad", [0, 5, 16])
+def test_blur_edges(ours, w, h, pad, monkeypatch):
+    """The blurred image at its tiles' edges: mirrored columns and rows, part
+    tiles, 16-byte and other pitches."""
+    monkeypatch.setattr(G, "pitched", lambda gray: pitched(gray, (-w) % 16 + 16 if pad == 16 else pad))
+    g = np.random.default_rng(w * h).integers(0, 256, (h, w), dtype=np.uint8)
+    _, _, blurred, (st2, st3, _) = G.detect_describe(ours, g, 20, 50)
+    assert (st2, st3) == (0, 0) and np.array_equal(blurred, s2s3.blur(g))
