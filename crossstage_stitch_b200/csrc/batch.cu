@@ -63,7 +63,7 @@ void set_attributes_once() {
     static std::once_flag flag;
     std::call_once(flag, [] {
         static_assert(kTables <= 20, "table offsets");
-        cudaFuncSetAttribute(s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>>,
+        cudaFuncSetAttribute(s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>, s2s3::kSortThreads>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              s2s3::kSortCap * static_cast<int>(sizeof(std::uint64_t)));
         using Src = s5k::JobTable<SearchJob>;
@@ -219,6 +219,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     }
     sort_smem = s2s3::sort_smem_bytes(max_cand);
     rank_fallback = max_cand > s2s3::kSortCap;
+    small_sorts = max_cand <= s2s3::kSortSmall;
     desc_keys = s2s3::desc_keys(keypoints);
     search_smem = s5k::search_smem_bytes(max_cap_m, true);
     finish_smem = s5k::finish_smem_bytes(max_cap_m);
@@ -662,8 +663,14 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
             s2s3::rank_topk_kernel<DetSrc>
                 <<<det_blocks[s2s3::kHarrisKind] * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, 0);
     } else {
-        if (go(det_blocks[s2s3::kSortKind]))
-            s2s3::sort_topk_kernel<DetSrc><<<det_blocks[s2s3::kSortKind], s2s3::kSortThreads, sort_smem, s>>>(det);
+        const auto sort = [&](auto threads) {
+            constexpr int kThreads = decltype(threads)::value;
+            s2s3::sort_topk_kernel<DetSrc, kThreads><<<det_blocks[s2s3::kSortKind], kThreads, sort_smem, s>>>(det);
+        };
+        if (go(det_blocks[s2s3::kSortKind])) {
+            if (small_sorts) sort(std::integral_constant<int, s2s3::kSortSmallThreads>{});
+            else sort(std::integral_constant<int, s2s3::kSortThreads>{});
+        }
         if (rank_fallback && go(det_blocks[s2s3::kHarrisKind]))
             s2s3::rank_topk_kernel<DetSrc>
                 <<<det_blocks[s2s3::kHarrisKind] * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, s2s3::kSortCap);

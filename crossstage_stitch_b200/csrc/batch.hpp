@@ -56,6 +56,7 @@ public:
     int search_blocks = 0, fit_blocks = 0;
     int sort_smem = 0, search_smem = 0, finish_smem = 0;
     bool rank_fallback = false;  // a job has more candidates than the sort takes
+    bool small_sorts = false;    // no job has more than kSortSmall candidates
     bool rank = false;           // every job's candidates are ranked, not sorted
     int desc_keys = 0;           // keypoints per describe block
     int hpw = 8;

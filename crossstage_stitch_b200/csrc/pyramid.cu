@@ -175,7 +175,7 @@ bool enable_pyramid_sort_smem() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(sort_topk_kernel<DetSrc>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ok[dev] = cudaFuncSetAttribute(sort_topk_kernel<DetSrc, kSortThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kSortCap * static_cast<int>(sizeof(std::uint64_t))) == cudaSuccess;
     });
     return ok[dev];
@@ -248,7 +248,7 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
         if (max_cand > kSortCap || rank_pays(blocks(kHarrisKind), blocks(kSortKind), max_cand))
             launch_chained(rank_topk_kernel<DetSrc>, blocks(kHarrisKind) * kRankPer, kRankThreads, 0, stream, det, 0);
         else
-            launch_chained(sort_topk_kernel<DetSrc>, blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream, det);
+            launch_chained(sort_topk_kernel<DetSrc, kSortThreads>, blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream, det);
         launches += 4;
         launch_chained(blur_tiles_kernel<DesSrc, true>, std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), kBlurThreads, 0, stream,
             des, at_offset<uint2>(ws, l.blur_list), queue + 1, 0);

@@ -116,7 +116,7 @@ template <class Src> bool enable_sort_smem() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(sort_topk_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ok[dev] = cudaFuncSetAttribute(sort_topk_kernel<Src, kSortThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kSortCap * static_cast<int>(sizeof(std::uint64_t))) == cudaSuccess;
     });
     return ok[dev];
@@ -159,7 +159,7 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
     if (l.candidates > kSortCap || rank_pays(harris_blocks, 1, l.candidates))
         launch_chained(rank_topk_kernel<Src>, harris_blocks * kRankPer, kRankThreads, 0, stream, src, 0);
     else
-        launch_chained(sort_topk_kernel<Src>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src);
+        launch_chained(sort_topk_kernel<Src, kSortThreads>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src);
     note_launches(4);
     return launch_status();
 }

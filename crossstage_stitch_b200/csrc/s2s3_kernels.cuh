@@ -210,7 +210,8 @@ constexpr int kRankThreads = 512;
 constexpr int kRankPer = kHarrisThreads / kRankKeys;  // rank blocks per harris block
 constexpr int kRankTile = 1024;      // keys staged at a time
 constexpr int kSortCap = 16384;    // candidates sorted in shared memory by one block
-constexpr int kSortThreads = 1024;
+constexpr int kSortThreads = 1024, kSortSmallThreads = 256;
+constexpr int kSortSmall = 1024;    // most candidates of any job of a launch of the small sort blocks
 constexpr int kSortChunk = 64;      // keys a warp sorts in registers (2 per lane)
 constexpr int kBlurTileW = 64, kBlurTileH = 64;
 constexpr int kDescWarps = 8;
@@ -970,9 +971,15 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
 }
 
 // One block per job: bitonic sort (descending) of up to kSortCap keys in
-// shared memory, then the first min(K, selected) become the keypoints.
-template <class Src>
-__global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_constant__ Src src) {
+// shared memory, then the first min(K, selected) become the keypoints. Bound by
+// instruction issue and barriers on the SMs that have a block: with at most
+// kSortSmall candidates a job, blocks of 256 threads leave eight jobs to an SM
+// (1024 jobs of 64 pairs at 8 layers, K = 2000: 45 us with 1024 threads, 31 with
+// 512, 29 with 256; 128 to 256 jobs: 16 to 18 us either way), while larger jobs
+// want them all (30 mixed pairs, K up to 8000: 83, 86 and 100 us, and 106 in two
+// launches that divide the jobs).
+template <class Src, int kThreads>
+__global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_constant__ Src src) {
     wait_for_previous();
     extern __shared__ std::uint64_t sk[];
     DetectJob j;
@@ -982,7 +989,7 @@ __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_co
     if (n > kSortCap || n == 0) return;
     int N = kSortChunk;  // at least one 64-key chunk (zero keys pad and sort last)
     while (N < n) N <<= 1;
-    for (int i = threadIdx.x; i < N; i += kSortThreads) sk[i] = i < n ? j.keys[i] : 0ull;
+    for (int i = threadIdx.x; i < N; i += kThreads) sk[i] = i < n ? j.keys[i] : 0ull;
     __syncthreads();
     // Bitonic network, keys unique: a compare-exchange of i < q = i + s puts
     // the larger key first where (i & k) == 0 (those runs end up descending).
@@ -990,7 +997,7 @@ __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_co
     // c*64 + lane and c*64 + lane + 32 of chunk c; wider ones in shared memory.
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto chunk_pass = [&](int k_lo, int k_hi, int s_top) {
-        for (int c = warp; c < N / kSortChunk; c += kSortThreads / 32) {
+        for (int c = warp; c < N / kSortChunk; c += kThreads / 32) {
             const int e0 = c * kSortChunk + lane;
             std::uint64_t v0 = sk[e0], v1 = sk[e0 + 32];
             for (int k = k_lo; k <= k_hi; k <<= 1) {
@@ -1019,8 +1026,8 @@ __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_co
     chunk_pass(2, kSortChunk, kSortChunk / 2);  // runs up to 64 keys: registers only
     for (int k = 2 * kSortChunk; k <= N; k <<= 1) {
         for (int s = k >> 1; s >= kSortChunk; s >>= 1) {
-            for (int t = threadIdx.x; t < (N >> 1); t += kSortThreads) {
-                const int i = (t / s) * (s << 1) + (t % s);
+            for (int t = threadIdx.x; t < (N >> 1); t += kThreads) {
+                const int i = 2 * t - (t & (s - 1));  // the t-th key without bit s
                 const int q = i + s;
                 const std::uint64_t a = sk[i], b = sk[q];
                 const bool descending = (i & k) == 0;
@@ -1031,7 +1038,7 @@ __global__ __launch_bounds__(kSortThreads) void sort_topk_kernel(const __grid_co
         chunk_pass(k, k, kSortChunk / 2);
     }
     const int limit = min(n, j.max_keypoints);
-    for (int i = threadIdx.x; i < limit; i += kSortThreads) write_keypoint(j, i, sk[i]);
+    for (int i = threadIdx.x; i < limit; i += kThreads) write_keypoint(j, i, sk[i]);
 }
 
 // Top-K by counting: the rank of a key is the number of larger keys (keys are

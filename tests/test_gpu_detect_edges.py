@@ -4,7 +4,9 @@ around the ranked and the listed ties, candidate counts around the rank
 kernel's blocks and tiles, aligned and odd pitches, saturated windows."""
 import numpy as np
 import pytest
+import torch
 
+from crossstage_stitch_b200 import batch, stages
 from oracle import pyramid, s2s3
 from tests import gpu_util as G
 from tests.test_gpu_pyramid import run_pyramid
@@ -97,3 +99,21 @@ def test_blur_edges(ours, w, h, pad, monkeypatch):
     g = np.random.default_rng(w * h).integers(0, 256, (h, w), dtype=np.uint8)
     _, _, blurred, (st2, st3, _) = G.detect_describe(ours, g, 20, 50)
     assert (st2, st3) == (0, 0) and np.array_equal(blurred, s2s3.blur(g))
+
+
+@pytest.mark.parametrize("k", [33, 512, 513])
+def test_batched_sort_blocks(cuda, k):
+    """20 pairs: more jobs than are ranked; 66 and 1024 candidates a job are
+    sorted by small blocks, 1026 by large ones."""
+    rng = np.random.default_rng(k)
+    grays = [rng.integers(0, 256, (150 + i, 170), dtype=np.uint8) for i in range(40)]
+    images = [torch.from_numpy(g).cuda() for g in grays]
+    b = batch.Batch([batch.pair_desc(images[2 * i], images[2 * i + 1],
+                                     stages.Knobs(max_keypoints=k, fast_threshold=10, hypotheses=64, seed=i))
+                     for i in range(20)])
+    b.enqueue()
+    torch.cuda.synchronize()
+    for i in range(0, 40, 7):
+        got = b.outputs(i // 2)["kp_a" if i % 2 == 0 else "kp_b"]
+        want = s2s3.detect_and_describe(grays[i], 10, k)[0]
+        assert want.shape[0] == k and np.array_equal(got, want)
