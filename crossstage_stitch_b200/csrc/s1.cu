@@ -69,15 +69,24 @@ __device__ __forceinline__ int s1_pixel(const Params& p, int xd, int yd) {
 }
 
 // Source bytes [0, kBytes) at p of a row, in words, for the integer modes. With
-// p 8- or 4-byte aligned they come from 8- or 4-byte loads; otherwise from
+// p 16-, 8- or 4-byte aligned they come from loads of that size; otherwise from
 // the aligned words around them, shifted, when those lie inside [first, last)
 // (the image's bytes), and byte by byte at its ends.
 template <int kBytes>
 __device__ __forceinline__ void load_bytes(const std::uint8_t* p, const std::uint8_t* first, const std::uint8_t* last,
                                            std::uint32_t (&w)[kBytes / 4]) {
-    const int off = static_cast<int>(reinterpret_cast<std::uintptr_t>(p) & 7);
+    const int off = static_cast<int>(reinterpret_cast<std::uintptr_t>(p) & 15);
     constexpr int kWords = kBytes / 4;
-    if (off == 0 && kBytes % 8 == 0) {
+    if (off == 0 && kBytes % 16 == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords / 4; ++i) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
+            w[4 * i] = v.x;
+            w[4 * i + 1] = v.y;
+            w[4 * i + 2] = v.z;
+            w[4 * i + 3] = v.w;
+        }
+    } else if ((off & 7) == 0 && kBytes % 8 == 0) {
 #pragma unroll
         for (int i = 0; i < kWords / 2; ++i) {
             const uint2 v = __ldg(reinterpret_cast<const uint2*>(p) + i);
@@ -114,34 +123,49 @@ template <int kWords> __device__ __forceinline__ int gray_at(const std::uint32_t
     return static_cast<int>(__dp2a_hi(3735u, rgb, rg) >> 15);
 }
 
-// Four adjacent outputs of an exact kFactor x kFactor average (1: none), all
-// inside the output, in the bytes of a word.
-template <int kFactor> __device__ __forceinline__ std::uint32_t s1_quad(const Params& p, int x, int y) {
-    constexpr int kBytes = 12 * kFactor;
+// kOut adjacent outputs (a multiple of 4) of an exact kFactor x kFactor average
+// (1: none), all inside the output, in the bytes of words.
+template <int kFactor, int kOut>
+__device__ __forceinline__ void s1_words(const Params& p, int x, int y, std::uint32_t (&out)[kOut / 4]) {
+    constexpr int kBytes = 3 * kFactor * kOut;
     const std::uint8_t* last = p.src + static_cast<std::size_t>(p.orig_h - 1) * p.src_pitch + 3 * static_cast<std::size_t>(p.orig_w);
-    int sum[4] = {};
+    int sum[kOut] = {};
+    std::uint32_t w[kFactor == 2 ? 2 : 1][kBytes / 4];  // both rows of a half-size output in flight
 #pragma unroll
     for (int dy = 0; dy < kFactor; ++dy) {
-        std::uint32_t w[kBytes / 4];
-        load_bytes<kBytes>(p.src + static_cast<std::size_t>(kFactor * y + dy) * p.src_pitch + 3 * kFactor * static_cast<std::size_t>(x),
-                           p.src, last, w);
+        if (kFactor != 2 || dy == 0) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+            for (int d = 0; d < (kFactor == 2 ? 2 : 1); ++d)
+                load_bytes<kBytes>(p.src + static_cast<std::size_t>(kFactor * y + dy + d) * p.src_pitch + 3 * kFactor * static_cast<std::size_t>(x),
+                                   p.src, last, w[d]);
+        }
 #pragma unroll
-            for (int dx = 0; dx < kFactor; ++dx) sum[k] += gray_at(w, 3 * (kFactor * k + dx));
+        for (int k = 0; k < kOut; ++k)
+#pragma unroll
+            for (int dx = 0; dx < kFactor; ++dx) sum[k] += gray_at(w[kFactor == 2 ? dy : 0], 3 * (kFactor * k + dx));
     }
-    std::uint32_t out = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int v = kFactor == 1 ? sum[k] : kFactor == 2 ? (sum[k] + 2) >> 2 : __float2int_rn(__fmul_rn(static_cast<float>(sum[k]), 0.0625f));
-        out |= static_cast<std::uint32_t>(v) << (8 * k);
+    for (int q = 0; q < kOut / 4; ++q) {
+        out[q] = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int t = sum[4 * q + k];
+            const int v = kFactor == 1 ? t : kFactor == 2 ? (t + 2) >> 2 : __float2int_rn(__fmul_rn(static_cast<float>(t), 0.0625f));
+            out[q] |= static_cast<std::uint32_t>(v) << (8 * k);
+        }
     }
-    return out;
+}
+
+template <int kFactor> __device__ __forceinline__ std::uint32_t s1_quad(const Params& p, int x, int y) {
+    std::uint32_t out[1];
+    s1_words<kFactor, 4>(p, x, y, out);
+    return out[0];
 }
 
 // Outputs x .. x + 3 (those inside) of row y. The integer modes are bound by
 // memory: they read words and write one (4K pair to half size, 54 MB: 22 us
-// byte by byte, 14 us; the measured copy rate would take 8.3).
+// byte by byte, 14 us so, 12 us by the 48-byte runs of s1_long; the measured
+// copy rate would take 8.3).
 __device__ __forceinline__ void s1_outputs(const Params& p, int x, int y) {
     std::uint8_t* dst = p.dst + static_cast<std::size_t>(y) * p.dst_pitch + x;
     if (p.mode < 3 && x + 4 <= p.work_w) {
@@ -159,14 +183,41 @@ __device__ __forceinline__ void s1_outputs(const Params& p, int x, int y) {
         if (x + k < p.work_w) dst[k] = static_cast<std::uint8_t>(s1_pixel(p, x + k, y));
 }
 
-constexpr int kS1BlockX = 32, kS1BlockY = 8;  // 32 x 4-output columns x 8 rows per block
+// Outputs of a thread of the per-image and per-pair kernel: 48 source bytes of
+// a row in the integer modes, 4 outputs in the others.
+__host__ __device__ constexpr int s1_run(int mode) { return mode < 3 ? 16 >> mode : 4; }
+
+// Outputs x .. x + s1_run - 1 (those inside) of row y, as one run of 16-byte
+// loads and whole stores where the row allows it, by fours otherwise.
+template <int kFactor> __device__ __forceinline__ void s1_long(const Params& p, int x, int y) {
+    constexpr int kOut = 16 / kFactor;
+    std::uint8_t* dst = p.dst + static_cast<std::size_t>(y) * p.dst_pitch + x;
+    const std::uint8_t* src = p.src + static_cast<std::size_t>(kFactor * y) * p.src_pitch + 3 * kFactor * static_cast<std::size_t>(x);
+    if (x + kOut <= p.work_w && (reinterpret_cast<std::uintptr_t>(dst) & (kOut - 1)) == 0 &&
+        ((reinterpret_cast<std::uintptr_t>(src) | static_cast<std::uintptr_t>(p.src_pitch)) & 15) == 0) {
+        std::uint32_t out[kOut / 4];
+        s1_words<kFactor, kOut>(p, x, y, out);
+        if constexpr (kOut == 16) *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+        else if constexpr (kOut == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(out[0], out[1]);
+        else *reinterpret_cast<std::uint32_t*>(dst) = out[0];
+        return;
+    }
+    for (int q = 0; q < kOut && x + q < p.work_w; q += 4) s1_outputs(p, x + q, y);
+}
+
+constexpr int kS1BlockX = 16, kS1BlockY = 16;  // runs of columns x rows per block
 
 __global__ __launch_bounds__(kS1BlockX * kS1BlockY) void s1_kernel(const __grid_constant__ Pair pair) {
     const Params& p = pair.img[blockIdx.z];
-    const int x = 4 * (blockIdx.x * kS1BlockX + threadIdx.x);
+    const int x = s1_run(p.mode) * (blockIdx.x * kS1BlockX + threadIdx.x);
     const int y = blockIdx.y * kS1BlockY + threadIdx.y;
     if (y >= p.work_h || x >= p.work_w) return;
-    s1_outputs(p, x, y);
+    switch (p.mode) {
+        case 0: s1_long<1>(p, x, y); break;
+        case 1: s1_long<2>(p, x, y); break;
+        case 2: s1_long<4>(p, x, y); break;
+        default: s1_outputs(p, x, y);
+    }
 }
 
 // Batched form: one launch over the images of many requests; each block
@@ -265,13 +316,14 @@ Status scale_info(int w, int h, double s, ScaleInfo* out) {
 }
 
 Status launch(const Pair& pair, int images, cudaStream_t stream) {
-    int mw = pair.img[0].work_w, mh = pair.img[0].work_h;
-    if (images == 2) {
-        mw = mw > pair.img[1].work_w ? mw : pair.img[1].work_w;
-        mh = mh > pair.img[1].work_h ? mh : pair.img[1].work_h;
+    int runs = 0, mh = 0;
+    for (int z = 0; z < images; ++z) {
+        const Params& p = pair.img[z];
+        runs = max(runs, ceil_div(p.work_w, s1_run(p.mode)));
+        mh = max(mh, p.work_h);
     }
     const dim3 block(kS1BlockX, kS1BlockY);
-    const dim3 grid(ceil_div(ceil_div(mw, 4), kS1BlockX), ceil_div(mh, kS1BlockY), images);
+    const dim3 grid(ceil_div(runs, kS1BlockX), ceil_div(mh, kS1BlockY), images);
     s1_kernel<<<grid, block, 0, stream>>>(pair);
     note_launches(1);
     return launch_status();

@@ -38,3 +38,27 @@ def test_loads(cuda, factor, w, h, offset, pad):
     got = out[offset:].view(h, out_pitch).cpu().numpy()
     assert np.array_equal(got[:, :w], c_oracle.s1(rgb, w, h))
     assert (got[:, w:] == 0x5a).all() and (out[:offset] == 0x5a).all()
+
+
+@pytest.mark.parametrize("factor", [1, 2, 4])
+@pytest.mark.parametrize("w,h", [(15, 2), (16, 17), (20, 5), (37, 33), (263, 6)])
+@pytest.mark.parametrize("out_offset", [0, 4, 8])
+def test_runs(cuda, factor, w, h, out_offset):
+    """48-byte runs of 16-byte aligned rows and their last, shorter one; an
+    output that the run's store does not fit."""
+    rng = np.random.default_rng(w + h)
+    sw, sh = w * factor, h * factor
+    rgb = rng.integers(0, 256, (sh, sw, 3), dtype=np.uint8)
+    pitch, out_pitch = (3 * sw + 15) // 16 * 16, (w + 15) // 16 * 16
+    rows = torch.zeros((sh, pitch), dtype=torch.uint8, device="cuda")
+    rows[:, :3 * sw] = torch.from_numpy(rgb.reshape(sh, 3 * sw)).cuda()
+    out = torch.full((out_offset + h * out_pitch,), 0x5a, dtype=torch.uint8, device="cuda")
+    si = ScaleInfo()
+    st = _abi.load().stitch_s1_preprocess_single(
+        C.byref(ImageView(rows.data_ptr(), sw, sh, pitch, 0)), 1.0 / factor,
+        C.byref(ImageView(out.data_ptr() + out_offset, w, h, out_pitch, 1)), C.byref(si), stream())
+    torch.cuda.synchronize()
+    assert st == 0
+    got = out[out_offset:].view(h, out_pitch).cpu().numpy()
+    assert np.array_equal(got[:, :w], c_oracle.s1(rgb, w, h))
+    assert (got[:, w:] == 0x5a).all() and (out[:out_offset] == 0x5a).all()
