@@ -46,8 +46,6 @@ bool detect_layout(int w, int h, int k, DetectLayout* out) {
     l.params = lay.take(1, sizeof(SelectParams));
     l.keys = lay.take(static_cast<std::size_t>(l.candidates), sizeof(std::uint64_t));
     l.maxima = lay.take(std::max<std::size_t>(cells, 1), sizeof(std::uint64_t));
-    l.max_ties = static_cast<int>(std::min<std::size_t>(cells, kTieCap));
-    l.ties = lay.take(static_cast<std::size_t>(std::max(l.max_ties, 1)), sizeof(std::uint32_t));
     if (!lay.ok) return false;
     l.total = lay.cursor;
     *out = l;
@@ -80,8 +78,6 @@ DetectJob make_detect_job(const ImageView& im, const s2::Config& c, const Keypoi
     j.harris_k = c.harris_k;
     j.maxima = at_offset<std::uint64_t>(ws, l.maxima);
     j.max_maxima = l.max_maxima;
-    j.ties = at_offset<std::uint32_t>(ws, l.ties);
-    j.max_ties = l.max_ties;
     j.hist = at_offset<std::uint32_t>(ws, l.hist);
     j.params = at_offset<SelectParams>(ws, l.params);
     j.keys = at_offset<std::uint64_t>(ws, l.keys);

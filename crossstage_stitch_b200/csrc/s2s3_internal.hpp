@@ -10,8 +10,8 @@ namespace stitch::b200::s2s3 {
 // histogram bins and then the kDetectCounters counters, zeroed together
 // (hist_bytes) before each run.
 struct DetectLayout {
-    std::size_t maxima, hist, params, keys, ties, total;
-    int max_maxima, max_ties, candidates, tiles_x, tiles, select_blocks;
+    std::size_t maxima, hist, params, keys, total;
+    int max_maxima, candidates, tiles_x, tiles, select_blocks;
     static constexpr std::size_t hist_bytes = kHistWords * sizeof(std::uint32_t);
 };
 

@@ -51,8 +51,6 @@ struct alignas(16) DetectJob {  // 16-byte multiple: copied into shared memory i
                                    // all zeroed before the FAST launch
     SelectParams* params;
     std::uint64_t* keys;           // [candidates]
-    std::uint32_t* ties;           // raster indices of the maxima at the selection threshold
-    int max_ties;                  // capacity of `ties`
     // output
     float* x;
     float* y;
@@ -196,7 +194,7 @@ constexpr int kSelectPx = 65536;   // image pixels per select block (a job's max
                                    // by ceil(W * H / kSelectPx) blocks)
 constexpr int kFastThreads = 256;
 constexpr int kFastCtasPerSm = 7;  // resident FAST blocks per SM (shared memory); the persistent grid is 148 x this
-constexpr int kTieCap = 16384;      // tie list entries; more ties are picked from the maxima list itself
+constexpr int kTieCap = 16384;      // most tie list entries; more ties are picked from the maxima list itself
 constexpr int kTieRank = 1024;      // ties ranked against each other in shared memory
 // Largest offset of a rotated rBRIEF sample from its keypoint: the pattern's
 // coordinates lie within a radius of 18.39 px (|x|, |y| <= 13), so a rotated
@@ -703,6 +701,18 @@ __device__ __forceinline__ SelectParams select_params(const std::uint32_t* hist,
     return *out;
 }
 
+// The list of the maxima at the selection threshold (their raster indices), in
+// the entries of the maxima list that its n maxima leave over.
+struct TieList {
+    std::uint32_t* at;
+    std::uint32_t room;
+};
+
+__device__ __forceinline__ TieList tie_list(const DetectJob& j, std::uint32_t n) {
+    const std::uint32_t left = static_cast<std::uint32_t>(j.max_maxima) - n;  // two ties fit an entry
+    return {reinterpret_cast<std::uint32_t*>(j.maxima + n), min(left, kTieCap / 2u) * 2u};
+}
+
 // The first `p.ties` maxima at the threshold score in raster order, when they
 // cannot all be kept (the reference's raster-order scatter of the first ties,
 // src/s2_s3/s2.cu:182-235), by the 256 threads of one block, into keys[above,
@@ -710,15 +720,16 @@ __device__ __forceinline__ SelectParams select_params(const std::uint32_t* hist,
 // outgrew their list (then an entry counts only with the threshold's score).
 // A few ties are ranked against each other; more go through a
 // most-significant-digit radix select of the p.ties-th smallest raster index.
-__device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams& p, std::uint32_t listed) {
+__device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams& p, std::uint32_t listed,
+                                          const TieList& list) {
     __shared__ __align__(16) std::uint32_t buf[kTieRank];  // staged ties, or the 256 radix bins
     __shared__ std::uint32_t pick[2];        // digit, maxima before it
     std::uint32_t* ctr = j.counters();
     const std::uint32_t T = p.threshold, total = j.hist[T];
     const int t = threadIdx.x;
-    if (total <= kTieRank && total <= static_cast<std::uint32_t>(j.max_ties)) {
+    if (total <= kTieRank && total <= list.room) {
         const int n = static_cast<int>(total), padded = (n + 3) / 4 * 4;
-        for (int i = t; i < padded; i += 256) buf[i] = i < n ? __ldcg(j.ties + i) : 0xffffffffu;
+        for (int i = t; i < padded; i += 256) buf[i] = i < n ? __ldcg(list.at + i) : 0xffffffffu;
         __syncthreads();
         for (int i = t; i < n; i += 256) {
             const std::uint32_t px = buf[i];
@@ -731,11 +742,11 @@ __device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams
         }
         return;
     }
-    const bool own = total <= static_cast<std::uint32_t>(j.max_ties);
+    const bool own = total <= list.room;
     const std::uint32_t n = own ? total : listed;
     const auto entry = [&](std::uint32_t i, std::uint32_t& px) {  // whether entry i is a tie
         if (own) {
-            px = __ldcg(j.ties + i);
+            px = __ldcg(list.at + i);
             return true;
         }
         const std::uint64_t e = j.maxima[i];
@@ -810,6 +821,7 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
     const bool all_ties = p.ties == j.hist[p.threshold];
     std::uint32_t* ctr = j.counters();
     const std::uint32_t n = min(ctr[kListed], static_cast<std::uint32_t>(j.max_maxima));
+    const TieList list = tie_list(j, n);
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     // ties go behind the keys above the threshold, or to their list
@@ -836,7 +848,7 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
         bt = __shfl_sync(0xffffffffu, bt, 0) + __popc(mt & below);
         if (above && ba < p.above) j.keys[ba] = px;  // always true when list and histogram agree
         if (tie && all_ties && bt < p.ties) j.keys[p.above + bt] = px;
-        if (tie && !all_ties && bt < static_cast<std::uint32_t>(j.max_ties)) j.ties[bt] = px;
+        if (tie && !all_ties && bt < list.room) list.at[bt] = px;
     }
     if (all_ties || p.selected == 0) return;
     __threadfence();  // this block's list entries, before it counts as done
@@ -846,7 +858,7 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
     __syncthreads();
     if (!last) return;
     __threadfence();
-    pick_ties(j, p, n);
+    pick_ties(j, p, n, list);
 }
 
 // ------------------------------------------------------------- Harris

@@ -201,8 +201,9 @@ int stitch_pyramid_detect_describe(const stitch_image_view* image, const stitch_
 /* No reference counterpart. Chooses the exact binary matcher of the calling
  * host thread's later S4 launches (stitch_s4_* calls) and of the batch plans
  * and servers it creates afterwards: 0 the __popc tile kernel, 1 (the
- * default) the tcgen05 kind::i8 tensor-core kernel (descriptor bits as +-1
- * int8, Hamming = (256 - dot) / 2) with 256 train rows per MMA stage, 2 and
+ * default) the tcgen05 kind::i8 tensor-core kernel (query bits as +-1, train
+ * bits as 0 and 1, int8: Hamming = the query's bits set + dot) with 256 train
+ * rows per MMA stage, 2 and
  * 3 the same kernel with 128 and 64 train rows per stage (smaller blocks,
  * more of them per SM), 4 the pipelined tensor-core kernel (train-stage
  * expansion, MMAs and the top-2 epilogue of consecutive stages overlapped by

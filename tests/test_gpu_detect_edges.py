@@ -1,7 +1,8 @@
 """S2/S3 where the selection, the rank sort, the Harris loads, the describe
-rounds, the blur, FAST and the resize change path, bit for bit against the oracle: tie counts
-around the ranked and the listed ties, candidate counts around the rank
-kernel's blocks and tiles, aligned and odd pitches, saturated windows."""
+rounds, the blur, FAST and the resize change path, bit for bit against the
+oracle: tie counts around the ranked and the listed ties, candidate counts
+around the rank kernel's blocks and tiles, aligned and odd pitches, tile and
+band edges, saturated windows."""
 import numpy as np
 import pytest
 import torch
