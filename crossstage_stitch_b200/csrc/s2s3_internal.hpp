@@ -36,9 +36,9 @@ DescribeJob make_describe_job(const ImageView& im, const Keypoints& kp, const De
 // sort_topk_kernel. Measured, a rank block costs about 9.5 ns (a block has
 // some microseconds of latency, 592 run at once), and so does a key of the
 // largest job, padded to a power of two, per wave of sort blocks (one per job,
-// two per SM). K = 2000 at 8 layers: 4 pairs 20 us either way, 8 pairs 31
-// ranked, 21 sorted, 64 pairs 170 and 62; single level: 8 pairs 25 and 49;
-// K = 8000 at 8 layers, 2 pairs: 29 and 49.
+// two per SM). K = 2000 at 8 layers: 3 pairs 12 us ranked, 18 sorted, 4 pairs 20
+// and 16, 8 pairs 31 and 18, 64 pairs 170 and 29 (small sort blocks); single
+// level: 8 pairs 25 and 49; K = 8000 at 8 layers, 2 pairs: 29 and 49.
 inline bool rank_pays(long long harris_blocks, int jobs, int max_candidates) {
     long long keys = 1024;
     while (keys < max_candidates) keys *= 2;
