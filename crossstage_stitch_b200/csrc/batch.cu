@@ -41,6 +41,20 @@ template <class T> T* at(void* base, std::size_t off) { return at_offset<T>(base
 
 const ImageView& view(const stitch_image_view& v) { return *reinterpret_cast<const ImageView*>(&v); }
 
+// Rows of a resize tile: tall tiles share more of a tile's own work, but leave
+// fewer blocks, so they need two waves of them at the first resized layer. 64
+// pairs at 512x512 (2048 such tiles): layers 96 us by 64 rows, 94 by 128; 30
+// mixed pairs (about 10,000): 301 and 268.
+int resize_tile_rows(const std::vector<stitch_pair_desc>& pairs) {
+    long long tiles = 0;
+    for (const auto& q : pairs)
+        for (const auto* im : {&q.image_a, &q.image_b})
+            if (q.pyramid.levels > 1)
+                tiles += static_cast<long long>(ceil_div(static_cast<int>(im->width / q.pyramid.scale_factor), s2s3::kResizeTileW)) *
+                         ceil_div(static_cast<int>(im->height / q.pyramid.scale_factor), s2s3::kResizeTallH);
+    return tiles >= 2 * 5 * kSmCount ? s2s3::kResizeTallH : s2s3::kResizeTileH;
+}
+
 // Clears the counts and histograms at the start of the workspace. A kernel,
 // not a memset: a graph replay then holds no copy-engine work before its
 // first stage kernel, so it never queues behind an image upload running on
@@ -114,6 +128,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
         }
     }
     // 2. jobs per image: one single-level job, or one per pyramid layer
+    resize_tile_h = tuning.resize_tile_h ? tuning.resize_tile_h : resize_tile_rows(pairs);
     n_det = n_layers = n_resize = 0;
     max_levels = 1;
     for (int i = 0; i < n; ++i) {
@@ -130,7 +145,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
             }
             if (!s2s3::pyramid_layout(im.width, im.height, q.s2.max_keypoints, q.pyramid.levels,
                                       q.pyramid.scale_factor, &o.pyr[s],
-                                      tuning.resize_tile_h ? tuning.resize_tile_h : s2s3::kResizeTileH)) {
+                                      resize_tile_h)) {
                 if (bad_pair) *bad_pair = i;
                 return Status::INVALID_ARGUMENT;
             }
@@ -637,10 +652,13 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
     mark();  // tables uploaded, counts cleared
     for (int kind = 0; kind + 1 < max_levels; ++kind)  // layer kind + 1 of every pyramid image
         if (go(rs_blocks[kind])) {
-            switch (tuning.resize_tile_h) {
+            switch (resize_tile_h) {
                 case 16: s2s3::resize_kernel<RsSrc, 16><<<rs_blocks[kind], 256, 0, s>>>(rs, kind); break;
                 case 32: s2s3::resize_kernel<RsSrc, 32><<<rs_blocks[kind], 256, 0, s>>>(rs, kind); break;
-                default: s2s3::resize_kernel<RsSrc, s2s3::kResizeTileH><<<rs_blocks[kind], 256, 0, s>>>(rs, kind);
+                case s2s3::kResizeTileH:
+                    s2s3::resize_kernel<RsSrc, s2s3::kResizeTileH><<<rs_blocks[kind], 256, 0, s>>>(rs, kind);
+                    break;
+                default: s2s3::resize_kernel<RsSrc, s2s3::kResizeTallH><<<rs_blocks[kind], 256, 0, s>>>(rs, kind);
             }
         }
     mark();

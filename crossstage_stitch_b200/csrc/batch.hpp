@@ -54,6 +54,7 @@ public:
     int rs_blocks[s2s3::kMaxLevels] = {};  // resize launch of layer kind + 1
     int knn_blocks = 0, merge_blocks = 0, n_knn = 0;
     int search_blocks = 0, fit_blocks = 0;
+    int resize_tile_h = s2s3::kResizeTileH;  // output rows of a resize block
     int sort_smem = 0, search_smem = 0, finish_smem = 0;
     bool rank_fallback = false;  // a job has more candidates than the sort takes
     bool small_sorts = false;    // no job has more than kSortSmall candidates

@@ -63,7 +63,7 @@ bool pyramid_layout(int w, int h, int k, int levels, float sf, PyramidLayout* ou
         !valid_pyramid(levels, sf))
         return false;
     PyramidLayout l{};
-    if (resize_tile_h < 16 || resize_tile_h > kResizeTileH || resize_tile_h % 16) return false;
+    if (resize_tile_h < 16 || resize_tile_h > kResizeTallH || resize_tile_h % 16) return false;
     l.resize_tile_h = resize_tile_h;
     l.plan = level_plan(w, h, k, levels, sf);
     const int n = l.plan.levels;

@@ -82,7 +82,7 @@ struct PyramidLayout {
     std::size_t total;
 };
 
-// resize_tile_h: 64 rows per resize block when many images share a launch;
+// resize_tile_h: 64 or 128 rows per resize block when many images share a launch;
 // a single image's pyramid (kSingleResizeTileH) takes 16 to fill the GPU.
 constexpr int kSingleResizeTileH = 16;
 bool pyramid_layout(int w, int h, int k, int levels, float scale_factor, PyramidLayout* out,

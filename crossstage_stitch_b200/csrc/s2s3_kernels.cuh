@@ -225,7 +225,8 @@ __host__ __device__ inline int desc_keys(long long keypoints) {
     return kDescWarps * rounds;
 }
 constexpr int kEdge = 31;
-constexpr int kResizeTileW = 128, kResizeTileH = 64;  // tallest tile; a job's tile_h may be smaller
+constexpr int kResizeTileW = 128, kResizeTileH = 64;  // the tile of a launch over many images
+constexpr int kResizeTallH = 128;                     // and of one with tiles enough for it (resize_tile_rows)
 constexpr int kMaxLevels = 16;
 static_assert(kMaxLevels <= kMapKinds && kDetectKinds <= kMapKinds, "block map kinds");
 
@@ -1116,7 +1117,7 @@ __device__ __forceinline__ int2 linear_exact_tap(int v, int src, double scale) {
     return make_int2(static_cast<int>(fl), static_cast<int>(rint((f - fl) * 256.0)));
 }
 
-// One block = one tile of 128 x kTileH (16..64) layer pixels:
+// One block = one tile of 128 x kTileH (16..128) layer pixels:
 //   1. per-column and per-row taps in shared memory (double, as above);
 //   2. the tile's exact source window (rows of the first and last row taps,
 //      columns from the first column tap rounded down to 16 bytes) is
@@ -1141,8 +1142,9 @@ __device__ __forceinline__ int2 linear_exact_tap(int v, int src, double scale) {
 // 1..7 of 128 images of 512x512: 133 us walking every source row with the
 // output rows tested inside (34 instructions per pixel), 104 with this loop
 // (21), 96 with six blocks per SM instead of five; 30 mixed pairs: 442, 328
-// and 303 us.
-constexpr int kRawStride = 256;  // bytes of a staged source row: 16 chunks of 16
+// and 303 us. A third of that is made per tile (taps, window, selectors), so
+// tiles of 128 rows take 94 and 268 us.
+constexpr int kRawStride = 208;  // bytes of a staged source row: 13 chunks of 16
 template <int kTileH> __host__ __device__ constexpr int resize_raw_rows() { return kTileH * 3 / 2 + 6; }
 
 // Four output pixels of one row from the h of its upper and lower source rows.
@@ -1154,8 +1156,8 @@ __device__ __forceinline__ std::uint32_t resize_quad(const std::uint32_t (&ha)[4
 }
 
 template <class Src, int kTileH>
-__global__ __launch_bounds__(256, 6) void resize_kernel(const __grid_constant__ Src src, int kind) {
-    static_assert(kTileH >= 16 && kTileH <= kResizeTileH && kTileH % 16 == 0, "resize tile height");
+__global__ __launch_bounds__(256, kTileH > kResizeTileH ? 5 : 6) void resize_kernel(const __grid_constant__ Src src, int kind) {
+    static_assert(kTileH >= 16 && kTileH <= kResizeTallH && kResizeTileW + kTileH <= 256 && kTileH % 16 == 0, "resize tile height");
     constexpr int kBand = kTileH / 8, kRows = resize_raw_rows<kTileH>();
     __shared__ int2 xtap[kResizeTileW];
     __shared__ int2 ytap[kTileH];

@@ -324,12 +324,12 @@ int stitch_batch_create(int n_pairs, const stitch_pair_desc* pairs, stitch_batch
  * per plan by an autotuner (results never depend on them); 0 in a field
  * keeps its default. fast_ctas_per_sm: resident FAST blocks per SM in the
  * persistent FAST grid, 1..7 (default 7); blur_ctas_per_sm: the same for the
- * on-demand blur, 1..6 (default 6); matcher: 1 + an S4 matcher kind (0..4,
+ * on-demand blur, 1..6 (default 5); matcher: 1 + an S4 matcher kind (0..4,
  * as for stitch_s4_set_matcher), or 0 for the creating thread's choice;
  * search_hpw: MSAC hypotheses per warp (a block has 8 warps), 4, 8, 16 or 32
  * (default: the largest up to 16 that still fills a wave of four blocks per
  * SM); resize_tile_h: pyramid rows per resize block, 16, 32 or 64 (default
- * 64). */
+ * 64, and 128 in batches of enough tiles). */
 typedef struct stitch_batch_tuning {
     int fast_ctas_per_sm;
     int blur_ctas_per_sm;

@@ -118,3 +118,21 @@ def test_batched_sort_blocks(cuda, k):
         got = b.outputs(i // 2)["kp_a" if i % 2 == 0 else "kp_b"]
         want = s2s3.detect_and_describe(grays[i], 10, k)[0]
         assert want.shape[0] == k and np.array_equal(got, want)
+
+
+def test_batch_of_many_resize_tiles(cuda):
+    """Layers resized by tall tiles (two waves of 128 rows at the first resized
+    layer; odd sizes, part tiles) equal the per-pair call's."""
+    rng = np.random.default_rng(12)
+    pairs = [[rng.integers(0, 256, (h, w), dtype=np.uint8) for _ in range(2)] for w, h in ((3841, 2159), (3700, 2301))]
+    images = [[torch.from_numpy(g).cuda() for g in p] for p in pairs]
+    knobs = stages.Knobs(max_keypoints=1000, fast_threshold=40, hypotheses=64, levels=4, seed=3)
+    b = batch.Batch([batch.pair_desc(ia, ib, knobs) for ia, ib in images])
+    b.enqueue()
+    torch.cuda.synchronize()
+    runner = stages.PairRunner(3841, 2301, 1000, max_r=64)
+    for i, (ga, gb) in enumerate(pairs):
+        runner.run(ga, gb, knobs)
+        want, got = runner.download(), b.outputs(i)
+        for key in ("kp_a", "kp_b", "desc_a", "desc_b"):
+            assert np.array_equal(got[key], want[key]), (i, key)
