@@ -72,21 +72,16 @@ enum Table {
     kDetJobs, kDetPrefix, kDesJobs, kDesPrefix, kKnnJobs, kKnnPrefix, kMergePrefix, kAccJobs, kAccPrefix,
     kPairJobs, kPairPrefix, kSearchJobs, kSearchPrefix, kFitPrefix, kRsJobs, kRsPrefix, kBlockMap, kTables
 };
+static_assert(kTables <= 20, "table offsets");
 
-void set_attributes_once() {
-    static std::once_flag flag;
-    std::call_once(flag, [] {
-        static_assert(kTables <= 20, "table offsets");
-        cudaFuncSetAttribute(s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>, s2s3::kSortThreads>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             s2s3::kSortCap * static_cast<int>(sizeof(std::uint64_t)));
-        using Src = s5k::JobTable<SearchJob>;
-        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 32>), true);
-        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 64>), true);
-        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 128>), true);
-        s5k::enable_search_smem_once(reinterpret_cast<const void*>(s5k::search_kernel<Src, true, 256>), true);
-        s5k::enable_finish_smem_once(reinterpret_cast<const void*>(s5k::finish_kernel<s5k::JobTable<PairIO>>));
-    });
+// Opts the kernels in to their shared memory on the current device; false if it refuses.
+bool enable_kernels() {
+    using Src = s5k::JobTable<SearchJob>;
+    return enable_smem<s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>, s2s3::kSortThreads>>(
+               s2s3::kSortCap * static_cast<int>(sizeof(std::uint64_t))) &&
+           s5k::enable_search_smem<Src, true, 32>() && s5k::enable_search_smem<Src, true, 64>() &&
+           s5k::enable_search_smem<Src, true, 128>() && s5k::enable_search_smem<Src, true, 256>() &&
+           s5k::enable_finish_smem<s5k::JobTable<PairIO>>();
 }
 
 }  // namespace
@@ -595,9 +590,9 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
                      const unsigned char* device_tables) {
     if (!ws || !aligned(ws, kWorkspaceAlign)) return Status::INVALID_ARGUMENT;
     if (bytes < total) return Status::INSUFFICIENT_WORKSPACE;
-    set_attributes_once();
     const Status st = stage_tables(ws);
     if (st != Status::OK) return st;
+    if (!enable_kernels()) return Status::CUDA_ERROR;
     const unsigned char* T = device_tables;
     if (!T) {
         unsigned char* W = at<unsigned char>(ws, tables);

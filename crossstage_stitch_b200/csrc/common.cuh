@@ -6,6 +6,7 @@
 #include <climits>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 
 #include "stage_api.hpp"
 
@@ -47,6 +48,20 @@ inline void launch_chained(void (*kernel)(P...), int grid, int block, int smem, 
 
 __device__ __forceinline__ void wait_for_previous() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Opts a kernel in to `most` bytes of dynamic shared memory on the current
+// device; false if the device refuses. Once per device: the attribute belongs to
+// the device it was set on, and a process may use several.
+template <auto kKernel> bool enable_smem(int most) {
+    static std::once_flag flags[64];
+    static bool ok[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::call_once(flags[dev], [&] {
+        ok[dev] = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+    });
+    return ok[dev];
 }
 
 inline Status launch_status() {

@@ -91,16 +91,6 @@ int search_smem_bytes(int match_capacity, bool prefit) {
     return (n + (n & 1)) * static_cast<int>(sizeof(float4));  // staged two by two
 }
 
-bool enable_finish_smem_once(const void* fn) {
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, finish_smem_bytes(kFinishStage)) ==
-           cudaSuccess;
-}
-
-bool enable_search_smem_once(const void* fn, bool prefit) {
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                search_smem_bytes(INT_MAX, prefit)) == cudaSuccess;
-}
-
 }  // namespace stitch::b200::s5k
 
 namespace stitch::s5 {
@@ -110,11 +100,16 @@ using namespace ::stitch::b200::s5k;
 
 namespace {
 
+using SearchSrc = OneJob<SearchJob>;
+
+bool enable_kernels() {
+    return enable_search_smem<SearchSrc, false, 8>() && enable_search_smem<SearchSrc, false, 16>() &&
+           enable_search_smem<SearchSrc, false, 32>() && enable_search_smem<SearchSrc, false, 64>() &&
+           enable_finish_smem<OneJob<PairIO>>();
+}
+
 template <int kGroup> void launch_search(const SearchJob& sj, int match_capacity, cudaStream_t stream) {
-    using Src = OneJob<SearchJob>;
-    static const bool smem_ok =
-        enable_search_smem_once(reinterpret_cast<const void*>(search_kernel<Src, false, kGroup>), false);
-    (void)smem_ok;
+    using Src = SearchSrc;
     launch_chained(search_kernel<Src, false, kGroup>, sj.io.search_blocks, kSearchThreads, search_smem_bytes(match_capacity, false), stream, Src{sj});
 }
 
@@ -133,6 +128,7 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
     const Status chk = check_and_build(a, b, matches, scale_a, scale_b, config, inlier_mask, output, workspace,
                                        workspace_bytes, &io);
     if (chk != Status::OK) return chk;
+    if (!enable_kernels()) return Status::CUDA_ERROR;
     const int count = config.hypotheses - config.previous_hypotheses;
     // Hypotheses per block (8 * hpw) as few as keep the blocks, one per SM, in
     // one wave: a block's fit (one thread per hypothesis) takes about as long
@@ -153,9 +149,6 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
         note_launches(1);
         if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;
     }
-    static const bool finish_ok =
-        enable_finish_smem_once(reinterpret_cast<const void*>(finish_kernel<OneJob<PairIO>>));
-    (void)finish_ok;
     launch_chained(finish_kernel<OneJob<PairIO>>, 1, kFinishThreads, finish_smem_bytes(matches.capacity), stream, OneJob<PairIO>{io});
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;

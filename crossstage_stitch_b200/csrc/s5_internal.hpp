@@ -18,7 +18,13 @@ int plan_search(int count, int hpw);
 // Dynamic shared memory of a search block, with or without the models fitted
 // beforehand.
 int search_smem_bytes(int match_capacity, bool prefit);
-bool enable_search_smem_once(const void* fn, bool prefit);
-bool enable_finish_smem_once(const void* fn);
+// Opt the kernels of a job source in to their shared memory on the current
+// device; false if it refuses.
+template <class Src, bool kPrefit, int kGroup> bool enable_search_smem() {
+    return enable_smem<search_kernel<Src, kPrefit, kGroup>>(search_smem_bytes(INT_MAX, kPrefit));
+}
+template <class Src> bool enable_finish_smem() {
+    return enable_smem<finish_kernel<Src>>(finish_smem_bytes(kFinishStage));
+}
 
 }  // namespace stitch::b200::s5k
