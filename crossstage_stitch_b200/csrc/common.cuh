@@ -21,16 +21,20 @@ void note_launches(int n);
 
 // Launches of the per-image and per-pair calls: a kernel may be scheduled while
 // the one before it on the stream still runs, and holds at
-// wait_for_previous(), the first statement of every kernel launched this way
-// that touches memory, until that one has completed and its writes are
-// visible. Every kernel waits (whatever its blocks do afterwards), so "the one
-// before" has itself waited for all earlier work. A kernel lets the next one
-// be scheduled only once it has been released itself: let go before the wait,
-// several waiting kernels pile up on the chip and the blocks of the working
-// ones are placed unevenly (512x512 pair 219 us that way, 184 this way). These
-// calls are chains of some thirty short dependent kernels, in which the launch
-// latency is a large part: VGA single-level pair 133 -> 100 us, 512x512 at 8
-// layers 233 -> 184 us. The batched chain launches plainly.
+// wait_for_previous() until that one has completed and its writes are visible.
+// Before the wait a kernel reads its launch parameters and constant tables only,
+// and writes nothing but shared memory. Every kernel waits (whatever its blocks
+// do afterwards), so "the one before" has itself waited for all earlier work.
+// What the launch before writes is read by plain loads: a read-only load (__ldg)
+// promises that nobody writes during the whole kernel, the part before its wait
+// included, and the compiler may move it there. (Launches further back have
+// completed when a kernel starts.) A kernel lets the next one be scheduled only
+// once it has been released itself: let go before the wait, several waiting
+// kernels pile up on the chip and the blocks of the working ones are placed
+// unevenly (512x512 pair 219 us that way, 184 this way). These calls are chains
+// of some thirty short dependent kernels, in which the launch latency is a large
+// part: VGA single-level pair 133 -> 100 us, 512x512 at 8 layers 233 -> 184 us.
+// The batched chain launches plainly.
 template <class... P, class... A>
 inline void launch_chained(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg{};

@@ -1242,8 +1242,9 @@ __global__ __launch_bounds__(256, kTileH > kResizeTileH ? 5 : 6) void resize_ker
             std::uint32_t ha[4], hb[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const std::uint32_t wa = __ldg(A + tx[k].x) | (static_cast<std::uint32_t>(__ldg(A + xb[k])) << 8);
-                const std::uint32_t wb = __ldg(B + tx[k].x) | (static_cast<std::uint32_t>(__ldg(B + xb[k])) << 8);
+                // plain loads: the launch before may be the one that writes this layer's source
+                const std::uint32_t wa = A[tx[k].x] | (static_cast<std::uint32_t>(A[xb[k]]) << 8);
+                const std::uint32_t wb = B[tx[k].x] | (static_cast<std::uint32_t>(B[xb[k]]) << 8);
                 ha[k] = __dp2a_lo(wx[k], wa, 0u);
                 hb[k] = __dp2a_lo(wx[k], wb, 0u);
             }

@@ -240,7 +240,8 @@ __device__ __forceinline__ std::uint32_t pm_one4(std::uint32_t n) {
 }
 
 // kWords consecutive words of a descriptor row from `src` (16-byte aligned
-// row), zeros when src is null.
+// row), zeros when src is null. Plain loads: the describe kernel that writes the
+// rows may be the launch before, which this kernel overlaps (launch_chained).
 template <int kWords> struct Words {
     std::uint32_t w[kWords];
 };
@@ -250,14 +251,14 @@ template <int kWords> __device__ __forceinline__ Words<kWords> load_words(const 
         if constexpr (kWords >= 4) {
 #pragma unroll
             for (int i = 0; i < kWords / 4; ++i) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + i);
+                const uint4 v = reinterpret_cast<const uint4*>(src)[i];
                 r.w[4 * i] = v.x; r.w[4 * i + 1] = v.y; r.w[4 * i + 2] = v.z; r.w[4 * i + 3] = v.w;
             }
         } else if constexpr (kWords == 2) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+            const uint2 v = *reinterpret_cast<const uint2*>(src);
             r.w[0] = v.x; r.w[1] = v.y;
         } else {
-            r.w[0] = __ldg(reinterpret_cast<const std::uint32_t*>(src));
+            r.w[0] = *reinterpret_cast<const std::uint32_t*>(src);
         }
     }
     return r;
