@@ -9,11 +9,13 @@ height), captured as its own CUDA graph; BucketedBatch replays the graphs on
 a few streams so that the buckets' kernels overlap. Results never depend on
 the shapes: every plan equals the per-pair stages bit for bit.
 
-Tuner picks a bucket's shapes by coordinate descent from the defaults, one
-field at a time over its candidate values, timing the sub-batch's graph with
-CUDA events on the device (median of a few replays), and caches the choice
-in a JSON file keyed by (GPU name, bucket, K class): the STITCH_TUNE_CACHE
-path, else ~/.cache/crossstage_stitch_b200/tuning.json.
+Tuner picks a bucket's shapes by coordinate descent from the untuned plan's
+(every field 0), one field at a time over its candidate values, timing the
+sub-batch's graph with CUDA events on the device (median of a few replays), and
+caches the choice in a JSON file keyed by (GPU name, bucket, K class): the
+STITCH_TUNE_CACHE path, else ~/.cache/crossstage_stitch_b200/tuning.json. A
+cached choice is taken as it is: after an update of the library delete the file,
+since the shapes were measured with the kernels before.
 """
 from __future__ import annotations
 
@@ -29,14 +31,16 @@ from .stages import Knobs
 
 BUCKETS = (("vga", 640 * 480), ("720p", 1280 * 720), ("1080p", 1920 * 1080), ("4k", 3840 * 2160))
 K_CLASSES = (("k500", 1000), ("k2000", 4000), ("k8000", 1 << 30))
-# candidate values of each tuning field, the default first
+# candidate values of each tuning field beside 0, the plan's own choice
 SPACE = {
     "fast_ctas_per_sm": (7, 6, 4),
-    "resize_tile_h": (64, 32, 16),
-    "blur_ctas_per_sm": (6, 4),
+    "resize_tile_h": (64, 32, 16),   # 0: 128 in batches of enough tiles, else 64
+    "blur_ctas_per_sm": (5, 6, 4),
     "matcher": (2, 5),          # 1 + matcher kind: tensor cores, pipelined tensor cores
-    "search_hpw": (0, 8, 32),   # 0: chosen from the batch size
+    "search_hpw": (8, 32),      # 0: chosen from the batch size
 }
+# fields where 0 is the first candidate in every plan, which is not timed again
+FIXED = ("fast_ctas_per_sm", "blur_ctas_per_sm")
 
 
 def bucket_of(w_a: int, h_a: int, w_b: int, h_b: int) -> str:
@@ -95,10 +99,10 @@ class Tuner:
         key = self.key(group)
         if key in self.table:
             return dict(self.table[key]["tuning"])
-        best = {f: vals[0] for f, vals in SPACE.items()}
+        best = dict.fromkeys(SPACE, 0)
         default_ms = best_ms = self.time_plan(pairs, best)
         for field, vals in SPACE.items():
-            for v in vals[1:]:
+            for v in vals[1:] if field in FIXED else vals:
                 trial = dict(best, **{field: v})
                 ms = self.time_plan(pairs, trial)
                 if ms < best_ms:
