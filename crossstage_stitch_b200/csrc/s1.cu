@@ -13,7 +13,8 @@
 //   host      src/s1/s1.cu:209-320 argument order, one launch for a pair
 //
 // Both images of a pair run in one launch (blockIdx.z selects the image);
-// each thread produces 4 horizontally adjacent outputs.
+// each thread produces 4 horizontally adjacent outputs, or those of 48 source
+// bytes in the integer modes.
 #include <cmath>
 
 #include "s1_internal.hpp"
@@ -183,18 +184,23 @@ __device__ __forceinline__ void s1_outputs(const Params& p, int x, int y) {
         if (x + k < p.work_w) dst[k] = static_cast<std::uint8_t>(s1_pixel(p, x + k, y));
 }
 
-// Outputs of a thread of the per-image and per-pair kernel: 48 source bytes of
-// a row in the integer modes, 4 outputs in the others.
-__host__ __device__ constexpr int s1_run(int mode) { return mode < 3 ? 16 >> mode : 4; }
+// Outputs of a thread of s1_kernel<true>: 48 source bytes of a row in the
+// integer modes.
+__host__ __device__ constexpr int s1_run(int mode) { return 16 >> mode; }
 
-// Outputs x .. x + s1_run - 1 (those inside) of row y, as one run of 16-byte
-// loads and whole stores where the row allows it, by fours otherwise.
+// Whether an image goes by such runs: an integer mode, rows that 16-byte loads
+// and whole stores fit.
+inline bool s1_runs(const Params& p) {
+    return p.mode < 3 && ((reinterpret_cast<std::uintptr_t>(p.src) | static_cast<std::uintptr_t>(p.src_pitch)) & 15) == 0 &&
+           ((reinterpret_cast<std::uintptr_t>(p.dst) | static_cast<std::uintptr_t>(p.dst_pitch)) &
+            static_cast<std::uintptr_t>(s1_run(p.mode) - 1)) == 0;
+}
+
+// Outputs x .. x + s1_run - 1 of row y as one run, by fours at the row's end.
 template <int kFactor> __device__ __forceinline__ void s1_long(const Params& p, int x, int y) {
     constexpr int kOut = 16 / kFactor;
     std::uint8_t* dst = p.dst + static_cast<std::size_t>(y) * p.dst_pitch + x;
-    const std::uint8_t* src = p.src + static_cast<std::size_t>(kFactor * y) * p.src_pitch + 3 * kFactor * static_cast<std::size_t>(x);
-    if (x + kOut <= p.work_w && (reinterpret_cast<std::uintptr_t>(dst) & (kOut - 1)) == 0 &&
-        ((reinterpret_cast<std::uintptr_t>(src) | static_cast<std::uintptr_t>(p.src_pitch)) & 15) == 0) {
+    if (x + kOut <= p.work_w) {
         std::uint32_t out[kOut / 4];
         s1_words<kFactor, kOut>(p, x, y, out);
         if constexpr (kOut == 16) *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
@@ -207,16 +213,27 @@ template <int kFactor> __device__ __forceinline__ void s1_long(const Params& p, 
 
 constexpr int kS1BlockX = 16, kS1BlockY = 16;  // runs of columns x rows per block
 
-__global__ __launch_bounds__(kS1BlockX * kS1BlockY) void s1_kernel(const __grid_constant__ Pair pair) {
+// kRuns: every image of the call goes by runs (s1_runs); else a thread has four
+// outputs. Two kernels, since the runs take 64 registers, four blocks to an SM:
+// in one kernel the float filter, which is bound by its dependent loads and
+// sums, had half of its warps (3840x2160 pair at 0.6: 89 us; 80 at eight blocks;
+// 3839x2157 at 0.25: 53 both, and 61 at six blocks, where the last wave is nearly
+// empty), and rows that no run fits were read 48 bytes apart by fours (3839x2157
+// pair at 1: 36 us; 23 four outputs at a time).
+template <bool kRuns>
+__global__ __launch_bounds__(kS1BlockX * kS1BlockY, kRuns ? 4 : 8) void s1_kernel(const __grid_constant__ Pair pair) {
     const Params& p = pair.img[blockIdx.z];
-    const int x = s1_run(p.mode) * (blockIdx.x * kS1BlockX + threadIdx.x);
-    const int y = blockIdx.y * kS1BlockY + threadIdx.y;
+    const int column = blockIdx.x * kS1BlockX + threadIdx.x, y = blockIdx.y * kS1BlockY + threadIdx.y;
+    const int x = (kRuns ? s1_run(p.mode) : 4) * column;
     if (y >= p.work_h || x >= p.work_w) return;
-    switch (p.mode) {
-        case 0: s1_long<1>(p, x, y); break;
-        case 1: s1_long<2>(p, x, y); break;
-        case 2: s1_long<4>(p, x, y); break;
-        default: s1_outputs(p, x, y);
+    if constexpr (!kRuns) {
+        s1_outputs(p, x, y);
+    } else {
+        switch (p.mode) {
+            case 0: s1_long<1>(p, x, y); break;
+            case 1: s1_long<2>(p, x, y); break;
+            default: s1_long<4>(p, x, y);
+        }
     }
 }
 
@@ -316,15 +333,18 @@ Status scale_info(int w, int h, double s, ScaleInfo* out) {
 }
 
 Status launch(const Pair& pair, int images, cudaStream_t stream) {
-    int runs = 0, mh = 0;
+    bool by_runs = true;
+    for (int z = 0; z < images; ++z) by_runs = by_runs && s1_runs(pair.img[z]);
+    int columns = 0, mh = 0;
     for (int z = 0; z < images; ++z) {
         const Params& p = pair.img[z];
-        runs = max(runs, ceil_div(p.work_w, s1_run(p.mode)));
+        columns = max(columns, ceil_div(p.work_w, by_runs ? s1_run(p.mode) : 4));
         mh = max(mh, p.work_h);
     }
     const dim3 block(kS1BlockX, kS1BlockY);
-    const dim3 grid(ceil_div(runs, kS1BlockX), ceil_div(mh, kS1BlockY), images);
-    s1_kernel<<<grid, block, 0, stream>>>(pair);
+    const dim3 grid(ceil_div(columns, kS1BlockX), ceil_div(mh, kS1BlockY), images);
+    if (by_runs) s1_kernel<true><<<grid, block, 0, stream>>>(pair);
+    else s1_kernel<false><<<grid, block, 0, stream>>>(pair);
     note_launches(1);
     return launch_status();
 }
