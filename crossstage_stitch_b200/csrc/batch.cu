@@ -281,7 +281,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
                 }
             }
         }
-    rank = s2s3::rank_pays(det_total[s2s3::kHarrisKind], det_total[s2s3::kSortKind], max_cand);
+    rank_below = s2s3::rank_pays(det_total[s2s3::kHarrisKind], det_total[s2s3::kSortKind], max_cand) ? INT_MAX : 0;
     std::size_t map_entries = 0;
     for (int kind = 0; kind < s2s3::kDetectKinds; ++kind) {
         det_first[kind] = map_entries;
@@ -671,22 +671,26 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
     if (go(det_blocks[s2s3::kHarrisKind]))
         s2s3::harris_kernel<DetSrc><<<det_blocks[s2s3::kHarrisKind], s2s3::kHarrisThreads, 0, s>>>(det);
     mark();
-    if (rank) {
-        if (go(det_blocks[s2s3::kHarrisKind]))
-            s2s3::rank_topk_kernel<DetSrc>
-                <<<det_blocks[s2s3::kHarrisKind] * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, 0);
-    } else {
+    // top-K: jobs of up to rank_below keys ranked, of up to kSortCap sorted, the others ranked
+    const int harris_blocks = det_blocks[s2s3::kHarrisKind];
+    const auto rank_wide = [&](int above, int below) {
+        s2s3::rank_wide_kernel<DetSrc><<<s2s3::kRankGrid, s2s3::kRankThreads, 0, s>>>(det, above, below, harris_blocks);
+    };
+    if (rank_below > 0 && go(harris_blocks)) {
+        const long long slices = static_cast<long long>(harris_blocks) * s2s3::kRankPer;
+        if (slices > s2s3::kRankDirect) rank_wide(0, rank_below);
+        else s2s3::rank_topk_kernel<DetSrc><<<static_cast<int>(slices), s2s3::kRankThreads, 0, s>>>(det, 0, rank_below);
+    }
+    if (rank_below < s2s3::kSortCap) {
         const auto sort = [&](auto threads) {
             constexpr int kThreads = decltype(threads)::value;
-            s2s3::sort_topk_kernel<DetSrc, kThreads><<<det_blocks[s2s3::kSortKind], kThreads, sort_smem, s>>>(det);
+            s2s3::sort_topk_kernel<DetSrc, kThreads><<<det_blocks[s2s3::kSortKind], kThreads, sort_smem, s>>>(det, rank_below);
         };
         if (go(det_blocks[s2s3::kSortKind])) {
             if (small_sorts) sort(std::integral_constant<int, s2s3::kSortSmallThreads>{});
             else sort(std::integral_constant<int, s2s3::kSortThreads>{});
         }
-        if (rank_fallback && go(det_blocks[s2s3::kHarrisKind]))
-            s2s3::rank_topk_kernel<DetSrc>
-                <<<det_blocks[s2s3::kHarrisKind] * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, s2s3::kSortCap);
+        if (rank_fallback && go(harris_blocks)) rank_wide(s2s3::kSortCap, INT_MAX);
     }
     mark();
     if (go(tiles > 0 && blur_total > 0 ? 1 : 0))

@@ -58,7 +58,7 @@ public:
     int sort_smem = 0, search_smem = 0, finish_smem = 0;
     bool rank_fallback = false;  // a job has more candidates than the sort takes
     bool small_sorts = false;    // no job has more than kSortSmall candidates
-    bool rank = false;           // every job's candidates are ranked, not sorted
+    int rank_below = 0;          // jobs of at most so many keys are ranked, not sorted
     int desc_keys = 0;           // keypoints per describe block
     int hpw = 8;
     // binary matcher of this plan's S4 launches (s4k::kMatcherPopc or

@@ -152,11 +152,14 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
     const int harris_blocks = ceil_div(l.candidates, kHarrisThreads);
     launch_chained(harris_kernel<Src>, harris_blocks, kHarrisThreads, 0, stream, src);
     if (!record(e_harris, stream)) return Status::CUDA_ERROR;
+    int launches = 4;
     if (l.candidates > kSortCap || rank_pays(harris_blocks, 1, l.candidates))
-        launch_chained(rank_topk_kernel<Src>, harris_blocks * kRankPer, kRankThreads, 0, stream, src, 0);
+        launches = 3 + launch_rank<Src>(harris_blocks, l.candidates, [&](auto kernel, int blocks, auto... args) {
+            launch_chained(kernel, blocks, kRankThreads, 0, stream, src, args...);
+        });
     else
-        launch_chained(sort_topk_kernel<Src, kSortThreads>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src);
-    note_launches(4);
+        launch_chained(sort_topk_kernel<Src, kSortThreads>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src, 0);
+    note_launches(launches);
     return launch_status();
 }
 

@@ -984,7 +984,8 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
 }
 
 // One block per job: bitonic sort (descending) of up to kSortCap keys in
-// shared memory, then the first min(K, selected) become the keypoints. Bound by
+// shared memory, then the first min(K, selected) become the keypoints. Jobs with
+// at most `above` keys (0 at least) are left to the ranking. Bound by
 // instruction issue and barriers on the SMs that have a block: with at most
 // kSortSmall candidates a job, blocks of 256 threads leave eight jobs to an SM
 // (1024 jobs of 64 pairs at 8 layers, K = 2000: 45 us with 1024 threads, 31 with
@@ -992,14 +993,14 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
 // want them all (30 mixed pairs, K up to 8000: 83, 86 and 100 us, and 106 in two
 // launches that divide the jobs).
 template <class Src, int kThreads>
-__global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_constant__ Src src) {
+__global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_constant__ Src src, int above) {
     wait_for_previous();
     extern __shared__ std::uint64_t sk[];
     DetectJob j;
     int local;
     if (!src.find(blockIdx.x, kSortKind, &j, &local)) return;
     const int n = static_cast<int>(j.params->selected);
-    if (n > kSortCap || n == 0) return;
+    if (n > kSortCap || n <= above) return;
     int N = kSortChunk;  // at least one 64-key chunk (zero keys pad and sort last)
     while (N < n) N <<= 1;
     for (int i = threadIdx.x; i < N; i += kThreads) sk[i] = i < n ? j.keys[i] : 0ull;
@@ -1057,12 +1058,13 @@ __global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_consta
 // Top-K by counting: the rank of a key is the number of larger keys (keys are
 // unique). A block ranks kRankKeys keys, one per lane; its 16 warps share the
 // comparisons with every key of the job, staged kRankTile at a time. Jobs with
-// at most `above` keys are left to the sort. Counting n keys costs n^2
+// at most `above` keys are left to the sort, those with more than `below` to
+// rank_wide_kernel. Counting n keys costs n^2
 // comparisons, but spread over the whole chip, where the sort has one block
 // per job: one 512x512 image, 8 layers: 12 -> 6 us; 4K, K = 8000: 46 -> 14 us.
 // rank_pays draws the line between the two.
 template <class Src>
-__global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_constant__ Src src, int above) {
+__global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_constant__ Src src, int above, int below) {
     wait_for_previous();
     __shared__ __align__(16) std::uint64_t tile[kRankTile];
     __shared__ int part[kRankThreads / 32][kRankKeys];
@@ -1072,7 +1074,7 @@ __global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_co
     if (!src.find(blockIdx.x / kRankPer, kHarrisKind, &j, &local)) return;
     const int first = (local * kRankPer + static_cast<int>(blockIdx.x % kRankPer)) * kRankKeys;
     const int n = static_cast<int>(j.params->selected);
-    if (n <= above || first >= n) return;  // block-uniform
+    if (n <= above || n > below || first >= n) return;  // block-uniform
     const int t = threadIdx.x, k = t % kRankKeys, slice = t / kRankKeys;
     const int slot = first + k;
     const std::uint64_t key = slot < n ? j.keys[slot] : ~0ull;
@@ -1096,6 +1098,96 @@ __global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_co
         for (int v = 1; v < kRankThreads / 32; ++v) rank += part[v][k];
         if (rank < j.max_keypoints) write_keypoint(j, rank, key);
     }
+}
+
+// The same with kRankGrid blocks, each of which looks for the harris blocks that
+// hold keys among its share of the launch with all its threads, and kRankWide keys per
+// lane, for two kinds of launches:
+// - of batches that would take more than kRankDirect blocks above. A slice without
+//   keys, whose job lookup is a chain of loads, costs 2.2 ns as a block of its own:
+//   32 pairs of 800x600, K = 20000, some 400 keypoints each, sort and rank 210 us
+//   so, 54 here (an image's own launch has no lookup: 0.4 ns);
+// - of jobs of very many keys, which fill the chip's block slots all the same: a key
+//   read from shared memory is compared four times. 64 jobs of 40000 keys: 18.3 ms
+//   above, 14.4 here; one of 400000: 27.1 and 22.0.
+constexpr int kRankDirect = 12 * 148, kRankGrid = 8 * 148, kRankWide = 4;
+constexpr int kRankMany = 1 << 17;  // an image's jobs of more keys are ranked here
+static_assert(kRankKeys * kRankWide == kHarrisThreads, "a block ranks a harris block's keys");
+
+template <class Src>
+__global__ __launch_bounds__(kRankThreads, 3) void rank_wide_kernel(const __grid_constant__ Src src, int above, int below, int harris_blocks) {
+    wait_for_previous();
+    __shared__ __align__(16) std::uint64_t tile[kRankTile];
+    __shared__ int part[kRankThreads / 32][kHarrisThreads];
+    __shared__ int found[kRankThreads], n_found;
+    const int t = threadIdx.x, lane = t % 32, warp = t / 32, grid = gridDim.x;
+    // first key and key count of harris block b; false when it has nothing to rank
+    const auto lookup = [&](int b, DetectJob* j, int* first, int* n) {
+        int local;
+        if (!src.find(b, kHarrisKind, j, &local)) return false;
+        *first = local * kHarrisThreads;
+        *n = static_cast<int>(j->params->selected);
+        return *n > above && *n <= below && *first < *n;
+    };
+    for (int base = blockIdx.x; base < harris_blocks; base += grid * kRankThreads) {
+        if (t == 0) n_found = 0;
+        __syncthreads();
+        {
+            const long long mine = base + static_cast<long long>(grid) * t;
+            DetectJob j;
+            int first, n;
+            if (mine < harris_blocks && lookup(static_cast<int>(mine), &j, &first, &n))
+                found[atomicAdd(&n_found, 1)] = static_cast<int>(mine);
+        }
+        __syncthreads();
+        const int todo = n_found;
+        for (int f = 0; f < todo; ++f) {
+            DetectJob j;
+            int first, n;
+            lookup(found[f], &j, &first, &n);
+            std::uint64_t key[kRankWide];
+            int rank[kRankWide];
+#pragma unroll
+            for (int p = 0; p < kRankWide; ++p) {
+                const int slot = first + 32 * p + lane;
+                key[p] = slot < n ? j.keys[slot] : ~0ull;
+                rank[p] = 0;
+            }
+            for (int b0 = 0; b0 < n; b0 += kRankTile) {
+                if (b0 || f) __syncthreads();
+#pragma unroll
+                for (int i = t; i < kRankTile; i += kRankThreads) tile[i] = b0 + i < n ? j.keys[b0 + i] : 0ull;
+                __syncthreads();
+                const int m = min(kRankTile, (n - b0 + 1) / 2 * 2);  // keys past n are 0, never larger
+#pragma unroll 4
+                for (int i = 2 * warp; i < m; i += 2 * (kRankThreads / 32)) {
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(tile + i);
+#pragma unroll
+                    for (int p = 0; p < kRankWide; ++p) rank[p] += (q.x > key[p]) + (q.y > key[p]);
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < kRankWide; ++p) part[warp][32 * p + lane] = rank[p];
+            __syncthreads();
+            if (t < kHarrisThreads && first + t < n) {
+                int r = 0;
+#pragma unroll
+                for (int v = 0; v < kRankThreads / 32; ++v) r += part[v][t];
+                if (r < j.max_keypoints) write_keypoint(j, r, j.keys[first + t]);
+            }
+        }
+        __syncthreads();  // found, n_found and part are read before they are written again
+    }
+}
+
+// Launches the ranking of one image's jobs of up to max_candidates candidates, in
+// all `harris_blocks` blocks of them, through go(kernel, blocks, arguments after
+// the source ...). Returns the launches.
+template <class Src, class Go> inline int launch_rank(int harris_blocks, int max_candidates, Go go) {
+    const bool many = max_candidates > kRankMany;
+    go(rank_topk_kernel<Src>, harris_blocks * kRankPer, 0, many ? kRankMany : INT_MAX);
+    if (many) go(rank_wide_kernel<Src>, kRankGrid, kRankMany, INT_MAX, harris_blocks);
+    return many ? 2 : 1;
 }
 
 // ------------------------------------------------------ pyramid layers

@@ -2,8 +2,9 @@
 // the first alone: the built objects are linked to the CUDA runtime below, which
 // keeps kernel attributes per device, as the real one does, and refuses a launch
 // with more than 48 KB of dynamic shared memory of a kernel that was not opted
-// in on the current device. Nothing runs on a GPU. Built and run by
-// tests/test_multi_device.py.
+// in on the current device. It also checks the blocks of a batch whose jobs have
+// far more candidates than keys may be there. Nothing runs on a GPU. Built and run
+// by tests/test_multi_device.py.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -22,7 +23,10 @@ bool refuse_attributes = false;
 std::map<std::pair<int, const void*>, std::size_t> opted;
 cudaError_t last = cudaSuccess;
 
-cudaError_t launch(const void* kernel, std::size_t smem) {
+unsigned rank_blocks = 0;  // most blocks of 512 threads, the ranking's, of a launch
+
+cudaError_t launch(const void* kernel, dim3 grid, dim3 block, std::size_t smem) {
+    if (block.x == 512 && grid.x > rank_blocks) rank_blocks = grid.x;
     const auto it = opted.find({device, kernel});
     const std::size_t limit = it == opted.end() ? 48 * 1024 : it->second;
     ++launches;
@@ -69,8 +73,12 @@ cudaError_t cudaFuncSetAttribute(const void* kernel, cudaFuncAttribute a, int va
     if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) opted[{device, kernel}] = static_cast<std::size_t>(value);
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* kernel, dim3, dim3, void**, std::size_t smem, cudaStream_t) { return launch(kernel, smem); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel, void**) { return launch(kernel, c->dynamicSmemBytes); }
+cudaError_t cudaLaunchKernel(const void* kernel, dim3 grid, dim3 block, void**, std::size_t smem, cudaStream_t) {
+    return launch(kernel, grid, block, smem);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel, void**) {
+    return launch(kernel, c->gridDim, c->blockDim, c->dynamicSmemBytes);
+}
 cudaError_t cudaMemcpyAsync(void*, const void*, std::size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaMemcpy2DAsync(void*, std::size_t, const void*, std::size_t, std::size_t, std::size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaMemcpyFromSymbol(void* d, const void*, std::size_t n, std::size_t, cudaMemcpyKind) { return std::memset(d, 0, n), cudaSuccess; }
@@ -152,12 +160,13 @@ int detect_and_match(const Buffers& b, int k) {
     return st;
 }
 
-int batch(const Buffers& b, int k, int levels, const stitch_batch_tuning* tuning) {
-    const std::vector<stitch_pair_desc> pairs = {pair(b, k, 2000, levels), pair(b, 500, 500, levels)};
+int batch(const Buffers& b, int k, int levels, const stitch_batch_tuning* tuning, int copies = 1) {
+    std::vector<stitch_pair_desc> pairs(copies, pair(b, k, 2000, levels));
+    pairs.push_back(pair(b, 500, 500, levels));
     stitch_batch* plan = nullptr;
     std::size_t bytes = 0;
     int bad = -1;
-    int st = stitch_batch_create_tuned(2, pairs.data(), tuning, &plan, &bytes, &bad);
+    int st = stitch_batch_create_tuned(static_cast<int>(pairs.size()), pairs.data(), tuning, &plan, &bytes, &bad);
     if (st) return st;
     void* ws = host_memory(bytes);
     st = stitch_batch_enqueue(plan, ws, bytes, nullptr, nullptr);
@@ -185,6 +194,10 @@ int main() {
         }
         if (refused) return std::printf("device %d: %d launches refused\n", d, refused), 1;
     }
+    // 32 pairs of 2 x 40000 candidates: a block per 32 of them would be 80,000 blocks
+    rank_blocks = 0;
+    if (const int st = batch(b, 20000, 1, nullptr, 32)) return std::printf("large batch: status %d\n", st), 1;
+    if (rank_blocks == 0 || rank_blocks > 2000) return std::printf("%u blocks of the ranking\n", rank_blocks), 1;
     // a device that refuses the attribute: an error, and no launch that would fail
     cudaSetDevice(3);
     refuse_attributes = true;
