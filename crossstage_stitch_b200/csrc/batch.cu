@@ -168,7 +168,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     Layout lay;
     const std::size_t counts = lay.take(3 * static_cast<std::size_t>(n) + n_layers, sizeof(int));
     hists = lay.take(static_cast<std::size_t>(std::max(n_det, 1)) * s2s3::kHistWords, sizeof(std::uint32_t));
-    queue = lay.take(2, sizeof(std::uint32_t));
+    queue = lay.take(8, sizeof(std::uint32_t));  // FAST tile queue, blur-list count, -, -, RankTotals
     blur_flags = lay.take(std::max<std::size_t>(blur_total, 1), sizeof(std::uint32_t));
     zeroed = lay.cursor;
     blur_list = lay.take(std::max<std::size_t>(blur_total, 1), sizeof(uint2));
@@ -260,6 +260,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     std::fill(std::begin(des_total), std::end(des_total), 0);
     std::fill(std::begin(rs_total), std::end(rs_total), 0);
     std::fill(std::begin(s45_total), std::end(s45_total), 0);
+    float sum = 0.0f, squares = 0.0f;  // of the candidates that a job's sort takes
     bool map_fits = alloc_staging && n_det < (1 << 16) && n_resize < (1 << 16);
     for (int i = 0; i < n; ++i)
         for (int s = 0; s < 2; ++s) {
@@ -267,6 +268,11 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
             for (int l = 0; l < L; ++l) {
                 int db[s2s3::kDetectKinds], sb[s2s3::kDescribeKinds];
                 job_blocks(i, s, l, db, sb);
+                if (db[s2s3::kSortKind]) {
+                    const float c = static_cast<float>(std::min((off[i].pyramid[s] ? off[i].pyr[s].det[l] : off[i].det[s]).candidates, s2s3::kSortCap));
+                    sum += c;
+                    squares += c * c;
+                }
                 for (int kind = 0; kind < s2s3::kDetectKinds; ++kind) {
                     det_total[kind] += db[kind];
                     map_fits = map_fits && db[kind] < (1 << 16);
@@ -281,7 +287,11 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
                 }
             }
         }
-    rank_below = s2s3::rank_pays(det_total[s2s3::kHarrisKind], det_total[s2s3::kSortKind], max_cand) ? INT_MAX : 0;
+    topk = kSorted;
+    if (s2s3::rank_pays(det_total[s2s3::kHarrisKind], det_total[s2s3::kSortKind], max_cand))
+        topk = s2s3::rank_cost(squares, sum, std::min(max_cand, s2s3::kSortCap), det_total[s2s3::kSortKind], rank_wide()) <= 1.25f
+                   ? kRanked  // deciding would cost more than it could gain
+                   : kByCounts;
     std::size_t map_entries = 0;
     for (int kind = 0; kind < s2s3::kDetectKinds; ++kind) {
         det_first[kind] = map_entries;
@@ -658,6 +668,7 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
         }
     mark();
     std::uint32_t* q = at<std::uint32_t>(ws, queue);  // FAST tile queue, then the blur-list count
+    auto* totals = reinterpret_cast<s2s3::RankTotals*>(q + 4);
     const int tiles = det_blocks[s2s3::kFastKind];
     if (go(tiles))
         s2s3::fast_kernel<DetSrc><<<std::min(tiles, kSmCount * (tuning.fast_ctas_per_sm ? tuning.fast_ctas_per_sm
@@ -665,32 +676,32 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
                                     s2s3::kFastThreads, 0, s>>>(det, q, tiles);
     mark();
     if (go(det_blocks[s2s3::kSelectKind])) {
-        s2s3::select_kernel<DetSrc><<<det_blocks[s2s3::kSelectKind], 256, 0, s>>>(det);
+        s2s3::select_kernel<DetSrc><<<det_blocks[s2s3::kSelectKind], 256, 0, s>>>(det, topk == kByCounts ? totals : nullptr);
     }
     mark();
     if (go(det_blocks[s2s3::kHarrisKind]))
         s2s3::harris_kernel<DetSrc><<<det_blocks[s2s3::kHarrisKind], s2s3::kHarrisThreads, 0, s>>>(det);
     mark();
-    // top-K: jobs of up to rank_below keys ranked, of up to kSortCap sorted, the others ranked
     const int harris_blocks = det_blocks[s2s3::kHarrisKind];
-    const auto rank_wide = [&](int above, int below) {
-        s2s3::rank_wide_kernel<DetSrc><<<s2s3::kRankGrid, s2s3::kRankThreads, 0, s>>>(det, above, below, harris_blocks);
+    const s2s3::RankChoice choice{topk == kByCounts ? totals : nullptr, det_blocks[s2s3::kSortKind], rank_wide()};
+    const int cap = s2s3::kSortCap, below = topk == kRanked ? INT_MAX : cap;
+    const auto wide = [&](int above, int most, const s2s3::RankChoice& c) {
+        s2s3::rank_wide_kernel<DetSrc><<<s2s3::kRankGrid, s2s3::kRankThreads, 0, s>>>(det, above, most, harris_blocks, c);
     };
-    if (rank_below > 0 && go(harris_blocks)) {
-        const long long slices = static_cast<long long>(harris_blocks) * s2s3::kRankPer;
-        if (slices > s2s3::kRankDirect) rank_wide(0, rank_below);
-        else s2s3::rank_topk_kernel<DetSrc><<<static_cast<int>(slices), s2s3::kRankThreads, 0, s>>>(det, 0, rank_below);
+    if (topk != kSorted && go(harris_blocks)) {
+        if (rank_wide()) wide(0, below, choice);
+        else s2s3::rank_topk_kernel<DetSrc><<<harris_blocks * s2s3::kRankPer, s2s3::kRankThreads, 0, s>>>(det, below, choice);
     }
-    if (rank_below < s2s3::kSortCap) {
+    if (topk != kRanked) {
         const auto sort = [&](auto threads) {
             constexpr int kThreads = decltype(threads)::value;
-            s2s3::sort_topk_kernel<DetSrc, kThreads><<<det_blocks[s2s3::kSortKind], kThreads, sort_smem, s>>>(det, rank_below);
+            s2s3::sort_topk_kernel<DetSrc, kThreads><<<det_blocks[s2s3::kSortKind], kThreads, sort_smem, s>>>(det, choice);
         };
         if (go(det_blocks[s2s3::kSortKind])) {
             if (small_sorts) sort(std::integral_constant<int, s2s3::kSortSmallThreads>{});
             else sort(std::integral_constant<int, s2s3::kSortThreads>{});
         }
-        if (rank_fallback && go(harris_blocks)) rank_wide(s2s3::kSortCap, INT_MAX);
+        if (rank_fallback && go(harris_blocks)) wide(cap, INT_MAX, s2s3::RankChoice{});
     }
     mark();
     if (go(tiles > 0 && blur_total > 0 ? 1 : 0))

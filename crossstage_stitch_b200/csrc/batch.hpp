@@ -44,8 +44,8 @@ public:
     int n_resize = 0;  // resize jobs (layers 1.. of every pyramid image)
     int max_levels = 1;
     // zeroed head of the workspace: counts, then FAST histograms and counters
-    // u32[n_det][kHistWords], the FAST tile queue and blur-list count (2
-    // words), the blur-tile flags u32[blur_total]; `zeroed` bytes in all.
+    // u32[n_det][kHistWords], the FAST tile queue, the blur-list count and the
+    // RankTotals (8 words), the blur-tile flags u32[blur_total]; `zeroed` bytes in all.
     // The blur list uint2[blur_total] follows the head.
     std::size_t hists = 0, queue = 0, blur_flags = 0, zeroed = 0, blur_list = 0;
     std::size_t blur_total = 0;
@@ -58,7 +58,11 @@ public:
     int sort_smem = 0, search_smem = 0, finish_smem = 0;
     bool rank_fallback = false;  // a job has more candidates than the sort takes
     bool small_sorts = false;    // no job has more than kSortSmall candidates
-    int rank_below = 0;          // jobs of at most so many keys are ranked, not sorted
+    enum TopK { kSorted, kRanked, kByCounts };
+    TopK topk = kSorted;         // kByCounts: decided on the device (RankChoice)
+    bool rank_wide() const {     // which ranking kernel
+        return static_cast<long long>(det_total[s2s3::kHarrisKind]) * s2s3::kRankPer > s2s3::kRankDirect;
+    }
     int desc_keys = 0;           // keypoints per describe block
     int hpw = 8;
     // binary matcher of this plan's S4 launches (s4k::kMatcherPopc or

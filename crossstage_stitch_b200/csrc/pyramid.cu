@@ -243,7 +243,7 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
     if (blocks(kFastKind)) {
         launch_chained(fast_kernel<DetSrc>, std::min(blocks(kFastKind), kSmCount * kFastCtasPerSm), kFastThreads, 0, stream,
             det, queue, blocks(kFastKind));
-        launch_chained(select_kernel<DetSrc>, blocks(kSelectKind), 256, 0, stream, det);
+        launch_chained(select_kernel<DetSrc>, blocks(kSelectKind), 256, 0, stream, det, nullptr);
         launch_chained(harris_kernel<DetSrc>, blocks(kHarrisKind), kHarrisThreads, 0, stream, det);
         launches += 4;
         if (max_cand > kSortCap || rank_pays(blocks(kHarrisKind), blocks(kSortKind), max_cand))
@@ -251,7 +251,7 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
                 launch_chained(kernel, grid, kRankThreads, 0, stream, det, args...);
             }) - 1;
         else
-            launch_chained(sort_topk_kernel<DetSrc, kSortThreads>, blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream, det, 0);
+            launch_chained(sort_topk_kernel<DetSrc, kSortThreads>, blocks(kSortKind), kSortThreads, sort_smem_bytes(max_cand), stream, det, RankChoice{});
         launch_chained(blur_tiles_kernel<DesSrc, true>, std::max(1, std::min(l.blur_first[n], kSmCount * kBlurCtasPerSm)), kBlurThreads, 0, stream,
             des, at_offset<uint2>(ws, l.blur_list), queue + 1, 0);
         ++launches;

@@ -147,7 +147,7 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
     const int fast_grid = std::min(l.tiles, kSmCount * kFastCtasPerSm);
     launch_chained(fast_kernel<Src>, fast_grid, kFastThreads, 0, stream, src, src.job.counters() + kTileQueue, l.tiles);
     if (!record(e_fast, stream)) return Status::CUDA_ERROR;
-    launch_chained(select_kernel<Src>, l.select_blocks, 256, 0, stream, src);
+    launch_chained(select_kernel<Src>, l.select_blocks, 256, 0, stream, src, nullptr);
     if (!record(e_select, stream)) return Status::CUDA_ERROR;
     const int harris_blocks = ceil_div(l.candidates, kHarrisThreads);
     launch_chained(harris_kernel<Src>, harris_blocks, kHarrisThreads, 0, stream, src);
@@ -158,7 +158,7 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
             launch_chained(kernel, blocks, kRankThreads, 0, stream, src, args...);
         });
     else
-        launch_chained(sort_topk_kernel<Src, kSortThreads>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src, 0);
+        launch_chained(sort_topk_kernel<Src, kSortThreads>, 1, kSortThreads, sort_smem_bytes(l.candidates), stream, src, RankChoice{});
     note_launches(launches);
     return launch_status();
 }

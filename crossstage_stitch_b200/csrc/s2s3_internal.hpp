@@ -32,13 +32,12 @@ DetectJob make_detect_job(const ImageView& im, const s2::Config& c, const Keypoi
                           const DetectLayout& l);
 DescribeJob make_describe_job(const ImageView& im, const Keypoints& kp, const Descriptors& out, void* ws,
                               const DescribeLayout& l);
-// Whether rank_topk_kernel orders a launch's jobs faster than
-// sort_topk_kernel. Measured, a rank block costs about 9.5 ns (a block has
-// some microseconds of latency, 592 run at once), and so does a key of the
-// largest job, padded to a power of two, per wave of sort blocks (one per job,
-// two per SM). K = 2000 at 8 layers: 3 pairs 12 us ranked, 18 sorted, 4 pairs 20
-// and 16, 8 pairs 31 and 18, 64 pairs 170 and 29 (small sort blocks); single
-// level: 8 pairs 25 and 49; K = 8000 at 8 layers, 2 pairs: 29 and 49.
+// Whether rank_topk_kernel may order a launch's jobs faster than
+// sort_topk_kernel, by their capacities: always for one image; a rank block costs
+// about 9.5 ns (a block has some microseconds of latency, 592 run at once), and so
+// does a key of the largest job, padded to a power of two, per wave of sort blocks
+// (one per job, two per SM). K = 2000 at 8 layers: 3 pairs 12 us ranked, 18 sorted,
+// 4 pairs 20 and 18, 8 pairs 28 and 18, 64 pairs 94 and 46.
 inline bool rank_pays(long long harris_blocks, int jobs, int max_candidates) {
     long long keys = 1024;
     while (keys < max_candidates) keys *= 2;

@@ -30,6 +30,13 @@ struct SelectParams {
     std::uint32_t selected;   // above + ties
 };
 
+// Keys of the jobs of a batch that the sort takes, summed up by the selection
+// (zeroed per run).
+struct RankTotals {
+    unsigned long long squares;
+    std::uint32_t sum, largest;
+};
+
 // Per-job counters of the detect kernels, after the 256 histogram bins.
 enum DetectCounter {
     kListed, kAboveWritten, kTiesWritten, kTileQueue,
@@ -806,7 +813,7 @@ __device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams
 // them in the last block saves a launch. Select and ties together, 512x512:
 // 18.5 -> 7 us, 4K: 67 -> 23 us.
 template <class Src>
-__global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src src) {
+__global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src src, RankTotals* totals) {
     wait_for_previous();
     __shared__ std::uint32_t suffix[257];
     __shared__ SelectParams sp;
@@ -818,6 +825,11 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
     if (local == 0 && threadIdx.x == 0) {
         *j.params = p;
         *j.count = static_cast<int>(min(p.selected, static_cast<std::uint32_t>(j.max_keypoints)));
+        if (totals && p.selected <= kSortCap) {
+            atomicAdd(&totals->squares, static_cast<unsigned long long>(p.selected) * p.selected);
+            atomicAdd(&totals->sum, p.selected);
+            atomicMax(&totals->largest, p.selected);
+        }
     }
     const bool all_ties = p.ties == j.hist[p.threshold];
     std::uint32_t* ctr = j.counters();
@@ -983,9 +995,33 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
     if (j.blur_marks) mark_blur_tiles(j, static_cast<int>(x), static_cast<int>(y));
 }
 
+// Time of ranking `jobs` jobs with `sum` keys in all, `squares` comparisons and
+// `largest` keys in one, by that of sorting them. Measured in ns: the ranking takes 8 us,
+// 4 ns per 32 keys and a rate, 4 comparisons per ps in slices of 32 keys and 6.4 in
+// wide ones; the sort 6 us and 10.2 ns per key of the largest job, padded to a power of
+// two, for every wave of blocks (one per job, two per SM). 800x600 noise, K keypoints
+// at one level, ranked and sorted: 4 pairs, K = 1000 18 and 26 us, 4000 102 and 90, 8000
+// 315 and 186; 8 pairs, K = 2000 57 and 45; 16 pairs, K = 4000 312 and 90.
+__host__ __device__ inline float rank_cost(float squares, float sum, int largest, int jobs, bool wide) {
+    int keys = 1024;
+    while (keys < largest) keys *= 2;
+    const float rank = 8000.0f + 0.125f * sum + 4.0f * jobs + (wide ? 0.156e-3f : 0.25e-3f) * squares;
+    return rank / (6000.0f + 10.2f * keys * ((jobs + 2 * 148 - 1) / (2 * 148)));
+}
+
+// Where the capacities leave it open (totals not null), the kernels of both ways are
+// launched and decide by the keys that are there: the idle one costs 3 to 5 us.
+struct RankChoice {
+    const RankTotals* totals;
+    int jobs;
+    bool wide;
+    __device__ __forceinline__ bool ranked() const {
+        return rank_cost(static_cast<float>(totals->squares), static_cast<float>(totals->sum), static_cast<int>(totals->largest), jobs, wide) <= 1.0f;
+    }
+};
+
 // One block per job: bitonic sort (descending) of up to kSortCap keys in
-// shared memory, then the first min(K, selected) become the keypoints. Jobs with
-// at most `above` keys (0 at least) are left to the ranking. Bound by
+// shared memory, then the first min(K, selected) become the keypoints. Bound by
 // instruction issue and barriers on the SMs that have a block: with at most
 // kSortSmall candidates a job, blocks of 256 threads leave eight jobs to an SM
 // (1024 jobs of 64 pairs at 8 layers, K = 2000: 45 us with 1024 threads, 31 with
@@ -993,14 +1029,15 @@ __device__ __forceinline__ void write_keypoint(const DetectJob& j, int rank, std
 // want them all (30 mixed pairs, K up to 8000: 83, 86 and 100 us, and 106 in two
 // launches that divide the jobs).
 template <class Src, int kThreads>
-__global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_constant__ Src src, int above) {
+__global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_constant__ Src src, RankChoice choice) {
     wait_for_previous();
+    if (choice.totals && choice.ranked()) return;
     extern __shared__ std::uint64_t sk[];
     DetectJob j;
     int local;
     if (!src.find(blockIdx.x, kSortKind, &j, &local)) return;
     const int n = static_cast<int>(j.params->selected);
-    if (n > kSortCap || n <= above) return;
+    if (n > kSortCap || n == 0) return;
     int N = kSortChunk;  // at least one 64-key chunk (zero keys pad and sort last)
     while (N < n) N <<= 1;
     for (int i = threadIdx.x; i < N; i += kThreads) sk[i] = i < n ? j.keys[i] : 0ull;
@@ -1058,14 +1095,14 @@ __global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_consta
 // Top-K by counting: the rank of a key is the number of larger keys (keys are
 // unique). A block ranks kRankKeys keys, one per lane; its 16 warps share the
 // comparisons with every key of the job, staged kRankTile at a time. Jobs with
-// at most `above` keys are left to the sort, those with more than `below` to
-// rank_wide_kernel. Counting n keys costs n^2
+// more than `below` keys are left to rank_wide_kernel. Counting n keys costs n^2
 // comparisons, but spread over the whole chip, where the sort has one block
 // per job: one 512x512 image, 8 layers: 12 -> 6 us; 4K, K = 8000: 46 -> 14 us.
 // rank_pays draws the line between the two.
 template <class Src>
-__global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_constant__ Src src, int above, int below) {
+__global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_constant__ Src src, int below, RankChoice choice) {
     wait_for_previous();
+    if (choice.totals && !choice.ranked()) return;
     __shared__ __align__(16) std::uint64_t tile[kRankTile];
     __shared__ int part[kRankThreads / 32][kRankKeys];
     static_assert(kRankKeys == 32, "one key per lane");
@@ -1074,7 +1111,7 @@ __global__ __launch_bounds__(kRankThreads) void rank_topk_kernel(const __grid_co
     if (!src.find(blockIdx.x / kRankPer, kHarrisKind, &j, &local)) return;
     const int first = (local * kRankPer + static_cast<int>(blockIdx.x % kRankPer)) * kRankKeys;
     const int n = static_cast<int>(j.params->selected);
-    if (n <= above || n > below || first >= n) return;  // block-uniform
+    if (n > below || first >= n) return;  // block-uniform
     const int t = threadIdx.x, k = t % kRankKeys, slice = t / kRankKeys;
     const int slot = first + k;
     const std::uint64_t key = slot < n ? j.keys[slot] : ~0ull;
@@ -1115,8 +1152,10 @@ constexpr int kRankMany = 1 << 17;  // an image's jobs of more keys are ranked h
 static_assert(kRankKeys * kRankWide == kHarrisThreads, "a block ranks a harris block's keys");
 
 template <class Src>
-__global__ __launch_bounds__(kRankThreads, 3) void rank_wide_kernel(const __grid_constant__ Src src, int above, int below, int harris_blocks) {
+__global__ __launch_bounds__(kRankThreads, 3) void rank_wide_kernel(const __grid_constant__ Src src, int above, int below, int harris_blocks,
+                                                                     RankChoice choice) {
     wait_for_previous();
+    if (choice.totals && !choice.ranked()) return;
     __shared__ __align__(16) std::uint64_t tile[kRankTile];
     __shared__ int part[kRankThreads / 32][kHarrisThreads];
     __shared__ int found[kRankThreads], n_found;
@@ -1185,8 +1224,8 @@ __global__ __launch_bounds__(kRankThreads, 3) void rank_wide_kernel(const __grid
 // the source ...). Returns the launches.
 template <class Src, class Go> inline int launch_rank(int harris_blocks, int max_candidates, Go go) {
     const bool many = max_candidates > kRankMany;
-    go(rank_topk_kernel<Src>, harris_blocks * kRankPer, 0, many ? kRankMany : INT_MAX);
-    if (many) go(rank_wide_kernel<Src>, kRankGrid, kRankMany, INT_MAX, harris_blocks);
+    go(rank_topk_kernel<Src>, harris_blocks * kRankPer, many ? kRankMany : INT_MAX, RankChoice{});
+    if (many) go(rank_wide_kernel<Src>, kRankGrid, kRankMany, INT_MAX, harris_blocks, RankChoice{});
     return many ? 2 : 1;
 }
 

@@ -49,3 +49,21 @@ def test_batch(cuda, levels):
         assert np.array_equal(got, want), i
         seen.add(len(want))
     assert min(seen) == 0 and (levels > 1 or max(seen) == 20000)
+
+
+@pytest.mark.parametrize("pairs,k,thr", [(3, 4000, 5), (3, 4000, 140), (8, 2000, 5), (8, 2000, 140), (4, 20000, 5)])
+def test_batch_decides_by_counts(cuda, pairs, k, thr):
+    """Capacities that leave ranking or sorting open: many keys (sorted) and few
+    (ranked), by a block per slice and by wide slices; jobs past the sort too."""
+    rng = np.random.default_rng(pairs)
+    grays = [rng.integers(0, 256, (410 + 40 * (i % 4), 620), dtype=np.uint8) for i in range(2 * pairs)]
+    images = [torch.from_numpy(g).cuda() for g in grays]
+    b = batch.Batch([batch.pair_desc(images[2 * i], images[2 * i + 1], stages.Knobs(
+        max_keypoints=k, fast_threshold=thr, hypotheses=64, seed=i, levels=1)) for i in range(pairs)])
+    for _ in range(2):  # the counts are summed up anew in every run
+        b.enqueue()
+    torch.cuda.synchronize()
+    for i in (0, 3, 2 * pairs - 1):
+        got = b.outputs(i // 2)["kp_a" if i % 2 == 0 else "kp_b"]
+        want = s2s3.detect_and_describe(grays[i], thr, k)[0]
+        assert np.array_equal(got, want) and (len(want) == min(k, 20000) or thr == 140 or k == 20000), (i, len(want))
