@@ -229,7 +229,6 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
     }
     sort_smem = s2s3::sort_smem_bytes(max_cand);
     rank_fallback = max_cand > s2s3::kSortCap;
-    small_sorts = max_cand <= s2s3::kSortSmall;
     desc_keys = s2s3::desc_keys(keypoints);
     search_smem = s5k::search_smem_bytes(max_cap_m, true);
     finish_smem = s5k::finish_smem_bytes(max_cap_m);
@@ -287,6 +286,7 @@ Status Plan::build(int n_pairs, const stitch_pair_desc* p, int* bad_pair, bool a
                 }
             }
         }
+    sort_threads = s2s3::sort_threads(max_cand, det_total[s2s3::kSortKind]);
     topk = kSorted;
     if (s2s3::rank_pays(det_total[s2s3::kHarrisKind], det_total[s2s3::kSortKind], max_cand))
         topk = s2s3::rank_cost(squares, sum, std::min(max_cand, s2s3::kSortCap), det_total[s2s3::kSortKind], rank_wide()) <= 1.25f
@@ -698,8 +698,11 @@ Status Plan::enqueue(void* ws, std::size_t bytes, stitch_homography_result* host
             s2s3::sort_topk_kernel<DetSrc, kThreads><<<det_blocks[s2s3::kSortKind], kThreads, sort_smem, s>>>(det, choice);
         };
         if (go(det_blocks[s2s3::kSortKind])) {
-            if (small_sorts) sort(std::integral_constant<int, s2s3::kSortSmallThreads>{});
-            else sort(std::integral_constant<int, s2s3::kSortThreads>{});
+            switch (sort_threads) {
+                case 256: sort(std::integral_constant<int, 256>{}); break;
+                case 512: sort(std::integral_constant<int, 512>{}); break;
+                default: sort(std::integral_constant<int, s2s3::kSortThreads>{});
+            }
         }
         if (rank_fallback && go(harris_blocks)) wide(cap, INT_MAX, s2s3::RankChoice{});
     }

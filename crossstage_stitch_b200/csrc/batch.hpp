@@ -57,7 +57,7 @@ public:
     int resize_tile_h = s2s3::kResizeTileH;  // output rows of a resize block
     int sort_smem = 0, search_smem = 0, finish_smem = 0;
     bool rank_fallback = false;  // a job has more candidates than the sort takes
-    bool small_sorts = false;    // no job has more than kSortSmall candidates
+    int sort_threads = s2s3::kSortThreads;
     enum TopK { kSorted, kRanked, kByCounts };
     TopK topk = kSorted;         // kByCounts: decided on the device (RankChoice)
     bool rank_wide() const {     // which ranking kernel

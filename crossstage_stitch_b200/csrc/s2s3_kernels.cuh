@@ -215,8 +215,14 @@ constexpr int kRankThreads = 512;
 constexpr int kRankPer = kHarrisThreads / kRankKeys;  // rank blocks per harris block
 constexpr int kRankTile = 1024;      // keys staged at a time
 constexpr int kSortCap = 16384;    // candidates sorted in shared memory by one block
-constexpr int kSortThreads = 1024, kSortSmallThreads = 256;
-constexpr int kSortSmall = 1024;    // most candidates of any job of a launch of the small sort blocks
+constexpr int kSortThreads = 1024;
+// Threads of a batch's sort blocks: few where a job has few keys for them or many
+// jobs share an SM. Noise of 500x400, us with 256, 512 and 1024 threads: 64 jobs of 1000
+// candidates 24, 18, 18; 512 jobs of up to 868 (8 layers) 37, 31, 39; 1024 of them 46,
+// 46, 59, and at 512x512 29, 31, 45; 512 jobs of up to 434 19, 23, 28.
+constexpr int sort_threads(int max_candidates, int jobs) {
+    return max_candidates <= 512 || (max_candidates <= 1024 && jobs >= 6 * 148) ? 256 : max_candidates <= 1024 ? 512 : kSortThreads;
+}
 constexpr int kSortChunk = 64;      // keys a warp sorts in registers (2 per lane)
 constexpr int kBlurTileW = 64, kBlurTileH = 64;
 constexpr int kDescWarps = 8;
@@ -1022,12 +1028,9 @@ struct RankChoice {
 
 // One block per job: bitonic sort (descending) of up to kSortCap keys in
 // shared memory, then the first min(K, selected) become the keypoints. Bound by
-// instruction issue and barriers on the SMs that have a block: with at most
-// kSortSmall candidates a job, blocks of 256 threads leave eight jobs to an SM
-// (1024 jobs of 64 pairs at 8 layers, K = 2000: 45 us with 1024 threads, 31 with
-// 512, 29 with 256; 128 to 256 jobs: 16 to 18 us either way), while larger jobs
-// want them all (30 mixed pairs, K up to 8000: 83, 86 and 100 us, and 106 in two
-// launches that divide the jobs).
+// instruction issue and barriers on the SMs that have a block; sort_threads has the
+// batched blocks' sizes (30 mixed pairs, K up to 8000, want 1024 threads: 83 us, 86
+// with 512, 100 with 256, and 106 in two launches that divide the jobs).
 template <class Src, int kThreads>
 __global__ __launch_bounds__(kThreads) void sort_topk_kernel(const __grid_constant__ Src src, RankChoice choice) {
     wait_for_previous();

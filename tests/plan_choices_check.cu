@@ -1,5 +1,5 @@
 // Host-only check of the kernels that batch::Plan::build chooses for a batch:
-// how the candidates are ordered. Built and run by tests/test_plan_choices.py on
+// how the candidates are ordered and by what blocks. Built and run by tests/test_plan_choices.py on
 // the CPU: build() with alloc_staging = false touches no device.
 #include <cstdio>
 #include <vector>
@@ -49,6 +49,16 @@ int main() {
     for (const Shape s : {Shape{64, 512, 512, 2000, 8}, Shape{32, 800, 600, 2000, 1}, Shape{8, 800, 600, 8000, 8}}) {
         Plan p;
         if (!build(s, &p) || p.topk != Plan::kSorted) return fail("not sorted", s);
+    }
+    // sort blocks
+    const struct {
+        Shape s;
+        int threads;
+    } sorts[] = {{{32, 800, 600, 500, 1}, 512},  {{64, 800, 600, 256, 1}, 256},  {{8, 512, 512, 2000, 8}, 512},
+                 {{64, 512, 512, 2000, 8}, 256}, {{64, 512, 512, 1000, 8}, 256}, {{32, 800, 600, 513, 1}, 1024}};
+    for (const auto& c : sorts) {
+        Plan p;
+        if (!build(c.s, &p) || p.sort_threads != c.threads) return fail("other sort blocks", c.s);
     }
     std::printf("plan choices ok\n");
     return 0;
