@@ -124,6 +124,7 @@ template <class Job> struct OneJob {
         return true;
     }
     __device__ Job at(int /*index*/) const { return job; }
+    __device__ int count() const { return 1; }
 };
 
 // Device table: prefix[kind * (n + 1) + i] is the first block of job i for
@@ -158,6 +159,7 @@ template <class Job> struct JobTable {
         return true;
     }
     __device__ Job at(int index) const { return jobs[index]; }
+    __device__ int count() const { return n; }
 };
 
 // A few jobs passed by value (the layers of one image's pyramid):
@@ -175,6 +177,7 @@ template <class Job, int kJobs, int kKinds> struct InlineTable {
         return true;
     }
     __device__ Job at(int index) const { return jobs[index]; }
+    __device__ int count() const { return n; }
 };
 
 // Launch kinds of the detect table: kFastKind entries are the FAST tiles of
@@ -1734,7 +1737,7 @@ __device__ __forceinline__ int rotated_sample(const std::uint8_t* centre, std::u
     return centre[static_cast<int>(__float_as_uint(cy) * stride + __float_as_uint(cx) + bias)];
 }
 
-// A warp describes keys / kDescWarps keypoints (the block stages the pattern
+// A warp describes up to keys / kDescWarps keypoints (the block stages the pattern
 // and the disc weights once): first the intensity-centroid moments over the
 // radius-15 disc of the unblurred image of each (kept on lane r for the r-th),
 // then all their angles at once, one per lane (float fastAtan2, cos/sin
@@ -1775,12 +1778,22 @@ __global__ __launch_bounds__(kDescWarps * 32, kDescCtasPerSm) void describe_kern
         if (local == 0 && threadIdx.x == 0) atomicAdd(j.out_count, count);
         for (int m = 0; m < j.level; ++m) base += j.level_counts[m];
     }
-    if (local * keys >= count) return;
+    // keypoints per block: `keys` follows from the capacities; where fewer are there,
+    // as many as still fill the chip if every job has this one's (desc_keys), with
+    // blocks enough for all. 1279x717, K = 60000, some 4000 there: S3 40 us by `keys`,
+    // 15 so; 4 pairs of 800x600, K = 8000, 2100 there: this kernel 43 and 31 us.
+    int per = keys;
+    if (keys > kDescWarps && count < j.capacity) {
+        const int blocks = (j.capacity + keys - 1) / keys;
+        per = min(keys, desc_keys(static_cast<long long>(count) * src.count()));
+        while (per < keys && per * blocks < count) per *= 2;
+    }
+    if (local * per >= count) return;
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int pitch = j.pitch, blur_pitch = j.blur_pitch;
-    const int first = local * keys + (threadIdx.x >> 5);  // the warp's r-th keypoint is first + r * kDescWarps
-    const int rounds = min(keys / kDescWarps, (count - first + kDescWarps - 1) / kDescWarps);
+    const int first = local * per + (threadIdx.x >> 5);  // the warp's r-th keypoint is first + r * kDescWarps
+    const int rounds = min(per / kDescWarps, (count - first + kDescWarps - 1) / kDescWarps);
     if (rounds <= 0) return;
     // keypoint r on lane r: position (x = -1: too near the edge), moments, then cos and sin
     int x = -1, y = 0;
