@@ -1,5 +1,5 @@
 // Host-only check of the kernels that batch::Plan::build chooses for a batch:
-// how the candidates are ordered and by what blocks. Built and run by tests/test_plan_choices.py on
+// how the candidates are ordered and by what blocks, the rows of a resize tile. Built and run by tests/test_plan_choices.py on
 // the CPU: build() with alloc_staging = false touches no device.
 #include <cstdio>
 #include <vector>
@@ -60,6 +60,17 @@ int main() {
         Plan p;
         if (!build(c.s, &p) || p.sort_threads != c.threads) return fail("other sort blocks", c.s);
     }
+    // resize tiles: 128 rows from two waves of them on, 64 below; the tuning's value where it has one
+    const struct {
+        Shape s;
+        int rows;
+    } tiles[] = {{{2, 3700, 2159, 1000, 4}, 128}, {{2, 3700, 2100, 1000, 4}, 64}, {{64, 512, 512, 2000, 8}, 128}, {{8, 512, 512, 2000, 8}, 64}};
+    for (const auto& c : tiles)
+        for (const int tuned : {0, 32}) {
+            Plan p;
+            p.tuning.resize_tile_h = tuned;
+            if (!build(c.s, &p) || p.resize_tile_h != (tuned ? tuned : c.rows)) return fail("other resize tiles", c.s);
+        }
     std::printf("plan choices ok\n");
     return 0;
 }
