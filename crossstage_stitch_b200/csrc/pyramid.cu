@@ -1,7 +1,7 @@
 // Scale-pyramid S2/S3 of one image: layers 1..L-1 resized in a chain, then
 // S2 and S3 of every layer in the same launches (the layers' jobs travel as
-// kernel parameters; the FAST kernel also writes each layer's blur), each
-// layer's keypoints and descriptors written by the describe kernel straight
+// kernel parameters; the blur of the tiles that keypoints sample is one launch
+// over all layers), each layer's keypoints and descriptors written by the describe kernel straight
 // into the image's concatenated outputs in level-0 coordinates.
 //
 // The reference has no pyramid (docs/decisions/s2-s3-orb.md:84): its S2/S3

@@ -4,7 +4,10 @@
 // Every kernel reads its image and buffers from a "job". A job source is
 // either one job passed by value (the per-image stage call) or a device table
 // of jobs plus a block-prefix array (the batched chain, where one launch
-// covers every image of every pair). Results are identical either way.
+// covers every image of every pair). Results are identical either way, but for
+// the blur: the pyramid and batched paths fuse its products and sums, the
+// per-image S3 call rounds each as the reference does, and on noise some 3 blurred
+// pixels of a million differ by one (first_taps).
 //
 // Reference semantics (file:line in the reference tree):
 //   FAST score        src/s2_s3/s2.cu:37-67   (cornerScore<16>, circle order)
@@ -182,8 +185,9 @@ template <class Job, int kJobs, int kKinds> struct InlineTable {
 
 // Launch kinds of the detect table: kFastKind entries are the FAST tiles of
 // each job (looked up by tile index from the persistent FAST kernel's
-// queue), kSelectKind blocks walk a job's maxima list, kSortKind is one
-// block per job (tie selection, then the top-K sort).
+// queue), kSelectKind blocks walk a job's maxima list (a job's last one picks its
+// ties), kHarrisKind blocks have kHarrisThreads candidates each (the ranking divides
+// them further), kSortKind is one block per job, the top-K sort.
 enum DetectKind { kFastKind = 0, kSelectKind = 1, kHarrisKind = 2, kSortKind = 3, kDetectKinds = 4 };
 enum DescribeKind { kBlurKind = 0, kDescKind = 1, kDescribeKinds = 2 };
 

@@ -131,8 +131,8 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
     if (!enable_kernels()) return Status::CUDA_ERROR;
     const int count = config.hypotheses - config.previous_hypotheses;
     // Hypotheses per block (8 * hpw) as few as keep the blocks, one per SM, in
-    // one wave: a block's fit (one thread per hypothesis) takes about as long
-    // for 8 models as for 64.
+    // one wave: a block fits 32 at a time, eight lanes each, which takes about as
+    // long for 8 models as for 32.
     io.hpw = count <= 8 * kSmCount ? 1 : count <= 16 * kSmCount ? 2 : count <= 32 * kSmCount ? 4 : 8;
     io.search_blocks = plan_search(count, io.hpw);
     launch_chained(prepare_kernel<OneJob<PairIO>>, 1, kPrepareThreads, 0, stream, OneJob<PairIO>{io});

@@ -17,8 +17,8 @@
 //                             src/s5/s5.cu:139-212
 //
 // Layout of the work: a block of the search owns 8 * HPW consecutive
-// hypotheses. Their models (fitted one per thread, in this kernel or by
-// fit_kernel) are first bounded from below and above in FP32, all of them over
+// hypotheses. Their models (fitted here by eight lanes each, or one per thread
+// by fit_kernel) are first bounded from below and above in FP32, all of them over
 // all matches; the few whose lower bound does not exceed the smallest loss
 // known to the pair are then scored exactly, by 128 threads that play the
 // reference's 128 virtual lanes, so that the per-lane sums and the reduction
@@ -675,7 +675,8 @@ __global__ __launch_bounds__(kFitThreads, 3) void fit_kernel(const __grid_consta
 // FP32 bounds of a model's loss L = sum of min(r^2, tau^2), r = |H b - a|.
 // With u = 2^-24, the coordinate bounds Ax, Ay, Bx, By of the pair and the
 // FP32 evaluation of X, Y, Z (two FMAs on rounded entries each), 1/Z (one
-// approximate reciprocal, relative error 2u) and d = X (1/Z) - ax (one FMA):
+// approximate reciprocal, for which the PTX ISA states one unit in the last place
+// over the full range: a relative error of 2u) and d = X (1/Z) - ax (one FMA):
 //   |Z' - Z| <= EZ = 4u (|h6| Bx + |h7| By + |h8|) + 2e-15, likewise EX, EY,
 //   e = |r' - r| <= c0 + c1 |1/Z'|, W = 4 tau + Ax + Ay,
 //   c0 = 2.2u W + 4u tau,  c1 = 1.5 (W EZ + EX + EY),

@@ -142,8 +142,8 @@ class PairRunner:
     the runner beside image A's on the caller's, between an event of the
     caller's stream and one the caller's stream waits for: to the caller all
     work is on their stream. One image leaves most of the chip idle (512x512
-    pair 176 -> 130 us, 4K 664 -> 601 us). With another stage library everything stays on the
-    caller's stream."""
+    pair 176 -> 130 us, 4K 664 -> 575 us). With another stage library everything
+    stays on the caller's stream."""
 
     def __init__(self, max_w: int, max_h: int, max_k: int, max_r: int = 8192, device: str | int = "cuda",
                  cross_check: bool = False, stage_lib=None):
