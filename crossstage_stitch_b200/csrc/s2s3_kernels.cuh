@@ -40,13 +40,12 @@ struct RankTotals {
     std::uint32_t sum, largest;
 };
 
-// Per-job counters of the detect kernels, after the 256 histogram bins.
-enum DetectCounter {
-    kListed, kAboveWritten, kTiesWritten, kTileQueue,
-    kTiesListed,   // maxima at the threshold listed in `ties`
-    kSelectDone,   // select blocks that have finished
-    kDetectCounters
-};
+// Per-job counters of the detect kernels, after the 256 histogram bins. kTies
+// counts the maxima at the threshold written behind the keys above it, or listed
+// (TieList). Scores start at 1, so bin 0 of the histogram counts the select blocks
+// that have finished: a word more would take the smallest workspaces.
+enum DetectCounter { kListed, kAboveWritten, kTies, kTileQueue, kDetectCounters };
+constexpr int kSelectDoneBin = 0;
 constexpr int kHistWords = 256 + kDetectCounters;  // one job's histogram and counters
 
 struct alignas(16) DetectJob {  // 16-byte multiple: copied into shared memory in 16-byte chunks
@@ -57,7 +56,7 @@ struct alignas(16) DetectJob {  // 16-byte multiple: copied into shared memory i
     // workspace
     std::uint64_t* maxima;         // NMS maxima listed by the FAST kernel: (score << 32) | raster index
     int max_maxima;                // capacity of `maxima`
-    std::uint32_t* hist;           // [256] scores of the listed maxima, then DetectCounter words;
+    std::uint32_t* hist;           // [256] scores of the listed maxima (bin 0: kSelectDoneBin), then DetectCounter words;
                                    // all zeroed before the FAST launch
     SelectParams* params;
     std::uint64_t* keys;           // [candidates]
@@ -745,7 +744,7 @@ __device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams
                                           const TieList& list) {
     __shared__ __align__(16) std::uint32_t buf[kTieRank];  // staged ties, or the 256 radix bins
     __shared__ std::uint32_t pick[2];        // digit, maxima before it
-    std::uint32_t* ctr = j.counters();
+    __shared__ std::uint32_t written;
     const std::uint32_t T = p.threshold, total = j.hist[T];
     const int t = threadIdx.x;
     if (total <= kTieRank && total <= list.room) {
@@ -790,6 +789,7 @@ __device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams
             while (d < 255 && run + buf[d] < need) run += buf[d++];
             pick[0] = d;
             pick[1] = run;
+            written = 0;
         }
         __syncthreads();
         prefix |= pick[0] << shift;
@@ -804,7 +804,7 @@ __device__ __forceinline__ void pick_ties(const DetectJob& j, const SelectParams
         const bool keep = i < n && entry(i, px) && px <= prefix;
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         std::uint32_t b = 0;
-        if (lane == 0 && m) b = atomicAdd(&ctr[kTiesWritten], static_cast<std::uint32_t>(__popc(m)));
+        if (lane == 0 && m) b = atomicAdd(&written, static_cast<std::uint32_t>(__popc(m)));
         b = __shfl_sync(0xffffffffu, b, 0) + __popc(m & below);
         if (keep && b < p.ties) j.keys[p.above + b] = px;
     }
@@ -851,7 +851,7 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     // ties go behind the keys above the threshold, or to their list
-    std::uint32_t* const tie_count = &ctr[all_ties ? kTiesWritten : kTiesListed];
+    std::uint32_t* const tie_count = &ctr[kTies];
     const std::uint32_t stride = static_cast<std::uint32_t>(j.select_blocks) * 256u;
     for (std::uint32_t i0 = static_cast<std::uint32_t>(local) * 256u; i0 < n; i0 += stride) {  // block-uniform
         const std::uint32_t i = i0 + threadIdx.x;
@@ -880,7 +880,7 @@ __global__ __launch_bounds__(256) void select_kernel(const __grid_constant__ Src
     __threadfence();  // this block's list entries, before it counts as done
     __syncthreads();
     if (threadIdx.x == 0)
-        last = atomicAdd(&ctr[kSelectDone], 1u) == static_cast<std::uint32_t>(j.select_blocks) - 1u;
+        last = atomicAdd(&j.hist[kSelectDoneBin], 1u) == static_cast<std::uint32_t>(j.select_blocks) - 1u;
     __syncthreads();
     if (!last) return;
     __threadfence();
