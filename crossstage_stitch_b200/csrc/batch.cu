@@ -20,7 +20,6 @@
 #include <algorithm>
 #include <iterator>
 #include <cstring>
-#include <mutex>
 #include <type_traits>
 
 #include "batch.hpp"
@@ -77,8 +76,7 @@ static_assert(kTables <= 20, "table offsets");
 // Opts the kernels in to their shared memory on the current device; false if it refuses.
 bool enable_kernels() {
     using Src = s5k::JobTable<SearchJob>;
-    return enable_smem<s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>, s2s3::kSortThreads>>(
-               s2s3::kSortCap * static_cast<int>(sizeof(std::uint64_t))) &&
+    return enable_smem<s2s3::sort_topk_kernel<s2s3::JobTable<DetectJob>, s2s3::kSortThreads>>(s2s3::kSortSmem) &&
            s5k::enable_search_smem<Src, true, 32>() && s5k::enable_search_smem<Src, true, 64>() &&
            s5k::enable_search_smem<Src, true, 128>() && s5k::enable_search_smem<Src, true, 256>() &&
            s5k::enable_finish_smem<s5k::JobTable<PairIO>>();

@@ -3,10 +3,10 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <climits>
 #include <cstddef>
 #include <cstdint>
-#include <mutex>
 
 #include "stage_api.hpp"
 
@@ -54,18 +54,23 @@ __device__ __forceinline__ void wait_for_previous() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Opts a kernel in to `most` bytes of dynamic shared memory on the current
-// device; false if the device refuses. Once per device: the attribute belongs to
-// the device it was set on, and a process may use several.
+// Unique id of the current context (ids are never reused within a process); 0
+// when there is none or it cannot be read.
+unsigned long long current_context_id();
+
+// Opts a kernel in to `most` bytes of dynamic shared memory in the current
+// context; false if the device refuses. Once per context: the attribute belongs to
+// the context it was set in, and a process may use several devices, or one again
+// after a reset.
 template <auto kKernel> bool enable_smem(int most) {
-    static std::once_flag flags[64];
-    static bool ok[64];
+    static std::atomic<unsigned long long> done[64];  // by device: the context that has it
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
-    });
-    return ok[dev];
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return false;
+    const unsigned long long context = dev < 64 ? current_context_id() : 0;
+    if (context && done[dev].load(std::memory_order_relaxed) == context) return true;
+    if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return false;
+    if (dev < 64) done[dev].store(current_context_id(), std::memory_order_relaxed);  // the call may have made the context
+    return true;
 }
 
 inline Status launch_status() {

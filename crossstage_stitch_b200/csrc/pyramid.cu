@@ -11,7 +11,6 @@
 // and each layer runs the reference's single-level S2/S3 unchanged.
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "s2s3_internal.hpp"
 
@@ -169,18 +168,6 @@ using DetSrc = InlineTable<DetectJob, kMaxLevels, kDetectKinds>;
 using DesSrc = InlineTable<DescribeJob, kMaxLevels, kDescribeKinds>;
 static_assert(sizeof(DetSrc) <= 4096 && sizeof(DesSrc) <= 4096, "layer tables must fit the kernel parameters");
 
-bool enable_pyramid_sort_smem() {
-    static std::once_flag flags[64];
-    static bool ok[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(sort_topk_kernel<DetSrc, kSortThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kSortCap * static_cast<int>(sizeof(std::uint64_t))) == cudaSuccess;
-    });
-    return ok[dev];
-}
-
 }  // namespace
 
 Status pyramid_workspace_bytes(int w, int h, const s2::Config& c, int levels, float sf, std::size_t* bytes) {
@@ -212,7 +199,7 @@ Status pyramid_detect_describe(const ImageView& image, const s2::Config& c, int 
         return Status::CUDA_ERROR;
     const int n = l.plan.levels;
     if (n == 0 || c.max_keypoints == 0) return launch_status();
-    if (!enable_pyramid_sort_smem()) return Status::CUDA_ERROR;
+    if (!enable_smem<sort_topk_kernel<DetSrc, kSortThreads>>(kSortSmem)) return Status::CUDA_ERROR;
     PyramidJobs jobs;
     std::uint32_t* queue = at_offset<std::uint32_t>(ws, l.queue);
     const PyramidShared sh{at_offset<int>(ws, l.counts), at_offset<std::uint32_t>(ws, l.hists),

@@ -7,7 +7,6 @@
 // these kernels need).
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "s2s3_internal.hpp"
 
@@ -104,20 +103,6 @@ int sort_smem_bytes(int candidates) {
 
 namespace {
 
-// Opt the shared-memory sort kernels in to more than 48 KB of dynamic shared
-// memory, once per device.
-template <class Src> bool enable_sort_smem() {
-    static std::once_flag flags[64];
-    static bool ok[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(sort_topk_kernel<Src, kSortThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kSortCap * static_cast<int>(sizeof(std::uint64_t))) == cudaSuccess;
-    });
-    return ok[dev];
-}
-
 bool record(cudaEvent_t ev, cudaStream_t s) { return !ev || cudaEventRecord(ev, s) == cudaSuccess; }
 
 Status detect(const ImageView& image, const s2::Config& config, const Keypoints& output, void* ws,
@@ -140,7 +125,7 @@ Status detect(const ImageView& image, const s2::Config& config, const Keypoints&
     if (!ws || !aligned(ws, kWorkspaceAlign)) return Status::INVALID_ARGUMENT;
     if (ws_bytes < l.total) return Status::INSUFFICIENT_WORKSPACE;
     using Src = OneJob<DetectJob>;
-    if (!enable_sort_smem<Src>()) return Status::CUDA_ERROR;
+    if (!enable_smem<sort_topk_kernel<Src, kSortThreads>>(kSortSmem)) return Status::CUDA_ERROR;
     const Src src{make_detect_job(image, config, output, ws, l)};
     if (cudaMemsetAsync(src.job.hist, 0, DetectLayout::hist_bytes, stream) != cudaSuccess)
         return Status::CUDA_ERROR;

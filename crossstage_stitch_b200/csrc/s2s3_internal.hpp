@@ -43,8 +43,9 @@ inline bool rank_pays(long long harris_blocks, int jobs, int max_candidates) {
     while (keys < max_candidates) keys *= 2;
     return harris_blocks * kRankPer <= keys * ceil_div(jobs, 2 * kSmCount);
 }
-// Dynamic shared memory of sort_topk_kernel for `candidates` keys.
+// Dynamic shared memory of sort_topk_kernel for `candidates` keys, and the most.
 int sort_smem_bytes(int candidates);
+constexpr int kSortSmem = kSortCap * static_cast<int>(sizeof(std::uint64_t));
 
 // ------------------------------------------------------- scale pyramid
 

@@ -1,8 +1,6 @@
 // S4 layout and job builders shared by the per-pair call and the batched chain.
 #pragma once
 
-#include <mutex>
-
 #include <type_traits>
 
 #include "s4_kernels.cuh"
@@ -36,31 +34,6 @@ bool valid_matcher(int kind);
 // OK, with *required the workspace bytes the call needs.
 Status check_match_args(const Keypoints& a, const Descriptors& da, const Keypoints& b, const Descriptors& db,
                         const s4::Config& config, const Matches& output, std::size_t* required);
-// Opts the tensor-core kernel for a job source in to its shared memory
-// (once per device); false if the device refuses.
-template <class Src, int kRowsB> bool enable_tc_smem() {
-    static std::once_flag flags[64];
-    static bool ok[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(knn_tc_kernel<Src, kRowsB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       TcShape<kRowsB>::smem) == cudaSuccess;
-    });
-    return ok[dev];
-}
-// Launches the tensor-core matcher of `kind` over `blocks` blocks.
-template <class Src> bool enable_pipe_smem() {
-    static std::once_flag flags[64];
-    static bool ok[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::call_once(flags[dev], [&] {
-        ok[dev] = cudaFuncSetAttribute(knn_tc_pipe_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kPipeSmem) == cudaSuccess;
-    });
-    return ok[dev];
-}
 // Launches the tensor-core matcher: chained (launch_chained) for the per-pair
 // call, plainly in the batched chain.
 template <class Src> bool launch_tc(int kind, int blocks, const Src& src, cudaStream_t s) {
@@ -69,11 +42,15 @@ template <class Src> bool launch_tc(int kind, int blocks, const Src& src, cudaSt
         else kernel<<<blocks, threads, smem, s>>>(src);
         return true;
     };
-    if (kind == kMatcherTensorPipe) return enable_pipe_smem<Src>() && go(knn_tc_pipe_kernel<Src>, kPipeThreads, kPipeSmem);
+    const auto tc = [&](auto rows) {
+        constexpr int kRows = decltype(rows)::value, smem = TcShape<kRows>::smem;
+        return enable_smem<knn_tc_kernel<Src, kRows>>(smem) && go(knn_tc_kernel<Src, kRows>, kTcThreads, smem);
+    };
+    if (kind == kMatcherTensorPipe) return enable_smem<knn_tc_pipe_kernel<Src>>(kPipeSmem) && go(knn_tc_pipe_kernel<Src>, kPipeThreads, kPipeSmem);
     switch (tc_rows(kind)) {
-        case 64: return enable_tc_smem<Src, 64>() && go(knn_tc_kernel<Src, 64>, kTcThreads, TcShape<64>::smem);
-        case 128: return enable_tc_smem<Src, 128>() && go(knn_tc_kernel<Src, 128>, kTcThreads, TcShape<128>::smem);
-        default: return enable_tc_smem<Src, 256>() && go(knn_tc_kernel<Src, 256>, kTcThreads, TcShape<256>::smem);
+        case 64: return tc(std::integral_constant<int, 64>{});
+        case 128: return tc(std::integral_constant<int, 128>{});
+        default: return tc(std::integral_constant<int, 256>{});
     }
 }
 constexpr int tc_blocks_per_sm(int kind) {

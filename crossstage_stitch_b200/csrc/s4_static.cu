@@ -25,7 +25,6 @@
 // stitch_s4_match reports them; then requests whose S4 workspace would exceed
 // kScratchBytes fail with INSUFFICIENT_WORKSPACE, before anything is
 // enqueued. No cudaMalloc, cudaFree or allocating library routine is called.
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -40,45 +39,6 @@ constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_s4_scratch[kScratchBytes];
 
-using CtxGetCurrent = CUresult (*)(CUcontext*);
-using CtxGetId = CUresult (*)(CUcontext, unsigned long long*);
-
-struct DriverCalls {
-    CtxGetCurrent get_current = nullptr;
-    CtxGetId get_id = nullptr;
-};
-
-// cuCtxGetCurrent and cuCtxGetId through the runtime's driver entry points
-// (the library links no libcuda); both null when the driver lacks them.
-const DriverCalls& driver_calls() {
-    static const DriverCalls calls = [] {
-        DriverCalls c;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess && p)
-            c.get_current = reinterpret_cast<CtxGetCurrent>(p);
-        p = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess && p)
-            c.get_id = reinterpret_cast<CtxGetId>(p);
-        if (!c.get_current || !c.get_id) c = DriverCalls{};
-        return c;
-    }();
-    return calls;
-}
-
-// Unique id of the current context (ids are never reused within a process);
-// 0 when there is none or it cannot be read.
-unsigned long long current_context_id() {
-    const DriverCalls& d = driver_calls();
-    if (!d.get_current) return 0;
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (d.get_current(&ctx) != CUDA_SUCCESS || !ctx || d.get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-    return id;
-}
-
 struct Cached {
     unsigned long long context = 0;  // 0: nothing cached
     void* address = nullptr;
@@ -92,7 +52,7 @@ Cached g_cache[kMaxDevices];
 void* scratch_on_current_device() {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-    const unsigned long long ctx = current_context_id();
+    const unsigned long long ctx = stitch::b200::current_context_id();
     std::lock_guard<std::mutex> hold(g_lock);
     Cached& c = g_cache[dev];
     if (ctx != 0 && c.context == ctx) return c.address;
@@ -102,7 +62,7 @@ void* scratch_on_current_device() {
         return nullptr;
     }
     // the lookup makes the device's primary context current if it was not
-    const unsigned long long now = ctx != 0 ? ctx : current_context_id();
+    const unsigned long long now = ctx != 0 ? ctx : stitch::b200::current_context_id();
     c = Cached{now, now != 0 ? p : nullptr};
     return p;
 }

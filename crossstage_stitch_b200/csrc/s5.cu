@@ -102,9 +102,11 @@ namespace {
 
 using SearchSrc = OneJob<SearchJob>;
 
-bool enable_kernels() {
-    return enable_search_smem<SearchSrc, false, 8>() && enable_search_smem<SearchSrc, false, 16>() &&
-           enable_search_smem<SearchSrc, false, 32>() && enable_search_smem<SearchSrc, false, 64>() &&
+bool enable_kernels(int hpw) {
+    return (hpw == 1   ? enable_search_smem<SearchSrc, false, 8>()
+            : hpw == 2 ? enable_search_smem<SearchSrc, false, 16>()
+            : hpw == 4 ? enable_search_smem<SearchSrc, false, 32>()
+                       : enable_search_smem<SearchSrc, false, 64>()) &&
            enable_finish_smem<OneJob<PairIO>>();
 }
 
@@ -128,13 +130,13 @@ Status estimate(const Keypoints& a, const Keypoints& b, const Matches& matches, 
     const Status chk = check_and_build(a, b, matches, scale_a, scale_b, config, inlier_mask, output, workspace,
                                        workspace_bytes, &io);
     if (chk != Status::OK) return chk;
-    if (!enable_kernels()) return Status::CUDA_ERROR;
     const int count = config.hypotheses - config.previous_hypotheses;
     // Hypotheses per block (8 * hpw) as few as keep the blocks, one per SM, in
     // one wave: a block fits 32 at a time, eight lanes each, which takes about as
     // long for 8 models as for 32.
     io.hpw = count <= 8 * kSmCount ? 1 : count <= 16 * kSmCount ? 2 : count <= 32 * kSmCount ? 4 : 8;
     io.search_blocks = plan_search(count, io.hpw);
+    if (!enable_kernels(io.hpw)) return Status::CUDA_ERROR;
     launch_chained(prepare_kernel<OneJob<PairIO>>, 1, kPrepareThreads, 0, stream, OneJob<PairIO>{io});
     note_launches(1);
     if (cudaGetLastError() != cudaSuccess) return Status::CUDA_ERROR;

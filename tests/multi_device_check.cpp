@@ -2,9 +2,10 @@
 // the first alone: the built objects are linked to the CUDA runtime below, which
 // keeps kernel attributes per device, as the real one does, and refuses a launch
 // with more than 48 KB of dynamic shared memory of a kernel that was not opted
-// in on the current device. It also checks the blocks of a batch whose jobs have
-// far more candidates than keys may be there. Nothing runs on a GPU. Built and run
-// by tests/test_multi_device.py.
+// in on the current device; a reset takes the attributes away. It also checks the
+// blocks of a batch whose jobs have far more candidates than keys may be there.
+// Nothing runs on a GPU. Built and run by tests/test_multi_device.py.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -18,7 +19,9 @@
 
 namespace {
 
-int device = 0, launches = 0, refused = 0;
+int device = 0, launches = 0, refused = 0, set = 0;
+bool with_ids = false;                // whether the driver tells contexts apart
+unsigned long long context[8] = {1, 2, 3, 4, 5, 6, 7, 8};
 bool refuse_attributes = false;
 std::map<std::pair<int, const void*>, std::size_t> opted;
 cudaError_t last = cudaSuccess;
@@ -70,6 +73,7 @@ cudaError_t cudaSetDevice(int d) { return device = d, cudaSuccess; }
 cudaError_t cudaGetLastError() { return std::exchange(last, cudaSuccess); }
 cudaError_t cudaFuncSetAttribute(const void* kernel, cudaFuncAttribute a, int value) {
     if (refuse_attributes) return last = cudaErrorInvalidValue;
+    ++set;
     if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) opted[{device, kernel}] = static_cast<std::size_t>(value);
     return cudaSuccess;
 }
@@ -89,7 +93,13 @@ cudaError_t cudaFree(void* p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, std::size_t n, unsigned) { return *p = host_memory(n), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaGetSymbolAddress(void** p, const void*) { return *p = &device, cudaSuccess; }
-cudaError_t cudaGetDriverEntryPoint(const char*, void**, unsigned long long, cudaDriverEntryPointQueryResult*) { return cudaErrorNotSupported; }
+CUresult current(CUcontext* c) { return *c = reinterpret_cast<CUcontext>(&context[device]), CUDA_SUCCESS; }
+CUresult context_id(CUcontext c, unsigned long long* id) { return *id = *reinterpret_cast<unsigned long long*>(c), CUDA_SUCCESS; }
+cudaError_t cudaGetDriverEntryPoint(const char* name, void** p, unsigned long long, cudaDriverEntryPointQueryResult* q) {
+    *p = reinterpret_cast<void*>(!std::strcmp(name, "cuCtxGetCurrent") ? reinterpret_cast<void (*)()>(current) : reinterpret_cast<void (*)()>(context_id));
+    *q = cudaDriverEntryPointSuccess;
+    return with_ids ? cudaSuccess : cudaErrorNotSupported;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t*, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
@@ -177,8 +187,9 @@ int batch(const Buffers& b, int k, int levels, const stitch_batch_tuning* tuning
 
 }  // namespace
 
-int main() {
+int main(int argc, char**) {
     const Buffers b;
+    with_ids = argc > 1;
     for (int d = 0; d < 3; ++d) {
         cudaSetDevice(d);
         for (const int k : {100, 2000, 8193}) {
@@ -194,6 +205,18 @@ int main() {
         }
         if (refused) return std::printf("device %d: %d launches refused\n", d, refused), 1;
     }
+    // a reset: another context without the attributes; and, the contexts known, no attribute is set twice
+    cudaSetDevice(1);
+    opted.clear();
+    context[1] = 100;
+    {
+        if (const int st = estimate(b, 8193, 2000)) return std::printf("after a reset: estimate: status %d\n", st), 1;
+        if (const int st = detect_and_match(b, 8193)) return std::printf("after a reset: stages: status %d\n", st), 1;
+        if (const int st = batch(b, 8193, 8, nullptr)) return std::printf("after a reset: batch: status %d\n", st), 1;
+    }
+    const int before_again = set;
+    estimate(b, 8193, 2000), detect_and_match(b, 8193), batch(b, 8193, 8, nullptr);
+    if (with_ids && set != before_again) return std::printf("attributes set again\n"), 1;
     // 32 pairs of 2 x 40000 candidates: a block per 32 of them would be 80,000 blocks
     rank_blocks = 0;
     if (const int st = batch(b, 20000, 1, nullptr, 32)) return std::printf("large batch: status %d\n", st), 1;

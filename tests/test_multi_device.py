@@ -1,6 +1,6 @@
-"""Every call works on each GPU of one process: the kernels that need more
-shared memory than a launch may have by default are opted in on every device.
-The check (tests/multi_device_check.cpp) links the built objects to a CUDA
+"""Every call works on each GPU of one process, and after a device reset: the
+kernels that need more shared memory than a launch may have by default are opted in
+in every context, whether the driver gives contexts an id or not. The check (tests/multi_device_check.cpp) links the built objects to a CUDA
 runtime of its own and runs on the CPU."""
 import shutil
 import subprocess
@@ -26,6 +26,7 @@ def test_calls_on_every_device_of_a_process():
                "-pthread", "-o", str(exe)]
         built = subprocess.run(cmd, capture_output=True, text=True)
         assert built.returncode == 0, built.stderr[-4000:]
-        out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
-        assert out.returncode == 0, (out.returncode, out.stdout, out.stderr)
-        assert "devices ok" in out.stdout
+        for ids in ([], ["ids"]):
+            out = subprocess.run([str(exe), *ids], capture_output=True, text=True, timeout=120)
+            assert out.returncode == 0, (out.returncode, out.stdout, out.stderr)
+            assert "devices ok" in out.stdout
