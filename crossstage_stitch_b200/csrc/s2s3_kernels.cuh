@@ -20,6 +20,8 @@
 //   describe          src/s2_s3/s3.cu:75-157
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace stitch::b200::s2s3 {
@@ -1288,6 +1290,14 @@ __device__ __forceinline__ int2 linear_exact_tap(int v, int src, double scale) {
 constexpr int kRawStride = 208;  // bytes of a staged source row: 13 chunks of 16
 template <int kTileH> __host__ __device__ constexpr int resize_raw_rows() { return kTileH * 3 / 2 + 6; }
 
+// A source byte read in place. Read-only loads may pass the stores to the other layer
+// (2 pairs of 799x601, ratio 2, 4 layers: layers 22 us with them, 25 with plain ones),
+// but a chained launch may overlap the one that writes its source (launch_chained).
+template <class Src> __device__ __forceinline__ std::uint32_t source_byte(const std::uint8_t* p) {
+    if constexpr (std::is_same_v<Src, JobTable<ResizeJob>>) return __ldg(p);
+    else return *p;
+}
+
 // Four output pixels of one row from the h of its upper and lower source rows.
 __device__ __forceinline__ std::uint32_t resize_quad(const std::uint32_t (&ha)[4], const std::uint32_t (&hb)[4], std::uint32_t wy) {
     std::uint32_t v[4];
@@ -1383,9 +1393,8 @@ __global__ __launch_bounds__(256, kTileH > kResizeTileH ? 5 : 6) void resize_ker
             std::uint32_t ha[4], hb[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                // plain loads: the launch before may be the one that writes this layer's source
-                const std::uint32_t wa = A[tx[k].x] | (static_cast<std::uint32_t>(A[xb[k]]) << 8);
-                const std::uint32_t wb = B[tx[k].x] | (static_cast<std::uint32_t>(B[xb[k]]) << 8);
+                const std::uint32_t wa = source_byte<Src>(A + tx[k].x) | (source_byte<Src>(A + xb[k]) << 8);
+                const std::uint32_t wb = source_byte<Src>(B + tx[k].x) | (source_byte<Src>(B + xb[k]) << 8);
                 ha[k] = __dp2a_lo(wx[k], wa, 0u);
                 hb[k] = __dp2a_lo(wx[k], wb, 0u);
             }
