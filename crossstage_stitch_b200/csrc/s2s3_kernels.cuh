@@ -1772,18 +1772,23 @@ __global__ __launch_bounds__(kDescWarps * 32, kDescCtasPerSm) void describe_kern
         wait_for_previous();
         return;
     }
-    {
+    // word loads of the disc need 4-byte aligned rows (block-uniform)
+    const bool words = ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 3) == 0;
+    const auto stage = [&] {  // depends on the job and on constants alone
         const int p = threadIdx.x;  // 256 threads, one pattern pair each
         const int4 q = kOrbPattern[p];
         pat[p & 7][p >> 3] = make_float4(static_cast<float>(q.x), static_cast<float>(q.y), static_cast<float>(q.z),
                                          static_cast<float>(q.w));
-    }
-    // word loads of the disc need 4-byte aligned rows (block-uniform)
-    const bool words = ((reinterpret_cast<std::uintptr_t>(j.image) | static_cast<std::uintptr_t>(j.pitch)) & 3) == 0;
-    if (words)
-        for (int e = threadIdx.x; e < static_cast<int>(sizeof(DiscTable) / 16); e += kDescWarps * 32)
-            reinterpret_cast<uint4*>(&disc)[e] = __ldg(reinterpret_cast<const uint4*>(&kDiscTable) + e);
-    wait_for_previous();  // what stands above depends on the job and on constants alone
+        if (words)
+            for (int e = threadIdx.x; e < static_cast<int>(sizeof(DiscTable) / 16); e += kDescWarps * 32)
+                reinterpret_cast<uint4*>(&disc)[e] = __ldg(reinterpret_cast<const uint4*>(&kDiscTable) + e);
+    };
+    // a chained launch stages beside the launch before it, a batch's block once it
+    // knows that it has keypoints (32 pairs, K = 20000, 2100 there: 183 -> 161 us; 64
+    // pairs at 512x512, K = 2000, 1460 there: 165 -> 166)
+    constexpr bool kChained = !std::is_same_v<Src, JobTable<DescribeJob>>;
+    if constexpr (kChained) stage();
+    wait_for_previous();
     // The grid covers the capacity; blocks past the keypoint count leave now.
     const int count = min(*j.count, j.capacity);
     int base = 0;  // first output row of this layer
@@ -1792,16 +1797,19 @@ __global__ __launch_bounds__(kDescWarps * 32, kDescCtasPerSm) void describe_kern
         for (int m = 0; m < j.level; ++m) base += j.level_counts[m];
     }
     // keypoints per block: `keys` follows from the capacities; where fewer are there,
-    // as many as still fill the chip if every job has this one's (desc_keys), with
-    // blocks enough for all. 1279x717, K = 60000, some 4000 there: S3 40 us by `keys`,
-    // 15 so; 4 pairs of 800x600, K = 8000, 2100 there: this kernel 43 and 31 us.
+    // as few as keep the launch in one wave if every job has this one's, with blocks
+    // enough for all. 1279x717, K = 60000, some 4000 there: S3 40 us by `keys`, 15 so;
+    // this kernel, 800x600: 4 pairs, K = 8000, 2100 there 43 and 32 us; 32 pairs at 8
+    // layers, K = 1000, 350 there 51 and 50 (54 where the chip is only to be filled).
     int per = keys;
     if (keys > kDescWarps && count < j.capacity) {
         const int blocks = (j.capacity + keys - 1) / keys;
-        per = min(keys, desc_keys(static_cast<long long>(count) * src.count()));
-        while (per < keys && per * blocks < count) per *= 2;
+        per = kDescWarps;
+        const int most = 148 * kDescCtasPerSm / src.count();
+        while (per < keys && (per * blocks < count || per * most < count)) per *= 2;
     }
     if (local * per >= count) return;
+    if constexpr (!kChained) stage();
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int pitch = j.pitch, blur_pitch = j.blur_pitch;
